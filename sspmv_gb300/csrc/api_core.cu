@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "csr_stream.cuh"
 #include "plan.cuh"
 
 namespace sspmv {
@@ -62,6 +63,7 @@ void free_plan(sspmv_features *f, sspmv_stream_t s) {
         free_plan(&p->sub->f, s);
         delete p->sub;
     }
+    free_stream_plan(p->stream, s);
     for (void *e : p->extra) dfree(e, s);
     delete p;
     f->priv = nullptr;

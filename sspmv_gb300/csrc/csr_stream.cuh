@@ -1,0 +1,48 @@
+// csr_stream.cuh -- the nonzero-split stream kernel (csr_stream.cu): device
+// view of a row-ordered run of nonzeros, its plan and its launchers.  Used by
+// CSR (default kernel), the short tails of the sliced formats and the request
+// server's batches.
+#pragma once
+
+#include "common.cuh"
+#include "plan.cuh"
+
+namespace sspmv {
+
+// What the kernel reads besides x and y: the nonzeros in row order and the
+// plan's arrays (StreamPlan).
+struct StreamView {
+    const int32_t *col = nullptr;
+    const void *val = nullptr;
+    const int4 *rec = nullptr;
+    const int4 *split = nullptr;
+    const uint8_t *ends = nullptr;
+    const int32_t *nzrow = nullptr;
+    const int32_t *empty = nullptr;
+    int64_t windows = 0;
+    uint32_t nnz = 0;
+    int32_t window = 0;
+    int32_t nempty = 0;
+    int32_t nsplit = 0;
+    int32_t vec = 0;  // 16-byte aligned col and val: vector loads
+};
+
+// Builds (once) the stream plan of m rows given by row_offset (m + 1
+// entries, nnz > 0); row_offset is not read after the call's work on `s`.
+sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset, int32_t value_type,
+                                sspmv_stream_t s);
+void free_stream_plan(StreamPlan &sp, sspmv_stream_t s);
+StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, const void *val);
+
+// The kernel steps through X and Y in 32-bit byte strides.
+inline bool stream_takes_strides(int64_t ldx, int64_t ldy, size_t value_bytes) {
+    return (uint64_t)ldx * value_bytes <= 0xffffffffu && (uint64_t)ldy * value_bytes <= 0xffffffffu;
+}
+
+// Y = alpha * A * X + beta * Y on the rows of the plan, K right-hand sides
+// (1, 2, 4 or 8): one launch, and one more where rows are split.
+template <typename V, int K>
+sspmv_status launch_stream_view(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta, V *y,
+                                int64_t ldy, sspmv_stream_t s);
+
+}  // namespace sspmv

@@ -25,8 +25,26 @@ struct MergePlan {
 
 constexpr int kMaxK = 8;  // right-hand sides handled per pass
 
+// Schedule of the stream kernel (csr_stream.cu): the nonzeros cut into windows
+// of `window` elements.
+struct StreamPlan {
+    int window = 0;            // 0: not built
+    int64_t windows = 0;
+    int4 *rec = nullptr;       // [windows] first element, end element, first row, flags: 1 the first row began in an
+                               // earlier window, 2 the last one goes on past the window
+    int4 *split = nullptr;     // [nsplit] split rows: first window, last window, ordinal
+    int64_t nsplit = 0;
+    uint8_t *ends = nullptr;   // bit e: nonzero e is the last of its row
+    void *tail_val = nullptr;  // [windows * kMaxK] piece of the split row that goes on past the window
+    void *head_val = nullptr;  // [windows * kMaxK] last piece of the split row that ends in the window
+    int32_t *nzrow = nullptr;  // y row of the i-th nonempty row (null: i itself)
+    int32_t *empty = nullptr;  // rows without nonzeros
+    int64_t nempty = 0;
+};
+
 struct Plan {
     int kind = 0;
+    StreamPlan stream;
     MergePlan merge[2];     // [0]: tile for k <= 4, [1]: tile for k == 8
     int param = 0;          // kernel parameter set by sspmv_set_kernel (0 = library choice)
     void *extra[12] = {nullptr};  // format-specific device buffers

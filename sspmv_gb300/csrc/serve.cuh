@@ -1,18 +1,19 @@
 // serve.cuh -- device-side batch description shared by the request server
-// (server.cu) and the batched stream CSR kernels (spmv_csr.cu).
+// (server.cu) and the batched stream CSR kernels (csr_stream.cu).
 //
 // A batch holds many independent requests y = alpha*A*X + beta*Y on CSR
 // matrices of any size.  Requests are grouped by (value type, k); group g =
 // 4 * (value_type == F64) + log2(k) for k in {1, 2, 4, 8}.  Within a group the
-// 256-nonzero chunks of all requests are numbered consecutively (item i owns
-// global chunks [chunk_begin, chunk_begin + num_chunks)), and one persistent
-// kernel per group walks the global chunks.  Each request is cut into exactly
-// the chunks the single-matrix stream kernel uses (the matrix's own
-// row_start), so a request's result does not depend on what else is in the
+// windows of all requests are numbered consecutively (item i owns global
+// windows [window_begin, window_begin + windows of its matrix)), and one
+// persistent kernel per group walks the global windows.  Each request is cut
+// into exactly the windows the single-matrix stream kernel uses (the matrix's
+// own plan), so a request's result does not depend on what else is in the
 // batch.
 #pragma once
 
 #include "common.cuh"
+#include "csr_stream.cuh"
 
 namespace sspmv {
 
@@ -24,44 +25,42 @@ inline int batch_group(int32_t value_type, int32_t k) {
 }
 
 struct BatchItem {
-    const int32_t *row_offset;
-    const int32_t *col_index;
-    const void *values;
-    const int32_t *row_start;  // num_chunks + 1 rows holding each chunk's first nonzero
+    StreamView view;
     const void *x;
     void *y;
     int64_t ldx, ldy;
     double alpha, beta;
-    int64_t chunk_begin;  // first global chunk of this item in its group
-    int64_t nnz;
-    int32_t m;
-    int32_t num_chunks;
-    int32_t vec;          // 16-byte aligned col_index / values: vector loads
-    int32_t xvec;         // X rows aligned for vector loads (xrow_vec)
+    int64_t window_begin;  // first global window of this item in its group
+    int64_t split_begin;   // first global split row likewise
+    int32_t xvec;          // X rows aligned for vector loads (xrow_vec)
+    int32_t yvec;          // Y rows likewise
 };
 
 struct BatchHeader {
     int32_t item_begin[kBatchGroups];    // first item of each group (items are stored group by group)
     int32_t n_items[kBatchGroups];
-    int64_t total_chunks[kBatchGroups];
-    int64_t carry_base[kBatchGroups];    // first carry slot of each group
+    int64_t total_windows[kBatchGroups];
+    int64_t total_splits[kBatchGroups];
+    int64_t slot_base[kBatchGroups];     // first split-row slot of each group
 };
 
-// Carry slots of one batch workspace (one per chunk): a row index, an end
-// flag and kMaxK carry and head values of up to 8 bytes.
-constexpr size_t kBatchSlotBytes = 4 + 4 + 2 * 8 * 8;
+// Split-row slots of one batch workspace (one per window): kMaxK values of up
+// to 8 bytes for each of a window's two pieces.
+constexpr size_t kBatchSlotBytes = 2 * kMaxK * 8;
 
-// The stream kernel's plan of a matrix (built once): row of each chunk's first
-// nonzero, chunk count, longest run of empty rows.
-sspmv_status csr_stream_plan(const sspmv_csr *A, const int32_t **row_start, int64_t *num_chunks, int32_t *max_gap,
-                             sspmv_stream_t s);
-// Whether the stream kernel (and so the batched kernel) takes the matrix.
-bool csr_stream_takes(int64_t num_nnzs, int32_t max_gap);
+// Slots for a batch of `requests` matrices of `chunks` 256-nonzero chunks in
+// all: a window holds at least 480 nonzeros (window_size), so a matrix has no
+// more windows than chunks.
+inline int64_t batch_slots(int64_t chunks, int64_t requests) { return chunks + requests; }
+
+// The stream kernel's view of a matrix with nonzeros (its plan built on the
+// first call).
+sspmv_status csr_stream_view(const sspmv_csr *A, StreamView *view, sspmv_stream_t s);
 
 // Persistent grid size of group g (SMs x resident CTAs of its batch kernel).
 unsigned csr_batch_grid(int g);
 
-// Launches group g's batched stream kernel and its fix-up kernel on stream s.
+// Launches group g's batched stream kernel and its split-row kernel on stream s.
 // Header and items are read from device memory when the kernels run, so the
 // launches can be captured once and replayed for every batch.
 sspmv_status launch_csr_batch_group(int g, const BatchHeader *d_hdr, const BatchItem *d_items, void *carry,

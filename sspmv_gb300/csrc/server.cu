@@ -73,8 +73,8 @@ struct Matrix {
     int64_t bytes = 0;
     int64_t refs = 0;        // requests in batches not yet completed (or being formed)
     uint64_t last_use = 0;   // LRU clock
-    const int32_t *row_start = nullptr;  // CSR stream plan: first row of each 256-nonzero chunk
-    int64_t chunks = 0;
+    StreamView view;                     // CSR: what the batched stream kernel reads
+    int64_t chunks = 0;                  // 256-nonzero chunks (max_batch_tiles counts these)
     bool batchable = false;              // the batched stream kernel takes this matrix
     // The plan of a matrix (carry buffers) is shared by its per-request
     // launches: launches on different streams are ordered through this event.
@@ -123,8 +123,8 @@ struct Batch {
     sspmv_status st = SSPMV_OK;
 };
 
-// Device bytes a resident matrix holds (arrays; plans counted as chunk
-// starts + carries).
+// Device bytes a resident matrix holds (arrays; plans counted at a bound of
+// their window records and split-row slots).
 int64_t device_bytes(const Matrix &M) {
     const int64_t V = (int64_t)vsize(M.vt), m = M.m, nnz = M.nnz;
     const int64_t plan = 2 * ((m + nnz) / 1024 + 2) * 152;
@@ -196,7 +196,7 @@ void release(Matrix &M) {
     if (M.ev) cudaEventDestroy(M.ev);
     M.ev = nullptr;
     M.ev_stream = nullptr;
-    M.row_start = nullptr;
+    M.view = StreamView();
     M.batchable = false;
     M.resident = false;
 }
@@ -207,6 +207,7 @@ struct Server {
     sspmv_server_config cfg{};
     int device = 0;
     size_t desc_bytes = 0, in_bytes = 0, out_bytes = 0;
+    int64_t slots = 0;  // split-row slots of a workspace
     std::vector<Workspace> ws;
     cudaStream_t load_stream = nullptr;
     cudaStream_t capture_stream = nullptr;  // idle stream the batch graphs are captured on
@@ -258,7 +259,8 @@ sspmv_status Server::init() {
         SSPMV_CUDA_TRY(cudaMalloc(&w.d_out, out_bytes));
         SSPMV_CUDA_TRY(cudaMallocHost(&w.h_in, in_bytes));
         SSPMV_CUDA_TRY(cudaMallocHost(&w.h_out, out_bytes));
-        SSPMV_CUDA_TRY(cudaMalloc(&w.carry, (size_t)cfg.max_batch_tiles * kBatchSlotBytes));
+        slots = batch_slots(cfg.max_batch_tiles, cfg.max_batch_requests);
+        SSPMV_CUDA_TRY(cudaMalloc(&w.carry, (size_t)slots * kBatchSlotBytes));
     }
     SSPMV_CUDA_TRY(cudaStreamCreateWithFlags(&load_stream, cudaStreamNonBlocking));
     SSPMV_CUDA_TRY(cudaStreamCreateWithFlags(&capture_stream, cudaStreamNonBlocking));
@@ -339,9 +341,9 @@ sspmv_status Server::load(Matrix &M) {
     sspmv_status st = SSPMV_OK;
     if (M.fmt == SSPMV_FMT_CSR) {
         M.dev.csr = csr;
-        int32_t gap = 0;
-        st = csr_stream_plan(&M.dev.csr, &M.row_start, &M.chunks, &gap, s);
-        M.batchable = st == SSPMV_OK && csr_stream_takes(M.nnz, gap);
+        if (M.nnz > 0) st = csr_stream_view(&M.dev.csr, &M.view, s);
+        M.chunks = (M.nnz + 255) / 256;
+        M.batchable = st == SSPMV_OK && M.nnz > 0;
     } else {
         st = convert(&csr, M, s);
         cudaStreamSynchronize(load_stream);
@@ -461,7 +463,8 @@ void Server::worker_loop() {
             r->stage_x = !on_device && (int64_t)r->x_bytes <= cfg.stage_limit_bytes;
             r->stage_y = !on_device && (int64_t)r->y_bytes <= cfg.stage_limit_bytes;
             const bool batched = !per_request && M.fmt == SSPMV_FMT_CSR && M.batchable &&
-                                 (k == 1 || k == 2 || k == 4 || k == 8);
+                                 (k == 1 || k == 2 || k == 4 || k == 8) &&
+                                 stream_takes_strides(r->r.ldx, r->r.ldy, V);
             const int64_t t = batched ? M.chunks : 0;
             const size_t xa = up256(r->x_bytes), ya = up256(r->y_bytes);
             const bool fits = x_front + x_back + xa <= in_cap && y_front + y_back + ya <= out_bytes &&
@@ -507,7 +510,7 @@ void Server::worker_loop() {
     }
 }
 
-// The workspace's batch graph: every group's stream kernel and fix-up as
+// The workspace's batch graph: every group's two kernels as
 // parallel branches (a group without requests in a batch exits at once), so
 // one graph serves every batch and is captured before the first one.
 // Captured on an idle stream (kernel arguments name only this workspace's
@@ -534,7 +537,7 @@ sspmv_status Server::ensure_graph(Workspace &w) {
             cudaStream_t bs = g == 0 ? cs : side[g - 1];
             if (g > 0) cudaStreamWaitEvent(bs, evs[0], 0);
             if (st == SSPMV_OK)
-                st = launch_csr_batch_group(g, d_hdr, d_items, w.carry, cfg.max_batch_tiles,
+                st = launch_csr_batch_group(g, d_hdr, d_items, w.carry, slots,
                                             reinterpret_cast<sspmv_stream_t>(bs));
             if (g > 0) {
                 cudaEventRecord(evs[g], bs);
@@ -561,7 +564,7 @@ sspmv_status Server::launch_groups(Workspace &w, uint32_t mask) {
         BatchItem *d_items = reinterpret_cast<BatchItem *>(w.d_in + sizeof(BatchHeader));
         sspmv_stream_t s = reinterpret_cast<sspmv_stream_t>(w.stream);
         for (int g = 0; g < kBatchGroups; g++)
-            if (mask & (1u << g)) SSPMV_TRY(launch_csr_batch_group(g, d_hdr, d_items, w.carry, cfg.max_batch_tiles, s));
+            if (mask & (1u << g)) SSPMV_TRY(launch_csr_batch_group(g, d_hdr, d_items, w.carry, slots, s));
         return SSPMV_OK;
     }
     SSPMV_TRY(ensure_graph(w));
@@ -598,38 +601,34 @@ void Server::issue(Batch &b) {
     }
     BatchItem *items = reinterpret_cast<BatchItem *>(w.h_in + sizeof(BatchHeader));
     int fill[kBatchGroups] = {0};
-    int64_t group_tiles[kBatchGroups] = {0};
+    int64_t group_tiles[kBatchGroups] = {0}, group_splits[kBatchGroups] = {0};
     uint32_t mask = 0;
     for (Request *r : b.reqs) {
         if (r->group < 0) continue;
         const int g = r->group;
         const Matrix &M = *r->mat;
         BatchItem &it = items[hdr.item_begin[g] + fill[g]++];
-        it.row_offset = M.dev.csr.row_offset;
-        it.col_index = M.dev.csr.col_index;
-        it.values = M.dev.csr.values;
-        it.row_start = M.row_start;
+        it.view = M.view;
         it.x = r->d_x;
         it.y = r->d_y;
         it.ldx = r->r.ldx;
         it.ldy = r->r.ldy;
         it.alpha = r->r.alpha;
         it.beta = r->r.beta;
-        it.chunk_begin = group_tiles[g];
-        it.nnz = M.nnz;
-        it.m = (int32_t)M.m;
-        it.num_chunks = (int32_t)M.chunks;
-        it.vec = ((reinterpret_cast<uintptr_t>(M.dev.csr.col_index) | reinterpret_cast<uintptr_t>(M.dev.csr.values)) &
-                  15) == 0;
+        it.window_begin = group_tiles[g];
+        it.split_begin = group_splits[g];
         it.xvec = xrow_vec(r->d_x, r->r.ldx, g >= 4 ? 8 : 4, r->r.k);
-        group_tiles[g] += M.chunks;
+        it.yvec = xrow_vec(r->d_y, r->r.ldy, g >= 4 ? 8 : 4, r->r.k);
+        group_tiles[g] += M.view.windows;
+        group_splits[g] += M.view.nsplit;
         mask |= 1u << g;
     }
     int64_t carry = 0;
     for (int g = 0; g < kBatchGroups; g++) {
         hdr.n_items[g] = counts[g];
-        hdr.total_chunks[g] = group_tiles[g];
-        hdr.carry_base[g] = carry;
+        hdr.total_windows[g] = group_tiles[g];
+        hdr.total_splits[g] = group_splits[g];
+        hdr.slot_base[g] = carry;
         carry += group_tiles[g];
     }
     std::memcpy(w.h_in, &hdr, sizeof(hdr));

@@ -427,10 +427,8 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
             p->sub = new (std::nothrow) sspmv_csr();
             if (!p->sub) return fail(SSPMV_OUT_OF_MEMORY, "overflow matrix allocation failed");
             SSPMV_TRY(sspmv_csr_wrap(p->sub, f->value_type, nshort, v.n, optr[(size_t)nshort], dptr, ocol, oval));
-            const int32_t *rs = nullptr;
-            int64_t nch = 0;
-            int32_t gap = 0;
-            SSPMV_TRY(csr_stream_plan(p->sub, &rs, &nch, &gap, s));  // built now, not inside a later SpMV
+            StreamView v2;
+            SSPMV_TRY(csr_stream_view(p->sub, &v2, s));  // built now, not inside a later SpMV
         }
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
     }

@@ -3,9 +3,9 @@
 // Replaces LeSpMV_csr (src/spmv_csr.cpp:165-185) and its three CPU kernels
 // (serial, OpenMP per row, nnz-balanced row partition).
 //
-// Default kernel (kernel_flag 0): the nonzero-split stream kernel (see
-// csr_stream_kernel); matrices with long runs of empty rows fall back to
-// merge-path.  kernel_flag 4: the pipelined thread-per-row kernel for
+// Default kernel (kernel_flag 0): the nonzero-split stream kernel
+// (csr_stream.cu); a matrix without nonzeros runs merge-path.  kernel_flag 4:
+// the pipelined thread-per-row kernel for
 // matrices whose rows all have at most 12 nonzeros (csr_pipe_kernel).
 // kernel_flag 3: the row-block kernel for matrices whose rows are all short
 // (csr_rowblock_kernel; one launch, no fix-up).  kernel_flag 2: merge-path.
@@ -32,6 +32,7 @@
 #include "primitives.cuh"
 #include "spmv_common.cuh"
 #include "csr_pipe.cuh"
+#include "csr_stream.cuh"
 #include "serve.cuh"
 
 namespace sspmv {
@@ -758,780 +759,18 @@ sspmv_status launch_rowblock(const sspmv_csr *A, Plan *p, V alpha, const V *x, i
     return SSPMV_OK;
 }
 
-// ------------------------------------------------------- stream kernel --
-// kernel_flag 0: nonzero-split "stream" kernel.  A warp takes 256 consecutive
-// nonzeros, lane l the 8 at 8l (vector loads of columns and values, all 8
-// gathers issued before use for k <= 2).  A lane finds the row of its first
-// nonzero by binary search inside the warp's row range (row_start of the
-// chunk, from the plan) and walks row_offset from there; a nonzero ends its
-// row when row_offset[r + 1] == e + 1.  Rows that start and end inside a lane
-// are written by it; the open sums before a lane's first row end and after
-// its last are joined by one segmented shuffle scan per warp, rows crossing
-// warps by a fix-up in chunk order (deterministic, no atomics).  The lane that
-// ends a row also writes the empty rows right after it (and the lane holding
-// nonzero 0 the empty rows before it); matrices with a run of more than
-// kStreamMaxGap empty rows use the merge-path kernel instead.
-constexpr int kStreamPerLane = 8;
-constexpr int kStreamChunk = 32 * kStreamPerLane;
-constexpr int kStreamMaxGap = 256;
-
-__global__ void stream_row_starts(int64_t nt, int m, int64_t nnz, const int32_t *__restrict__ rp,
-                                  int32_t *__restrict__ row_start) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t > nt) return;
-    const int64_t e = t * kStreamChunk;
-    if (e >= nnz) {
-        row_start[t] = m;
-        return;
-    }
-    int lo = 0, hi = m - 1;  // last row r with rp[r] <= e: the row holding nonzero e
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (rp[mid] <= e) lo = mid;
-        else hi = mid - 1;
-    }
-    row_start[t] = lo;
-}
-
-// Longest run of empty rows (runs longer than kStreamMaxGap stop counting).
-__global__ void stream_max_gap(int m, const int32_t *__restrict__ rp, int *__restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        if (rp[i + 1] != rp[i] || (i > 0 && rp[i] == rp[i - 1])) continue;  // not the start of an empty run
-        int len = 0;
-        for (int64_t j = i; j < m && rp[j + 1] == rp[j] && len <= kStreamMaxGap; j++) len++;
-        atomicMax(out, len);
-    }
-}
-
-template <typename V>
-__device__ __forceinline__ void stream_load8(const int32_t *__restrict__ ci, const V *__restrict__ cv, int64_t e0,
-                                             int nv, bool vec, int (&c)[8], V (&a)[8]) {
-    if (vec && nv == 8) {
-        const int4 c0 = __ldcs(reinterpret_cast<const int4 *>(ci + e0));
-        const int4 c1 = __ldcs(reinterpret_cast<const int4 *>(ci + e0 + 4));
-        c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
-        if constexpr (sizeof(V) == 8) {
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const double2 v = __ldcs(reinterpret_cast<const double2 *>(cv + e0) + h);
-                a[2 * h] = v.x;
-                a[2 * h + 1] = v.y;
-            }
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const float4 v = __ldcs(reinterpret_cast<const float4 *>(cv + e0) + h);
-                a[4 * h] = v.x; a[4 * h + 1] = v.y; a[4 * h + 2] = v.z; a[4 * h + 3] = v.w;
-            }
-        }
-        return;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        c[u] = u < nv ? ld_stream(ci + e0 + u) : 0;
-        a[u] = u < nv ? ld_stream(cv + e0 + u) : V(0);
-    }
-}
-
-// The stream kernel for FP64 with k = 8 right-hand sides: groups of G = k
-// lanes share a run of 8G consecutive nonzeros, lane q of a group owning column q,
-// so each gathered row X[col, 0:k] (k consecutive values) is read by G
-// adjacent lanes in one coalesced access instead of k scattered loads by one
-// lane.  A group walks its nonzeros in order (loads of 8 in flight) with the
-// row logic of the per-lane form; the groups' open sums are joined by a
-// segmented shuffle scan with stride G.
-template <typename V, int K, int G>
-__device__ __forceinline__ void stream_chunk_cols(
-    int m, int64_t nnz, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const V *__restrict__ cv,
-    const V *__restrict__ x, int64_t ldx, V alpha, V beta, V *__restrict__ y, int64_t ldy,
-    const int32_t *__restrict__ row_start, const int64_t w, const int64_t slot, int32_t *__restrict__ carry_row,
-    int32_t *__restrict__ has_end, V *__restrict__ carry_val, V *__restrict__ head_val) {
-    static_assert(K % G == 0 && 32 % G == 0, "group shape");
-    constexpr int KL = K / G;                 // columns per lane
-    constexpr int NG = 32 / G;                // groups per warp
-    constexpr int EPG = kStreamChunk / NG;    // nonzeros per group (8G)
-    constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x & 31, gi = lane / G, q0 = (lane % G) * KL;
-    const int64_t j0 = w * kStreamChunk;
-    if (j0 >= nnz) return;  // warp-uniform
-    const int64_t j1 = min(j0 + (int64_t)kStreamChunk, nnz);
-    const int64_t e0 = j0 + (int64_t)gi * EPG;
-    const int nv = (int)max((int64_t)0, min((int64_t)EPG, j1 - e0));
-    const int ra = __ldg(row_start + w);
-    const bool head_open = __ldg(rp + ra) < j0;
-    int r = ra;
-    if (nv > 0) {
-        int lo = ra, hi = min(__ldg(row_start + w + 1), m - 1);
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(rp + mid) <= e0) lo = mid;
-            else hi = mid - 1;
-        }
-        r = lo;
-    }
-    if (e0 == 0 && nv > 0) {  // empty rows before the first nonzero
-        for (int r2 = 0; r2 < r; r2++) {
-            V *yp = y + (int64_t)r2 * ldy + q0;
-#pragma unroll
-            for (int q = 0; q < KL; q++) yp[q] = axpby(alpha, V(0), beta, yp + q);
-        }
-    }
-    int rend = nv > 0 ? __ldg(rp + r + 1) : 0;
-    V seg[KL], head[KL];
-#pragma unroll
-    for (int q = 0; q < KL; q++) seg[q] = head[q] = V(0);
-    bool any_end = false, last_open = false;
-    int head_row = -1, last_row = -1;
-    constexpr int SB = 8;  // nonzeros whose loads are in flight together
-    for (int s0 = 0; s0 < nv; s0 += SB) {  // group-uniform
-        int c[SB];
-        V a[SB], xv[SB][KL];
-#pragma unroll
-        for (int u = 0; u < SB; u++) {
-            const bool ok = s0 + u < nv;
-            c[u] = ok ? ld_stream(ci + e0 + s0 + u) : 0;
-            a[u] = ok ? ld_stream(cv + e0 + s0 + u) : V(0);
-        }
-#pragma unroll
-        for (int u = 0; u < SB; u++)
-#pragma unroll
-            for (int q = 0; q < KL; q++)
-                xv[u][q] = s0 + u < nv ? ld_x(x + (int64_t)c[u] * ldx + q0 + q) : V(0);
-#pragma unroll
-        for (int u = 0; u < SB; u++) {
-            if (s0 + u < nv) {
-                const int64_t e = e0 + s0 + u;
-                while (rend <= e) rend = __ldg(rp + (++r) + 1);
-#pragma unroll
-                for (int q = 0; q < KL; q++) seg[q] += a[u] * xv[u][q];
-                last_row = r;
-                last_open = rend != e + 1;
-                if (!last_open) {
-                    if (!any_end) {
-                        any_end = true;
-                        head_row = r;
-#pragma unroll
-                        for (int q = 0; q < KL; q++) head[q] = seg[q];
-                    } else {
-                        V *yp = y + (int64_t)r * ldy + q0;
-#pragma unroll
-                        for (int q = 0; q < KL; q++) yp[q] = axpby(alpha, seg[q], beta, yp + q);
-                    }
-#pragma unroll
-                    for (int q = 0; q < KL; q++) seg[q] = V(0);
-                    for (int r2 = r + 1; r2 < m && __ldg(rp + r2 + 1) == e + 1; r2++) {
-                        V *yp = y + (int64_t)r2 * ldy + q0;
-#pragma unroll
-                        for (int q = 0; q < KL; q++) yp[q] = axpby(alpha, V(0), beta, yp + q);
-                    }
-                }
-            }
-        }
-    }
-    V S[KL];
-#pragma unroll
-    for (int q = 0; q < KL; q++) S[q] = seg[q];
-    bool f = any_end;
-#pragma unroll
-    for (int o = 1; o < NG; o <<= 1) {
-        V up[KL];
-#pragma unroll
-        for (int q = 0; q < KL; q++) up[q] = __shfl_up_sync(kFull, S[q], o * G);
-        const bool fu = __shfl_up_sync(kFull, f, o * G);
-        if (gi >= o) {
-            if (!f) {
-#pragma unroll
-                for (int q = 0; q < KL; q++) S[q] += up[q];
-            }
-            f = f || fu;
-        }
-    }
-    V cin[KL];
-#pragma unroll
-    for (int q = 0; q < KL; q++) {
-        cin[q] = __shfl_up_sync(kFull, S[q], G);
-        if (gi == 0) cin[q] = V(0);
-    }
-    if (any_end) {
-        V tot[KL];
-#pragma unroll
-        for (int q = 0; q < KL; q++) tot[q] = head[q] + cin[q];
-        if (head_row == ra && head_open) {
-            V *hp = head_val + slot * kMaxK + q0;
-#pragma unroll
-            for (int q = 0; q < KL; q++) hp[q] = tot[q];
-        } else {
-            V *yp = y + (int64_t)head_row * ldy + q0;
-#pragma unroll
-            for (int q = 0; q < KL; q++) yp[q] = axpby(alpha, tot[q], beta, yp + q);
-        }
-    }
-    const bool chunk_end = __any_sync(kFull, any_end);
-    if (nv > 0 && e0 + nv == j1) {  // the group holding the chunk's last nonzero
-        if (q0 == 0) {
-            has_end[slot] = chunk_end ? 1 : 0;
-            carry_row[slot] = last_open ? last_row : -1;
-        }
-        if (last_open) {
-            V *cp = carry_val + slot * kMaxK + q0;
-#pragma unroll
-            for (int q = 0; q < KL; q++) cp[q] = S[q];
-        }
-    }
-}
-
-// Chunk w (nonzeros 256w ..) of one matrix, run by one warp; `slot` indexes
-// the carry arrays.  Shared by the single-matrix kernel and the batched
-// serving kernel.
-template <typename V, int K, bool PLAIN = false>
-__device__ __forceinline__ void stream_chunk_lanes(
-    int m, int64_t nnz, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const V *__restrict__ cv,
-    const V *__restrict__ x, int64_t ldx, V alpha, V beta, V *__restrict__ y, int64_t ldy,
-    const int32_t *__restrict__ row_start, const int64_t w, const int64_t slot, int32_t *__restrict__ carry_row,
-    int32_t *__restrict__ has_end, V *__restrict__ carry_val, V *__restrict__ head_val, int vec, int xvec) {
-    constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    constexpr bool plain = PLAIN;  // alpha == 1 and beta == 0: y = sum
-    const int64_t j0 = w * kStreamChunk;
-    if (j0 >= nnz) return;  // warp-uniform
-    const int64_t j1 = min(j0 + (int64_t)kStreamChunk, nnz);
-    const int64_t e0 = j0 + (int64_t)lane * kStreamPerLane;
-    const int nv = (int)max((int64_t)0, min((int64_t)kStreamPerLane, j1 - e0));
-    int c[8];
-    V a[8];
-    stream_load8<V>(ci, cv, e0, nv, vec != 0, c, a);
-    const int ra = __ldg(row_start + w);
-    const bool head_open = __ldg(rp + ra) < j0;  // the chunk's first row began in an earlier chunk
-    int r = ra;
-    if (nv > 0) {
-        int lo = ra, hi = min(__ldg(row_start + w + 1), m - 1);
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(rp + mid) <= e0) lo = mid;
-            else hi = mid - 1;
-        }
-        r = lo;
-    }
-    V xv[K <= 2 ? 8 : 1][K];
-    if constexpr (K <= 2) {
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (u < nv) {
-                ld_xrow<V, K>(x, c[u], ldx, xvec != 0, xv[u]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < K; q++) xv[u][q] = V(0);
-            }
-        }
-    }
-    if (e0 == 0 && nv > 0) {  // empty rows before the first nonzero
-        for (int r2 = 0; r2 < r; r2++) {
-            V *yp = y + (int64_t)r2 * ldy;
-#pragma unroll
-            for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, V(0), beta, yp + q);
-        }
-    }
-    int rend = nv > 0 ? __ldg(rp + r + 1) : 0;
-    V seg[K], head[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) seg[q] = head[q] = V(0);
-    bool any_end = false, last_open = false;
-    int head_row = -1, last_row = -1;
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        if (u < nv) {
-            const int64_t e = e0 + u;
-            while (rend <= e) rend = __ldg(rp + (++r) + 1);  // skip empty rows
-            if constexpr (K <= 2) {
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] += a[u] * xv[u][q];
-            } else {
-                V xr[K];
-                ld_xrow<V, K>(x, c[u], ldx, xvec != 0, xr);
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] += a[u] * xr[q];
-            }
-            last_row = r;
-            last_open = rend != e + 1;
-            if (!last_open) {  // row r ends at e
-                if (!any_end) {
-                    any_end = true;
-                    head_row = r;
-#pragma unroll
-                    for (int q = 0; q < K; q++) head[q] = seg[q];
-                } else {
-                    V *yp = y + (int64_t)r * ldy;
-#pragma unroll
-                    for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, seg[q], beta, yp + q);
-                }
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] = V(0);
-                for (int r2 = r + 1; r2 < m && __ldg(rp + r2 + 1) == e + 1; r2++) {  // empty rows after r
-                    V *yp = y + (int64_t)r2 * ldy;
-#pragma unroll
-                    for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, V(0), beta, yp + q);
-                }
-            }
-        }
-    }
-    V S[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) S[q] = seg[q];
-    bool f = any_end;
-    const int span = unflagged_run(f);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        if (o > span) break;  // warp-uniform
-        V up[K];
-#pragma unroll
-        for (int q = 0; q < K; q++) up[q] = __shfl_up_sync(kFull, S[q], o);
-        const bool fu = __shfl_up_sync(kFull, f, o);
-        if (lane >= o) {
-            if (!f) {
-#pragma unroll
-                for (int q = 0; q < K; q++) S[q] += up[q];
-            }
-            f = f || fu;
-        }
-    }
-    V cin[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) {
-        cin[q] = __shfl_up_sync(kFull, S[q], 1);
-        if (lane == 0) cin[q] = V(0);
-    }
-    if (any_end) {
-        V tot[K];
-#pragma unroll
-        for (int q = 0; q < K; q++) tot[q] = head[q] + cin[q];
-        if (head_row == ra && head_open) {
-            V *hp = head_val + slot * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) hp[q] = tot[q];
-        } else {
-            V *yp = y + (int64_t)head_row * ldy;
-#pragma unroll
-            for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, tot[q], beta, yp + q);
-        }
-    }
-    const bool chunk_end = __any_sync(kFull, any_end);
-    if (nv > 0 && e0 + nv == j1) {  // the lane holding the chunk's last nonzero
-        has_end[slot] = chunk_end ? 1 : 0;
-        carry_row[slot] = last_open ? last_row : -1;
-        if (last_open) {
-            V *cp = carry_val + slot * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) cp[q] = S[q];
-        }
-    }
-}
-
-// The chunk of a matrix without empty rows: the rows starting inside the
-// chunk are read once (row_offset[ra ..], one row per lane per step) and
-// marked as bits in shared memory (one 8-bit word per lane, position p of the
-// chunk at word p / 8, bit p % 8); each lane then knows which of its 8
-// nonzeros end a row (the next position starts one) and, by a prefix count of
-// the bits, the row of its first nonzero -- no search and no chain of
-// dependent loads on row_offset.  The arithmetic (per-lane sums in nonzero
-// order, the segmented scan, the carry slots) is that of stream_chunk_lanes,
-// so both give the same bits.  sbits: the warp's 33 words of shared memory.
-template <typename V, int K, bool PLAIN = false>
-__device__ __forceinline__ void stream_chunk_fast(
-    int m, int64_t nnz, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const V *__restrict__ cv,
-    const V *__restrict__ x, int64_t ldx, V alpha, V beta, V *__restrict__ y, int64_t ldy, const int ra,
-    const int last, const int64_t w, const int64_t slot, int32_t *__restrict__ carry_row,
-    int32_t *__restrict__ has_end, V *__restrict__ carry_val, V *__restrict__ head_val, int vec, int xvec,
-    uint32_t *__restrict__ sbits) {
-    constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    constexpr bool plain = PLAIN;  // alpha == 1 and beta == 0: y = sum
-    const int64_t j0 = w * kStreamChunk;
-    const int64_t j1 = min(j0 + (int64_t)kStreamChunk, nnz);
-    const int64_t e0 = j0 + (int64_t)lane * kStreamPerLane;
-    const int nv = (int)max((int64_t)0, min((int64_t)kStreamPerLane, j1 - e0));
-    int c[8];
-    V a[8];
-    stream_load8<V>(ci, cv, e0, nv, vec != 0, c, a);
-    sbits[lane] = 0u;
-    if (lane == 0) sbits[32] = 0u;
-    __syncwarp();
-    // rows ra .. last (last = one past the row holding the chunk's end): mark
-    // each start p in (0, 256] (p = 256: a row starting right after the chunk)
-    bool head_open = false;
-    for (int r0 = ra; r0 <= last; r0 += 32) {  // warp-uniform
-        const int rr = r0 + lane;
-        if (rr <= last) {
-            const int64_t p = (int64_t)__ldg(rp + rr) - j0;
-            if (p > 0 && p <= kStreamChunk) atomicOr(sbits + (p >> 3), 1u << (p & 7));
-            if (rr == ra) head_open = p < 0;  // the chunk's first row began in an earlier chunk
-        }
-    }
-    head_open = __shfl_sync(kFull, head_open, 0);
-    __syncwarp();
-    const uint32_t starts = sbits[lane], starts_next = sbits[lane + 1];
-    // bit u of `ends`: nonzero u ends its row (a row starts at e0 + u + 1)
-    const uint32_t ends = (starts >> 1) | ((starts_next & 1u) << 7);
-    // the lane's first row: ra + the starts in (j0, e0]
-    int before = __popc(starts);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(kFull, before, o);
-        if (lane >= o) before += t;
-    }
-    before -= __popc(starts);  // starts in lanes before this one
-    const int pos = before + (int)(starts & 1u);
-    V xv[K <= 2 ? 8 : 1][K];
-    if constexpr (K <= 2) {
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (u < nv) {
-                ld_xrow<V, K>(x, c[u], ldx, xvec != 0, xv[u]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < K; q++) xv[u][q] = V(0);
-            }
-        }
-    }
-    int r = ra + pos;
-    V seg[K], head[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) seg[q] = head[q] = V(0);
-    bool any_end = false, last_open = false;
-    int head_row = -1, last_row = -1;
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        if (u < nv) {
-            if constexpr (K <= 2) {
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] += a[u] * xv[u][q];
-            } else {
-                V xr[K];
-                ld_xrow<V, K>(x, c[u], ldx, xvec != 0, xr);
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] += a[u] * xr[q];
-            }
-            last_row = r;
-            last_open = !((ends >> u) & 1u);
-            if (!last_open) {  // row r ends here
-                if (!any_end) {
-                    any_end = true;
-                    head_row = r;
-#pragma unroll
-                    for (int q = 0; q < K; q++) head[q] = seg[q];
-                } else {
-                    V *yp = y + (int64_t)r * ldy;
-#pragma unroll
-                    for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, seg[q], beta, yp + q);
-                }
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] = V(0);
-                r++;
-            }
-        }
-    }
-    V S[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) S[q] = seg[q];
-    bool f = any_end;
-    const int span = unflagged_run(f);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        if (o > span) break;  // warp-uniform
-        V up[K];
-#pragma unroll
-        for (int q = 0; q < K; q++) up[q] = __shfl_up_sync(kFull, S[q], o);
-        const bool fu = __shfl_up_sync(kFull, f, o);
-        if (lane >= o) {
-            if (!f) {
-#pragma unroll
-                for (int q = 0; q < K; q++) S[q] += up[q];
-            }
-            f = f || fu;
-        }
-    }
-    V cin[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) {
-        cin[q] = __shfl_up_sync(kFull, S[q], 1);
-        if (lane == 0) cin[q] = V(0);
-    }
-    if (any_end) {
-        V tot[K];
-#pragma unroll
-        for (int q = 0; q < K; q++) tot[q] = head[q] + cin[q];
-        if (head_row == ra && head_open) {
-            V *hp = head_val + slot * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) hp[q] = tot[q];
-        } else {
-            V *yp = y + (int64_t)head_row * ldy;
-#pragma unroll
-            for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, tot[q], beta, yp + q);
-        }
-    }
-    const bool chunk_end = __any_sync(kFull, any_end);
-    if (nv > 0 && e0 + nv == j1) {  // the lane holding the chunk's last nonzero
-        has_end[slot] = chunk_end ? 1 : 0;
-        carry_row[slot] = last_open ? last_row : -1;
-        if (last_open) {
-            V *cp = carry_val + slot * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) cp[q] = S[q];
-        }
-    }
-}
-
-// One lane per nonzero run (stream_chunk_lanes), except FP64 with k = 8:
-// column groups (stream_chunk_cols), which read each 64-byte row of X with
-// one coalesced access (measured 1.3-1.4x faster there; slower for FP32 and
-// mixed for k = 4).
-template <typename V, int K, bool PLAIN = false>
-__device__ __forceinline__ void stream_chunk(
-    int m, int64_t nnz, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const V *__restrict__ cv,
-    const V *__restrict__ x, int64_t ldx, V alpha, V beta, V *__restrict__ y, int64_t ldy,
-    const int32_t *__restrict__ row_start, const int64_t w, const int64_t slot, int32_t *__restrict__ carry_row,
-    int32_t *__restrict__ has_end, V *__restrict__ carry_val, V *__restrict__ head_val, int vec, int xvec,
-    int no_empty, uint32_t *__restrict__ sbits) {
-    if constexpr (K == 8 && sizeof(V) == 8) {
-        stream_chunk_cols<V, K, K>(m, nnz, rp, ci, cv, x, ldx, alpha, beta, y, ldy, row_start, w, slot, carry_row,
-                                   has_end, carry_val, head_val);
-    } else {
-        if (no_empty && w * kStreamChunk < nnz) {  // warp-uniform
-            const int ra = __ldg(row_start + w);
-            const int last = min(__ldg(row_start + w + 1), m - 1) + 1;
-            stream_chunk_fast<V, K, PLAIN>(m, nnz, rp, ci, cv, x, ldx, alpha, beta, y, ldy, ra, last, w, slot,
-                                           carry_row, has_end, carry_val, head_val, vec, xvec, sbits);
-            return;
-        }
-        stream_chunk_lanes<V, K, PLAIN>(m, nnz, rp, ci, cv, x, ldx, alpha, beta, y, ldy, row_start, w, slot,
-                                        carry_row, has_end, carry_val, head_val, vec, xvec);
-    }
-}
-
-#define SSPMV_STREAM_KERNEL_BODY                                                                          \
-    __shared__ uint32_t s_bits[kBlock / 32][33];                                                          \
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;                              \
-    stream_chunk<V, K, PLAIN>(m, nnz, rp, ci, cv, x, ldx, alpha, beta, y, ldy, row_start, w, w, carry_row,    \
-                              has_end, carry_val, head_val, vec, xvec, no_empty, s_bits[threadIdx.x >> 5]);
-
-// PLAIN: alpha == 1 and beta == 0 (y = sum), instantiated for k = 1: the
-// rows' writes then carry no FP64 multiply.
-template <typename V, int K, bool PLAIN = false>
-__global__ void __launch_bounds__(kBlock) csr_stream_kernel(
-    int m, int64_t nnz, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const V *__restrict__ cv,
-    const V *__restrict__ x, int64_t ldx, V alpha, V beta, V *__restrict__ y, int64_t ldy,
-    const int32_t *__restrict__ row_start, int32_t *__restrict__ carry_row, int32_t *__restrict__ has_end,
-    V *__restrict__ carry_val, V *__restrict__ head_val, int vec, int xvec, int no_empty) {
-    SSPMV_STREAM_KERNEL_BODY
-}
-
-// The same kernel held to six resident CTAs per SM (at most 42 registers):
-// measured 5-8% faster for FP32 at k = 1; FP64 slows down when squeezed.
-template <typename V, int K, bool PLAIN = false>
-__global__ void __launch_bounds__(kBlock, 6) csr_stream_kernel_occ6(
-    int m, int64_t nnz, const int32_t *__restrict__ rp, const int32_t *__restrict__ ci, const V *__restrict__ cv,
-    const V *__restrict__ x, int64_t ldx, V alpha, V beta, V *__restrict__ y, int64_t ldy,
-    const int32_t *__restrict__ row_start, int32_t *__restrict__ carry_row, int32_t *__restrict__ has_end,
-    V *__restrict__ carry_val, V *__restrict__ head_val, int vec, int xvec, int no_empty) {
-    SSPMV_STREAM_KERNEL_BODY
-}
-#undef SSPMV_STREAM_KERNEL_BODY
-
-// Rows crossing chunks: a thread per chunk; the chunk where the row starts
-// adds the later chunks' pieces (chain_sum).
-template <typename V, int K>
-__global__ void csr_stream_fixup(int64_t nt, const int32_t *__restrict__ rp, const int32_t *__restrict__ carry_row,
-                                 const int32_t *__restrict__ has_end, const V *__restrict__ carry_val,
-                                 const V *__restrict__ head_val, V alpha, V beta, V *__restrict__ y, int64_t ldy) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t - (threadIdx.x & 31) >= nt) return;  // whole warp past the end
-    const int r = t < nt ? carry_row[t] : -1;
-    const bool mine = r >= 0 && (int64_t)rp[r] >= t * kStreamChunk;  // open here and began here
-    V tot[K];
-    chain_sum<V, K>(mine, t, nt, 0, has_end, carry_val, head_val, tot);
-    if (mine) {
-        V *yp = y + (int64_t)r * ldy;
-#pragma unroll
-        for (int q = 0; q < K; q++) yp[q] = axpby(alpha, tot[q], beta, yp + q);
-    }
-}
-
-// Plan slots of the stream kernel (CSR matrices use no other extra slots):
-// extra[0] row_start[nt + 1], extra[1] carry_row/has_end [2 nt], extra[2]
-// carry values, extra[3] head values; extra_i[0] = nt, extra_i[1] = longest
-// empty-row run (capped just above kStreamMaxGap).
-sspmv_status ensure_stream_plan(const sspmv_csr *A, Plan *p, sspmv_stream_t s) {
-    if (p->extra[0]) return SSPMV_OK;
-    std::lock_guard<PlanMutex> g(plan_mutex());
-    if (p->extra[0]) return SSPMV_OK;
-    const int64_t m = A->f.num_rows, nnz = A->f.num_nnzs;
-    const int64_t nt = std::max<int64_t>((nnz + kStreamChunk - 1) / kStreamChunk, 1);
-    const size_t sv = vsize(A->f.value_type);
-    int32_t *starts = nullptr, *ints = nullptr;
-    unsigned char *cvals = nullptr, *hvals = nullptr;
-    int *gap = nullptr;
-    SSPMV_TRY(dalloc(&starts, (size_t)nt + 1, s));
-    SSPMV_TRY(dalloc(&ints, (size_t)nt * 2, s));
-    SSPMV_TRY(dalloc(&cvals, (size_t)nt * kMaxK * sv, s));
-    SSPMV_TRY(dalloc(&hvals, (size_t)nt * kMaxK * sv, s));
-    SSPMV_TRY(dalloc(&gap, 1, s));
-    SSPMV_CUDA_TRY(cudaMemsetAsync(gap, 0, sizeof(int), cu(s)));
-    stream_row_starts<<<grid_for(nt + 1, 256), 256, 0, cu(s)>>>(nt, (int)m, nnz, A->row_offset, starts);
-    SSPMV_LAUNCH_CHECK();
-    stream_max_gap<<<grid_for(m, 256, (int64_t)num_sms() * 16), 256, 0, cu(s)>>>((int)m, A->row_offset, gap);
-    SSPMV_LAUNCH_CHECK();
-    int hgap = 0;
-    SSPMV_CUDA_TRY(cudaMemcpyAsync(&hgap, gap, sizeof(int), cudaMemcpyDeviceToHost, cu(s)));
-    SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
-    dfree(gap, s);
-    p->extra_i[0] = nt;
-    p->extra_i[1] = hgap;
-    p->extra[1] = ints;
-    p->extra[2] = cvals;
-    p->extra[3] = hvals;
-    p->extra[0] = starts;  // published last
-    return SSPMV_OK;
-}
-
 template <typename V, int K>
 sspmv_status launch_stream(const sspmv_csr *A, Plan *p, V alpha, const V *x, int64_t ldx, V beta, V *y,
                            int64_t ldy, sspmv_stream_t s) {
-    if (A->f.num_nnzs == 0) return launch_merge<V, K>(A, p, alpha, x, ldx, beta, y, ldy, s);
-    SSPMV_TRY(ensure_stream_plan(A, p, s));
-    if (p->extra_i[1] > kStreamMaxGap) return launch_merge<V, K>(A, p, alpha, x, ldx, beta, y, ldy, s);
-    const int64_t nt = p->extra_i[0];
-    int32_t *ints = (int32_t *)p->extra[1];
-    const int vec = ((reinterpret_cast<uintptr_t>(A->col_index) | reinterpret_cast<uintptr_t>(A->values)) & 15) == 0;
-    const unsigned grid = grid_for(nt * 32, kBlock);
-    const int no_empty = p->extra_i[1] == 0 ? 1 : 0;
-    const int xvec = xrow_vec(x, ldx, sizeof(V), K);
-    auto go = [&](auto kernel) {
-        kernel<<<grid, kBlock, 0, cu(s)>>>((int)A->f.num_rows, A->f.num_nnzs, A->row_offset, A->col_index,
-                                           (const V *)A->values, x, ldx, alpha, beta, y, ldy,
-                                           (const int32_t *)p->extra[0], ints, ints + nt, (V *)p->extra[2],
-                                           (V *)p->extra[3], vec, xvec, no_empty);
-    };
-    const bool plain = alpha == V(1) && beta == V(0);
-    if constexpr (sizeof(V) == 4 && K == 1) {
-        if (plain) go(csr_stream_kernel_occ6<V, K, true>);
-        else go(csr_stream_kernel_occ6<V, K>);
-    } else if constexpr (K == 1) {
-        if (plain) go(csr_stream_kernel<V, K, true>);
-        else go(csr_stream_kernel<V, K>);
-    } else {
-        go(csr_stream_kernel<V, K>);
-    }
-    SSPMV_LAUNCH_CHECK();
-    if (nt > 1) {
-        csr_stream_fixup<V, K><<<grid_for(nt, 256), 256, 0, cu(s)>>>(nt, A->row_offset, ints, ints + nt,
-                                                                     (const V *)p->extra[2], (const V *)p->extra[3],
-                                                                     alpha, beta, y, ldy);
-        SSPMV_LAUNCH_CHECK();
-    }
-    return SSPMV_OK;
+    if (A->f.num_nnzs == 0 || !stream_takes_strides(ldx, ldy, sizeof(V)))
+        return launch_merge<V, K>(A, p, alpha, x, ldx, beta, y, ldy, s);
+    StreamView v;
+    SSPMV_TRY(csr_stream_view(A, &v, s));
+    return launch_stream_view<V, K>(v, p->stream, alpha, x, ldx, beta, y, ldy, s);
 }
 
-// ---------------------------------------------------- batched (serving) --
-// Index of the item owning global chunk gc: the last item whose chunk_begin
-// is <= gc (items of a group have increasing chunk_begin).
-__device__ __forceinline__ int batch_item_of(const BatchItem *__restrict__ items, int n, int64_t gc) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&items[mid].chunk_begin) <= gc) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// Persistent stream kernel over the chunks of every request of group g:
-// warp i of the grid takes global chunks i, i + warps, ...  A request is cut
-// into the chunks a lone sspmv_spmm_csr call uses (the matrix's own
-// row_start), and its carries go to per-batch slots, so its result does not
-// depend on the rest of the batch and equals the single-request call's.
-template <typename V, int K>
-__global__ void __launch_bounds__(kBlock) csr_batch_kernel(int g, const BatchHeader *__restrict__ hdr,
-                                                           const BatchItem *__restrict__ all_items,
-                                                           int32_t *__restrict__ carry_row,
-                                                           int32_t *__restrict__ has_end, V *__restrict__ carry_val,
-                                                           V *__restrict__ head_val) {
-    const int n = hdr->n_items[g];
-    const int64_t total = hdr->total_chunks[g];
-    const int64_t base = hdr->carry_base[g];
-    const BatchItem *items = all_items + hdr->item_begin[g];
-    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t gc = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; gc < total; gc += warps) {
-        const BatchItem *q = items + batch_item_of(items, n, gc);
-        stream_chunk<V, K>(q->m, q->nnz, q->row_offset, q->col_index, (const V *)q->values, (const V *)q->x, q->ldx,
-                           (V)q->alpha, (V)q->beta, (V *)q->y, q->ldy, q->row_start, gc - q->chunk_begin, base + gc,
-                           carry_row, has_end, carry_val, head_val, q->vec, q->xvec, 0, nullptr);
-    }
-}
-
-// The batched counterpart of csr_stream_fixup: one thread per global chunk.
-template <typename V, int K>
-__global__ void csr_batch_fixup(int g, const BatchHeader *__restrict__ hdr, const BatchItem *__restrict__ all_items,
-                                const int32_t *__restrict__ carry_row, const int32_t *__restrict__ has_end,
-                                const V *__restrict__ carry_val, const V *__restrict__ head_val) {
-    const int n = hdr->n_items[g];
-    const int64_t total = hdr->total_chunks[g];
-    const int64_t base = hdr->carry_base[g];
-    const BatchItem *items = all_items + hdr->item_begin[g];
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    // warp-uniform trip count: lane l takes global chunk w0 + l of each round
-    for (int64_t w0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; w0 < total; w0 += stride) {
-        const int64_t gc = w0 + lane;
-        const BatchItem *q = gc < total ? items + batch_item_of(items, n, gc) : items;
-        const int64_t t = gc - q->chunk_begin, nt = q->num_chunks;
-        const int64_t slot = base + gc;
-        const int r = gc < total && nt > 1 ? carry_row[slot] : -1;
-        const bool mine = r >= 0 && (int64_t)q->row_offset[r] >= t * kStreamChunk;
-        V tot[K];
-        const int64_t shift = slot - t;  // chunk u of this lane's item lives in slot u + shift
-        chain_sum<V, K>(mine, t, nt, shift, has_end, carry_val, head_val, tot);
-        if (mine) {
-            V *yp = (V *)q->y + (int64_t)r * q->ldy;
-            const V alpha = (V)q->alpha, beta = (V)q->beta;
-#pragma unroll
-            for (int c = 0; c < K; c++) yp[c] = axpby(alpha, tot[c], beta, yp + c);
-        }
-    }
-}
-
-// Resident CTAs per SM of csr_batch_kernel<V, K>.
-template <typename V, int K>
-int batch_blocks_per_sm() {
-    static int blocks = 0;
-    if (blocks == 0) {
-        int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, csr_batch_kernel<V, K>, kBlock, 0) != cudaSuccess ||
-            b < 1)
-            b = 1;
-        blocks = b;
-    }
-    return blocks;
-}
-
-template <typename V, int K>
-sspmv_status launch_batch_vk(int g, const BatchHeader *hdr, const BatchItem *items, void *carry, int64_t slots,
-                             sspmv_stream_t s) {
-    unsigned char *c = (unsigned char *)carry;
-    int32_t *carry_row = (int32_t *)c;
-    int32_t *has_end = (int32_t *)(c + (size_t)slots * 4);
-    V *carry_val = (V *)(c + (size_t)slots * 8);
-    V *head_val = (V *)(c + (size_t)slots * (8 + kMaxK * 8));
-    const unsigned grid = (unsigned)(num_sms() * batch_blocks_per_sm<V, K>());
-    csr_batch_kernel<V, K><<<grid, kBlock, 0, cu(s)>>>(g, hdr, items, carry_row, has_end, carry_val, head_val);
-    SSPMV_LAUNCH_CHECK();
-    csr_batch_fixup<V, K><<<(unsigned)num_sms() * 4, 256, 0, cu(s)>>>(g, hdr, items, carry_row, has_end, carry_val,
-                                                                        head_val);
-    SSPMV_LAUNCH_CHECK();
-    return SSPMV_OK;
-}
-
-// kernel_flag 0 (default): stream kernel (merge-path for matrices it does
-// not take; the request server's batched CSR work sums in the same order, so
+// kernel_flag 0 (default): stream kernel (merge-path for a matrix without
+// nonzeros; the request server's batched CSR work sums in the same order, so
 // a request's result does not depend on whether it was batched); 1: vector;
 // 2: merge-path; 3: row-block; 4: pipelined thread per row (3 and 4 fall
 // back to the default on matrices they do not take).
@@ -1611,47 +850,12 @@ sspmv_status ensure_merge_plan(Plan *p, int which, int64_t m, int64_t nnz, const
     return SSPMV_OK;
 }
 
-sspmv_status csr_stream_plan(const sspmv_csr *A, const int32_t **row_start, int64_t *num_chunks, int32_t *max_gap,
-                             sspmv_stream_t s) {
+sspmv_status csr_stream_view(const sspmv_csr *A, StreamView *view, sspmv_stream_t s) {
     Plan *p = get_plan(&A->f);
     if (!p) return fail(SSPMV_OUT_OF_MEMORY, "plan allocation failed");
-    SSPMV_TRY(ensure_stream_plan(A, p, s));
-    *row_start = (const int32_t *)p->extra[0];
-    *num_chunks = p->extra_i[0];
-    *max_gap = (int32_t)p->extra_i[1];
+    SSPMV_TRY(ensure_stream_plan(p->stream, A->f.num_rows, A->f.num_nnzs, A->row_offset, A->f.value_type, s));
+    *view = stream_view(p->stream, A->f.num_nnzs, A->col_index, A->values);
     return SSPMV_OK;
-}
-
-bool csr_stream_takes(int64_t num_nnzs, int32_t max_gap) { return num_nnzs > 0 && max_gap <= kStreamMaxGap; }
-
-unsigned csr_batch_grid(int g) {
-    int b = 1;
-    switch (g) {
-    case 0: b = batch_blocks_per_sm<float, 1>(); break;
-    case 1: b = batch_blocks_per_sm<float, 2>(); break;
-    case 2: b = batch_blocks_per_sm<float, 4>(); break;
-    case 3: b = batch_blocks_per_sm<float, 8>(); break;
-    case 4: b = batch_blocks_per_sm<double, 1>(); break;
-    case 5: b = batch_blocks_per_sm<double, 2>(); break;
-    case 6: b = batch_blocks_per_sm<double, 4>(); break;
-    default: b = batch_blocks_per_sm<double, 8>(); break;
-    }
-    return (unsigned)(num_sms() * b);
-}
-
-sspmv_status launch_csr_batch_group(int g, const BatchHeader *d_hdr, const BatchItem *d_items, void *carry,
-                                    int64_t carry_slots, sspmv_stream_t s) {
-    switch (g) {
-    case 0: return launch_batch_vk<float, 1>(g, d_hdr, d_items, carry, carry_slots, s);
-    case 1: return launch_batch_vk<float, 2>(g, d_hdr, d_items, carry, carry_slots, s);
-    case 2: return launch_batch_vk<float, 4>(g, d_hdr, d_items, carry, carry_slots, s);
-    case 3: return launch_batch_vk<float, 8>(g, d_hdr, d_items, carry, carry_slots, s);
-    case 4: return launch_batch_vk<double, 1>(g, d_hdr, d_items, carry, carry_slots, s);
-    case 5: return launch_batch_vk<double, 2>(g, d_hdr, d_items, carry, carry_slots, s);
-    case 6: return launch_batch_vk<double, 4>(g, d_hdr, d_items, carry, carry_slots, s);
-    case 7: return launch_batch_vk<double, 8>(g, d_hdr, d_items, carry, carry_slots, s);
-    }
-    return fail(SSPMV_INVALID_ARG, "batch group %d out of range", g);
 }
 
 }  // namespace sspmv
