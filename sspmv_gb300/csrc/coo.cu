@@ -6,19 +6,23 @@
 //
 // SpMV (LeSpMV_coo, src/spmv_coo.cpp:161-182).  The reference scales y by
 // beta, then scatters alpha*a*x with OpenMP atomics (and skips the scaling
-// when beta == 0, leaving stale y).  Here, for row-sorted COO, each warp takes
-// 256 consecutive nonzeros and reduces runs of equal rows with a segmented
-// shuffle scan (kernel_flag 0, default); kernel_flag 1 uses CTA tiles of 2048
-// nonzeros staged in shared memory with a block-wide segmented scan.  Rows
-// that cross chunk boundaries are finished by a second kernel in a fixed
-// order, and rows with no nonzeros (listed once, when the plan is built) get
-// y = beta*y.  No atomics: results are deterministic.  Unsorted COO
-// (row_sorted == 0) uses a scale pass plus an atomic scatter, like the
-// reference.
+// when beta == 0, leaving stale y).  Here row-sorted COO runs the stream
+// kernel (csr_stream.cu; kernel_flag 0, default): its plan holds the rows'
+// ends as one bit per nonzero, so the 4 bytes of a row index per nonzero are
+// read when the plan is built and not by the product.  Uniform 4M x 32 FP64
+// (134M nonzeros): 600 us with the row indices streamed by a kernel of its
+// own (loads of row, column and value per lane, segmented scan keyed by row),
+// 535 us now (power-law 1M FP32 88 -> 73 us).  kernel_flag 1 uses CTA tiles of 2048 nonzeros staged in shared
+// memory with a block-wide segmented scan; rows that cross tiles are finished
+// by a second kernel in a fixed order, and rows with no nonzeros (listed once,
+// when the plan is built) get y = beta*y.  No atomics: results are
+// deterministic.  Unsorted COO (row_sorted == 0) uses a scale pass plus an
+// atomic scatter, like the reference.
 #include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
+#include "csr_stream.cuh"
 #include "plan.cuh"
 #include "primitives.cuh"
 #include "spmv_common.cuh"
@@ -271,191 +275,6 @@ __global__ void __launch_bounds__(kBlock) coo_tile_kernel(
     }
 }
 
-// Warp kernel (default): a warp takes kWarpChunk = 256 consecutive nonzeros,
-// lane l the 8 consecutive ones at 8l (vector loads of rows, columns and
-// values; all 8 gathers of x issued before use for k <= 2).  Each lane sums
-// its nonzeros in order, writing every row that starts and ends inside its 8;
-// the open sum before its first row end (head) and after its last (tail) are
-// joined across lanes by one segmented shuffle scan keyed by "lane has a row
-// end".  The row that ends first in a lane gets head + the carried tail sum;
-// a row that began before the warp's chunk is left in head_val for the
-// fix-up, and the chunk's open last row in carry_val.  No shared memory, no
-// barriers, one shuffle scan per 256 nonzeros.
-constexpr int kCooPerLane = 8;
-constexpr int kWarpChunk = 32 * kCooPerLane;
-
-template <typename V>
-struct Vec2 {
-    using T = double2;
-};
-template <>
-struct Vec2<float> {
-    using T = float4;
-};
-
-// Loads this lane's 8 consecutive nonzeros (n_valid of them exist).
-template <typename V>
-__device__ __forceinline__ void coo_load8(const int32_t *__restrict__ ri, const int32_t *__restrict__ ci,
-                                          const V *__restrict__ cv, int64_t e0, int nv, bool vec, int (&r)[8],
-                                          int (&c)[8], V (&a)[8]) {
-    if (vec && nv == 8) {
-        const int4 r0 = __ldcs(reinterpret_cast<const int4 *>(ri + e0));
-        const int4 r1 = __ldcs(reinterpret_cast<const int4 *>(ri + e0 + 4));
-        const int4 c0 = __ldcs(reinterpret_cast<const int4 *>(ci + e0));
-        const int4 c1 = __ldcs(reinterpret_cast<const int4 *>(ci + e0 + 4));
-        r[0] = r0.x; r[1] = r0.y; r[2] = r0.z; r[3] = r0.w; r[4] = r1.x; r[5] = r1.y; r[6] = r1.z; r[7] = r1.w;
-        c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
-        if constexpr (sizeof(V) == 8) {
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const double2 v = __ldcs(reinterpret_cast<const double2 *>(cv + e0) + h);
-                a[2 * h] = v.x;
-                a[2 * h + 1] = v.y;
-            }
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const float4 v = __ldcs(reinterpret_cast<const float4 *>(cv + e0) + h);
-                a[4 * h] = v.x; a[4 * h + 1] = v.y; a[4 * h + 2] = v.z; a[4 * h + 3] = v.w;
-            }
-        }
-        return;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        r[u] = u < nv ? ld_stream(ri + e0 + u) : -1;
-        c[u] = u < nv ? ld_stream(ci + e0 + u) : 0;
-        a[u] = u < nv ? ld_stream(cv + e0 + u) : V(0);
-    }
-}
-
-// k = 1: four (FP64) or five (FP32) resident CTAs per SM, the best of 3-6
-// measured on uniform, power-law and banded rows.
-template <typename V, int K, bool PLAIN = false>
-__global__ void __launch_bounds__(kBlock, K == 1 ? (sizeof(V) == 4 ? 5 : 4) : 1) coo_warp_kernel(
-    int64_t nnz, const int32_t *__restrict__ ri, const int32_t *__restrict__ ci, const V *__restrict__ cv,
-    const V *__restrict__ x, int64_t ldx, V alpha, V beta, V *__restrict__ y, int64_t ldy,
-    int32_t *__restrict__ carry_row, int32_t *__restrict__ has_end, V *__restrict__ carry_val,
-    V *__restrict__ head_val, int vec, int xvec) {
-    constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    constexpr bool plain = PLAIN;  // alpha == 1 and beta == 0: y = sum
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t j0 = w * kWarpChunk;
-    if (j0 >= nnz) return;  // warp-uniform
-    const int64_t j1 = min(j0 + (int64_t)kWarpChunk, nnz);
-    const int64_t e0 = j0 + (int64_t)lane * kCooPerLane;
-    const int nv = (int)max((int64_t)0, min((int64_t)kCooPerLane, j1 - e0));
-    int r[8], c[8];
-    V a[8];
-    coo_load8<V>(ri, ci, cv, e0, nv, vec != 0, r, c, a);
-    const int first_row = __shfl_sync(kFull, r[0], 0);
-    const bool head_open = j0 > 0 && __ldg(ri + j0 - 1) == first_row;  // chunk starts inside a row
-    // row of the nonzero after this lane's last one
-    int next = __shfl_down_sync(kFull, r[0], 1);
-    if (nv > 0 && e0 + nv == j1) next = j1 < nnz ? __ldg(ri + j1) : -1;
-    V xv[K <= 2 ? 8 : 1][K];
-    if constexpr (K <= 2) {
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            if (u < nv) {
-                ld_xrow<V, K>(x, c[u], ldx, xvec != 0, xv[u]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < K; q++) xv[u][q] = V(0);
-            }
-        }
-    }
-    V seg[K], head[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) seg[q] = head[q] = V(0);
-    bool any_end = false;
-    int head_row = -1, last_row = -1;
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        if (u < nv) {
-            last_row = r[u];
-            if constexpr (K <= 2) {
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] += a[u] * xv[u][q];
-            } else {
-                V xr[K];
-                ld_xrow<V, K>(x, c[u], ldx, xvec != 0, xr);
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] += a[u] * xr[q];
-            }
-            const int rn = u + 1 < nv ? r[u + 1] : next;
-            if (rn != r[u]) {  // r[u] ends here
-                if (!any_end) {
-                    any_end = true;
-                    head_row = r[u];
-#pragma unroll
-                    for (int q = 0; q < K; q++) head[q] = seg[q];
-                } else {
-                    V *yp = y + (int64_t)r[u] * ldy;
-#pragma unroll
-                    for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, seg[q], beta, yp + q);
-                }
-#pragma unroll
-                for (int q = 0; q < K; q++) seg[q] = V(0);
-            }
-        }
-    }
-    // segmented inclusive scan of the open tails; a lane with a row end starts a segment
-    V S[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) S[q] = seg[q];
-    bool f = any_end;
-    const int span = unflagged_run(f);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        if (o > span) break;  // warp-uniform
-        V up[K];
-#pragma unroll
-        for (int q = 0; q < K; q++) up[q] = __shfl_up_sync(kFull, S[q], o);
-        const bool fu = __shfl_up_sync(kFull, f, o);
-        if (lane >= o) {
-            if (!f) {
-#pragma unroll
-                for (int q = 0; q < K; q++) S[q] += up[q];
-            }
-            f = f || fu;
-        }
-    }
-    V cin[K];  // tail sums carried into this lane's first row
-#pragma unroll
-    for (int q = 0; q < K; q++) {
-        cin[q] = __shfl_up_sync(kFull, S[q], 1);
-        if (lane == 0) cin[q] = V(0);
-    }
-    if (any_end) {
-        V tot[K];
-#pragma unroll
-        for (int q = 0; q < K; q++) tot[q] = head[q] + cin[q];
-        if (head_row == first_row && head_open) {
-            V *hp = head_val + w * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) hp[q] = tot[q];
-        } else {
-            V *yp = y + (int64_t)head_row * ldy;
-#pragma unroll
-            for (int q = 0; q < K; q++) yp[q] = row_out(plain, alpha, tot[q], beta, yp + q);
-        }
-    }
-    const bool chunk_end = __any_sync(kFull, any_end);
-    // the lane holding the chunk's last nonzero reports the open last row
-    if (nv > 0 && e0 + nv == j1) {
-        const bool open = next == last_row;
-        has_end[w] = chunk_end ? 1 : 0;
-        carry_row[w] = open ? last_row : -1;
-        if (open) {
-            V *cp = carry_val + w * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) cp[q] = S[q];
-        }
-    }
-}
-
 template <typename V, int K>
 __global__ void coo_fixup(int64_t ntiles, const int32_t *__restrict__ ri, int tile,
                           const int32_t *__restrict__ carry_row, const int32_t *__restrict__ has_end,
@@ -480,15 +299,36 @@ __global__ void coo_fixup(int64_t ntiles, const int32_t *__restrict__ ri, int ti
     }
 }
 
-struct CooPlan {
-    int64_t ntiles[2] = {0, 0};
-    int32_t *carry_row[2] = {nullptr, nullptr};
-    int32_t *has_end[2] = {nullptr, nullptr};
-    void *carry_val[2] = {nullptr, nullptr};
-    void *head_val[2] = {nullptr, nullptr};
-};
+// rp[i] = first nonzero whose row is i or more (rows ascending).
+__global__ void sorted_row_offsets(int64_t m, int64_t nnz, const int32_t *__restrict__ ri, int32_t *__restrict__ rp) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= m; i += (int64_t)gridDim.x * blockDim.x) {
+        int64_t lo = 0, hi = nnz;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (ri[mid] < i) lo = mid + 1;
+            else hi = mid;
+        }
+        rp[i] = (int32_t)lo;
+    }
+}
 
-// extra[0..]: carry buffers per tile size, extra[10] = absent-row list (extra[6..8]: warp chunks)
+// The stream kernel's plan, from row offsets made for it and freed again.
+sspmv_status ensure_coo_stream_plan(const sspmv_coo *A, Plan *p, sspmv_stream_t s) {
+    if (p->stream.window) return SSPMV_OK;
+    std::lock_guard<PlanMutex> g(plan_mutex());
+    if (p->stream.window) return SSPMV_OK;
+    const int64_t m = A->f.num_rows, nnz = A->f.num_nnzs;
+    int32_t *rp = nullptr;
+    SSPMV_TRY(dalloc(&rp, (size_t)m + 1, s));
+    sorted_row_offsets<<<grid_for(m + 1, 256, (int64_t)num_sms() * 32), 256, 0, cu(s)>>>(m, nnz, A->row_index, rp);
+    note_launch();
+    sspmv_status st = cudaGetLastError() == cudaSuccess ? SSPMV_OK : fail(SSPMV_CUDA_ERROR, "coo row offsets");
+    if (st == SSPMV_OK) st = ensure_stream_plan(p->stream, m, nnz, rp, A->f.value_type, s);
+    dfree(rp, s);
+    return st;
+}
+
+// Tile kernel: extra[0..]: carry buffers per tile size, extra[10] = absent-row list
 sspmv_status ensure_coo_plan(const sspmv_coo *A, Plan *p, int which, int tile, sspmv_stream_t s) {
     if (p->extra[which * 3]) return SSPMV_OK;
     std::lock_guard<PlanMutex> g(plan_mutex());
@@ -547,9 +387,13 @@ sspmv_status coo_pass(const sspmv_coo *A, Plan *p, V alpha, const V *x, int64_t 
         }
         return SSPMV_OK;
     }
-    const bool warp_kernel = A->f.kernel_flag != 1;
-    const int tile = warp_kernel ? kWarpChunk : CooShape<K>::tile;
-    const int which = warp_kernel ? 2 : (K <= 4 ? 0 : 1);
+    if (A->f.kernel_flag != 1 && nnz > 0 && stream_takes_strides(ldx, ldy, sizeof(V))) {
+        SSPMV_TRY(ensure_coo_stream_plan(A, p, s));
+        return launch_stream_view<V, K>(stream_view(p->stream, nnz, A->col_index, A->values), p->stream, alpha, x, ldx,
+                                        beta, y, ldy, s);
+    }
+    const int tile = CooShape<K>::tile;
+    const int which = K <= 4 ? 0 : 1;
     SSPMV_TRY(ensure_coo_plan(A, p, which, tile, s));
     const int64_t nt = p->extra_i[which * 3];
     int32_t *ints = (int32_t *)p->extra[which * 3];
@@ -560,26 +404,6 @@ sspmv_status coo_pass(const sspmv_coo *A, Plan *p, V alpha, const V *x, int64_t 
         SSPMV_LAUNCH_CHECK();
     }
     if (nnz == 0) return SSPMV_OK;
-    if (warp_kernel) {
-        const int vec = ((reinterpret_cast<uintptr_t>(A->row_index) | reinterpret_cast<uintptr_t>(A->col_index) |
-                          reinterpret_cast<uintptr_t>(A->values)) & 15) == 0;
-        auto go = [&](auto kernel) {
-            kernel<<<grid_for(nt * 32, kBlock), kBlock, 0, cu(s)>>>(
-                nnz, A->row_index, A->col_index, (const V *)A->values, x, ldx, alpha, beta, y, ldy, ints, ints + nt,
-                (V *)p->extra[which * 3 + 1], (V *)p->extra[which * 3 + 2], vec, xrow_vec(x, ldx, sizeof(V), K));
-        };
-        if (K == 1 && alpha == V(1) && beta == V(0)) go(coo_warp_kernel<V, K, K == 1>);
-        else go(coo_warp_kernel<V, K>);
-        SSPMV_LAUNCH_CHECK();
-        if (nt > 1) {
-            coo_fixup<V, K><<<grid_for(nt, 256), 256, 0, cu(s)>>>(nt, A->row_index, tile, ints, ints + nt,
-                                                                  (const V *)p->extra[which * 3 + 1],
-                                                                  (const V *)p->extra[which * 3 + 2], alpha, beta, y,
-                                                                  ldy);
-            SSPMV_LAUNCH_CHECK();
-        }
-        return SSPMV_OK;
-    }
     const size_t smem = (size_t)tile * K * sizeof(V) + (size_t)tile * 4;
     static std::atomic<bool> attr{false};  // set after the attribute call returns
     if (!attr.load(std::memory_order_acquire)) {

@@ -1,5 +1,5 @@
 // csr_stream.cu -- the nonzero-split stream kernel on sm_103a: CSR's default
-// SpMV / SpMM, the short tails of the sliced formats and the request server's
+// SpMV / SpMM, row-sorted COO's, the short tails of the sliced formats and the request server's
 // batches.
 //
 // The nonzeros are cut into windows of T elements (window_size); a warp owns
