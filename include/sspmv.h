@@ -221,8 +221,8 @@ sspmv_status sspmv_release_plan(sspmv_features *f, sspmv_stream_t stream);
  * format's LeSpMV entry, param a kernel parameter (0 lets the library
  * choose): CSR vector kernel: lanes per row 1..32; CSR row-block kernel:
  * nonzeros per block window (512, 1024, 2048, 4096); S-ELL, SELL-c-sigma,
- * SELL-c-R: the slots a row's thread reads before the rest of the row moves
- * to the overflow CSR pass (default: a cost model over the row lengths).
+ * SELL-c-R: the longest row a thread multiplies on its own; longer rows run
+ * the CSR stream kernel (default: a cost model over the row lengths).
  * Used by the autotuner. */
 sspmv_status sspmv_set_kernel(sspmv_features *f, int32_t kernel_flag, int32_t param);
 
@@ -251,8 +251,7 @@ sspmv_status sspmv_delete_csr(sspmv_csr *A);
 
 /* ---------------- SpMV / SpMM ---------------- */
 /* LeSpMV_csr (src/spmv_csr.cpp:165-185).  kernel_flag 0 (default):
- * nonzero-split stream kernel (256 nonzeros per warp; matrices with runs of
- * more than 256 empty rows use merge-path); 2: nnz-balanced merge-path
+ * nonzero-split stream kernel; 2: nnz-balanced merge-path
  * kernel; 1: vector-per-row kernel (param: lanes per row, 1..32); 3: row-block
  * kernel for matrices whose rows all have at most 64 nonzeros (one CTA per
  * block of whole rows, param: nonzeros per block window, 512..4096; one
@@ -601,7 +600,7 @@ typedef enum { SSPMV_SERVE_BATCHED = 0, SSPMV_SERVE_PER_REQUEST = 1 } sspmv_serv
 typedef struct {
     int32_t mode;               /* sspmv_serve_mode */
     int32_t max_batch_requests; /* 0: 1024 */
-    int64_t max_batch_tiles;    /* 256-nonzero chunks (carry slots) per batch; 0: 1 << 20 */
+    int64_t max_batch_tiles;    /* 256-nonzero chunks per batch; 0: 1 << 20 */
     int64_t arena_bytes;        /* per batch in flight, device staging for X and for Y each; 0: 512 MiB */
     int64_t stage_limit_bytes;  /* X / Y up to this size are packed through pinned staging; 0: 1 MiB */
     int64_t hbm_budget_bytes;   /* resident matrices; 0: 120e9 */

@@ -59,10 +59,6 @@ void free_plan(sspmv_features *f, sspmv_stream_t s) {
         dfree(mp.carry_val, s);
         dfree(mp.head_val, s);
     }
-    if (p->sub) {
-        free_plan(&p->sub->f, s);
-        delete p->sub;
-    }
     free_stream_plan(p->stream, s);
     for (void *e : p->extra) dfree(e, s);
     delete p;

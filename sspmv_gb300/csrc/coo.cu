@@ -323,7 +323,7 @@ sspmv_status ensure_coo_stream_plan(const sspmv_coo *A, Plan *p, sspmv_stream_t 
     sorted_row_offsets<<<grid_for(m + 1, 256, (int64_t)num_sms() * 32), 256, 0, cu(s)>>>(m, nnz, A->row_index, rp);
     note_launch();
     sspmv_status st = cudaGetLastError() == cudaSuccess ? SSPMV_OK : fail(SSPMV_CUDA_ERROR, "coo row offsets");
-    if (st == SSPMV_OK) st = ensure_stream_plan(p->stream, m, nnz, rp, A->f.value_type, s);
+    if (st == SSPMV_OK) st = ensure_stream_plan(p->stream, m, nnz, rp, nullptr, A->f.value_type, s);
     dfree(rp, s);
     return st;
 }

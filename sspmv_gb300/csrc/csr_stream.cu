@@ -1,5 +1,5 @@
 // csr_stream.cu -- the nonzero-split stream kernel on sm_103a: CSR's default
-// SpMV / SpMM, row-sorted COO's, the short tails of the sliced formats and the request server's
+// SpMV / SpMM, row-sorted COO's, the long rows of the sliced formats and the request server's
 // batches.
 //
 // The nonzeros are cut into windows of T elements (window_size); a warp owns
@@ -588,13 +588,13 @@ void free_stream_plan(StreamPlan &sp, sspmv_stream_t s) {
     dfree(sp.ends, s);
     dfree(sp.tail_val, s);
     dfree(sp.head_val, s);
-    dfree(sp.nzrow, s);
+    if (sp.owns_nzrow) dfree(sp.nzrow, s);
     dfree(sp.empty, s);
     sp = StreamPlan();
 }
 
-sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset, int32_t value_type,
-                                sspmv_stream_t s) {
+sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
+                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s) {
     if (sp.window) return SSPMV_OK;
     std::lock_guard<PlanMutex> g(plan_mutex());
     if (sp.window) return SSPMV_OK;
@@ -612,6 +612,7 @@ sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const in
         SSPMV_LAUNCH_CHECK();
         SSPMV_CUDA_TRY(cudaMemcpyAsync(h, count, sizeof(h), cudaMemcpyDeviceToHost, cu(s)));
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
+        q.nzrow = const_cast<int32_t *>(row_map);
         if (h[0] > 0) {
             q.nempty = (int64_t)h[0];
             SSPMV_TRY(dalloc(&pos, (size_t)m, s));
@@ -619,6 +620,7 @@ sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const in
             SSPMV_LAUNCH_CHECK();
             SSPMV_TRY(exclusive_scan_i32(pos, pos, m, nullptr, s));
             SSPMV_TRY(dalloc(&q.nzrow, (size_t)(m - q.nempty), s));
+            q.owns_nzrow = true;
             SSPMV_TRY(dalloc(&q.empty, (size_t)q.nempty, s));
             stream_row_lists<<<grid, 256, 0, cu(s)>>>(m, row_offset, pos, q.nzrow, q.empty);
             SSPMV_LAUNCH_CHECK();

@@ -1,6 +1,6 @@
 // csr_stream.cuh -- the nonzero-split stream kernel (csr_stream.cu): device
 // view of a row-ordered run of nonzeros, its plan and its launchers.  Used by
-// CSR (default kernel), the short tails of the sliced formats and the request
+// CSR (default kernel), the long rows of the sliced formats and the request
 // server's batches.
 #pragma once
 
@@ -29,8 +29,9 @@ struct StreamView {
 
 // Builds (once) the stream plan of m rows given by row_offset (m + 1
 // entries, nnz > 0); row_offset is not read after the call's work on `s`.
-sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset, int32_t value_type,
-                                sspmv_stream_t s);
+// row_map: y row of each row (rows then all nonempty; null: the row itself), owned by the caller and kept as long as the plan.
+sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
+                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s);
 void free_stream_plan(StreamPlan &sp, sspmv_stream_t s);
 StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, const void *val);
 

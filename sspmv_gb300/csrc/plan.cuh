@@ -38,6 +38,7 @@ struct StreamPlan {
     void *tail_val = nullptr;  // [windows * kMaxK] piece of the split row that goes on past the window
     void *head_val = nullptr;  // [windows * kMaxK] last piece of the split row that ends in the window
     int32_t *nzrow = nullptr;  // y row of the i-th nonempty row (null: i itself)
+    bool owns_nzrow = false;
     int32_t *empty = nullptr;  // rows without nonzeros
     int64_t nempty = 0;
 };
@@ -49,12 +50,11 @@ struct Plan {
     int param = 0;          // kernel parameter set by sspmv_set_kernel (0 = library choice)
     void *extra[12] = {nullptr};  // format-specific device buffers
     int64_t extra_i[12] = {0};
-    sspmv_csr *sub = nullptr;     // a library-made CSR view over extra buffers (its own plan freed with this one)
 };
 
 // Guards plan creation.  Recursive: building one plan may build another
-// (a sliced matrix's overflow CSR gets its stream plan while its own plan is
-// being built).
+// (a sliced matrix's overflow rows get their stream plan while the matrix's
+// own plan is being built).
 using PlanMutex = std::recursive_mutex;
 PlanMutex &plan_mutex();
 Plan *get_plan(const sspmv_features *f);  // creates an empty plan if needed

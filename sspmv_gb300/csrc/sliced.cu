@@ -19,12 +19,13 @@
 // slice*(maxlen+1) + (maxlen - len) over rows fed in descending row order.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
+#include "csr_stream.cuh"
 #include "plan.cuh"
 #include "primitives.cuh"
-#include "serve.cuh"
 #include "spmv_common.cuh"
 
 namespace sspmv {
@@ -41,155 +42,89 @@ constexpr int kBlock = 256;
 // ------------------------------------------------------------------ SpMV --
 // A thread per stored row reads its slots (C consecutive rows read together)
 // up to its first padding slot, so a warp runs as long as its longest row.
-// Where a few long rows would keep most lanes of their warps idle, the
-// thread pass stops at a cap (chosen once per matrix by choose_cap): the rest
-// of each longer row (its "overflow") is copied once into compact arrays.
-// Short tails form a CSR matrix multiplied by the CSR stream kernel (every
-// lane busy whatever the row lengths); long tails are cut into pieces of one
-// row, a warp each; a fix-up adds each overflow row's thread partial and the
-// rest.  The compact copy also skips the padding of the short rows that
-// share a long row's chunk (slot-major storage puts them in the same sectors).
-constexpr int kSlots = 4;  // slots of a row whose loads are in flight together
+// Where a few long rows would keep most lanes of their warps idle, rows longer
+// than a cap (chosen once per matrix by choose_cap) are left out: they are
+// copied once into compact arrays, whole, and multiplied by the stream kernel
+// (csr_stream.cu), every lane busy whatever the row lengths, which writes
+// their y through the plan's row list.  The compact copy also skips the
+// padding of the short rows that share a long row's chunk (slot-major storage
+// puts them in the same sectors).  Moving only the part of a row past the cap
+// (the thread's partial sum, a CSR pass over short tails, a warp per 2048
+// elements of long ones and a pass that adds the three) took five launches one
+// after another: SELL-c-sigma (4096, 32) on power-law 1M FP64 146 us, two
+// launches now 102.
 
-template <typename V, int K, bool PLAIN = false>
-__global__ void __launch_bounds__(kBlock) sliced_spmv_kernel(
+// S: slots of a row whose loads are in flight together (column and value
+// loads of S slots, then their x gathers, then the FMAs in slot order).
+// FLAT (ELL of up to 12 slots in FP32): a row's slots loaded unconditionally
+// (a slot past the width reads the last one again, padding gathers x[0]) with
+// registers for all of them: two memory latencies per row instead of two per
+// four slots -- banded 1M FP32 27 -> 21 us, 5-point Laplacian 1M 18.4 -> 15 us.
+// With a test around each load the compiler holds a thread to 32 registers
+// and orders a load after another's use; in FP64, whose pipe is the bound,
+// that form at full occupancy is the faster one (banded 2M 56 us against 63
+// FLAT).
+template <typename V, int K, int S, bool FLAT>
+constexpr int sliced_min_ctas() {
+    if (K > 1) return K * sizeof(V) <= 16 ? 6 : 4;
+    return !FLAT ? 8 : S > 10 ? 4 : S > 8 ? 5 : S > 6 ? 6 : 7;
+}
+
+template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false>
+__global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sliced_spmv_kernel(
     int m, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
     const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
-    V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap, const int32_t *__restrict__ ovf_id,
-    V *__restrict__ ovf_part) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = div_nonneg(i, C);
-        const int r = (int)(i - c * C);
-        const int64_t base = ld_stream(chunk_ptr + c);
-        const int64_t wfull = div_nonneg(ld_stream(chunk_ptr + c + 1) - base, C);
-        const int64_t w = min(wfull, cap);
-        const int32_t *cp = col + base + r;
-        const V *vp = val + base + r;
-        V s[K];
+    V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const int64_t c = div_nonneg(i, C);
+    const int r = (int)(i - c * C);
+    const int64_t base = ld_stream(chunk_ptr + c);
+    const int64_t w = div_nonneg(ld_stream(chunk_ptr + c + 1) - base, C);
+    const int32_t *cp = col + base + r;
+    const V *vp = val + base + r;
+    if (w > cap && ld_stream(cp + cap * C) >= 0) return;  // longer than the cap: the stream kernel's row
+    V s[K];
 #pragma unroll
-        for (int q = 0; q < K; q++) s[q] = V(0);
-        int64_t k = 0;
-        for (; k + kSlots <= w; k += kSlots) {
-            int cc[kSlots];
-            V aa[kSlots];
+    for (int q = 0; q < K; q++) s[q] = V(0);
+    for (int64_t k = 0; k < w; k += S) {
+        int cc[S];
+        V aa[S];
 #pragma unroll
-            for (int u = 0; u < kSlots; u++) {
-                cc[u] = ld_stream(cp + (k + u) * C);
-                aa[u] = ld_stream(vp + (k + u) * C);
+        for (int u = 0; u < S; u++) {
+            cc[u] = -1;
+            aa[u] = V(0);
+            if (FLAT || k + u < w) {
+                const int64_t at = (FLAT ? min(k + u, w - 1) : k + u) * C;
+                cc[u] = ld_stream(cp + at);
+                aa[u] = ld_stream(vp + at);
             }
+            if (FLAT && k + u >= w) cc[u] = -1;
+        }
+        if constexpr (K == 1) {
+            V xv[S];
 #pragma unroll
-            for (int u = 0; u < kSlots; u++)
+            for (int u = 0; u < S; u++)
+                xv[u] = FLAT ? ld_x(x + (int64_t)max(cc[u], 0) * ldx) : cc[u] >= 0 ? ld_x(x + (int64_t)cc[u] * ldx) : V(0);
+#pragma unroll
+            for (int u = 0; u < S; u++)
+                if (cc[u] >= 0) s[0] += aa[u] * xv[u];  // never 0 * x[0]: x may hold Inf or NaN
+        } else {
+#pragma unroll
+            for (int u = 0; u < S; u++)
                 if (cc[u] >= 0) {
                     V xr[K];
                     ld_xrow<V, K>(x, cc[u], ldx, xvec, xr);
 #pragma unroll
                     for (int q = 0; q < K; q++) s[q] += aa[u] * xr[q];
                 }
-            if (cc[kSlots - 1] < 0) break;  // padding is a suffix of the row
         }
-        if (k + kSlots > w) {
-            for (; k < w; k++) {
-                const int cc = ld_stream(cp + k * C);
-                if (cc < 0) break;
-                const V aa = ld_stream(vp + k * C);
-                V xr[K];
-                ld_xrow<V, K>(x, cc, ldx, xvec, xr);
-#pragma unroll
-                for (int q = 0; q < K; q++) s[q] += aa * xr[q];
-            }
-        }
-        if (wfull > w && ld_stream(cp + w * C) >= 0) {  // the row goes on past the cap: overflow
-            V *op = ovf_part + (int64_t)ovf_id[i] * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) op[q] = s[q];
-            continue;
-        }
-        const int64_t row = reorder ? (int64_t)ld_stream(reorder + i) : i;
-        V *yp = y + row * ldy;
-#pragma unroll
-        for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, s[q], beta, yp + q);
+        if (cc[S - 1] < 0) break;  // padding is a suffix of the row
     }
-}
-
-// Long tails (kPieceMin nonzeros or more; 64 measured best against 256, 1024
-// and 4096) are cut into pieces of at most kPieceElems nonzeros of one row, a
-// warp per piece, lanes on consecutive elements; piece = {overflow row, first
-// element, end element} of the compact arrays.
-constexpr int64_t kPieceMin = 64;
-constexpr int64_t kPieceElems = 2048;
-
-template <typename V, int K>
-__global__ void __launch_bounds__(kBlock) sliced_piece_kernel(int64_t npieces, const int4 *__restrict__ pieces,
-                                                              const int32_t *__restrict__ ocol,
-                                                              const V *__restrict__ oval, const V *__restrict__ x,
-                                                              int64_t ldx, int xvec, V *__restrict__ partial) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (warp >= npieces) return;
-    const int4 pc = pieces[warp];
-    V s[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) s[q] = V(0);
-    int64_t e = (int64_t)pc.y + lane;
-    for (; e + 96 < pc.z; e += 128) {
-        int cc[4];
-        V aa[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            cc[u] = ld_stream(ocol + e + 32 * u);
-            aa[u] = ld_stream(oval + e + 32 * u);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            V xr[K];
-            ld_xrow<V, K>(x, cc[u], ldx, xvec, xr);
-#pragma unroll
-            for (int q = 0; q < K; q++) s[q] += aa[u] * xr[q];
-        }
-    }
-    for (; e < pc.z; e += 32) {
-        const int cc = ld_stream(ocol + e);
-        const V aa = ld_stream(oval + e);
-        V xr[K];
-        ld_xrow<V, K>(x, cc, ldx, xvec, xr);
-#pragma unroll
-        for (int q = 0; q < K; q++) s[q] += aa * xr[q];
-    }
-#pragma unroll
-    for (int q = 0; q < K; q++) s[q] = warp_sum(s[q]);
-    if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < K; q++) partial[warp * kMaxK + q] = s[q];
-    }
-}
-
-// One thread per overflow row o: its thread partial plus the rest of the row
-// -- the overflow CSR result y_ovf[o] (alpha = 1, beta = 0) for the first
-// nshort rows (short tails), the row's pieces in order for the others.
-template <typename V, int K>
-__global__ void sliced_overflow_fixup(int64_t nov, int64_t nshort, const int32_t *__restrict__ ovf_rows,
-                                      const int32_t *__restrict__ reorder, const V *__restrict__ ovf_part,
-                                      const V *__restrict__ y_ovf, const int32_t *__restrict__ piece_begin,
-                                      const V *__restrict__ partial, V alpha, V beta, V *__restrict__ y,
-                                      int64_t ldy) {
-    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nov) return;
-    V sum[K];
-#pragma unroll
-    for (int q = 0; q < K; q++) sum[q] = ovf_part[o * kMaxK + q];
-    if (o < nshort) {
-#pragma unroll
-        for (int q = 0; q < K; q++) sum[q] += y_ovf[o * kMaxK + q];
-    } else {
-        for (int32_t pc = piece_begin[o - nshort]; pc < piece_begin[o - nshort + 1]; pc++)
-#pragma unroll
-            for (int q = 0; q < K; q++) sum[q] += partial[(int64_t)pc * kMaxK + q];
-    }
-    const int64_t i = ovf_rows[o];
-    const int64_t row = reorder ? (int64_t)reorder[i] : i;
+    const int64_t row = reorder ? (int64_t)ld_stream(reorder + i) : i;
     V *yp = y + row * ldy;
 #pragma unroll
-    for (int q = 0; q < K; q++) yp[q] = axpby(alpha, sum[q], beta, yp + q);
+    for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, s[q], beta, yp + q);
 }
 
 // Plan building: stored length of every stored row (padding is a suffix:
@@ -211,30 +146,127 @@ __global__ void stored_row_lengths(int64_t m, int C, const int64_t *__restrict__
     }
 }
 
-// Overflow ids of the stored rows: ovf_id[rows[o]] = o.
-__global__ void set_overflow_ids(int64_t nov, const int32_t *__restrict__ rows, int32_t *__restrict__ ovf_id) {
-    const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (o < nov) ovf_id[rows[o]] = (int32_t)o;
+constexpr int kNumCaps = 12;  // the last: no cap
+struct CapList {
+    int64_t cap[kNumCaps];
+};
+constexpr int64_t kNoCap = INT64_MAX;
+
+// What the cost model needs of one cap: warp steps and longest row of the
+// thread pass without the rows past the cap, those rows and their nonzeros.
+struct CapStats {
+    unsigned long long slots, longest, rows, nnz;
+};
+
+// A warp per 32 stored rows (the rows a warp of the thread pass runs).
+__global__ void __launch_bounds__(kBlock) cap_stats(int64_t m, const int32_t *__restrict__ len, const CapList caps,
+                                                    CapStats *__restrict__ out) {
+    __shared__ CapStats s_out[kNumCaps];
+    const int lane = threadIdx.x & 31;
+    for (int t = threadIdx.x; t < kNumCaps; t += kBlock) s_out[t] = CapStats{0, 0, 0, 0};
+    __syncthreads();
+    unsigned long long slots = 0, longest = 0, rows = 0, nnz = 0;  // lane q: of cap q
+    const int64_t warps = ((int64_t)gridDim.x * kBlock) >> 5;
+    for (int64_t b = (((int64_t)blockIdx.x * kBlock + threadIdx.x) >> 5) * 32; b < m; b += warps * 32) {
+        const int l = b + lane < m ? len[b + lane] : 0;
+        const int most = __reduce_max_sync(0xffffffffu, l);
+#pragma unroll
+        for (int q = 0; q < kNumCaps; q++) {
+            unsigned mx = (unsigned)most, over = 0, n = 0;
+            if ((int64_t)most > caps.cap[q]) {  // warp-uniform
+                const bool past = (int64_t)l > caps.cap[q];
+                mx = __reduce_max_sync(0xffffffffu, past ? 0u : (unsigned)l);
+                over = __popc(__ballot_sync(0xffffffffu, past));
+                n = __reduce_add_sync(0xffffffffu, past ? (unsigned)l : 0u);
+            }
+            if (lane == q) {
+                slots += mx;
+                longest = max(longest, (unsigned long long)mx);
+                rows += over;
+                nnz += n;
+            }
+        }
+    }
+    if (lane < kNumCaps) {
+        atomicAdd(&s_out[lane].slots, slots);
+        atomicMax(&s_out[lane].longest, longest);
+        atomicAdd(&s_out[lane].rows, rows);
+        atomicAdd(&s_out[lane].nnz, nnz);
+    }
+    __syncthreads();
+    if (threadIdx.x < kNumCaps) {
+        CapStats *o = out + threadIdx.x;
+        const CapStats v = s_out[threadIdx.x];
+        atomicAdd(&o->slots, v.slots);
+        atomicMax(&o->longest, v.longest);
+        atomicAdd(&o->rows, v.rows);
+        atomicAdd(&o->nnz, v.nnz);
+    }
 }
 
-// Copies slots cap.. of each overflow row into the compact CSR arrays (one
-// warp per row).
+// Rows past the cap: a flag each, and their length.
+__global__ void overflow_flags(int64_t m, int64_t cap, const int32_t *__restrict__ len, int32_t *__restrict__ flag,
+                               int32_t *__restrict__ over) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+        const bool past = (int64_t)len[i] > cap;
+        flag[i] = past;
+        over[i] = past ? len[i] : 0;
+    }
+}
+
+// pos / off: the scans of flag and over.  Stored position, y row and first
+// compact element of every overflow row (optr[nov] = novf).
+__global__ void overflow_rows(int64_t m, int64_t cap, const int32_t *__restrict__ len, const int32_t *__restrict__ pos,
+                              const int32_t *__restrict__ off, const int32_t *__restrict__ reorder, int64_t nov,
+                              int32_t novf, int32_t *__restrict__ rows, int32_t *__restrict__ yrow,
+                              int32_t *__restrict__ optr) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
+        if (i == 0) optr[nov] = novf;
+        if ((int64_t)len[i] <= cap) continue;
+        const int32_t o = pos[i];
+        rows[o] = (int32_t)i;
+        yrow[o] = reorder ? reorder[i] : (int32_t)i;
+        optr[o] = off[i];
+    }
+}
+
+// Copies the overflow rows out of the slab: a block per kCopyTile consecutive
+// elements of the compact arrays (so that a row of 50k elements does not keep
+// one warp), each element's row by binary search among the block's rows.
+constexpr int kCopyTile = 2048;
+
 template <typename V>
-__global__ void copy_overflow(int64_t nov, int C, int64_t cap, const int32_t *__restrict__ ovf_rows,
-                              const int32_t *__restrict__ ovf_ptr, const int64_t *__restrict__ chunk_ptr,
-                              const int32_t *__restrict__ col, const V *__restrict__ val, int32_t *__restrict__ ocol,
-                              V *__restrict__ oval) {
-    const int lane = threadIdx.x & 31;
-    const int64_t o = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (o >= nov) return;
-    const int64_t i = ovf_rows[o];
-    const int64_t c = div_nonneg(i, C);
-    const int r = (int)(i - c * C);
-    const int64_t base = chunk_ptr[c] + cap * C + r;
-    const int64_t n = (int64_t)ovf_ptr[o + 1] - ovf_ptr[o], dst = ovf_ptr[o];
-    for (int64_t e = lane; e < n; e += 32) {
-        ocol[dst + e] = col[base + e * C];
-        oval[dst + e] = val[base + e * C];
+__global__ void __launch_bounds__(kBlock) copy_overflow(int64_t nov, int32_t novf, int C,
+                                                        const int32_t *__restrict__ rows,
+                                                        const int32_t *__restrict__ optr,
+                                                        const int64_t *__restrict__ chunk_ptr,
+                                                        const int32_t *__restrict__ col, const V *__restrict__ val,
+                                                        int32_t *__restrict__ ocol, V *__restrict__ oval) {
+    __shared__ int s_row[2];
+    const int64_t e0 = (int64_t)blockIdx.x * kCopyTile, e1 = min(e0 + (int64_t)kCopyTile, (int64_t)novf);
+    if (threadIdx.x < 2) {  // rows of the block's first and last element
+        const int64_t e = threadIdx.x ? e1 - 1 : e0;
+        int64_t lo = 0, hi = nov - 1;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi + 1) >> 1;
+            if (optr[mid] <= e) lo = mid;
+            else hi = mid - 1;
+        }
+        s_row[threadIdx.x] = (int)lo;
+    }
+    __syncthreads();
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += kBlock) {
+        int lo = s_row[0], hi = s_row[1];
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(optr + mid) <= e) lo = mid;
+            else hi = mid - 1;
+        }
+        const int64_t i = __ldg(rows + lo);
+        const int64_t c = div_nonneg(i, C);
+        const int64_t src = __ldg(chunk_ptr + c) + (e - __ldg(optr + lo)) * C + (i - c * C);
+        ocol[e] = col[src];
+        oval[e] = val[src];
     }
 }
 
@@ -245,198 +277,122 @@ struct SlicedView {
     const int32_t *reorder;
     const int32_t *col;
     const void *val;
-    int64_t nchunks;
-    int64_t n;  // columns
+    int64_t nchunks;  // 0: ELL
+    int32_t width;    // ELL
 };
 
 // Cost model of the cap, in picoseconds of GB300 time (fitted to measured
-// kernel times: the thread pass of S-ELL C=4 on a 4M-row power-law matrix,
-// the CSR stream kernel per nonzero on a 4M-row uniform matrix): the thread
-// pass costs kWarpSlotPs per warp and slot it runs (a warp runs as many slots
-// as its longest row, up to the cap), and no less than its longest thread:
-// kIterPs per 4 slots, each step a dependent chain of an HBM load and an x
-// gather (a 38k-slot row alone takes ~15 ms); the overflow costs kOvfNnzPs
-// per nonzero, kOvfRowPs per row (partial, CSR row, fix-up) and kOvfLaunchPs
-// for its extra launches.
+// times of power-law matrices of 0.1-4M rows at caps of 1 to 512).  A nonzero
+// costs kNnzPs in either kernel, its x gather; the thread pass no less than
+// kWarpSlotPs per warp and slot it runs (a warp runs as many slots as its
+// longest row within the cap), plus its longest thread's chain, kSlotChainPs
+// per slot (1M rows FP64, sigma = 4096: caps of 32, 128, 512 take 115, 171, 396
+// us); the overflow kOvfRowPs per row and kOvfLaunchPs for its launches.
 constexpr double kWarpSlotPs = 73.0;
-constexpr double kIterPs = 1.5e6;
-constexpr double kOvfNnzPs = 4.8;
+constexpr double kSlotChainPs = 0.5e6;
+constexpr double kNnzPs = 3.9;
 constexpr double kOvfRowPs = 20.0;
-constexpr double kOvfLaunchPs = 6.0e6;
-constexpr int64_t kCaps[] = {8, 12, 16, 24, 32, 48, 64, 96, 128, 256, 512};
-constexpr int64_t kNoCap = INT64_MAX;
+constexpr double kOvfLaunchPs = 4.0e6;
+constexpr CapList kCaps = {{8, 12, 16, 24, 32, 48, 64, 96, 128, 256, 512, kNoCap}};
 
-// The cap of least modelled time (kNoCap: no overflow), from the stored row
-// lengths (stored order: thread i runs stored row i, a warp 32 of them).
-int64_t choose_cap(const std::vector<int32_t> &len) {
-    const int64_t m = (int64_t)len.size();
-    constexpr int32_t H = 1024;  // exact histogram below H; longer rows listed
-    std::vector<int64_t> hist(H, 0);
-    std::vector<int32_t> longer, wmax((size_t)((m + 31) / 32), 0);
-    for (int64_t i = 0; i < m; i++) {
-        const int32_t l = len[(size_t)i];
-        int32_t &w = wmax[(size_t)(i >> 5)];
-        w = std::max(w, l);
-        if (l < H) hist[(size_t)l]++;
-        else longer.push_back(l);
-    }
-    double slots = 0;
-    int32_t longest = 0;
-    for (int32_t w : wmax) {
-        slots += w;
-        longest = std::max(longest, w);
-    }
-    auto thread_pass = [&](double warp_slots, int64_t slots_of_longest) {
-        return std::max(kWarpSlotPs * warp_slots, kIterPs * (double)((slots_of_longest + 3) / 4));
-    };
-    double best_cost = thread_pass(slots, longest);
-    int64_t best = kNoCap;
-    for (int64_t cap : kCaps) {
-        double thread = 0, ovn = 0, ovr = 0;
-        for (int32_t w : wmax) thread += (double)std::min<int64_t>(w, cap);
-        for (int64_t l = cap + 1; l < H; l++) {
-            ovn += (double)hist[(size_t)l] * (double)(l - cap);
-            ovr += (double)hist[(size_t)l];
-        }
-        for (int32_t l : longer)
-            if (l > cap) {
-                ovn += (double)(l - cap);
-                ovr += 1;
-            }
-        const double cost = thread_pass(thread, std::min<int64_t>(longest, cap)) + kOvfNnzPs * ovn +
-                            kOvfRowPs * ovr + (ovr > 0 ? kOvfLaunchPs : 0.0);
-        if (cost < best_cost) {
+// The candidate of least modelled time (ties: no cap, then the largest).
+int choose_cap(const CapStats (&st)[kNumCaps], int64_t total_nnz) {
+    int best = kNumCaps - 1;
+    double best_cost = 0;
+    for (int t = kNumCaps - 1; t >= 0; t--) {
+        const double thread = std::max(kWarpSlotPs * (double)st[t].slots,
+                                       kNnzPs * (double)(total_nnz - (int64_t)st[t].nnz)) +
+                              kSlotChainPs * (double)st[t].longest;
+        const double cost = thread + kNnzPs * (double)st[t].nnz + kOvfRowPs * (double)st[t].rows +
+                            (st[t].rows > 0 ? kOvfLaunchPs : 0.0);
+        if (t == kNumCaps - 1 || cost < best_cost) {
             best_cost = cost;
-            best = cap;
+            best = t;
         }
     }
     return best;
 }
 
 void free_overflow(Plan *p, sspmv_stream_t s) {
-    if (p->sub) {
-        free_plan(&p->sub->f, s);
-        delete p->sub;
-        p->sub = nullptr;
-    }
-    for (int e : {0, 1, 2, 3, 4, 5, 6, 7, 8, 9}) {
+    free_stream_plan(p->stream, s);
+    for (int e : {0, 1, 2}) {
         dfree(p->extra[e], s);
         p->extra[e] = nullptr;
     }
-    p->extra_i[1] = p->extra_i[4] = p->extra_i[5] = 0;
+    p->extra_i[1] = p->extra_i[4] = 0;
 }
 
 // Overflow plan of a sliced matrix, built on its first SpMV (and again after
-// sspmv_set_kernel changes the cap).  Overflow rows are ordered short tails
-// first, then long tails (kPieceMin nonzeros or more), their tails copied in
-// that order into the compact arrays.  extra[0] compact row offsets (nov+1;
-// its first nshort+1 entries are the short-tail CSR's row_offset), extra[1]
-// overflow rows (stored positions), extra[2] short-tail CSR result (nshort x
-// kMaxK), extra[3] pieces (int4), extra[4] thread partials of the overflow
-// rows, extra[5] / extra[6] compact columns / values, extra[7] piece partials,
-// extra[8] overflow id per stored row (-1: none), extra[9] first piece of each
-// long row (+1 entry); p->sub the short-tail CSR matrix (its stream plan built
-// here); extra_i[1] overflow rows, [2] the cap, [3] the kernel parameter the
-// plan was built for, [4] short-tail rows, [5] pieces, [7] built.
+// sspmv_set_kernel changes the cap).  extra[0] y row of every overflow row
+// (the stream plan's row list), extra[1] / extra[2] their columns / values;
+// p->stream the stream plan; extra_i[1] overflow rows, [2] the cap, [3] the
+// kernel parameter the plan was built for, [4] overflow nonzeros, [7] built.
 sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, Plan *p, sspmv_stream_t s) {
     if (p->extra_i[7] && p->extra_i[3] == p->param) return SSPMV_OK;
     std::lock_guard<PlanMutex> g(plan_mutex());
     if (p->extra_i[7] && p->extra_i[3] == p->param) return SSPMV_OK;
     p->extra_i[7] = 0;
     free_overflow(p, s);  // a plan for another cap, or one whose building failed
-    std::vector<int32_t> len((size_t)v.m);
-    {
-        int32_t *dlen = nullptr;
-        SSPMV_TRY(dalloc(&dlen, (size_t)v.m, s));
-        stored_row_lengths<<<grid_for(v.m, 256, (int64_t)num_sms() * 32), 256, 0, cu(s)>>>(v.m, v.C, v.chunk_ptr,
-                                                                                           v.col, dlen);
+    const int64_t m = v.m;
+    const unsigned grid = grid_for(m, 256, (int64_t)num_sms() * 32);
+    const size_t sv = vsize(f->value_type);
+    int32_t *len = nullptr, *pos = nullptr, *off = nullptr, *rows = nullptr, *optr = nullptr;
+    CapStats *dst = nullptr;
+    CapList caps = kCaps;
+    if (p->param > 0) caps.cap[0] = p->param;
+    int64_t nov = 0, novf = 0, cap = kNoCap;
+    auto build = [&]() -> sspmv_status {
+        SSPMV_TRY(dalloc(&len, (size_t)m, s));
+        SSPMV_TRY(dalloc(&dst, kNumCaps, s));
+        SSPMV_CUDA_TRY(cudaMemsetAsync(dst, 0, kNumCaps * sizeof(CapStats), cu(s)));
+        stored_row_lengths<<<grid, 256, 0, cu(s)>>>(m, v.C, v.chunk_ptr, v.col, len);
         SSPMV_LAUNCH_CHECK();
-        SSPMV_CUDA_TRY(cudaMemcpyAsync(len.data(), dlen, len.size() * 4, cudaMemcpyDeviceToHost, cu(s)));
+        cap_stats<<<grid_for(m, kBlock, (int64_t)num_sms() * 4), kBlock, 0, cu(s)>>>(m, len, caps, dst);
+        SSPMV_LAUNCH_CHECK();
+        CapStats st[kNumCaps];
+        SSPMV_CUDA_TRY(cudaMemcpyAsync(st, dst, sizeof(st), cudaMemcpyDeviceToHost, cu(s)));
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
-        dfree(dlen, s);
-    }
-    const int64_t cap = p->param > 0 ? (int64_t)p->param : choose_cap(len);
-    std::vector<int32_t> rows, long_rows;
-    int64_t total = 0;
-    for (int64_t i = 0; i < v.m; i++) {
-        const int64_t l = len[(size_t)i];
-        if (l <= cap) continue;
-        total += l - cap;
-        (l - cap >= kPieceMin ? long_rows : rows).push_back((int32_t)i);
-    }
-    if (total > 0x7fffffff) return fail(SSPMV_NOT_SUPPORTED, "overflow of the long rows exceeds the int32 range");
-    const int64_t nshort = (int64_t)rows.size();
-    rows.insert(rows.end(), long_rows.begin(), long_rows.end());
-    const int64_t nov = (int64_t)rows.size();
-    std::vector<int32_t> optr{0}, pbegin;
-    std::vector<int4> pieces;
-    for (int64_t o = 0; o < nov; o++) {
-        const int32_t o0 = optr.back(), n = len[(size_t)rows[(size_t)o]] - (int32_t)cap;
-        if (o >= nshort) {
-            pbegin.push_back((int32_t)pieces.size());
-            for (int64_t e = 0; e < n; e += kPieceElems)
-                pieces.push_back(make_int4((int)o, (int)(o0 + e), (int)(o0 + std::min<int64_t>(n, e + kPieceElems)), 0));
-        }
-        optr.push_back(o0 + n);
-    }
-    pbegin.push_back((int32_t)pieces.size());
-    const int64_t novf = optr.back(), npieces = (int64_t)pieces.size();
-    if (nov > 0) {
-        const size_t sv = vsize(f->value_type);
-        int32_t *dptr = nullptr, *drows = nullptr, *dov = nullptr, *ocol = nullptr, *dpb = nullptr;
-        int4 *dpieces = nullptr;
-        unsigned char *yov = nullptr, *opart = nullptr, *oval = nullptr, *ppart = nullptr;
-        // each buffer belongs to the plan as soon as it exists (free_overflow)
-        SSPMV_TRY(dalloc(&dptr, optr.size(), s));
-        p->extra[0] = dptr;
-        SSPMV_TRY(dalloc(&drows, rows.size(), s));
-        p->extra[1] = drows;
-        SSPMV_TRY(dalloc(&yov, (size_t)std::max<int64_t>(nshort, 1) * kMaxK * sv, s));
-        p->extra[2] = yov;
-        SSPMV_TRY(dalloc(&dpieces, pieces.size(), s));
-        p->extra[3] = dpieces;
-        SSPMV_TRY(dalloc(&opart, (size_t)nov * kMaxK * sv, s));
-        p->extra[4] = opart;
+        const int pick = p->param > 0 ? 0 : choose_cap(st, f->num_nnzs);
+        cap = caps.cap[pick];
+        nov = (int64_t)st[pick].rows;
+        novf = (int64_t)st[pick].nnz;
+        if (novf > 0x7fffffff) return fail(SSPMV_NOT_SUPPORTED, "overflow of the long rows exceeds the int32 range");
+        if (nov == 0) return SSPMV_OK;
+        int32_t *yrow = nullptr, *ocol = nullptr;
+        unsigned char *oval = nullptr;
+        SSPMV_TRY(dalloc(&pos, (size_t)m, s));
+        SSPMV_TRY(dalloc(&off, (size_t)m, s));
+        SSPMV_TRY(dalloc(&rows, (size_t)nov, s));
+        SSPMV_TRY(dalloc(&optr, (size_t)nov + 1, s));
+        // each kept buffer belongs to the plan as soon as it exists (free_overflow)
+        SSPMV_TRY(dalloc(&yrow, (size_t)nov, s));
+        p->extra[0] = yrow;
         SSPMV_TRY(dalloc(&ocol, (size_t)novf, s));
-        p->extra[5] = ocol;
+        p->extra[1] = ocol;
         SSPMV_TRY(dalloc(&oval, (size_t)novf * sv, s));
-        p->extra[6] = oval;
-        SSPMV_TRY(dalloc(&ppart, (size_t)std::max<int64_t>(npieces, 1) * kMaxK * sv, s));
-        p->extra[7] = ppart;
-        SSPMV_TRY(dalloc(&dov, (size_t)v.m, s));
-        p->extra[8] = dov;
-        SSPMV_TRY(dalloc(&dpb, pbegin.size(), s));
-        p->extra[9] = dpb;
-        SSPMV_CUDA_TRY(cudaMemcpyAsync(dptr, optr.data(), optr.size() * 4, cudaMemcpyHostToDevice, cu(s)));
-        SSPMV_CUDA_TRY(cudaMemcpyAsync(drows, rows.data(), rows.size() * 4, cudaMemcpyHostToDevice, cu(s)));
-        SSPMV_CUDA_TRY(cudaMemcpyAsync(dpb, pbegin.data(), pbegin.size() * 4, cudaMemcpyHostToDevice, cu(s)));
-        if (npieces > 0)
-            SSPMV_CUDA_TRY(cudaMemcpyAsync(dpieces, pieces.data(), pieces.size() * sizeof(int4),
-                                           cudaMemcpyHostToDevice, cu(s)));
-        SSPMV_CUDA_TRY(cudaMemsetAsync(dov, 0xff, (size_t)v.m * 4, cu(s)));
-        set_overflow_ids<<<grid_for(nov, 256), 256, 0, cu(s)>>>(nov, drows, dov);
+        p->extra[2] = oval;
+        overflow_flags<<<grid, 256, 0, cu(s)>>>(m, cap, len, pos, off);
+        SSPMV_LAUNCH_CHECK();
+        SSPMV_TRY(exclusive_scan_i32(pos, pos, m, nullptr, s));
+        SSPMV_TRY(exclusive_scan_i32(off, off, m, nullptr, s));
+        overflow_rows<<<grid, 256, 0, cu(s)>>>(m, cap, len, pos, off, v.reorder, nov, (int32_t)novf, rows, yrow, optr);
         SSPMV_LAUNCH_CHECK();
         SSPMV_TRY(dispatch_value(f->value_type, [&](auto tag) -> sspmv_status {
             using V = decltype(tag);
-            copy_overflow<V><<<grid_for(nov * 32, 256), 256, 0, cu(s)>>>(nov, v.C, cap, drows, dptr, v.chunk_ptr,
-                                                                         v.col, (const V *)v.val, ocol, (V *)oval);
+            copy_overflow<V><<<grid_for(novf, kCopyTile), kBlock, 0, cu(s)>>>(
+                nov, (int32_t)novf, v.C, rows, optr, v.chunk_ptr, v.col, (const V *)v.val, ocol, (V *)oval);
             SSPMV_LAUNCH_CHECK();
             return SSPMV_OK;
         }));
-        if (nshort > 0) {
-            p->sub = new (std::nothrow) sspmv_csr();
-            if (!p->sub) return fail(SSPMV_OUT_OF_MEMORY, "overflow matrix allocation failed");
-            SSPMV_TRY(sspmv_csr_wrap(p->sub, f->value_type, nshort, v.n, optr[(size_t)nshort], dptr, ocol, oval));
-            StreamView v2;
-            SSPMV_TRY(csr_stream_view(p->sub, &v2, s));  // built now, not inside a later SpMV
-        }
-        SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
-    }
+        return ensure_stream_plan(p->stream, nov, novf, optr, yrow, f->value_type, s);
+    };
+    const sspmv_status st = build();
+    for (void *t : {(void *)len, (void *)pos, (void *)off, (void *)rows, (void *)optr, (void *)dst}) dfree(t, s);
+    SSPMV_TRY(st);
     p->extra_i[1] = nov;
     p->extra_i[2] = nov > 0 ? cap : kNoCap;
     p->extra_i[3] = p->param;
-    p->extra_i[4] = nshort;
-    p->extra_i[5] = npieces;
+    p->extra_i[4] = novf;
     p->extra_i[7] = 1;
     return SSPMV_OK;
 }
@@ -444,32 +400,41 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
 template <typename V, int K>
 sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, int64_t ldx, V beta, V *y,
                            int64_t ldy, sspmv_stream_t s) {
-    const int64_t nov = p ? p->extra_i[1] : 0;
-    const unsigned grid = grid_for(v.m, kBlock, (int64_t)num_sms() * 16);
+    const int64_t nov = p && stream_takes_strides(ldx, ldy, sizeof(V)) ? p->extra_i[1] : 0;
+    if (nov > 0)  // the long rows first: the thread pass fills in behind them
+        SSPMV_TRY((launch_stream_view<V, K>(stream_view(p->stream, p->extra_i[4], (const int32_t *)p->extra[1],
+                                                        p->extra[2]),
+                                            p->stream, alpha, x, ldx, beta, y, ldy, s)));
+    // A thread per row and no grid stride: a fixed grid gave the same blocks the
+    // long rows at the head of every sigma slice (4M rows FP32, sigma = 4096:
+    // 580 us so, 328 with blocks scheduled as they finish).
+    const unsigned grid = grid_for(v.m, kBlock);
     const int xvec = xrow_vec(x, ldx, sizeof(V), K);
     auto go = [&](auto kernel) {
-        kernel<<<grid, kBlock, 0, cu(s)>>>(
-            (int)v.m, v.C, v.chunk_ptr, v.reorder, v.col, (const V *)v.val, x, ldx, xvec, alpha, beta, y, ldy,
-            nov > 0 ? p->extra_i[2] : kNoCap, nov > 0 ? (const int32_t *)p->extra[8] : nullptr,
-            nov > 0 ? (V *)p->extra[4] : nullptr);
+        kernel<<<grid, kBlock, 0, cu(s)>>>((int)v.m, v.C, v.chunk_ptr, v.reorder, v.col, (const V *)v.val, x, ldx,
+                                           xvec, alpha, beta, y, ldy, nov > 0 ? p->extra_i[2] : kNoCap);
     };
-    if (K == 1 && alpha == V(1) && beta == V(0)) go(sliced_spmv_kernel<V, K, K == 1>);  // y = sum
-    else go(sliced_spmv_kernel<V, K>);
-    SSPMV_LAUNCH_CHECK();
-    if (nov > 0) {
-        const int64_t nshort = p->extra_i[4], npieces = p->extra_i[5];
-        if (nshort > 0) SSPMV_TRY(sspmv_spmm_csr(1.0, p->sub, K, x, ldx, 0.0, p->extra[2], kMaxK, s));
-        if (npieces > 0) {
-            sliced_piece_kernel<V, K><<<grid_for(npieces * 32, kBlock), kBlock, 0, cu(s)>>>(
-                npieces, (const int4 *)p->extra[3], (const int32_t *)p->extra[5], (const V *)p->extra[6], x, ldx,
-                xvec, (V *)p->extra[7]);
-            SSPMV_LAUNCH_CHECK();
-        }
-        sliced_overflow_fixup<V, K><<<grid_for(nov, 256), 256, 0, cu(s)>>>(
-            nov, nshort, (const int32_t *)p->extra[1], v.reorder, (const V *)p->extra[4], (const V *)p->extra[2],
-            (const int32_t *)p->extra[9], (const V *)p->extra[7], alpha, beta, y, ldy);
-        SSPMV_LAUNCH_CHECK();
+    if constexpr (K == 1) {
+        const bool plain = alpha == V(1) && beta == V(0);  // y = sum
+        auto slots = [&](auto tag) {
+            constexpr int S = decltype(tag)::value;
+            constexpr bool flat = S > 4 && sizeof(V) == 4;  // only ELL takes S > 4
+            if (plain) go(sliced_spmv_kernel<V, K, S, true, flat>);
+            else go(sliced_spmv_kernel<V, K, S, false, flat>);
+        };
+        // ELL: all slots of a narrow row at once; wider rows and the chunked
+        // formats, whose rows differ in length, four at a time (six and eight
+        // were slower on power-law and uniform rows).
+        const int w = v.nchunks > 0 || v.width > 12 ? 4 : v.width;
+        if (w <= 4) slots(std::integral_constant<int, 4>());
+        else if (w <= 6) slots(std::integral_constant<int, 6>());
+        else if (w <= 8) slots(std::integral_constant<int, 8>());
+        else if (w <= 10) slots(std::integral_constant<int, 10>());
+        else slots(std::integral_constant<int, 12>());
+    } else {
+        go(sliced_spmv_kernel<V, K, 4>);
     }
+    SSPMV_LAUNCH_CHECK();
     return SSPMV_OK;
 }
 
@@ -792,7 +757,7 @@ extern "C" sspmv_status sspmv_spmm_ell(double alpha, const sspmv_ell *A, int32_t
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     Plan *p = get_plan(&A->f);
     SlicedView v{A->f.num_rows, (int32_t)std::max<int64_t>(A->f.num_rows, 1), (const int64_t *)p->extra[0], nullptr,
-                 A->col_index, A->values, 0, A->f.num_cols};
+                 A->col_index, A->values, 0, A->max_row_width};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -867,7 +832,7 @@ extern "C" sspmv_status sspmv_spmm_sell(double alpha, const sspmv_s_ell *A, int3
                                         double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->sliceWidth,   A->chunk_ptr,   nullptr,
-                 A->col_index,  A->values,     A->chunk_num,   A->f.num_cols};
+                 A->col_index,  A->values,     A->chunk_num, 0};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -941,7 +906,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_sigma(double alpha, const sspmv_sell_c
                                                 int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, A->f.num_cols};
+                 A->col_index,  A->values,         A->validchunkNum, 0};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1010,7 +975,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_R(double alpha, const sspmv_sell_c_R *
                                             int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, A->f.num_cols};
+                 A->col_index,  A->values,         A->validchunkNum, 0};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 

@@ -853,7 +853,7 @@ sspmv_status ensure_merge_plan(Plan *p, int which, int64_t m, int64_t nnz, const
 sspmv_status csr_stream_view(const sspmv_csr *A, StreamView *view, sspmv_stream_t s) {
     Plan *p = get_plan(&A->f);
     if (!p) return fail(SSPMV_OUT_OF_MEMORY, "plan allocation failed");
-    SSPMV_TRY(ensure_stream_plan(p->stream, A->f.num_rows, A->f.num_nnzs, A->row_offset, A->f.value_type, s));
+    SSPMV_TRY(ensure_stream_plan(p->stream, A->f.num_rows, A->f.num_nnzs, A->row_offset, nullptr, A->f.value_type, s));
     *view = stream_view(p->stream, A->f.num_nnzs, A->col_index, A->values);
     return SSPMV_OK;
 }
