@@ -3,6 +3,8 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstring>
+#include <cuda.h>
+#include <mutex>
 
 #include "common.cuh"
 #include "csr_stream.cuh"
@@ -18,9 +20,6 @@ void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 static thread_local int g_delete_nosync = 0;
 DeleteWithoutDeviceSync::DeleteWithoutDeviceSync() { g_delete_nosync++; }
 DeleteWithoutDeviceSync::~DeleteWithoutDeviceSync() { g_delete_nosync--; }
-void delete_barrier() {
-    if (g_delete_nosync == 0) cudaDeviceSynchronize();
-}
 
 void set_error(const char *fmt, ...) {
     va_list ap;
@@ -35,6 +34,108 @@ sspmv_status fail(sspmv_status s, const char *fmt, ...) {
     vsnprintf(g_last_error, sizeof(g_last_error), fmt, ap);
     va_end(ap);
     return s;
+}
+
+// Unique id of the calling thread's current CUDA context (0 if the driver
+// cannot tell), through the driver entry points the runtime hands out, so
+// no link against the driver library is needed.  A device reset
+// (cudaDeviceReset) ends the primary context and the next call gets a new
+// one with a new id: what is kept per context is then made again.
+unsigned long long current_context_id() {
+    using GetCurrent = CUresult (*)(CUcontext *);
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_current = reinterpret_cast<GetCurrent>(f);
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get_id = reinterpret_cast<GetId>(f);
+    });
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (get_current && get_id && get_current(&ctx) == CUDA_SUCCESS && ctx && get_id(ctx, &id) == CUDA_SUCCESS)
+        return id;
+    return 0;
+}
+
+namespace {
+constexpr int kMaxDevices = 64;
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long ctx = 0;
+};
+std::mutex g_pool_mutex;
+DevicePool g_pools[kMaxDevices];
+std::atomic<long long> g_live_blocks{0};
+
+// The current device's pool, made on first use (and again after a
+// cudaDeviceReset ended the context it belonged to).
+cudaError_t current_pool(cudaMemPool_t *out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    unsigned long long ctx = current_context_id();
+    if (ctx == 0 && (e = cudaSetDevice(dev)) == cudaSuccess) ctx = current_context_id();  // no context yet: made here
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> g(g_pool_mutex);
+    DevicePool &d = g_pools[dev];
+    if (!d.pool || d.ctx != ctx) {
+        cudaMemPoolProps props;
+        std::memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+        uint64_t keep = kPoolKeepBytes;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        d.pool = pool;
+        d.ctx = ctx;
+    }
+    *out = d.pool;
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = current_pool(&pool);
+    if (e != cudaSuccess) return e;
+    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    if (e == cudaErrorMemoryAllocation) {  // once more with nothing kept back
+        cudaGetLastError();
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    }
+    if (e == cudaSuccess) g_live_blocks.fetch_add(1, std::memory_order_relaxed);
+    return e;
+}
+
+void pool_free(void *p, cudaStream_t s) {
+    cudaFreeAsync(p, s);
+    g_live_blocks.fetch_sub(1, std::memory_order_relaxed);
+}
+
+DeleteScope::DeleteScope() {
+    if (g_delete_nosync == 0) cudaDeviceSynchronize();
+}
+DeleteScope::~DeleteScope() {
+    if (g_delete_nosync != 0 || g_live_blocks.load(std::memory_order_relaxed) != 0) return;
+    cudaMemPool_t pool = nullptr;
+    if (current_pool(&pool) != cudaSuccess) return;
+    cudaStreamSynchronize(nullptr);  // the frees just queued
+    cudaMemPoolTrimTo(pool, 0);
 }
 
 PlanMutex &plan_mutex() {
@@ -204,7 +305,7 @@ extern "C" sspmv_status sspmv_delete_csr(sspmv_csr *A) {
     if (!A) return SSPMV_OK;
     // The matrix may still be in use on any stream: wait for the device
     // before returning its memory.
-    delete_barrier();
+    const DeleteScope scope;
     free_plan(&A->f, nullptr);
     if (A->f.owns) {
         dfree(A->row_offset, nullptr);

@@ -589,7 +589,7 @@ extern "C" sspmv_status sspmv_coo_export(const sspmv_coo *A, int32_t *row_index,
 
 extern "C" sspmv_status sspmv_delete_coo(sspmv_coo *A) {
     if (!A) return SSPMV_OK;
-    delete_barrier();
+    const DeleteScope scope;
     free_plan(&A->f, nullptr);
     if (A->f.owns) {
         dfree(A->row_index, nullptr);

@@ -852,7 +852,7 @@ extern "C" sspmv_status sspmv_ell_export(const sspmv_ell *A, int32_t *col_index,
 
 extern "C" sspmv_status sspmv_delete_ell(sspmv_ell *A) {
     if (!A) return SSPMV_OK;
-    delete_barrier();
+    const DeleteScope scope;
     free_plan(&A->f, nullptr);
     if (A->f.owns) {
         dfree(A->col_index, nullptr);
@@ -914,7 +914,7 @@ extern "C" sspmv_status sspmv_sell_export(const sspmv_s_ell *A, int32_t *row_wid
 
 extern "C" sspmv_status sspmv_delete_sell(sspmv_s_ell *A) {
     if (!A) return SSPMV_OK;
-    delete_barrier();
+    const DeleteScope scope;
     free_plan(&A->f, nullptr);
     if (A->f.owns) {
         dfree(A->row_width, nullptr);
@@ -989,7 +989,7 @@ extern "C" sspmv_status sspmv_sell_c_sigma_export(const sspmv_sell_c_sigma *A, i
 
 extern "C" sspmv_status sspmv_delete_sell_c_sigma(sspmv_sell_c_sigma *A) {
     if (!A) return SSPMV_OK;
-    delete_barrier();
+    const DeleteScope scope;
     free_plan(&A->f, nullptr);
     if (A->f.owns) {
         dfree(A->reorder, nullptr);
@@ -1058,7 +1058,7 @@ extern "C" sspmv_status sspmv_sell_c_R_export(const sspmv_sell_c_R *A, int32_t *
 
 extern "C" sspmv_status sspmv_delete_sell_c_R(sspmv_sell_c_R *A) {
     if (!A) return SSPMV_OK;
-    delete_barrier();
+    const DeleteScope scope;
     free_plan(&A->f, nullptr);
     if (A->f.owns) {
         dfree(A->reorder, nullptr);

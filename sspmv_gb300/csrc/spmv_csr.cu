@@ -22,7 +22,6 @@
 // kernel_flag 1: vector-per-row kernel, `lanes` threads per row (2..32,
 // chosen from the mean row length, or set by the autotuner).
 #include <atomic>
-#include <cuda.h>
 #include <mutex>
 #include <type_traits>
 
@@ -922,34 +921,6 @@ constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mutex;
 void *g_noalloc_ptr[kNoAllocMaxDevices] = {nullptr};
 unsigned long long g_noalloc_ctx[kNoAllocMaxDevices] = {0};
-
-// Unique id of the calling thread's current CUDA context (0 if the driver
-// cannot tell), through the driver entry points the runtime hands out, so
-// no link against the driver library is needed.  A device reset
-// (cudaDeviceReset) ends the primary context and the next call gets a new
-// one with a new id: the array's address is then looked up again.
-unsigned long long current_context_id() {
-    using GetCurrent = CUresult (*)(CUcontext *);
-    using GetId = CUresult (*)(CUcontext, unsigned long long *);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void *f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_current = reinterpret_cast<GetCurrent>(f);
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            get_id = reinterpret_cast<GetId>(f);
-    });
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (get_current && get_id && get_current(&ctx) == CUDA_SUCCESS && ctx && get_id(ctx, &id) == CUDA_SUCCESS)
-        return id;
-    return 0;
-}
 
 // The scratch array's device address on the current device, looked up with
 // cudaGetSymbolAddress the first time this device (context) is seen.
