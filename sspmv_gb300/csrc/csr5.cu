@@ -16,20 +16,21 @@
 // tile_desc_offset slots the reference never writes are 0).
 //
 // SpMV (LeSpMV_csr5, src/spmv_csr5.cpp:439-457, which the reference builds for
-// double with AVX-512 only): one warp covers 32/omega tiles, a lane per tile
-// column.  Each lane sums its sigma products, closing a row segment at every
-// start bit; segments that run across lanes are joined with a segmented
-// shuffle scan keyed by segment number.  A tile's first and last rows can
-// cross tile boundaries: their pieces go to per-tile carries that a fix-up
-// kernel adds in tile order, so results are deterministic.  A row pass handles
-// the last tile (as CSR rows) and sets y = beta*y on empty rows.  Unlike the
-// reference, beta is applied to every row (the reference drops it on rows that
-// lie inside one tile, src/spmv_csr5.cpp:287-288).
+// double with AVX-512 only): a lane per tile column, 32 / omega tiles per step
+// of a warp, so that a warp's step is 32 sigma consecutive nonzeros, lane l
+// the sigma at l sigma (c5_window).  Row ends come from the stream kernel's
+// plan (csr_stream.cu: one bit per nonzero, a record per window), not from
+// the tile descriptors, and one segmented scan joins the lanes of all tiles of
+// a step; rows that cross a window are left in pieces and finished by the
+// split-row kernel in window order.  Deterministic.  Unlike the reference,
+// beta is applied to every row (the reference drops it on rows that lie inside
+// one tile, src/spmv_csr5.cpp:287-288).
 #include <algorithm>
 #include <cstring>
 #include <vector>
 
 #include "common.cuh"
+#include "csr_stream.cuh"
 #include "plan.cuh"
 #include "primitives.cuh"
 #include "spmv_common.cuh"
@@ -207,399 +208,244 @@ __global__ void c5_transpose(int64_t nnz, int32_t p, int32_t sigma, int32_t omeg
 }
 
 // ------------------------------------------------------------------ SpMV --
-struct C5View {
-    int32_t m, n, p, sigma, byo, bao, np;
-    int32_t xvec;  // X rows aligned for vector loads (xrow_vec), set per call
-    const int32_t *rp, *col;
-    const void *val;
-    const uint32_t *tp, *td;
-    const int32_t *tdo_ptr, *tdo;
+struct C5Shape {
+    int32_t sigma, omega, tiles;  // the last tile is stored in CSR order
 };
 
-template <int OMEGA>
-__device__ __forceinline__ uint32_t c5_bit(const uint32_t *d, int lane, int i, int bao, uint32_t d0) {
-    // bit for position i of this lane (packet 0 holds positions 0..31-bao)
-    const int glid = i + bao;
-    const uint32_t w = glid < 32 ? d0 : d[(glid / 32) * OMEGA + lane];
-    return (w >> (31 - glid % 32)) & 1u;
-}
-
-// SIG > 0: sigma known at compile time (16 or 32, descriptors of at most two
-// packets), so a lane's loop over its sigma nonzeros unrolls fully.
-template <typename V, int K, int OMEGA, int SIG, bool PLAIN = false>
-__global__ void __launch_bounds__(kBlock) csr5_tile_kernel(C5View A, const V *__restrict__ x, int64_t ldx, V alpha,
-                                                         V beta, V *__restrict__ y, int64_t ldy,
-                                                         int32_t *__restrict__ carry_row, int32_t *__restrict__ has_end,
-                                                         V *__restrict__ carry_val, V *__restrict__ head_val) {
-    constexpr int kGroups = 32 / OMEGA;
+// One window (rows that cross its ends are split), one warp.  A tile inside
+// one row is stored untransposed: its elements all belong to that row, so the
+// lanes add them up in the transposed order all the same.
+//
+// Bound like the stream kernel by the x gathers and the shuffles queued behind
+// them.  An earlier form read the tile pointer and descriptors before the
+// columns' addresses were known, scanned each tile on its own and left pieces
+// per tile, with a row pass for the last tile and a fix-up over all tiles:
+// power-law 1M FP64 (sigma 16, omega 8) 139 us, now 95.
+template <typename V, int K, int SIG, bool PLAIN>
+__device__ __forceinline__ void c5_window(const StreamView &A, const C5Shape g, const V *__restrict__ x, int64_t ldx,
+                                          int xvec, V alpha, V beta, V *__restrict__ y, int64_t ldy, const int64_t w,
+                                          V *__restrict__ tail_val, V *__restrict__ head_val) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr bool kSeed = sizeof(V) == 8;  // as the stream kernel
+    // nonzeros of a lane in flight together: for one FP64 right-hand side four
+    // with 18 CTAs per SM (uniform 3M x 32, sigma 32: 367 us; eight with 14: 388)
+    constexpr int kB = (K == 1 && sizeof(V) == 8) || K * sizeof(V) > 16 ? 4 : 8;
     const int lane = threadIdx.x & 31;
-    const int g = lane / OMEGA, xl = lane % OMEGA;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t t = warp * kGroups + g;
-    const bool active = t < (int64_t)A.p - 1;
-    const V *val = (const V *)A.val;
-    const int sigma = SIG > 0 ? SIG : A.sigma;
-    const int64_t tile = (int64_t)sigma * OMEGA;
-    const int64_t base = t * tile;
-
-    uint32_t tp0 = 0, tp1 = 0, d0 = 0;
-    int32_t yoff = 0;
-    if (active) {
-        tp0 = A.tp[t];
-        tp1 = A.tp[t + 1];
-        d0 = A.td[(size_t)t * OMEGA * A.np + xl];
-        yoff = (int32_t)(d0 >> (32 - A.byo));
-        if (xl == 0) yoff = 0;
-    }
-    const bool fast = tp0 == tp1;
-    const bool dirty = (tp0 >> 31) & 1u;
-    const int32_t row_start = (int32_t)(tp0 & 0x7FFFFFFFu);
-    const uint32_t *dl = A.td + (size_t)t * OMEGA * A.np;
-    const int32_t optr = (active && dirty) ? A.tdo_ptr[t] : 0;
-    // segment rel >= 1 of a tile with empty rows: tile_desc_offset holds its
-    // row counted from row_start + 1 (include/sparse_conversion.h:1290-1305)
-    auto map_row = [&](int32_t rel) -> int64_t {
-        if (rel == 0) return row_start;
-        return (int64_t)row_start + (dirty ? 1 + A.tdo[optr + rel - 1] : rel);
+    const int sigma = SIG > 0 ? SIG : g.sigma;
+    const V *val = static_cast<const V *>(A.val);
+    const int64_t tile = (int64_t)sigma * g.omega;
+    const int xl = lane & (g.omega - 1);
+    const int4 rec = __ldg(A.rec + w);
+    int row = rec.z;
+    bool head_split = rec.w & 1;
+    auto y_of = [&](int ordinal) {
+        return y + (int64_t)(A.nzrow ? __ldg(A.nzrow + ordinal) : ordinal) * ldy;
     };
-
-    V sum[K], head[K];
+    auto put = [&](int ordinal, const V(&sum)[K]) {
+        V *yp = y_of(ordinal);
 #pragma unroll
-    for (int q = 0; q < K; q++) sum[q] = head[q] = V(0);
-    bool seen = false;
-    int32_t rel = yoff;
-    // With at most two descriptor packets the lane's flags for positions
-    // 0..sigma-1 fit one 64-bit window: position i at bit 63 - i.
-    const bool window = SIG > 0 || A.np <= 2;
-    uint64_t bits = 0;
-    if (active && window)
-        bits = ((uint64_t)d0 << 32 | (A.np > 1 ? dl[OMEGA + xl] : 0u)) << A.bao;
-    auto bit_at = [&](int i) -> uint32_t {
-        if (window) return (uint32_t)(bits >> (63 - i)) & 1u;
-        return c5_bit<OMEGA>(dl, xl, i, A.bao, d0);
+        for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, sum[q], beta, yp + q);
     };
-    const uint32_t bit0 = active ? bit_at(0) : 0u;
-    if (active) {
-        // lane xl's i-th nonzero: p0 + i * step (tiles inside one row are
-        // stored untransposed)
-        const int64_t p0 = fast ? base + (int64_t)xl * sigma : base + xl;
-        const int64_t step = fast ? 1 : OMEGA;
-        // nonzeros whose loads (and x gathers) are in flight together: 8 for
-        // f32 at k = 1; 4 otherwise (deeper prefetch measured slower for f64)
-        constexpr int kU = (sizeof(V) == 4 && K == 1) ? 8 : 4;
+    V carry[K];  // the open row's sum over the earlier steps
 #pragma unroll
-        for (int i0 = 0; i0 < sigma; i0 += kU) {
-            int cc[kU];
-            V aa[kU], xv[kU][K];
+    for (int q = 0; q < K; q++) carry[q] = V(0);
+    bool later = false;
+    const int64_t wend = min((w + 1) * (int64_t)A.window, (int64_t)A.nnz);
+    for (int64_t b = w * (int64_t)A.window; b < wend; b += 32 * sigma) {  // warp-uniform
+        const int64_t e0 = b + (int64_t)lane * sigma;  // this lane's nonzeros e0 .. e0 + sigma - 1
+        const int64_t t = e0 / tile;
+        const bool csr_order = t == (int64_t)g.tiles - 1;
+        const int64_t p0 = csr_order ? e0 : t * tile + xl;
+        const int64_t step = csr_order ? 1 : g.omega;
+        const int nv = (int)max((int64_t)0, min((int64_t)sigma, (int64_t)A.nnz - e0));
+        // row ends of the lane, 8 at a time: bits e0 + i .. e0 + i + 7
+        auto ends8 = [&](int i) -> unsigned {
+            if (i >= nv) return 0u;
+            const int64_t e = e0 + i;
+            unsigned v = A.ends[e >> 3];
+            if (SIG == 0 && (e & 7)) v |= e + 8 - (e & 7) < (int64_t)A.nnz ? (unsigned)A.ends[(e >> 3) + 1] << 8 : 0u;
+            v >>= e & 7;
+            const int n = nv - i;
+            return v & (n >= 8 ? 0xffu : (1u << n) - 1u);
+        };
+        int mine = 0;
+        if constexpr (SIG > 0) {
 #pragma unroll
-            for (int u = 0; u < kU; u++) {
-                const int i = i0 + u;
-                cc[u] = 0;
-                aa[u] = V(0);
-                if (i < sigma) {
-                    const int64_t idx = p0 + (int64_t)i * step;
-                    cc[u] = ld_stream(A.col + idx);
-                    aa[u] = ld_stream(val + idx);
+            for (int i = 0; i < sigma; i += 8) mine += __popc(ends8(i));
+        } else {
+            for (int i = 0; i < sigma; i += 8) mine += __popc(ends8(i) & (sigma - i < 8 ? (1u << (sigma - i)) - 1u : 0xffu));
+        }
+        int pos = 0, nend = 0;  // rows ended in the lanes before this one, and in the step
+        const unsigned before = (1u << lane) - 1u;
+        for (int bit = 0; (1 << bit) <= sigma; bit++) {
+            const unsigned m = __ballot_sync(kFull, (mine >> bit) & 1);
+            pos += __popc(m & before) << bit;
+            nend += __popc(m) << bit;
+        }
+        const unsigned flags = __ballot_sync(kFull, mine != 0) & (before | (1u << lane));
+        const int dist = flags ? lane - (31 - __clz(flags)) : lane;
+
+        V sum[K], head[K];
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            sum[q] = kSeed && lane == 0 ? carry[q] : V(0);
+            head[q] = V(0);
+        }
+        bool first = true;
+        int idx = row + pos;
+#pragma unroll
+        for (int i = 0; i < sigma; i += kB) {
+            int c[kB];
+            V a[kB], xv[kB][K];
+#pragma unroll
+            for (int u = 0; u < kB; u++) {
+                c[u] = 0;
+                a[u] = V(0);
+                if (i + u < nv) {
+                    c[u] = ld_stream(A.col + p0 + (i + u) * step);
+                    a[u] = ld_stream(val + p0 + (i + u) * step);
                 }
             }
 #pragma unroll
-            for (int u = 0; u < kU; u++) {
-                if (i0 + u < sigma) {
-                    ld_xrow<V, K>(x, cc[u], ldx, A.xvec != 0, xv[u]);
+            for (int u = 0; u < kB; u++) {
+                if (i + u < nv) {
+                    ld_xrow<V, K>(x, c[u], ldx, xvec != 0, xv[u]);
                 } else {
 #pragma unroll
                     for (int q = 0; q < K; q++) xv[u][q] = V(0);
                 }
             }
+            const unsigned eb = ends8(i);
 #pragma unroll
-            for (int u = 0; u < kU; u++) {
-                const int i = i0 + u;
-                if (i >= sigma) break;
-                const uint32_t b = (xl == 0 && i == 0) ? 0u : (i == 0 ? bit0 : bit_at(i));
-                if (b) {
-                    if (!seen) {
+            for (int u = 0; u < kB; u++) {
+                if (SIG == 0 && i + u >= sigma) break;
+#pragma unroll
+                for (int q = 0; q < K; q++) sum[q] = fma(a[u], xv[u][q], sum[q]);
+                if ((eb >> u) & 1u) {
+                    if (first) {
+                        first = false;
 #pragma unroll
                         for (int q = 0; q < K; q++) head[q] = sum[q];
-                        seen = true;
                     } else {
-                        V *yp = y + map_row(rel) * ldy;
-#pragma unroll
-                        for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, sum[q], beta, yp + q);
+                        put(idx, sum);
                     }
-                    rel++;
+                    idx++;
 #pragma unroll
                     for (int q = 0; q < K; q++) sum[q] = V(0);
                 }
-#pragma unroll
-                for (int q = 0; q < K; q++) sum[q] += aa[u] * xv[u][q];
             }
         }
-    }
-    // segmented inclusive scan of the lanes' trailing runs, keyed by segment
-    int32_t key = rel;
-    // runs of equal keys never cross a tile's lanes (its first lane is flagged)
-    const int32_t key_up = __shfl_up_sync(0xffffffffu, key, 1, OMEGA);  // every lane shuffles (full mask)
-    const int span = unflagged_run(xl == 0 || key_up != key);
+        // segmented inclusive scan of the lanes' open sums
 #pragma unroll
-    for (int o = 1; o < OMEGA; o <<= 1) {
-        if (o > span) break;  // warp-uniform
-        const int32_t k2 = __shfl_up_sync(0xffffffffu, key, o, OMEGA);
-        V v2[K];
+        for (int o = 1; o < 32; o <<= 1) {
+            if (!__any_sync(kFull, dist >= o)) break;
 #pragma unroll
-        for (int q = 0; q < K; q++) v2[q] = __shfl_up_sync(0xffffffffu, sum[q], o, OMEGA);
-        if (xl >= o && k2 == key) {
-#pragma unroll
-            for (int q = 0; q < K; q++) sum[q] += v2[q];
+            for (int q = 0; q < K; q++) {
+                const V up = __shfl_up_sync(kFull, sum[q], o);
+                if (dist >= o) sum[q] += up;
+            }
         }
-    }
-    const int32_t kprev = __shfl_up_sync(0xffffffffu, key, 1, OMEGA);
-    V sprev[K];
+        V cin[K];
 #pragma unroll
-    for (int q = 0; q < K; q++) sprev[q] = __shfl_up_sync(0xffffffffu, sum[q], 1, OMEGA);
-    const uint32_t tile_bit0 = __shfl_sync(0xffffffffu, bit0, g * OMEGA, 32);
-    const bool carry = xl > 0 && kprev == yoff;
-    if (active && seen) {  // the segment numbered yoff closes at this lane's first start bit
-        V tot[K];
+        for (int q = 0; q < K; q++) cin[q] = __shfl_up_sync(kFull, sum[q], 1);
+        if (mine) {
+            if (lane > 0) {
 #pragma unroll
-        for (int q = 0; q < K; q++) tot[q] = head[q] + (carry ? sprev[q] : V(0));
-        if (yoff == 0 && !tile_bit0) {
-            V *hp = head_val + t * kMaxK;  // the tile's first row began in an earlier tile
+                for (int q = 0; q < K; q++) head[q] += cin[q];
+            }
+            if (!kSeed && pos == 0 && later) {
 #pragma unroll
-            for (int q = 0; q < K; q++) hp[q] = tot[q];
-        } else {
-            V *yp = y + map_row(yoff) * ldy;
+                for (int q = 0; q < K; q++) head[q] += carry[q];
+            }
+            if (head_split && pos == 0) {
+                V *hp = head_val + w * kMaxK;
 #pragma unroll
-            for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, tot[q], beta, yp + q);
-        }
-    }
-    if (active && xl == OMEGA - 1) {  // the tile's last run
-        const int64_t r = map_row(key);
-        const int64_t tile_end = base + tile;
-        const bool continues = (int64_t)A.rp[r + 1] > tile_end;
-        has_end[t] = (key > 0 || !continues) ? 1 : 0;
-        if (continues) {
-            carry_row[t] = (int32_t)r;
-            V *cp = carry_val + t * kMaxK;
-#pragma unroll
-            for (int q = 0; q < K; q++) cp[q] = sum[q];
-        } else {
-            carry_row[t] = -1;
-            if (key == 0 && !tile_bit0) {
-                V *hp = head_val + t * kMaxK;
-#pragma unroll
-                for (int q = 0; q < K; q++) hp[q] = sum[q];
+                for (int q = 0; q < K; q++) hp[q] = head[q];
             } else {
-                V *yp = y + r * ldy;
-#pragma unroll
-                for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, sum[q], beta, yp + q);
+                put(row + pos, head);
             }
         }
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            const V last = __shfl_sync(kFull, sum[q], 31);
+            carry[q] = kSeed || nend > 0 ? last : carry[q] + last;
+        }
+        if (nend > 0) head_split = false;
+        row += nend;
+        later = true;
+    }
+    if (A.nempty > 0) {  // rows without nonzeros: this window's share of the list
+        const int64_t i0 = A.nempty * w / A.windows, i1 = A.nempty * (w + 1) / A.windows;
+        for (int64_t i = i0 + lane; i < i1; i += 32) {
+            V *ye = y + (int64_t)__ldg(A.empty + i) * ldy;
+#pragma unroll
+            for (int q = 0; q < K; q++) ye[q] = beta == V(0) ? V(0) : beta * ye[q];
+        }
+    }
+    if ((rec.w & 2) && lane == 0) {
+        V *cp = tail_val + w * kMaxK;
+#pragma unroll
+        for (int q = 0; q < K; q++) cp[q] = carry[q];
     }
 }
 
-__global__ void count_empty_rows(int64_t rows, const int32_t *__restrict__ rp, unsigned long long *out) {
-    unsigned long long c = 0;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x)
-        c += rp[r] == rp[r + 1];
-    c = warp_sum(c);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
+constexpr int kC5Block = 64;
+template <typename V, int K, int SIG>
+constexpr int c5_min_ctas() {
+    return K == 1 ? (sizeof(V) == 8 ? 18 : SIG == 16 ? 20 : 18) : K * sizeof(V) <= 16 ? 10 : 8;
 }
 
-// y = beta*y on the empty rows before the tail tile (thread per row).
+template <typename V, int K, int SIG, bool PLAIN>
+__global__ void __launch_bounds__(kC5Block, (c5_min_ctas<V, K, SIG>())) csr5_kernel(
+    const StreamView A, const C5Shape g, const V *__restrict__ x, int64_t ldx, int xvec, V alpha, V beta,
+    V *__restrict__ y, int64_t ldy, V *__restrict__ tail_val, V *__restrict__ head_val) {
+    const int64_t w = (int64_t)blockIdx.x * (kC5Block / 32) + (threadIdx.x >> 5);
+    if (w >= A.windows) return;
+    c5_window<V, K, SIG, PLAIN>(A, g, x, ldx, xvec, alpha, beta, y, ldy, w, tail_val, head_val);
+}
+
 template <typename V, int K>
-__global__ void __launch_bounds__(kBlock) csr5_empty_rows(int64_t rows, const int32_t *__restrict__ rp, V beta,
-                                                        V *__restrict__ y, int64_t ldy) {
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x)
-        if (ld_stream(rp + r) == ld_stream(rp + r + 1)) {
-            V *yp = y + r * ldy;
+__global__ void csr5_no_nonzeros(int64_t m, V beta, V *__restrict__ y, int64_t ldy) {
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x)
 #pragma unroll
-            for (int q = 0; q < K; q++) yp[q] = beta == V(0) ? V(0) : beta * yp[q];
-        }
-}
-
-// Rows from the tail tile on (CSR dot products, warp per row; the first one is
-// clipped to the tail when it began earlier).
-template <typename V, int K>
-__global__ void __launch_bounds__(kBlock) csr5_rows_kernel(C5View A, int32_t tail_row, int64_t tail_start,
-                                                         const V *__restrict__ x, int64_t ldx, V alpha, V beta,
-                                                         V *__restrict__ y, int64_t ldy, int32_t *__restrict__ has_end,
-                                                         V *__restrict__ head_val) {
-    const int lane = threadIdx.x & 31;
-    const V *val = (const V *)A.val;
-    for (int64_t r = tail_row + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < A.m;
-         r += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        const int32_t rs = A.rp[r], re = A.rp[r + 1];
-        const bool clipped = r == tail_row && rs < tail_start;
-        const int64_t s0 = clipped ? tail_start : rs;
-        V s[K];
-#pragma unroll
-        for (int q = 0; q < K; q++) s[q] = V(0);
-        for (int64_t j = s0 + lane; j < re; j += 32) {
-            const V a = ld_stream(val + j);
-            V xr[K];
-            ld_xrow<V, K>(x, ld_stream(A.col + j), ldx, A.xvec != 0, xr);
-#pragma unroll
-            for (int q = 0; q < K; q++) s[q] += a * xr[q];
-        }
-#pragma unroll
-        for (int q = 0; q < K; q++) s[q] = warp_sum(s[q]);
-        if (lane == 0) {
-            if (clipped) {
-                V *hp = head_val + (int64_t)(A.p - 1) * kMaxK;
-#pragma unroll
-                for (int q = 0; q < K; q++) hp[q] = s[q];
-                has_end[A.p - 1] = 1;
-            } else {
-                V *yp = y + r * ldy;
-#pragma unroll
-                for (int q = 0; q < K; q++) yp[q] = axpby(alpha, s[q], beta, yp + q);
-            }
-        }
-    }
-}
-
-// Tiles 0..p-2 may leave a carry; the walk may reach the tail tile p-1, whose
-// head piece the row pass stored.
-template <typename V, int K>
-__global__ void csr5_fixup(int32_t ntiles, int64_t tile, const int32_t *__restrict__ rp,
-                           const int32_t *__restrict__ carry_row, const int32_t *__restrict__ has_end,
-                           const V *__restrict__ carry_val, const V *__restrict__ head_val, V alpha, V beta,
-                           V *__restrict__ y, int64_t ldy) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t - (threadIdx.x & 31) >= ntiles - 1) return;  // whole warp past the last full tile
-    const int32_t r = t < ntiles - 1 ? carry_row[t] : -1;
-    const bool mine = r >= 0 && (int64_t)rp[r] >= t * tile;  // open here and began in tile t
-    V tot[K];
-    chain_sum<V, K>(mine, t, ntiles, 0, has_end, carry_val, head_val, tot);
-    if (mine) {
-        V *yp = y + (int64_t)r * ldy;
-#pragma unroll
-        for (int q = 0; q < K; q++) yp[q] = axpby(alpha, tot[q], beta, yp + q);
-    }
-}
-
-C5View view_of(const sspmv_csr5 *A) {
-    C5View v;
-    v.xvec = 0;
-    v.m = (int32_t)A->f.num_rows;
-    v.n = (int32_t)A->f.num_cols;
-    v.p = A->_p;
-    v.sigma = A->sigma;
-    v.byo = A->bit_y_offset;
-    v.bao = A->bit_y_offset + A->bit_scansum_offset;
-    v.np = A->num_packets;
-    v.rp = A->row_offset;
-    v.col = A->col_index;
-    v.val = A->values;
-    v.tp = A->tile_ptr;
-    v.td = A->tile_desc;
-    v.tdo_ptr = A->tile_desc_offset_ptr;
-    v.tdo = A->tile_desc_offset;
-    return v;
-}
-
-// plan: extra[0] carry_row+has_end ints (2p), extra[1] carry_val, extra[2] head_val
-sspmv_status ensure_c5_plan(const sspmv_csr5 *A, Plan *pl, sspmv_stream_t s) {
-    if (pl->extra[0]) return SSPMV_OK;
-    std::lock_guard<PlanMutex> g(plan_mutex());
-    if (pl->extra[0]) return SSPMV_OK;
-    const int64_t p = std::max<int64_t>(A->_p, 1);
-    const size_t sv = vsize(A->f.value_type);
-    int32_t *ints = nullptr;
-    unsigned char *cv = nullptr, *hv = nullptr;
-    SSPMV_TRY(dalloc(&ints, (size_t)p * 2, s));
-    SSPMV_TRY(dalloc(&cv, (size_t)p * kMaxK * sv, s));
-    SSPMV_TRY(dalloc(&hv, (size_t)p * kMaxK * sv, s));
-    SSPMV_CUDA_TRY(cudaMemsetAsync(ints, 0, (size_t)p * 8, cu(s)));
-    // empty rows before the tail tile (they get y = beta*y in a separate pass)
-    const int64_t tail_row = A->_p > 0 ? A->tail_partition_start : 0;
-    unsigned long long *cnt = nullptr, h = 0;
-    SSPMV_TRY(dalloc(&cnt, 1, s));
-    SSPMV_CUDA_TRY(cudaMemsetAsync(cnt, 0, 8, cu(s)));
-    if (tail_row > 0) {
-        count_empty_rows<<<grid_for(tail_row, 256, (int64_t)num_sms() * 16), 256, 0, cu(s)>>>(tail_row, A->row_offset,
-                                                                                             cnt);
-        note_launch();
-    }
-    SSPMV_CUDA_TRY(cudaMemcpyAsync(&h, cnt, 8, cudaMemcpyDeviceToHost, cu(s)));
-    SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
-    dfree(cnt, s);
-    pl->extra_i[3] = (int64_t)h;
-    pl->extra[1] = cv;
-    pl->extra[2] = hv;
-    pl->extra[0] = ints;
-    return SSPMV_OK;
-}
-
-template <typename V, int K, int OMEGA>
-sspmv_status launch_c5_tiles(const C5View &v, V alpha, const V *x, int64_t ldx, V beta, V *y, int64_t ldy,
-                             int32_t *cr, int32_t *he, V *cv, V *hv, sspmv_stream_t s) {
-    const int64_t tiles = v.p - 1;
-    const int64_t warps = (tiles + (32 / OMEGA) - 1) / (32 / OMEGA);
-    const unsigned grid = grid_for(warps * 32, kBlock);
-    const int sig = (v.np <= 2 && (v.sigma == 16 || v.sigma == 32)) ? v.sigma : 0;
-    if constexpr (K == 1) {  // one right-hand side: sigma-specialised kernels
-        if (sig == 16) {
-            if (alpha == V(1) && beta == V(0))
-                csr5_tile_kernel<V, K, OMEGA, 16, true><<<grid, kBlock, 0, cu(s)>>>(v, x, ldx, alpha, beta, y, ldy, cr,
-                                                                                   he, cv, hv);
-            else
-                csr5_tile_kernel<V, K, OMEGA, 16><<<grid, kBlock, 0, cu(s)>>>(v, x, ldx, alpha, beta, y, ldy, cr, he,
-                                                                              cv, hv);
-            SSPMV_LAUNCH_CHECK();
-            return SSPMV_OK;
-        }
-        if (sig == 32) {
-            if (alpha == V(1) && beta == V(0))
-                csr5_tile_kernel<V, K, OMEGA, 32, true><<<grid, kBlock, 0, cu(s)>>>(v, x, ldx, alpha, beta, y, ldy, cr,
-                                                                                   he, cv, hv);
-            else
-                csr5_tile_kernel<V, K, OMEGA, 32><<<grid, kBlock, 0, cu(s)>>>(v, x, ldx, alpha, beta, y, ldy, cr, he,
-                                                                              cv, hv);
-            SSPMV_LAUNCH_CHECK();
-            return SSPMV_OK;
-        }
-    }
-    csr5_tile_kernel<V, K, OMEGA, 0><<<grid, kBlock, 0, cu(s)>>>(v, x, ldx, alpha, beta, y, ldy, cr, he, cv, hv);
-    SSPMV_LAUNCH_CHECK();
-    return SSPMV_OK;
+        for (int q = 0; q < K; q++) y[r * ldy + q] = beta == V(0) ? V(0) : beta * y[r * ldy + q];
 }
 
 template <typename V, int K>
 sspmv_status csr5_pass(const sspmv_csr5 *A, Plan *pl, V alpha, const V *x, int64_t ldx, V beta, V *y, int64_t ldy,
                        sspmv_stream_t s) {
-    SSPMV_TRY(ensure_c5_plan(A, pl, s));
-    C5View v = view_of(A);
-    v.xvec = xrow_vec(x, ldx, sizeof(V), K);
-    const int64_t p = std::max<int64_t>(A->_p, 1);
-    int32_t *cr = (int32_t *)pl->extra[0], *he = cr + p;
-    V *cv = (V *)pl->extra[1], *hv = (V *)pl->extra[2];
-    if (A->_p > 1) {
-        switch (A->omega) {
-        case 4: SSPMV_TRY((launch_c5_tiles<V, K, 4>(v, alpha, x, ldx, beta, y, ldy, cr, he, cv, hv, s))); break;
-        case 8: SSPMV_TRY((launch_c5_tiles<V, K, 8>(v, alpha, x, ldx, beta, y, ldy, cr, he, cv, hv, s))); break;
-        case 16: SSPMV_TRY((launch_c5_tiles<V, K, 16>(v, alpha, x, ldx, beta, y, ldy, cr, he, cv, hv, s))); break;
-        case 32: SSPMV_TRY((launch_c5_tiles<V, K, 32>(v, alpha, x, ldx, beta, y, ldy, cr, he, cv, hv, s))); break;
-        default: return fail(SSPMV_NOT_SUPPORTED, "CSR5 SpMV supports omega in {4, 8, 16, 32}");
-        }
-    }
-    const int64_t tail_start = A->_p > 0 ? (int64_t)(A->_p - 1) * A->sigma * A->omega : 0;
-    const int32_t tail_row = A->_p > 0 ? A->tail_partition_start : 0;
-    if (pl->extra_i[3] > 0) {  // empty rows before the tail tile
-        csr5_empty_rows<V, K><<<grid_for(tail_row, kBlock, (int64_t)num_sms() * 16), kBlock, 0, cu(s)>>>(
-            tail_row, A->row_offset, beta, y, ldy);
+    const int64_t m = A->f.num_rows, nnz = A->f.num_nnzs;
+    if (nnz == 0) {
+        csr5_no_nonzeros<V, K><<<grid_for(m, kBlock, (int64_t)num_sms() * 16), kBlock, 0, cu(s)>>>(m, beta, y, ldy);
         SSPMV_LAUNCH_CHECK();
+        return SSPMV_OK;
     }
-    csr5_rows_kernel<V, K><<<grid_for((A->f.num_rows - tail_row) * 32, kBlock, (int64_t)num_sms() * 32), kBlock, 0,
-                             cu(s)>>>(v, tail_row, tail_start, x, ldx, alpha, beta, y, ldy, he, hv);
+    if (A->_p > 1 && A->omega != 4 && A->omega != 8 && A->omega != 16 && A->omega != 32)
+        return fail(SSPMV_NOT_SUPPORTED, "CSR5 SpMV supports omega in {4, 8, 16, 32}");
+    const int ctas = A->f.value_type == SSPMV_F64 ? c5_min_ctas<double, 1, 16>() : c5_min_ctas<float, 1, 16>();
+    const int steps = window_steps(nnz, 32 * A->sigma, 32 * A->sigma, ctas * (kC5Block / 32));
+    SSPMV_TRY(ensure_stream_plan(pl->stream, m, nnz, A->row_offset, nullptr, A->f.value_type, s,
+                                 32 * A->sigma * steps, 0));
+    const StreamView v = stream_view(pl->stream, nnz, A->col_index, A->values);
+    // a single tile is in CSR order whatever omega is
+    const C5Shape g{A->sigma, A->_p > 1 ? A->omega : 32, A->_p};
+    const unsigned grid = grid_for(v.windows, kC5Block / 32);
+    V *tv = (V *)pl->stream.tail_val, *hv = (V *)pl->stream.head_val;
+    auto go = [&](auto kernel) {
+        kernel<<<grid, kC5Block, 0, cu(s)>>>(v, g, x, ldx, xrow_vec(x, ldx, sizeof(V), K), alpha, beta, y, ldy, tv, hv);
+    };
+    const bool plain = alpha == V(1) && beta == V(0);  // y = sum
+    if (A->sigma == 16) {
+        if (plain) go(csr5_kernel<V, K, 16, true>);
+        else go(csr5_kernel<V, K, 16, false>);
+    } else if (A->sigma == 32) {
+        if (plain) go(csr5_kernel<V, K, 32, true>);
+        else go(csr5_kernel<V, K, 32, false>);
+    } else {
+        go(csr5_kernel<V, K, 0, false>);
+    }
     SSPMV_LAUNCH_CHECK();
-    if (A->_p > 1) {
-        csr5_fixup<V, K><<<grid_for(A->_p - 1, 256), 256, 0, cu(s)>>>(A->_p, (int64_t)A->sigma * A->omega,
-                                                                     A->row_offset, cr, he, cv, hv, alpha, beta, y,
-                                                                     ldy);
-        SSPMV_LAUNCH_CHECK();
-    }
-    return SSPMV_OK;
+    return launch_split_rows<V, K>(v, pl->stream, alpha, beta, y, ldy, s);
 }
 
 }  // namespace

@@ -21,10 +21,8 @@
 // lane that ends it.  An earlier form that marked row starts in shared memory
 // (row_offset read per chunk, a five-step prefix scan, a second launch for rows
 // crossing 256-element chunks) took, per SpMV: 1024^2 Laplacian FP64 33.4 us
-// (now 23.2), uniform 2M x 32 FP64 315 us (271), banded 2M FP64 85 us (60),
-// power-law 4M FP32 with alpha and beta 339 us (274).  Windows of one step
-// (T = 224) were slower than two and more (a warp's start is paid once):
-// uniform FP32 247 against 242 us, power-law rows 442 against 365 us.  Columns
+// (now 21.2), uniform 2M x 32 FP64 315 us (271), banded 2M FP64 85 us (60),
+// power-law 4M FP32 with alpha and beta 339 us (272).  Columns
 // loaded a step ahead, a cp.async.bulk L2 prefetch of later windows and all
 // finished rows through shared memory were slower, too (fewer warps, or more
 // queued accesses).
@@ -50,6 +48,7 @@
 // code, so its result does not depend on the batch.
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "common.cuh"
 #include "csr_stream.cuh"
@@ -66,12 +65,22 @@ constexpr int kWarps = kBlock / 32;
 constexpr int kOver = 32;  // elements a warp reads past its window to finish its last row
 constexpr unsigned kFull = 0xffffffffu;
 
-// Two steps of 256 a warp, less what its last row may run past the window:
-// enough windows for every SM from a million nonzeros on.  Four steps where
-// there are windows to spare, from 16M nonzeros: power-law 4M FP32 277 us with
-// two steps, 274 with four; 1024^2 Laplacian FP64 (5M) 23.2 with two, 25.4
-// with four.
-int window_size(int64_t nnz) { return (nnz < ((int64_t)16 << 20) ? 512 : 1024) - kOver; }
+// Resident CTAs per SM the register budget is set for: the best of 16 to 24
+// (FP32) and 12 to 18 (FP64) for K = 1; spills and fewer warps cost about the
+// same beyond.
+template <typename V, int K>
+constexpr int stream_min_ctas() {
+    if (K == 1) return sizeof(V) == 8 ? 15 : 20;
+    return sizeof(V) == 8 ? 12 : 14;
+}
+
+// Elements per window: whole steps of 256 less what the last row may run past
+// the window, the number of steps by what the last wave of warps leaves idle
+// (window_steps).
+int window_size(int64_t nnz, int32_t value_type) {
+    const int ctas = value_type == SSPMV_F64 ? stream_min_ctas<double, 1>() : stream_min_ctas<float, 1>();
+    return 256 * window_steps(nnz, 256, 256 - kOver, ctas * kWarps) - kOver;
+}
 
 template <typename V, int K>
 struct StreamShape {
@@ -429,27 +438,31 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
     }
 }
 
-// Split row sp (first window, last window, ordinal), one warp: its pieces in
-// a fixed order -- lane l adds windows w0 + l, w0 + l + 32, ..., then a
-// shuffle tree.
+// Split row sp (first window, last window, ordinal), kSplitLanes lanes: its
+// pieces in a fixed order -- lane l adds windows w0 + l, w0 + l + 8, ..., then
+// a shuffle tree.  All lanes of the warp call it (any: whether the lane's row
+// exists).
+constexpr int kSplitLanes = 8;
+
 template <typename V, int K>
-__device__ __forceinline__ void stream_split_row(const int4 sp, const int32_t *__restrict__ nzrow,
+__device__ __forceinline__ void stream_split_row(bool any, const int4 sp, const int32_t *__restrict__ nzrow,
                                                  const StreamSlots<V> &sl, V alpha, V beta, V *__restrict__ y,
-                                                 uint32_t yrow) {
-    const int lane = threadIdx.x & 31;
+                                                 int64_t ldy) {
+    const int lane = threadIdx.x & (kSplitLanes - 1);
     V tot[K];
 #pragma unroll
     for (int q = 0; q < K; q++) tot[q] = V(0);
-    for (int u = sp.x + lane; u <= sp.y; u += 32) {
-        const V *p = (u == sp.y ? sl.head_val : sl.tail_val) + (u + sl.shift) * kMaxK;
+    if (any) {
+        for (int u = sp.x + lane; u <= sp.y; u += kSplitLanes) {
+            const V *p = (u == sp.y ? sl.head_val : sl.tail_val) + (u + sl.shift) * kMaxK;
 #pragma unroll
-        for (int q = 0; q < K; q++) tot[q] += p[q];
+            for (int q = 0; q < K; q++) tot[q] += p[q];
+        }
     }
 #pragma unroll
-    for (int q = 0; q < K; q++) tot[q] = warp_sum(tot[q]);
-    if (lane == 0) {
-        const uint32_t row = nzrow ? __ldg(nzrow + sp.z) : sp.z;
-        V *yp = reinterpret_cast<V *>(reinterpret_cast<char *>(y) + (uint64_t)row * yrow);
+    for (int q = 0; q < K; q++) tot[q] = warp_sum(tot[q], kSplitLanes);
+    if (any && lane == 0) {
+        V *yp = y + (int64_t)(nzrow ? __ldg(nzrow + sp.z) : sp.z) * ldy;
 #pragma unroll
         for (int q = 0; q < K; q++) yp[q] = scaled(alpha, tot[q], beta, beta == V(0) ? V(0) : yp[q]);
     }
@@ -458,18 +471,10 @@ __device__ __forceinline__ void stream_split_row(const int4 sp, const int32_t *_
 template <typename V, int K>
 __global__ void __launch_bounds__(256) csr_split_kernel(int64_t n, const int4 *__restrict__ split,
                                                         const int32_t *__restrict__ nzrow, const StreamSlots<V> sl,
-                                                        V alpha, V beta, V *__restrict__ y, uint32_t yrow) {
-    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i < n) stream_split_row<V, K>(__ldg(split + i), nzrow, sl, alpha, beta, y, yrow);
-}
-
-// Resident CTAs per SM the register budget is set for: the best of 16 to 24
-// (FP32) and 12 to 18 (FP64) for K = 1; spills and fewer warps cost about the
-// same beyond.
-template <typename V, int K>
-constexpr int stream_min_ctas() {
-    if (K == 1) return sizeof(V) == 8 ? 15 : 20;
-    return sizeof(V) == 8 ? 12 : 14;
+                                                        V alpha, V beta, V *__restrict__ y, int64_t ldy) {
+    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kSplitLanes;
+    const bool any = i < n;
+    stream_split_row<V, K>(any, any ? __ldg(split + i) : make_int4(0, -1, 0, 0), nzrow, sl, alpha, beta, y, ldy);
 }
 
 // PLAIN: alpha == 1 and beta == 0 (y = sum): row writes carry no FP64
@@ -492,18 +497,18 @@ int yrow_vec(const V *y, int64_t ldy, int k) {
 }
 
 // ------------------------------------------------------------------ plan --
-// A row that goes on more than kOver elements past its first window is split.
-__device__ __forceinline__ bool row_is_split(const int32_t *__restrict__ rp, int64_t row, int T) {
-    return (int64_t)rp[row + 1] > ((int64_t)(rp[row] / T) + 1) * T + kOver;
+// A row that goes on more than `over` elements past its first window is split.
+__device__ __forceinline__ bool row_is_split(const int32_t *__restrict__ rp, int64_t row, int T, int over) {
+    return (int64_t)rp[row + 1] > ((int64_t)(rp[row] / T) + 1) * T + over;
 }
 
 // out[0]: rows without nonzeros, out[1]: split rows.
-__global__ void stream_count_rows(int64_t m, int T, const int32_t *__restrict__ rp,
+__global__ void stream_count_rows(int64_t m, int T, int over, const int32_t *__restrict__ rp,
                                   unsigned long long *__restrict__ out) {
     unsigned long long n = 0, k = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
         n += rp[i + 1] == rp[i];
-        k += row_is_split(rp, i, T);
+        k += row_is_split(rp, i, T, over);
     }
     n = warp_sum(n);
     k = warp_sum(k);
@@ -548,7 +553,7 @@ __device__ __forceinline__ int first_row_from(const int32_t *__restrict__ rp, in
 
 // Window records, and the list of split rows (in any order: each is summed
 // on its own); nsplit starts at zero.
-__global__ void stream_windows(int64_t nw, int T, int m, int64_t nnz, const int32_t *__restrict__ rp,
+__global__ void stream_windows(int64_t nw, int T, int over, int m, int64_t nnz, const int32_t *__restrict__ rp,
                                const int32_t *__restrict__ pos, int4 *__restrict__ rec, int4 *__restrict__ split,
                                unsigned long long *__restrict__ nsplit) {
     const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -558,13 +563,13 @@ __global__ void stream_windows(int64_t nw, int T, int m, int64_t nnz, const int3
     auto ordinal = [&](int row) { return pos && row < m ? pos[row] : row; };
     int64_t eA = rp[r], eB;
     int first = ordinal(r), flags = 0;
-    if (eA > a && row_is_split(rp, r - 1, T)) {  // row r - 1 began in an earlier window
+    if (eA > a && row_is_split(rp, r - 1, T, over)) {  // row r - 1 began in an earlier window
         flags |= 1;
         eA = a;
         first = ordinal(r - 1);
     }
     if (r2 > r) {  // the last row that starts here
-        if (row_is_split(rp, r2 - 1, T)) {
+        if (row_is_split(rp, r2 - 1, T, over)) {
             flags |= 2;
             eB = b;
             split[atomicAdd(nsplit, 1ull)] = make_int4((int)w, (int)(((int64_t)rp[r2] - 1) / T), ordinal(r2 - 1), 0);
@@ -582,6 +587,28 @@ __global__ void stream_windows(int64_t nw, int T, int m, int64_t nnz, const int3
 
 }  // namespace
 
+// Warps of equal work run in waves of what the SMs hold, so few windows cost as
+// many steps as their last wave: 1024^2 Laplacian FP64 (4560 warps at once)
+// 23.2 us in 2.4 waves of two steps, 25.6 in 1.2 of four, 21.2 in one of five;
+// FP32 (6080) 14.9, 14.2 and 14.9.  kStart: a warp's start, in steps.  Many
+// waves overlap, and longer windows leave fewer rows to finish (power-law 4M
+// FP32: 289 us with one step, 275 with two, 272 with three to five).
+int window_steps(int64_t nnz, int step, int first, int warps_per_sm) {
+    constexpr double kStart = 0.35;
+    const double slots = (double)num_sms() * warps_per_sm;
+    int best = 1;
+    double best_cost = 0;
+    for (int n = 1; n <= 5; n++) {
+        const double waves = (double)nnz / ((double)(n - 1) * step + first) / slots;
+        const double cost = (waves <= 6 ? std::ceil(waves) : waves + 0.5) * (n + kStart);
+        if (n == 1 || cost < best_cost) {
+            best = n;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
 void free_stream_plan(StreamPlan &sp, sspmv_stream_t s) {
     dfree(sp.rec, s);
     dfree(sp.split, s);
@@ -594,11 +621,12 @@ void free_stream_plan(StreamPlan &sp, sspmv_stream_t s) {
 }
 
 sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
-                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s) {
+                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s, int window, int over) {
     if (sp.window) return SSPMV_OK;
     std::lock_guard<PlanMutex> g(plan_mutex());
     if (sp.window) return SSPMV_OK;
-    const int T = window_size(nnz);
+    const int T = window > 0 ? window : window_size(nnz, value_type);
+    if (over < 0) over = kOver;
     const int64_t nw = (nnz + T - 1) / T;
     const size_t sv = vsize(value_type);
     const unsigned grid = grid_for(m, 256, (int64_t)num_sms() * 16);
@@ -608,7 +636,7 @@ sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const in
     auto build = [&]() -> sspmv_status {
         SSPMV_TRY(dalloc(&count, 3, s));
         SSPMV_CUDA_TRY(cudaMemsetAsync(count, 0, 3 * sizeof(*count), cu(s)));
-        stream_count_rows<<<grid, 256, 0, cu(s)>>>(m, T, row_offset, count);
+        stream_count_rows<<<grid, 256, 0, cu(s)>>>(m, T, over, row_offset, count);
         SSPMV_LAUNCH_CHECK();
         SSPMV_CUDA_TRY(cudaMemcpyAsync(h, count, sizeof(h), cudaMemcpyDeviceToHost, cu(s)));
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
@@ -633,7 +661,7 @@ sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const in
         SSPMV_TRY(dalloc(&q.rec, (size_t)nw, s));
         q.nsplit = (int64_t)h[1];
         SSPMV_TRY(dalloc(&q.split, (size_t)q.nsplit, s));
-        stream_windows<<<grid_for(nw, 128), 128, 0, cu(s)>>>(nw, T, (int)m, nnz, row_offset, pos, q.rec, q.split,
+        stream_windows<<<grid_for(nw, 128), 128, 0, cu(s)>>>(nw, T, over, (int)m, nnz, row_offset, pos, q.rec, q.split,
                                                              count + 2);
         SSPMV_LAUNCH_CHECK();
         if (q.nsplit > 0) {
@@ -683,17 +711,25 @@ sspmv_status launch_stream_view(const StreamView &v, StreamPlan &sp, V alpha, co
     kernel<<<grid_for(v.windows, kWarps), kBlock, 0, cu(s)>>>(v, x, xrow, alpha, beta, y, yrow, sl,
                                                               xrow_vec(x, ldx, sizeof(V), K), yrow_vec(y, ldy, K));
     SSPMV_LAUNCH_CHECK();
-    if (v.nsplit > 0) {
-        csr_split_kernel<V, K><<<grid_for(v.nsplit * 32, 256), 256, 0, cu(s)>>>(v.nsplit, v.split, v.nzrow, sl, alpha,
-                                                                                beta, y, yrow);
-        SSPMV_LAUNCH_CHECK();
-    }
+    return launch_split_rows<V, K>(v, sp, alpha, beta, y, ldy, s);
+}
+
+template <typename V, int K>
+sspmv_status launch_split_rows(const StreamView &v, StreamPlan &sp, V alpha, V beta, V *y, int64_t ldy,
+                               sspmv_stream_t s) {
+    if (v.nsplit == 0) return SSPMV_OK;
+    const StreamSlots<V> sl{(V *)sp.tail_val, (V *)sp.head_val, 0};
+    csr_split_kernel<V, K><<<grid_for(v.nsplit * kSplitLanes, 256), 256, 0, cu(s)>>>(v.nsplit, v.split, v.nzrow, sl,
+                                                                                      alpha, beta, y, ldy);
+    SSPMV_LAUNCH_CHECK();
     return SSPMV_OK;
 }
 
 #define SSPMV_STREAM_INST(V, K)                                                                              \
     template sspmv_status launch_stream_view<V, K>(const StreamView &, StreamPlan &, V, const V *, int64_t, V, \
-                                                   V *, int64_t, sspmv_stream_t);
+                                                   V *, int64_t, sspmv_stream_t);                            \
+    template sspmv_status launch_split_rows<V, K>(const StreamView &, StreamPlan &, V, V, V *, int64_t,          \
+                                                  sspmv_stream_t);
 SSPMV_STREAM_INST(float, 1)
 SSPMV_STREAM_INST(float, 2)
 SSPMV_STREAM_INST(float, 4)
@@ -753,12 +789,16 @@ __global__ void __launch_bounds__(256) csr_batch_split_kernel(int g, const Batch
     const int64_t total = hdr->total_splits[g];
     const int64_t base = hdr->slot_base[g];
     const BatchItem *items = all_items + hdr->item_begin[g];
-    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < total; i += warps) {
-        const BatchItem *q = items + batch_item_of(items, n, i, &BatchItem::split_begin);
+    const int64_t stride = ((int64_t)gridDim.x * blockDim.x) / kSplitLanes;
+    const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kSplitLanes;
+    const int64_t w0 = i0 - (threadIdx.x & 31) / kSplitLanes;  // the warp's first row: trip count the same for its lanes
+    for (int64_t d = 0; w0 + d < total; d += stride) {
+        const int64_t i = i0 + d;
+        const bool any = i < total;
+        const BatchItem *q = items + (any ? batch_item_of(items, n, i, &BatchItem::split_begin) : 0);
         const StreamSlots<V> sl{tail_val, head_val, base + q->window_begin};
-        stream_split_row<V, K>(__ldg(q->view.split + (i - q->split_begin)), q->view.nzrow, sl, (V)q->alpha,
-                               (V)q->beta, (V *)q->y, (uint32_t)(q->ldy * (int64_t)sizeof(V)));
+        stream_split_row<V, K>(any, any ? __ldg(q->view.split + (i - q->split_begin)) : make_int4(0, -1, 0, 0),
+                               q->view.nzrow, sl, (V)q->alpha, (V)q->beta, (V *)q->y, q->ldy);
     }
 }
 

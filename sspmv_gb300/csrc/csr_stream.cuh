@@ -30,8 +30,15 @@ struct StreamView {
 // Builds (once) the stream plan of m rows given by row_offset (m + 1
 // entries, nnz > 0); row_offset is not read after the call's work on `s`.
 // row_map: y row of each row (rows then all nonempty; null: the row itself), owned by the caller and kept as long as the plan.
+// Steps per window (1 to 5) for nnz elements in steps of `step`, the first of
+// `first` elements, and warps_per_sm warps at once.
+int window_steps(int64_t nnz, int step, int first, int warps_per_sm);
+
+// window, over: elements per window and past it that its warp may read to
+// finish a row (0, -1: the stream kernel's own).
 sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
-                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s);
+                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s, int window = 0,
+                                int over = -1);
 void free_stream_plan(StreamPlan &sp, sspmv_stream_t s);
 StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, const void *val);
 
@@ -45,5 +52,11 @@ inline bool stream_takes_strides(int64_t ldx, int64_t ldy, size_t value_bytes) {
 template <typename V, int K>
 sspmv_status launch_stream_view(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta, V *y,
                                 int64_t ldy, sspmv_stream_t s);
+
+// Finishes the rows whose pieces a kernel over the plan's windows has left in
+// tail_val and head_val: one launch, none without such rows.
+template <typename V, int K>
+sspmv_status launch_split_rows(const StreamView &v, StreamPlan &sp, V alpha, V beta, V *y, int64_t ldy,
+                               sspmv_stream_t s);
 
 }  // namespace sspmv

@@ -49,9 +49,9 @@ struct BatchHeader {
 constexpr size_t kBatchSlotBytes = 2 * kMaxK * 8;
 
 // Slots for a batch of `requests` matrices of `chunks` 256-nonzero chunks in
-// all: a window holds at least 480 nonzeros (window_size), so a matrix has no
-// more windows than chunks.
-inline int64_t batch_slots(int64_t chunks, int64_t requests) { return chunks + requests; }
+// all: a window holds at least 224 nonzeros (window_size), so a matrix of c
+// chunks has at most 8 c / 7 + 1 windows.
+inline int64_t batch_slots(int64_t chunks, int64_t requests) { return chunks + (chunks + 6) / 7 + requests; }
 
 // The stream kernel's view of a matrix with nonzeros (its plan built on the
 // first call).

@@ -59,7 +59,7 @@ CASES = {
 }
 
 
-@pytest.mark.parametrize("T", [224, 480, 992])
+@pytest.mark.parametrize("T", [224, 480, 992, 1248])
 @pytest.mark.parametrize("case", list(CASES))
 def test_windows_cover_every_row_once(case, T):
     rp = row_offsets(CASES[case])
