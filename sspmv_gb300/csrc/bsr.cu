@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "csr_stream.cuh"
 #include "plan.cuh"
 #include "primitives.cuh"
 #include "spmv_common.cuh"
@@ -33,6 +34,7 @@ using namespace sspmv;
 namespace {
 
 constexpr int kBlock = 256;
+constexpr int kStreamBlock = 64;
 
 __global__ void bsr_keys(int64_t m, int32_t r, int32_t c, int64_t nb, const int32_t *__restrict__ rp,
                          const int32_t *__restrict__ ci, uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
@@ -145,120 +147,223 @@ __global__ void __launch_bounds__(kBlock) bsr_spmv_kernel(int m, int n, int r, i
 // a warp hold different numbers of blocks, and GB300's narrow FP64 pipe is
 // paid per warp instruction, however few lanes are active (profiled on 4x4
 // FP64 blocks, about one block per block row: the pipe 75-84% busy with a
-// third of its lanes doing FMAs).  This kernel streams blocks instead: lane
-// (g, q), g = lane / r, q = lane % r, multiplies row q of block kb + g by its
-// x segment, so each step of G = 32 / r blocks keeps all 32 lanes on FMAs.
-// Partial sums of one block row are joined by a segmented scan over the
-// groups (lanes q, q + r, q + 2r, ...; block_row[k] keys the segments), and a
-// block row running past the step carries into the next step.  Each warp owns
-// whole block rows (warp_row[w] .. warp_row[w + 1], cut every `per_warp`
-// blocks), so no partial sum leaves its warp: one launch, and the summation
-// order is fixed by the matrix alone.  r must be a power of two <= 32.
-template <typename V, int CB>
-__global__ void __launch_bounds__(kBlock) bsr_stream_kernel(
-    int64_t nwarps, int m, int n, int lr, const int32_t *__restrict__ warp_row, const int32_t *__restrict__ row_ptr,
-    const int32_t *__restrict__ block_row, const int32_t *__restrict__ bcol, const V *__restrict__ data,
-    const V *__restrict__ x, V alpha, V beta, V *__restrict__ y) {
-    const int r = 1 << lr, G = 32 >> lr;
+// third of its lanes doing FMAs).  This kernel streams blocks instead, as the
+// stream kernel (csr_stream.cu) streams nonzeros, on the same plan made of the
+// block rows: r lanes (lane q of the group takes row q of a block) walk B
+// consecutive blocks with all their loads in flight -- 16 bytes of a block's
+// row and of x at a time -- and restart at block row ends; the groups' open
+// sums are joined by one segmented scan per step of B * 32 / r blocks.  A warp
+// finishes the block rows that start in its window, so one launch and no
+// pieces; r must be a power of two <= 32.  With one block per group and step,
+// a scan for each, block_row read per block and values one at a time: 2M rows
+// of 4x4 blocks FP32 23.2 us, now 19.2 (FP64 54.0, now 40.0).  It moves 2.5
+// TB/s there: a chain of two dependent loads (the block's column, then x) at 32
+// warps a SM.  The next step's columns and blocks loaded before this step's
+// sums measured 19.6 us (more registers, fewer warps).
+template <typename V, int C>
+struct BsrShape {
+    static constexpr int kWords = (int)(C * sizeof(V) / 4);             // 4-byte words of a block's row
+    static constexpr int B = kWords >= 16 ? 1 : kWords <= 4 ? 4 : 16 / kWords;  // up to 16 words a lane in flight
+};
+
+// Resident CTAs per SM the register budget is set for: 2M rows of 4x4 blocks,
+// FP32 at 14 / 16 / 20 CTAs 19.6 / 19.2 / 20.1 us, FP64 at 16 / 20 43.8 /
+// 40.0 us; 1M rows of 8x8 FP64 at 16 / 20 (which spills) 54.9 / 57.9 us.
+template <typename V, int C>
+constexpr int bsr_ctas() {
+    return BsrShape<V, C>::kWords > 16 ? 8 : sizeof(V) == 8 && C == 4 ? 20 : 16;
+}
+
+// C values at p: vector loads when `vec` (p aligned to min(16, C values)).
+template <typename V, int C, bool STREAM>
+__device__ __forceinline__ void ld_run(const V *__restrict__ p, bool vec, V (&out)[C]) {
+    constexpr int kBytes = (int)(C * sizeof(V));
+    if constexpr (kBytes >= 16) {
+        if (vec) {
+#pragma unroll
+            for (int h = 0; h < kBytes / 16; h++) {
+                const float4 *src = reinterpret_cast<const float4 *>(p) + h;
+                const float4 t = STREAM ? __ldcs(src) : __ldg(src);
+                if constexpr (sizeof(V) == 4) {
+                    out[4 * h] = t.x; out[4 * h + 1] = t.y; out[4 * h + 2] = t.z; out[4 * h + 3] = t.w;
+                } else {
+                    out[2 * h] = __hiloint2double(__float_as_int(t.y), __float_as_int(t.x));
+                    out[2 * h + 1] = __hiloint2double(__float_as_int(t.w), __float_as_int(t.z));
+                }
+            }
+            return;
+        }
+    } else if constexpr (kBytes == 8 && sizeof(V) == 4) {
+        if (vec) {
+            const float2 *src = reinterpret_cast<const float2 *>(p);
+            const float2 t = STREAM ? __ldcs(src) : __ldg(src);
+            out[0] = t.x;
+            out[1] = t.y;
+            return;
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < C; e++) out[e] = STREAM ? ld_stream(p + e) : ld_x(p + e);
+}
+
+template <typename V, int C, bool PLAIN>
+__global__ void __launch_bounds__(kStreamBlock, (bsr_ctas<V, C>())) bsr_stream_kernel(
+    const StreamView A, int m, int n, int lr, const V *__restrict__ data, int dvec, const V *__restrict__ x, int xvec, V alpha,
+    V beta, V *__restrict__ y) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int B = BsrShape<V, C>::B;
+    constexpr bool kSeed = sizeof(V) == 8;
+    const int64_t w = (int64_t)blockIdx.x * (kStreamBlock / 32) + (threadIdx.x >> 5);
+    if (w >= A.windows) return;  // warp-uniform
+    const int r = 1 << lr, NG = 32 >> lr;
     const int lane = threadIdx.x & 31, g = lane >> lr, q = lane & (r - 1);
-    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (w >= nwarps) return;  // warp-uniform
-    const int64_t rc = (int64_t)r * CB;
-    const int rb0 = warp_row[w], rb1 = warp_row[w + 1];
-    const int k0 = row_ptr[rb0], k1 = row_ptr[rb1];
-    V carry = V(0);
-    int carry_row = -2;
-    const bool plain = alpha == V(1) && beta == V(0);  // y = sum, exactly alpha * sum
-    for (int kb = k0; kb < k1; kb += G) {
-        const int k = kb + g;
-        const bool valid = k < k1;
-        const int br = valid ? ld_stream(block_row + k) : -1;
-        V s = V(0);
-        if (valid) {
-            const int64_t x0 = (int64_t)ld_stream(bcol + k) * CB;
-            const V *blk = data + (int64_t)k * rc + q * CB;
-            if (x0 + CB <= n) {
-                V a[CB];
+    const int64_t rc = (int64_t)r * C;
+    const int4 rec = __ldg(A.rec + w);
+    const uint32_t eA = (uint32_t)rec.x, eB = (uint32_t)rec.y;
+    int row = rec.z;
+    auto put = [&](int ordinal, V sum) {
+        const int64_t i = ((int64_t)(A.nzrow ? __ldg(A.nzrow + ordinal) : ordinal) << lr) + q;
+        if (i < m) y[i] = row_out(PLAIN, alpha, sum, beta, y + i);
+    };
+    V carry = V(0);  // the open block row's sum over the earlier steps
+    const unsigned before = g == 0 ? 0u : 0xffffffffu >> (32 - (g << lr));  // lanes of the groups before this one
+    for (uint32_t b = eA & ~(uint32_t)(B - 1); b < eB && eA < eB; b += B * NG) {  // warp-uniform
+        const uint32_t e0 = b + (uint32_t)(B * g);
+        // which of the B blocks belong to the window, and which end a block row
+        unsigned in = 0;
 #pragma unroll
-                for (int e = 0; e < CB; e++) a[e] = ld_stream(blk + e);
+        for (int u = 0; u < B; u++) in |= (e0 + u >= eA && e0 + u < eB ? 1u : 0u) << u;
+        const unsigned eb = in ? (__ldg(A.ends + (e0 >> 3)) >> (e0 & 7)) & in : 0u;
+        int bc[B];
+        V a[B][C], xv[B][C];
 #pragma unroll
-                for (int e = 0; e < CB; e++) s += a[e] * ld_x(x + x0 + e);
+        for (int u = 0; u < B; u++) bc[u] = (in >> u) & 1u ? ld_stream(A.col + e0 + u) : 0;
+#pragma unroll
+        for (int u = 0; u < B; u++) {
+            if ((in >> u) & 1u) {
+                ld_run<V, C, true>(data + (int64_t)(e0 + u) * rc + q * C, dvec != 0, a[u]);
             } else {
-                for (int e = 0; e < CB && x0 + e < n; e++) s += ld_stream(blk + e) * ld_x(x + x0 + e);
+#pragma unroll
+                for (int e = 0; e < C; e++) a[u][e] = V(0);
             }
         }
-        // FP64 adds run on the same narrow pipe as the FMAs: the carry is
-        // added only when a row goes on from the previous step, and the scan
-        // runs only as deep as the longest segment of this step.
-        if (__shfl_sync(0xffffffffu, br, 0) == carry_row) {
-            if (g == 0) s += carry;
+#pragma unroll
+        for (int u = 0; u < B; u++) {
+            const int64_t x0 = (int64_t)bc[u] * C;
+            if (((in >> u) & 1u) && x0 + C <= n) {
+                ld_run<V, C, false>(x + x0, xvec != 0, xv[u]);
+            } else {  // the ragged last block column: its fill is no part of the product
+#pragma unroll
+                for (int e = 0; e < C; e++) {
+                    const bool ok = ((in >> u) & 1u) && x0 + e < n;
+                    xv[u][e] = ok ? ld_x(x + x0 + e) : V(0);
+                    if (!ok) a[u][e] = V(0);
+                }
+            }
         }
-        const int prev = __shfl_up_sync(0xffffffffu, br, r);
-        const unsigned heads = __ballot_sync(0xffffffffu, g == 0 || prev != br);  // lanes of segment heads
-        const int head_g = (31 - __clz(heads & (0xffffffffu >> (31 - lane)))) >> lr;
-        const int depth = __reduce_max_sync(0xffffffffu, (unsigned)(valid ? g - head_g : 0));
-        for (int off = 1; off <= depth; off <<= 1) {  // segmented inclusive scan over g
-            const int obr = __shfl_up_sync(0xffffffffu, br, off << lr);
-            const V os = __shfl_up_sync(0xffffffffu, s, off << lr);
-            if (g >= off && obr == br) s += os;
+        const int mine = __popc(eb);
+        int pos = 0, nend = 0;  // block rows ended in the groups before this one, and in the step
+#pragma unroll
+        for (int bit = 0; (1 << bit) <= B; bit++) {
+            const unsigned f = __ballot_sync(kFull, q == 0 && ((mine >> bit) & 1));
+            pos += __popc(f & before) << bit;
+            nend += __popc(f) << bit;
         }
-        int next = __shfl_down_sync(0xffffffffu, br, r);  // block row of block k + 1
-        if (g == G - 1) next = (k + 1 < k1) ? ld_stream(block_row + k + 1) : -1;
-        if (valid && next != br) {  // last block of row br
-            const int64_t row = ((int64_t)br << lr) + q;
-            if (row < m) y[row] = row_out(plain, alpha, s, beta, y + row);
+        const unsigned flags = __ballot_sync(kFull, mine != 0) & (before | (1u << lane));
+        const int dist = flags ? g - ((31 - __clz(flags)) >> lr) : g;
+        // FP64 carries the open sum through the FMAs; in FP32 the step's sum and
+        // each block's are taken apart, which keeps a long chain's rounding out
+        V sum = kSeed && g == 0 ? carry : V(0), head = V(0);
+        bool first = true;
+        int idx = row + pos;
+        auto end_row = [&](V total) {
+            if (first) {
+                first = false;
+                head = total;
+            } else {
+                put(idx, total);
+            }
+            idx++;
+        };
+        if constexpr (kSeed) {
+#pragma unroll
+            for (int u = 0; u < B; u++) {
+#pragma unroll
+                for (int e = 0; e < C; e++) sum = fma(a[u][e], xv[u][e], sum);
+                if ((eb >> u) & 1u) {
+                    end_row(sum);
+                    sum = V(0);
+                }
+            }
+        } else {
+            V part[B];
+#pragma unroll
+            for (int u = 0; u < B; u++) {
+                part[u] = V(0);
+#pragma unroll
+                for (int e = 0; e < C; e++) part[u] = fma(a[u][e], xv[u][e], part[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < B; u += 2) {  // by pairs of blocks
+                const V next = u + 1 < B ? part[u + 1 < B ? u + 1 : u] : V(0);
+                const bool end0 = (eb >> u) & 1u, end1 = u + 1 < B && ((eb >> (u + 1)) & 1u);
+                if (end0) end_row(sum + part[u]);
+                sum = end0 ? next : sum + (part[u] + next);
+                if (end1) {
+                    end_row(sum);
+                    sum = V(0);
+                }
+            }
         }
-        carry_row = __shfl_sync(0xffffffffu, br, (G - 1) << lr);
-        carry = __shfl_sync(0xffffffffu, s, ((G - 1) << lr) + q);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {  // segmented inclusive scan of the groups' open sums
+            if (!__any_sync(kFull, dist >= o)) break;
+            const V up = __shfl_up_sync(kFull, sum, o << lr);
+            if (dist >= o) sum += up;
+        }
+        const V cin = __shfl_up_sync(kFull, sum, r);
+        if (mine) {
+            if (g > 0) head += cin;
+            if (!kSeed && pos == 0) head += carry;
+            put(row + pos, head);
+        }
+        const V open = __shfl_sync(kFull, sum, ((NG - 1) << lr) + q);
+        carry = kSeed || nend > 0 ? open : carry + open;
+        row += nend;
     }
-    for (int b = rb0 + g; b < rb1; b += G) {  // empty block rows: y = beta * y
-        if (ld_stream(row_ptr + b) == ld_stream(row_ptr + b + 1)) {
-            const int64_t row = ((int64_t)b << lr) + q;
-            if (row < m) y[row] = axpby(alpha, V(0), beta, y + row);
+    if (A.nempty > 0) {  // block rows without blocks: y = beta * y, this window's share of the list
+        const int64_t i0 = A.nempty * w / A.windows, i1 = A.nempty * (w + 1) / A.windows;
+        for (int64_t t = lane; t < (i1 - i0) << lr; t += 32) {
+            const int64_t i = ((int64_t)__ldg(A.empty + i0 + (t >> lr)) << lr) + (t & (r - 1));
+            if (i < m) y[i] = beta == V(0) ? V(0) : beta * y[i];
         }
     }
 }
 
-__global__ void bsr_block_rows(int64_t mb, const int32_t *__restrict__ row_ptr, int32_t *__restrict__ block_row) {
-    for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < mb; b += (int64_t)gridDim.x * blockDim.x)
-        for (int32_t k = row_ptr[b]; k < row_ptr[b + 1]; k++) block_row[k] = (int32_t)b;
-}
-
-// warp_row[w] = the block row holding block w * per_warp (the last block row
-// starting at or before it); warp_row[0] = 0, warp_row[nwarps] = mb.
-__global__ void bsr_warp_rows(int64_t nwarps, int64_t mb, int64_t per_warp, const int32_t *__restrict__ row_ptr,
-                              int32_t *__restrict__ warp_row) {
-    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w <= nwarps; w += (int64_t)gridDim.x * blockDim.x) {
-        if (w == 0 || w == nwarps) {
-            warp_row[w] = w == 0 ? 0 : (int32_t)mb;
-            continue;
-        }
-        const int64_t k = w * per_warp;
-        int64_t lo = 0, hi = mb - 1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi + 1) >> 1;
-            if (row_ptr[mid] <= k) lo = mid;
-            else hi = mid - 1;
-        }
-        warp_row[w] = (int32_t)lo;
-    }
-}
-
-// Lane slots the thread-per-row kernel spends: every warp of 32 rows (32 / r
-// block rows) runs as many block iterations as its longest block row.
+// out[0]: lane slots the thread-per-row kernel spends (every warp of 32 rows,
+// 32 / r block rows, runs as many block iterations as its longest block row);
+// out[1]: block rows without blocks, for the stream plan.
 __global__ void bsr_row_kernel_slots(int64_t mb, int lr, const int32_t *__restrict__ row_ptr,
-                                     unsigned long long *__restrict__ slots) {
+                                     unsigned long long *__restrict__ out) {
     const int64_t per = 32 >> lr;
     const int64_t groups = (mb + per - 1) / per;
-    unsigned long long acc = 0;
+    unsigned long long acc = 0, empty = 0;
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < groups; w += (int64_t)gridDim.x * blockDim.x) {
         int32_t mx = 0;
         const int64_t b1 = min(mb, (w + 1) * per);
-        for (int64_t b = w * per; b < b1; b++) mx = max(mx, row_ptr[b + 1] - row_ptr[b]);
+        for (int64_t b = w * per; b < b1; b++) {
+            const int32_t len = row_ptr[b + 1] - row_ptr[b];
+            mx = max(mx, len);
+            empty += len == 0;
+        }
         acc += (unsigned long long)mx * (unsigned long long)per;
     }
     acc = warp_sum(acc);
-    if ((threadIdx.x & 31) == 0 && acc) atomicAdd(slots, acc);
+    empty = warp_sum(empty);
+    if ((threadIdx.x & 31) == 0) {
+        if (acc) atomicAdd(out, acc);
+        if (empty) atomicAdd(out + 1, empty);
+    }
 }
 
 int log2_exact(int64_t v) {
@@ -268,83 +373,59 @@ int log2_exact(int64_t v) {
 }
 
 // The block-stream kernel pays a segmented scan per step (about twice the
-// FP64 work of a thread whose lanes are all busy, measured); the thread-per-
-// row kernel pays for its idle lanes.  The stream kernel is chosen when the
-// thread kernel's lane slots exceed the blocks' by this factor.
+// FP64 work of a thread whose lanes are all busy); the thread-per-row kernel
+// pays for its idle lanes.  The stream kernel is chosen when the thread
+// kernel's lane slots exceed the blocks' by this factor.  Thread per row
+// against stream, 1M rows: even rows, 4x4 FP64 (banded) 58.7 / 89.0 us;
+// uneven rows, 4x4 FP32 (2M) 27.2 / 19.2.
 constexpr double kStreamWaste = 2.0;
 
-// extra_i[2]: 1 = block-stream kernel, 2 = thread-per-row kernel (decided once).
+// extra_i[2], decided once and published in one word: bits 0-1, 1 = block-stream
+// kernel, 2 = thread-per-row kernel; above them the block rows without blocks.
 sspmv_status choose_bsr_kernel(const sspmv_bsr *A, Plan *p, sspmv_stream_t s) {
     if (p->extra_i[2]) return SSPMV_OK;
     std::lock_guard<PlanMutex> guard(plan_mutex());
     if (p->extra_i[2]) return SSPMV_OK;
     const int lr = log2_exact(A->blockDim_r);
-    unsigned long long *d = nullptr, h = 0;
-    SSPMV_TRY(dalloc(&d, 1, s));
+    unsigned long long *d = nullptr, h[2] = {0, 0};
+    SSPMV_TRY(dalloc(&d, 2, s));
     auto body = [&]() -> sspmv_status {
         SSPMV_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(h), cu(s)));
         const int64_t groups = (A->mb + (32 >> lr) - 1) / (32 >> lr);
         bsr_row_kernel_slots<<<grid_for(groups, 256, (int64_t)num_sms() * 16), 256, 0, cu(s)>>>(A->mb, lr, A->row_ptr,
                                                                                               d);
         SSPMV_LAUNCH_CHECK();
-        SSPMV_CUDA_TRY(cudaMemcpyAsync(&h, d, sizeof(h), cudaMemcpyDeviceToHost, cu(s)));
+        SSPMV_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, cu(s)));
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
         return SSPMV_OK;
     };
     const sspmv_status st = body();
     dfree(d, s);
     if (st != SSPMV_OK) return st;
-    p->extra_i[2] = (double)h > kStreamWaste * (double)A->nnzb ? 1 : 2;
+    p->extra_i[2] = ((int64_t)h[1] << 2) | ((double)h[0] > kStreamWaste * (double)A->nnzb ? 1 : 2);
     return SSPMV_OK;
 }
 
-// Plan of the block-stream kernel: extra[0] = warp_row, extra[1] = block_row,
-// extra_i[0] = warps, extra_i[1] = blocks per warp.
-sspmv_status ensure_bsr_stream_plan(const sspmv_bsr *A, Plan *p, sspmv_stream_t s) {
-    if (p->extra[0]) return SSPMV_OK;
-    std::lock_guard<PlanMutex> guard(plan_mutex());
-    if (p->extra[0]) return SSPMV_OK;
-    const int lr = log2_exact(A->blockDim_r);
-    const int64_t G = 32 >> lr, nnzb = A->nnzb, mb = A->mb;
-    // enough warps to fill the GPU (48 per SM), at most 16 steps per warp
-    const int64_t steps = std::min<int64_t>(16, std::max<int64_t>(1, nnzb / (G * num_sms() * 48)));
-    const int64_t per_warp = G * steps;
-    const int64_t nwarps = std::max<int64_t>(1, (nnzb + per_warp - 1) / per_warp);
-    int32_t *wr = nullptr, *brow = nullptr;
-    SSPMV_TRY(dalloc(&wr, (size_t)nwarps + 1, s));
-    sspmv_status st = dalloc(&brow, (size_t)nnzb, s);
-    if (st != SSPMV_OK) {
-        dfree(wr, s);
-        return st;
-    }
-    bsr_warp_rows<<<grid_for(nwarps + 1, 256, (int64_t)num_sms() * 16), 256, 0, cu(s)>>>(nwarps, mb, per_warp,
-                                                                                      A->row_ptr, wr);
-    note_launch();
-    if (mb > 0) {
-        bsr_block_rows<<<grid_for(mb, 256, (int64_t)num_sms() * 16), 256, 0, cu(s)>>>(mb, A->row_ptr, brow);
-        note_launch();
-    }
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-        dfree(wr, s);
-        dfree(brow, s);
-        return fail(SSPMV_CUDA_ERROR, "bsr plan: %s", cudaGetErrorString(e));
-    }
-    p->extra_i[0] = nwarps;
-    p->extra_i[1] = per_warp;
-    p->extra[1] = brow;
-    p->extra[0] = wr;  // published last
-    return SSPMV_OK;
-}
-
-template <typename V, int CB>
+template <typename V, int C>
 sspmv_status launch_bsr_stream(const sspmv_bsr *A, Plan *p, V alpha, const V *x, V beta, V *y, sspmv_stream_t s) {
-    SSPMV_TRY(ensure_bsr_stream_plan(A, p, s));
-    const int64_t nwarps = p->extra_i[0];
-    const unsigned grid = (unsigned)((nwarps * 32 + kBlock - 1) / kBlock);
-    bsr_stream_kernel<V, CB><<<grid, kBlock, 0, cu(s)>>>(
-        nwarps, (int)A->f.num_rows, (int)A->f.num_cols, log2_exact(A->blockDim_r), (const int32_t *)p->extra[0],
-        A->row_ptr, (const int32_t *)p->extra[1], A->block_colindex, (const V *)A->block_data, x, alpha, beta, y);
+    // windows of whole steps less a block row's overhang; never split
+    const int lr = log2_exact(A->blockDim_r), step = BsrShape<V, C>::B * (32 >> lr);
+    const int64_t mean = A->mb > 0 ? (A->nnzb + A->mb - 1) / A->mb : 1;
+    const int slack = (int)std::min<int64_t>(step / 4, mean + 1);
+    const int n = window_steps(A->nnzb, step, step - slack, bsr_ctas<V, C>() * (kStreamBlock / 32));
+    const int64_t chosen = p->extra_i[2];
+    SSPMV_TRY(ensure_stream_plan(p->stream, A->mb, A->nnzb, A->row_ptr, nullptr, A->f.value_type, s,
+                                 step * n - slack, 0x7fffffff, chosen ? chosen >> 2 : -1));
+    const StreamView v = stream_view(p->stream, A->nnzb, A->block_colindex, A->block_data);
+    const size_t run = std::min<size_t>(16, C * sizeof(V));
+    const int xvec = reinterpret_cast<uintptr_t>(x) % run == 0 ? 1 : 0;
+    const int dvec = reinterpret_cast<uintptr_t>(A->block_data) % run == 0 ? 1 : 0;
+    auto go = [&](auto kernel) {
+        kernel<<<grid_for(v.windows, kStreamBlock / 32), kStreamBlock, 0, cu(s)>>>(
+            v, (int)A->f.num_rows, (int)A->f.num_cols, lr, (const V *)A->block_data, dvec, x, xvec, alpha, beta, y);
+    };
+    if (alpha == V(1) && beta == V(0)) go(bsr_stream_kernel<V, C, true>);  // y = sum
+    else go(bsr_stream_kernel<V, C, false>);
     SSPMV_LAUNCH_CHECK();
     return SSPMV_OK;
 }
@@ -355,7 +436,7 @@ sspmv_status launch_bsr_stream(const sspmv_bsr *A, Plan *p, V alpha, const V *x,
 // kernel_flag 1 is the thread-per-row kernel.
 template <typename V>
 bool try_bsr_stream(const sspmv_bsr *A, V alpha, const V *x, V beta, V *y, sspmv_stream_t s, sspmv_status *st) {
-    if (A->f.kernel_flag == 1 || A->nnzb > 0x7fffffff) return false;
+    if (A->f.kernel_flag == 1 || A->nnzb > 0x7fffffff || A->nnzb == 0) return false;
     const int lr = log2_exact(A->blockDim_r);
     if (lr < 0 || lr > 5) return false;
     if (A->blockDim_c != 1 && A->blockDim_c != 2 && A->blockDim_c != 4 && A->blockDim_c != 8 && A->blockDim_c != 16)
@@ -368,7 +449,7 @@ bool try_bsr_stream(const sspmv_bsr *A, V alpha, const V *x, V beta, V *y, sspmv
     if (A->f.kernel_flag != 2) {
         *st = choose_bsr_kernel(A, p, s);
         if (*st != SSPMV_OK) return true;
-        if (p->extra_i[2] != 1) return false;
+        if ((p->extra_i[2] & 3) != 1) return false;
     }
     switch (A->blockDim_c) {
     case 1: *st = launch_bsr_stream<V, 1>(A, p, alpha, x, beta, y, s); return true;

@@ -621,7 +621,8 @@ void free_stream_plan(StreamPlan &sp, sspmv_stream_t s) {
 }
 
 sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
-                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s, int window, int over) {
+                                const int32_t *row_map, int32_t value_type, sspmv_stream_t s, int window, int over,
+                                int64_t nempty) {
     if (sp.window) return SSPMV_OK;
     std::lock_guard<PlanMutex> g(plan_mutex());
     if (sp.window) return SSPMV_OK;
@@ -636,10 +637,14 @@ sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const in
     auto build = [&]() -> sspmv_status {
         SSPMV_TRY(dalloc(&count, 3, s));
         SSPMV_CUDA_TRY(cudaMemsetAsync(count, 0, 3 * sizeof(*count), cu(s)));
-        stream_count_rows<<<grid, 256, 0, cu(s)>>>(m, T, over, row_offset, count);
-        SSPMV_LAUNCH_CHECK();
-        SSPMV_CUDA_TRY(cudaMemcpyAsync(h, count, sizeof(h), cudaMemcpyDeviceToHost, cu(s)));
-        SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
+        if (nempty >= 0) {
+            h[0] = (unsigned long long)nempty;
+        } else {
+            stream_count_rows<<<grid, 256, 0, cu(s)>>>(m, T, over, row_offset, count);
+            SSPMV_LAUNCH_CHECK();
+            SSPMV_CUDA_TRY(cudaMemcpyAsync(h, count, sizeof(h), cudaMemcpyDeviceToHost, cu(s)));
+            SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
+        }
         q.nzrow = const_cast<int32_t *>(row_map);
         if (h[0] > 0) {
             q.nempty = (int64_t)h[0];

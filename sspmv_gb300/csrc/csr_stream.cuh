@@ -27,18 +27,21 @@ struct StreamView {
     int32_t vec = 0;  // 16-byte aligned col and val: vector loads
 };
 
-// Builds (once) the stream plan of m rows given by row_offset (m + 1
-// entries, nnz > 0); row_offset is not read after the call's work on `s`.
-// row_map: y row of each row (rows then all nonempty; null: the row itself), owned by the caller and kept as long as the plan.
 // Steps per window (1 to 5) for nnz elements in steps of `step`, the first of
 // `first` elements, and warps_per_sm warps at once.
 int window_steps(int64_t nnz, int step, int first, int warps_per_sm);
 
+// Builds (once) the stream plan of m rows given by row_offset (m + 1
+// entries, nnz > 0); row_offset is not read after the call's work on `s`.
+// row_map: y row of each row (rows then all nonempty; null: the row itself),
+// owned by the caller and kept as long as the plan.
 // window, over: elements per window and past it that its warp may read to
-// finish a row (0, -1: the stream kernel's own).
+// finish a row (0, -1: the stream kernel's own).  nempty: the rows without
+// elements where the caller has counted them and `over` leaves no row to split
+// (-1: counted here, which waits for the device).
 sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
                                 const int32_t *row_map, int32_t value_type, sspmv_stream_t s, int window = 0,
-                                int over = -1);
+                                int over = -1, int64_t nempty = -1);
 void free_stream_plan(StreamPlan &sp, sspmv_stream_t s);
 StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, const void *val);
 
