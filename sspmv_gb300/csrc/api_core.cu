@@ -153,13 +153,10 @@ Plan *get_plan(const sspmv_features *f) {
 void free_plan(sspmv_features *f, sspmv_stream_t s) {
     Plan *p = reinterpret_cast<Plan *>(f->priv);
     if (!p) return;
-    for (auto &mp : p->merge) {
-        dfree(mp.coords, s);
-        dfree(mp.carry_row, s);
-        dfree(mp.has_end, s);
-        dfree(mp.carry_val, s);
-        dfree(mp.head_val, s);
-    }
+    dfree(p->merge.carry_row, s);
+    dfree(p->merge.has_end, s);
+    dfree(p->merge.carry_val, s);
+    dfree(p->merge.head_val, s);
     free_stream_plan(p->stream, s);
     for (void *e : p->extra) dfree(e, s);
     delete p;

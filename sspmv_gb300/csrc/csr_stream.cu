@@ -99,54 +99,6 @@ struct StreamShape {
     static constexpr int kHot = KL * sizeof(V) == 16 ? 4 : 8;  // gathers of a lane in flight together
 };
 
-// Lane's 8 columns / values at e0 (zero past the last nonzero).
-__device__ __forceinline__ void load_cols8(const int32_t *__restrict__ col, uint32_t e0, uint32_t nnz, bool vec,
-                                           int (&c)[8]) {
-    if (vec && e0 + 8 <= nnz) {
-        const int4 p = __ldcs(reinterpret_cast<const int4 *>(col + e0));
-        const int4 q = __ldcs(reinterpret_cast<const int4 *>(col + e0) + 1);
-        c[0] = p.x; c[1] = p.y; c[2] = p.z; c[3] = p.w; c[4] = q.x; c[5] = q.y; c[6] = q.z; c[7] = q.w;
-        return;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) c[u] = e0 + u < nnz ? ld_stream(col + e0 + u) : 0;
-}
-
-template <typename V>
-__device__ __forceinline__ void load_vals8(const V *__restrict__ val, uint32_t e0, uint32_t nnz, bool vec,
-                                           V (&a)[8]) {
-    if (vec && e0 + 8 <= nnz) {
-        if constexpr (sizeof(V) == 8) {
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const double2 v = __ldcs(reinterpret_cast<const double2 *>(val + e0) + h);
-                a[2 * h] = v.x;
-                a[2 * h + 1] = v.y;
-            }
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const float4 v = __ldcs(reinterpret_cast<const float4 *>(val + e0) + h);
-                a[4 * h] = v.x; a[4 * h + 1] = v.y; a[4 * h + 2] = v.z; a[4 * h + 3] = v.w;
-            }
-        }
-        return;
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) a[u] = e0 + u < nnz ? ld_stream(val + e0 + u) : V(0);
-}
-
-// Bits u < N with lo <= e0 + u < hi.
-template <int N>
-__device__ __forceinline__ unsigned in_window(uint32_t e0, uint32_t lo, uint32_t hi) {
-    constexpr unsigned kAll = N == 32 ? 0xffffffffu : (1u << (N & 31)) - 1u;
-    if (e0 >= hi || e0 + N <= lo) return 0u;
-    unsigned m = kAll;
-    if (e0 < lo) m &= kAll << (lo - e0);
-    if (e0 + N > hi) m &= kAll >> (e0 + N - hi);
-    return m;
-}
-
 // End bits of the 8 G elements at e0 (a multiple of 8 G; the mask is padded
 // to whole words).
 template <int G>

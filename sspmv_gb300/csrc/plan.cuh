@@ -1,7 +1,7 @@
 // plan.cuh -- library-private per-matrix state hung off sspmv_features.priv.
 //
-// A plan caches what depends only on the sparsity structure (merge-path tile
-// coordinates, per-tile carry buffers, chosen launch shapes).  It is built on
+// A plan caches what depends only on the sparsity structure (windows of the
+// stream kernel, carry buffers, chosen launch shapes).  It is built on
 // the first SpMV of a matrix (or by the converter that made the matrix) and
 // freed by sspmv_delete_<fmt>.  Carry buffers are shared by all calls on one
 // matrix: calls on the same matrix must be ordered (one stream, or events).
@@ -12,15 +12,13 @@
 
 namespace sspmv {
 
-// Merge-path schedule over (row ends, nonzeros) for CSR-like kernels.
+// Scratch of the merge-path kernel: the pieces of rows that cross windows.
 struct MergePlan {
-    int tile_items = 0;       // merge items per CTA tile
-    int64_t num_tiles = 0;
-    int2 *coords = nullptr;   // num_tiles + 1 split points (row, nnz)
-    int32_t *carry_row = nullptr;
-    int32_t *has_end = nullptr;
-    void *carry_val = nullptr;  // num_tiles * kMaxK values
-    void *head_val = nullptr;   // num_tiles * kMaxK values
+    int64_t windows = 0;
+    int32_t *carry_row = nullptr;  // row that starts in the window and goes on past it, or -1
+    int32_t *has_end = nullptr;    // whether a row ends in the window
+    void *carry_val = nullptr;     // kMaxK values a window: sum of the row open at its end
+    void *head_val = nullptr;      // kMaxK values: sum of the first ended row, begun earlier
 };
 
 constexpr int kMaxK = 8;  // right-hand sides handled per pass
@@ -46,7 +44,7 @@ struct StreamPlan {
 struct Plan {
     int kind = 0;
     StreamPlan stream;
-    MergePlan merge[2];     // [0]: tile for k <= 4, [1]: tile for k == 8
+    MergePlan merge;
     int param = 0;          // kernel parameter set by sspmv_set_kernel (0 = library choice)
     void *extra[12] = {nullptr};  // format-specific device buffers
     int64_t extra_i[12] = {0};
@@ -60,9 +58,7 @@ PlanMutex &plan_mutex();
 Plan *get_plan(const sspmv_features *f);  // creates an empty plan if needed
 void free_plan(sspmv_features *f, sspmv_stream_t s);
 
-// Builds (once) the merge plan of a CSR-shaped structure: row_offset has m+1
-// entries and nnz = row_offset[m].
-sspmv_status ensure_merge_plan(Plan *p, int which, int64_t m, int64_t nnz, const int32_t *row_offset,
-                               int32_t value_type, sspmv_stream_t s);
+// Allocates (once) the merge-path scratch of a matrix.
+sspmv_status ensure_merge_plan(MergePlan &mp, int64_t m, int64_t nnz, int32_t value_type, sspmv_stream_t s);
 
 }  // namespace sspmv

@@ -8,16 +8,9 @@
 // the pipelined thread-per-row kernel for
 // matrices whose rows all have at most 12 nonzeros (csr_pipe_kernel).
 // kernel_flag 3: the row-block kernel for matrices whose rows are all short
-// (csr_rowblock_kernel; one launch, no fix-up).  kernel_flag 2: merge-path.
-// The (row end, nonzero)
-// merge sequence is cut into equal tiles of kTile items, so every CTA does the
-// same work whatever the row lengths (power-law rows up to 50k nonzeros and
-// empty rows alike).  A CTA stages its nonzeros' products a_ij * x_j into
-// shared memory with coalesced streaming loads, then each thread walks
-// kItems merge items and writes the rows it finishes.  Row pieces that cross
-// thread boundaries are joined by a block-wide segmented scan; rows that cross
-// tile boundaries leave (row, partial) carries in the plan and are finished by
-// a second kernel, in a fixed order, so results are deterministic.
+// (csr_rowblock_kernel; one launch, no fix-up).  kernel_flag 2: merge-path
+// (csr_merge_kernel), which needs no plan: also the allocation-free entry
+// point's kernel.
 //
 // kernel_flag 1: vector-per-row kernel, `lanes` threads per row (2..32,
 // chosen from the mean row length, or set by the autotuner).
@@ -39,234 +32,263 @@ namespace {
 
 constexpr int kBlock = 256;
 
-template <int K>
-struct MergeShape {
-    static constexpr int items = K <= 4 ? 8 : 4;     // merge items per thread
-    static constexpr int tile = kBlock * items;       // 2048 or 1024
-    static constexpr int which = K <= 4 ? 0 : 1;
-};
+// --------------------------------------------------------- merge path --
+// The (row end, nonzero) merge sequence cut into windows of kMergeItems items,
+// one per warp, whatever the row lengths; no plan: a warp finds its own start
+// (a 33-way search of row_offset, four dependent loads for 500k rows, hidden
+// by the other warps' gathers), turns the row ends of its window into end bits
+// and a row list in shared memory, and then runs steps of 256 nonzeros as the
+// stream kernel does -- 8 consecutive nonzeros a lane with all loads in flight,
+// one segmented scan of the open sums a step.  A row that crosses windows
+// leaves its pieces and is finished by a second kernel in a fixed order.  The
+// order of a row's additions depends on row_offset alone, not on K.
+// 8M nonzeros of power-law rows, 5% of them empty, K = 1: FP32 43.6 us + 7.4
+// for the second kernel (tiles of 2048 items staged in shared memory by 256
+// threads, split points from a kernel of their own: 12.6 + 48.7 + 8.8), the
+// whole call in FP64 100 -> 70 us; K = 8 on 200k rows, FP64, 331 -> 134 with
+// the scratch allocated for the call.  The gathers alone take 28 us: the rest
+// is shared-memory and shuffle work queued behind them and the row ends' round
+// trip.  Four steps a window measured the same.
+constexpr int kMergeBlock = 64;
+constexpr int kMergeWarps = kMergeBlock / 32;
+constexpr int kMergeSteps = 2;
+constexpr int kMergeItems = 256 * kMergeSteps - 8;  // its nonzeros, from an 8-aligned one on, fit the steps
 
-__global__ void merge_path_search(int64_t num_tiles, int tile_items, int m, int nnz,
-                                  const int32_t *__restrict__ row_offset, int2 *__restrict__ coords) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t > num_tiles) return;
-    int64_t total = (int64_t)m + nnz;
-    int64_t d = t * tile_items;
-    if (d > total) d = total;
-    int64_t lo = d - nnz > 0 ? d - nnz : 0;
-    int64_t hi = d < m ? d : m;
-    while (lo < hi) {
-        int64_t p = (lo + hi) >> 1;
-        if ((int64_t)row_offset[p + 1] <= d - p - 1) lo = p + 1;
-        else hi = p;
-    }
-    coords[t] = make_int2((int)lo, (int)(d - lo));
+inline int64_t merge_windows(int64_t m, int64_t nnz) {
+    return std::max<int64_t>((m + nnz + kMergeItems - 1) / kMergeItems, 1);
 }
 
+// Resident CTAs per SM the register budget is set for: K = 1, 2M rows, FP32, 20
+// (which spills) / 18 / 16 CTAs 178 / 157 / 160 us.
 template <typename V, int K>
-struct alignas(16) VecK {
-    V v[K];
-};
+constexpr int merge_ctas() {
+    return K == 1 ? (sizeof(V) == 8 ? 14 : 18) : K <= 4 ? 10 : 7;
+}
 
-// One merge-path tile (split points c0, c1) of one matrix; t indexes the
-// per-tile carry slots.  Used by the single-matrix kernel (one tile per CTA)
-// and by the batched serving kernel (a CTA loops over tiles of many
-// requests); the leading barrier makes back-to-back calls safe.
-template <typename V, int K>
-__device__ __forceinline__ void merge_tile(
-    int m, const int32_t *__restrict__ row_offset, const int32_t *__restrict__ col_index,
-    const V *__restrict__ values, const V *__restrict__ x, int64_t ldx, V alpha, V beta,
-    V *__restrict__ y, int64_t ldy, const int2 c0, const int2 c1, const int64_t t, int32_t *__restrict__ carry_row,
-    int32_t *__restrict__ has_end, V *__restrict__ carry_val, V *__restrict__ head_val,
-    unsigned char *__restrict__ smem_raw) {
-    constexpr int kItems = MergeShape<K>::items;
-    constexpr int kTile = MergeShape<K>::tile;
-    constexpr int kWarps = kBlock / 32;
-    V *s_prod = reinterpret_cast<V *>(smem_raw);                     // kTile * K
-    int *s_rowend = reinterpret_cast<int *>(s_prod + kTile * K);      // kTile + 1
-    __shared__ int s_wkey[kWarps];
-    __shared__ V s_wval[kWarps][K];
-    __shared__ V s_wpref[kWarps][K];
-    __shared__ V s_full[kBlock][K];
-    __shared__ int s_row0_start;
-    __syncthreads();
+// Rows whose end is among the first d items of the merge sequence (the warp's
+// lanes together): the smallest p with row_offset[p + 1] + p >= d.
+__device__ __forceinline__ int merge_split(const int32_t *__restrict__ row_offset, int64_t m, int64_t nnz, int64_t d,
+                                           int lane) {
+    int64_t lo = d > nnz ? d - nnz : 0, hi = d < m ? d : m;
+    while (lo < hi) {  // warp-uniform
+        const int64_t step = (hi - lo + 31) >> 5, p = lo + (lane + 1) * step - 1;
+        const unsigned ended =
+            __ballot_sync(0xffffffffu, p < hi && (int64_t)ld_x(row_offset + (p < hi ? p + 1 : 0)) + p < d);
+        const int64_t next = lo + __popc(ended) * step;
+        hi = min(hi, next + step - 1);
+        lo = min(next, hi);
+    }
+    return (int)lo;
+}
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int i0 = c0.x, j0 = c0.y;
-    const int nrows = c1.x - i0, nnzs = c1.y - j0;
+template <typename V, int K, bool PLAIN>
+__global__ void __launch_bounds__(kMergeBlock, (merge_ctas<V, K>())) csr_merge_kernel(
+    int64_t windows, int m, int nnz, const int32_t *__restrict__ row_offset, const int32_t *__restrict__ col_index,
+    const V *__restrict__ values, int vec, const V *__restrict__ x, int64_t ldx, int xvec, V alpha, V beta,
+    V *__restrict__ y, int64_t ldy, int32_t *__restrict__ carry_row, int32_t *__restrict__ has_end,
+    V *__restrict__ carry_val, V *__restrict__ head_val) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr bool kSeed = sizeof(V) == 8;  // as the stream kernel: FP32 adds the carry apart
+    constexpr int kHot = K == 1 ? 8 : K == 2 ? 4 : 2;  // gathers of a lane in flight together
+    __shared__ uint32_t s_ends[kMergeWarps][8 * kMergeSteps];
+    __shared__ unsigned short s_row[kMergeWarps][kMergeItems];
+    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t w = (int64_t)blockIdx.x * kMergeWarps + wi;
+    if (w >= windows) return;  // warp-uniform
+    uint32_t *ends = s_ends[wi];
+    unsigned short *rows = s_row[wi];
+    if (lane < 8 * kMergeSteps) ends[lane] = 0;
+    const int64_t d0 = w * kMergeItems, d1 = min(d0 + kMergeItems, (int64_t)m + nnz);
+    const int i0 = merge_split(row_offset, m, nnz, d0, lane);
+    const int j0 = (int)(d0 - i0), b = j0 & ~7;
+    __syncwarp();
 
-    // ---- stage row ends and products (coalesced, streaming) ----
-    // nrows + nnzs <= kTile = kBlock * kItems, so every thread owns at most
-    // kItems nonzeros and kItems row ends; all of its loads are issued before
-    // any is consumed (kItems independent chains in flight per thread).
-    {
-        int cidx[kItems];
-        V aval[kItems];
+    // rows that end in the window: end bits and row of the nonempty ones
+    int nr = 0, nne = 0, open_start;
+    bool head_split = false;  // the first nonempty one began in an earlier window
+    for (int base = 0, prev = row_offset[i0];; base += 32) {
+        const int64_t p = (int64_t)i0 + base + lane;
+        const int re = p < m ? ld_x(row_offset + p + 1) : 0;
+        const bool ended = p < m && re + p < d1;
+        int rs = __shfl_up_sync(kFull, re, 1);
+        if (lane == 0) rs = prev;
+        const bool some = ended && re > max(rs, j0);
+        const unsigned eb = __ballot_sync(kFull, ended), sb = __ballot_sync(kFull, some);
+        if (some) {
+            const int pos = re - 1 - b;
+            atomicOr(&ends[pos >> 5], 1u << (pos & 31));
+            rows[nne + __popc(sb & ((1u << lane) - 1u))] = (unsigned short)(base + lane);
+        } else if (ended) {
+            if (rs < j0) {  // all of the first row lies in earlier windows
 #pragma unroll
-        for (int u = 0; u < kItems; u++) {
-            const int k = tid + u * kBlock;
-            cidx[u] = 0;
-            aval[u] = V(0);
-            if (k < nnzs) {
-                cidx[u] = ld_stream(col_index + j0 + k);
-                aval[u] = ld_stream(values + j0 + k);
+                for (int q = 0; q < K; q++) head_val[w * K + q] = V(0);
+            } else {  // an empty row
+                V *yp = y + p * ldy;
+#pragma unroll
+                for (int q = 0; q < K; q++) yp[q] = beta == V(0) ? V(0) : beta * yp[q];
             }
         }
-        int rend[kItems];
-#pragma unroll
-        for (int u = 0; u < kItems; u++) {
-            const int k = tid + u * kBlock;
-            rend[u] = k < nrows ? ld_stream(row_offset + i0 + 1 + k) : 0;
+        if (base == 0) head_split = __ballot_sync(kFull, some && rs < j0) & 1u;
+        nr += __popc(eb);
+        nne += __popc(sb);
+        if (eb != kFull) {
+            open_start = __shfl_sync(kFull, rs, __popc(eb));
+            break;
         }
-        if (tid == 0) s_row0_start = i0 < m ? row_offset[i0] : 0;
-#pragma unroll
-        for (int u = 0; u < kItems; u++) {
-            const int k = tid + u * kBlock;
-            if (k < nnzs) {
-                const V *xp = x + (int64_t)cidx[u] * ldx;
-#pragma unroll
-                for (int r = 0; r < K; r++) s_prod[k * K + r] = aval[u] * ld_x(xp + r);
-            }
-            if (k < nrows) s_rowend[k] = rend[u];
-        }
+        prev = __shfl_sync(kFull, re, 31);
     }
-    __syncthreads();
+    const int j1 = (int)(d1 - i0 - nr);
+    if (lane == 0) {
+        carry_row[w] = i0 + nr < m && open_start >= j0 && open_start < j1 ? i0 + nr : -1;
+        has_end[w] = nr > 0;
+    }
+    __syncwarp();
 
-    // ---- per-thread merge over kItems items ----
-    const int total = nrows + nnzs;
-    const int d = min(tid * kItems, total);
-    int lo = max(d - nnzs, 0), hi = min(d, nrows);
-    while (lo < hi) {
-        int p = (lo + hi) >> 1;
-        if (s_rowend[p] <= j0 + d - p - 1) lo = p + 1;
-        else hi = p;
-    }
-    int ti = lo, tj = d - lo;
-    V sum[K];
+    V carry[K];  // the open row's sum over the earlier steps
 #pragma unroll
-    for (int r = 0; r < K; r++) sum[r] = V(0);
-    int first_row = -1;
-    V first_val[K];
+    for (int q = 0; q < K; q++) carry[q] = V(0);
+    int row = 0;  // ordinal among the window's nonempty rows of the first not yet finished
+    auto finished = [&](int idx, const V(&sum)[K]) {
+        V *yp = y + ((int64_t)i0 + rows[idx]) * ldy;
 #pragma unroll
-    for (int r = 0; r < K; r++) first_val[r] = V(0);
+        for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, sum[q], beta, yp + q);
+    };
+    for (int e = j0 < j1 ? b : j1; e < j1; e += 256) {  // warp-uniform
+        const uint32_t e0 = (uint32_t)e + 8u * lane;
+        const unsigned in = in_window<8>(e0, j0, j1);
+        int c[8];
+        V a[8];
+        if (in) {
+            load_cols8(col_index, e0, nnz, vec != 0, c);
+            load_vals8<V>(values, e0, nnz, vec != 0, a);
+        }
+        const unsigned ebits = (ends[(e0 - b) >> 5] >> ((e0 - b) & 31)) & 0xffu;
+        const int mine = __popc(ebits);
+        const unsigned before = (1u << lane) - 1u;
+        int pos = 0, nend = 0;  // rows ended in the lanes before this one, and in the step
 #pragma unroll
-    for (int s = 0; s < kItems; s++) {
-        if (ti < nrows && (tj >= nnzs || s_rowend[ti] <= j0 + tj)) {
-            if (first_row < 0) {
-                first_row = ti;
+        for (int bit = 0; bit < 4; bit++) {
+            const unsigned f = __ballot_sync(kFull, (mine >> bit) & 1);
+            pos += __popc(f & before) << bit;
+            nend += __popc(f) << bit;
+        }
+        const unsigned flags = __ballot_sync(kFull, mine != 0) & (before | (1u << lane));
+        const int dist = flags ? lane - (31 - __clz(flags)) : lane;
+        V sum[K], head[K];
 #pragma unroll
-                for (int r = 0; r < K; r++) first_val[r] = sum[r];
+        for (int q = 0; q < K; q++) {
+            sum[q] = kSeed && lane == 0 ? carry[q] : V(0);
+            head[q] = V(0);
+        }
+        bool first = true;
+        int idx = row + pos;
+#pragma unroll
+        for (int h = 0; h < 8; h += kHot) {
+            V xv[kHot][K];
+            if (in) {
+#pragma unroll
+                for (int u = 0; u < kHot; u++) ld_xrow<V, K>(x, c[h + u], ldx, xvec != 0, xv[u]);
+            }
+            if (in != 0xffu) {  // other windows' elements: theirs may be Inf or NaN
+#pragma unroll
+                for (int u = 0; u < kHot; u++)
+                    if (!((in >> (h + u)) & 1u)) {
+                        a[h + u] = V(0);
+#pragma unroll
+                        for (int q = 0; q < K; q++) xv[u][q] = V(0);
+                    }
+            }
+#pragma unroll
+            for (int u = 0; u < kHot; u++) {
+#pragma unroll
+                for (int q = 0; q < K; q++) sum[q] = fma(a[h + u], xv[u][q], sum[q]);
+                if ((ebits >> (h + u)) & 1u) {
+                    if (first) {
+                        first = false;
+#pragma unroll
+                        for (int q = 0; q < K; q++) head[q] = sum[q];
+                    } else {
+                        finished(idx, sum);
+                    }
+                    idx++;
+#pragma unroll
+                    for (int q = 0; q < K; q++) sum[q] = V(0);
+                }
+            }
+        }
+        // segmented inclusive scan of the lanes' open sums
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            if (!__any_sync(kFull, dist >= o)) break;
+#pragma unroll
+            for (int q = 0; q < K; q++) {
+                const V up = __shfl_up_sync(kFull, sum[q], o);
+                if (dist >= o) sum[q] += up;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            const V cin = __shfl_up_sync(kFull, sum[q], 1), last = __shfl_sync(kFull, sum[q], 31);
+            if (lane > 0) head[q] += cin;
+            if (!kSeed && pos == 0) head[q] += carry[q];
+            carry[q] = kSeed || nend > 0 ? last : carry[q] + last;
+        }
+        if (mine) {
+            if (head_split && pos == 0) {
+#pragma unroll
+                for (int q = 0; q < K; q++) head_val[w * K + q] = head[q];
             } else {
-                V *yp = y + (int64_t)(i0 + ti) * ldy;
-#pragma unroll
-                for (int r = 0; r < K; r++) yp[r] = axpby(alpha, sum[r], beta, yp + r);
+                finished(row + pos, head);
             }
-#pragma unroll
-            for (int r = 0; r < K; r++) sum[r] = V(0);
-            ti++;
-        } else if (tj < nnzs) {
-#pragma unroll
-            for (int r = 0; r < K; r++) sum[r] += s_prod[tj * K + r];
-            tj++;
         }
+        if (nend > 0) head_split = false;
+        row += nend;
     }
-
-    // ---- block-wide segmented inclusive scan of carry-outs keyed by row ----
-    int key = i0 + ti;
-    const int key_up = __shfl_up_sync(0xffffffffu, key, 1);  // every lane shuffles (full mask)
-    const int span = unflagged_run(lane == 0 || key_up != key);
+    if (lane == 0) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        if (o > span) break;  // warp-uniform
-        int k2 = __shfl_up_sync(0xffffffffu, key, o);
-        V v2[K];
-#pragma unroll
-        for (int r = 0; r < K; r++) v2[r] = __shfl_up_sync(0xffffffffu, sum[r], o);
-        if (lane >= o && k2 == key) {
-#pragma unroll
-            for (int r = 0; r < K; r++) sum[r] += v2[r];
-        }
-    }
-    if (lane == 31) {
-        s_wkey[warp] = key;
-#pragma unroll
-        for (int r = 0; r < K; r++) s_wval[warp][r] = sum[r];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 0; w < kWarps; w++) {
-            bool join = w > 0 && s_wkey[w] == s_wkey[w - 1];
-#pragma unroll
-            for (int r = 0; r < K; r++) s_wpref[w][r] = s_wval[w][r] + (join ? s_wpref[w - 1][r] : V(0));
-        }
-    }
-    __syncthreads();
-    if (warp > 0 && key == s_wkey[warp - 1]) {
-#pragma unroll
-        for (int r = 0; r < K; r++) sum[r] += s_wpref[warp - 1][r];
-    }
-#pragma unroll
-    for (int r = 0; r < K; r++) s_full[tid][r] = sum[r];
-    __syncthreads();
-
-    if (first_row >= 0) {
-        V tot[K];
-#pragma unroll
-        for (int r = 0; r < K; r++) tot[r] = first_val[r] + (tid > 0 ? s_full[tid - 1][r] : V(0));
-        if (first_row == 0 && s_row0_start < j0) {
-            V *hp = head_val + t * kMaxK;
-#pragma unroll
-            for (int r = 0; r < K; r++) hp[r] = tot[r];
-        } else {
-            V *yp = y + (int64_t)(i0 + first_row) * ldy;
-#pragma unroll
-            for (int r = 0; r < K; r++) yp[r] = axpby(alpha, tot[r], beta, yp + r);
-        }
-    }
-    if (tid == kBlock - 1) {
-        carry_row[t] = key;
-        has_end[t] = nrows > 0;
-        V *cp = carry_val + t * kMaxK;
-#pragma unroll
-        for (int r = 0; r < K; r++) cp[r] = sum[r];
+        for (int q = 0; q < K; q++) carry_val[w * K + q] = carry[q];
     }
 }
 
+// Finishes the rows that cross windows: the window where such a row starts
+// (carry_row >= 0) adds the following windows' pieces in order.
 template <typename V, int K>
-__global__ void __launch_bounds__(kBlock) csr_merge_kernel(
-    int m, const int32_t *__restrict__ row_offset, const int32_t *__restrict__ col_index,
-    const V *__restrict__ values, const V *__restrict__ x, int64_t ldx, V alpha, V beta,
-    V *__restrict__ y, int64_t ldy, const int2 *__restrict__ coords, int32_t *__restrict__ carry_row,
-    int32_t *__restrict__ has_end, V *__restrict__ carry_val, V *__restrict__ head_val) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int64_t t = blockIdx.x;
-    merge_tile<V, K>(m, row_offset, col_index, values, x, ldx, alpha, beta, y, ldy, coords[t], coords[t + 1], t,
-                     carry_row, has_end, carry_val, head_val, smem_raw);
-}
-
-// Finishes rows that cross tile boundaries: the tile where such a row starts
-// owns it and adds the following tiles' pieces in order.
-template <typename V, int K>
-__global__ void csr_merge_fixup(int64_t num_tiles, int m, const int32_t *__restrict__ row_offset,
-                                const int2 *__restrict__ coords, const int32_t *__restrict__ carry_row,
+__global__ void csr_merge_fixup(int64_t windows, const int32_t *__restrict__ carry_row,
                                 const int32_t *__restrict__ has_end, const V *__restrict__ carry_val,
-                                const V *__restrict__ head_val, V alpha, V beta, V *__restrict__ y,
-                                int64_t ldy) {
+                                const V *__restrict__ head_val, V alpha, V beta, V *__restrict__ y, int64_t ldy) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t - (threadIdx.x & 31) >= num_tiles) return;  // whole warp past the end
-    const int r = t < num_tiles ? carry_row[t] : m;
-    bool mine = false;
-    if (r < m) {
-        const int rs = row_offset[r];
-        mine = rs >= coords[t].y && rs < coords[t + 1].y;  // the row starts in tile t
-    }
+    if (t - (threadIdx.x & 31) >= windows) return;  // whole warp past the end
+    const int r = t < windows ? carry_row[t] : -1;
     V tot[K];
-    chain_sum<V, K>(mine, t, num_tiles, 0, has_end, carry_val, head_val, tot);
-    if (mine) {
+    chain_sum<V, K, K>(r >= 0, t, windows, 0, has_end, carry_val, head_val, tot);
+    if (r >= 0) {
         V *yp = y + (int64_t)r * ldy;
 #pragma unroll
         for (int q = 0; q < K; q++) yp[q] = axpby(alpha, tot[q], beta, yp + q);
     }
+}
+
+// y = alpha A x + beta y with the pieces of rows that cross windows in q
+// (arrays of q.windows entries, the values K apart).
+template <typename V, int K>
+sspmv_status run_merge(const sspmv_csr *A, const MergePlan &q, V alpha, const V *x, int64_t ldx, V beta, V *y,
+                       int64_t ldy, sspmv_stream_t s) {
+    const int vec = ((reinterpret_cast<uintptr_t>(A->col_index) | reinterpret_cast<uintptr_t>(A->values)) & 15) == 0;
+    auto go = [&](auto kernel) {
+        kernel<<<grid_for(q.windows, kMergeWarps), kMergeBlock, 0, cu(s)>>>(
+            q.windows, (int)A->f.num_rows, (int)A->f.num_nnzs, A->row_offset, A->col_index, (const V *)A->values, vec,
+            x, ldx, xrow_vec(x, ldx, sizeof(V), K), alpha, beta, y, ldy, q.carry_row, q.has_end, (V *)q.carry_val,
+            (V *)q.head_val);
+    };
+    if (alpha == V(1) && beta == V(0)) go(csr_merge_kernel<V, K, true>);  // y = sum
+    else go(csr_merge_kernel<V, K, false>);
+    SSPMV_LAUNCH_CHECK();
+    if (q.windows > 1) {
+        csr_merge_fixup<V, K><<<grid_for(q.windows, 256), 256, 0, cu(s)>>>(
+            q.windows, q.carry_row, q.has_end, (const V *)q.carry_val, (const V *)q.head_val, alpha, beta, y, ldy);
+        SSPMV_LAUNCH_CHECK();
+    }
+    return SSPMV_OK;
 }
 
 constexpr int kVecHoist = 6;
@@ -361,27 +383,8 @@ __global__ void __launch_bounds__(kBlock, (VS == 1 && K == 1) ? (sizeof(V) == 4 
 template <typename V, int K>
 sspmv_status launch_merge(const sspmv_csr *A, Plan *p, V alpha, const V *x, int64_t ldx, V beta, V *y,
                           int64_t ldy, sspmv_stream_t s) {
-    constexpr int which = MergeShape<K>::which;
-    SSPMV_TRY(ensure_merge_plan(p, which, A->f.num_rows, A->f.num_nnzs, A->row_offset, A->f.value_type, s));
-    MergePlan &mp = p->merge[which];
-    const size_t smem = (size_t)MergeShape<K>::tile * K * sizeof(V) + ((size_t)MergeShape<K>::tile + 1) * 4;
-    static std::atomic<bool> attr_set{false};  // set after the attribute call returns
-    if (!attr_set.load(std::memory_order_acquire)) {
-        SSPMV_CUDA_TRY(cudaFuncSetAttribute(csr_merge_kernel<V, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
-        attr_set.store(true, std::memory_order_release);
-    }
-    csr_merge_kernel<V, K><<<(unsigned)mp.num_tiles, kBlock, smem, cu(s)>>>(
-        (int)A->f.num_rows, A->row_offset, A->col_index, (const V *)A->values, x, ldx, alpha, beta, y, ldy,
-        mp.coords, mp.carry_row, mp.has_end, (V *)mp.carry_val, (V *)mp.head_val);
-    SSPMV_LAUNCH_CHECK();
-    if (mp.num_tiles > 1) {
-        csr_merge_fixup<V, K><<<grid_for(mp.num_tiles, 256), 256, 0, cu(s)>>>(
-            mp.num_tiles, (int)A->f.num_rows, A->row_offset, mp.coords, mp.carry_row, mp.has_end,
-            (const V *)mp.carry_val, (const V *)mp.head_val, alpha, beta, y, ldy);
-        SSPMV_LAUNCH_CHECK();
-    }
-    return SSPMV_OK;
+    SSPMV_TRY(ensure_merge_plan(p->merge, A->f.num_rows, A->f.num_nnzs, A->f.value_type, s));
+    return run_merge<V, K>(A, p->merge, alpha, x, ldx, beta, y, ldy, s);
 }
 
 template <typename V, int K, int VS>
@@ -825,27 +828,26 @@ sspmv_status spmm_csr_impl(double alpha, const sspmv_csr *A, int32_t k, const vo
     });
 }
 
-sspmv_status ensure_merge_plan(Plan *p, int which, int64_t m, int64_t nnz, const int32_t *row_offset,
-                               int32_t value_type, sspmv_stream_t s) {
-    MergePlan &mp = p->merge[which];
-    if (mp.coords) return SSPMV_OK;
+sspmv_status ensure_merge_plan(MergePlan &mp, int64_t m, int64_t nnz, int32_t value_type, sspmv_stream_t s) {
+    if (mp.windows) return SSPMV_OK;
     std::lock_guard<PlanMutex> g(plan_mutex());
-    if (mp.coords) return SSPMV_OK;
-    const int tile = which == 0 ? MergeShape<1>::tile : MergeShape<8>::tile;
-    const int64_t tiles = (m + nnz + tile - 1) / tile;
-    const int64_t nt = tiles > 0 ? tiles : 1;
+    if (mp.windows) return SSPMV_OK;
     MergePlan q;
-    q.tile_items = tile;
-    q.num_tiles = nt;
-    const size_t vs = vsize(value_type);
-    SSPMV_TRY(dalloc(&q.coords, (size_t)nt + 1, s));
-    SSPMV_TRY(dalloc(&q.carry_row, (size_t)nt, s));
-    SSPMV_TRY(dalloc(&q.has_end, (size_t)nt, s));
-    SSPMV_TRY(dalloc((unsigned char **)&q.carry_val, (size_t)nt * kMaxK * vs, s));
-    SSPMV_TRY(dalloc((unsigned char **)&q.head_val, (size_t)nt * kMaxK * vs, s));
-    merge_path_search<<<grid_for(nt + 1, 256), 256, 0, cu(s)>>>(nt, tile, (int)m, (int)nnz, row_offset, q.coords);
-    SSPMV_LAUNCH_CHECK();
+    const int64_t nw = merge_windows(m, nnz);
+    const size_t bytes = (size_t)nw * kMaxK * vsize(value_type);
+    sspmv_status st = dalloc(&q.carry_row, (size_t)nw, s);
+    if (st == SSPMV_OK) st = dalloc(&q.has_end, (size_t)nw, s);
+    if (st == SSPMV_OK) st = dalloc((unsigned char **)&q.carry_val, bytes, s);
+    if (st == SSPMV_OK) st = dalloc((unsigned char **)&q.head_val, bytes, s);
+    if (st != SSPMV_OK) {
+        dfree(q.carry_row, s);
+        dfree(q.has_end, s);
+        dfree(q.carry_val, s);
+        return st;
+    }
     mp = q;
+    std::atomic_thread_fence(std::memory_order_release);
+    mp.windows = nw;  // published last
     return SSPMV_OK;
 }
 
@@ -880,7 +882,7 @@ extern "C" double sspmv_algorithmic_bytes_csr(const sspmv_csr *A, int32_t k, int
 // ===================================================== allocation-free CSR ===
 //
 // sspmv_LeSpMV_csr_noalloc: the merge-path CSR SpMV (one right-hand side)
-// with its scratch -- tile split points and per-tile carries -- in a fixed
+// with its scratch -- the pieces of rows that cross windows -- in a fixed
 // device array that every GPU loading this library holds until the process
 // exits, so the call itself allocates nothing.
 //
@@ -894,26 +896,24 @@ extern "C" double sspmv_algorithmic_bytes_csr(const sspmv_csr *A, int32_t k, int
 // in device memory it allocates; this one does not.
 //
 // Limits and rules:
-//  - scratch is kNoAllocScratchBytes (16 MiB); a matrix needs
-//    ceil((num_rows + num_nnzs) / 2048) tiles of kNoAllocTileBytes each, so
-//    num_rows + num_nnzs may be at most kNoAllocMaxTiles * 2048 (about 238
-//    million); larger matrices get SSPMV_INVALID_ARG.
+//  - scratch is kNoAllocScratchBytes (16 MiB), of which a window of
+//    kMergeItems merge items takes kNoAllocWindowBytes; num_rows + num_nnzs
+//    may be at most kNoAllocMaxItems (about 238 million), which is within it;
+//    larger matrices get SSPMV_INVALID_ARG.
 //  - the first call on a device looks up the array's device address
 //    (cudaGetSymbolAddress) with that device current; make that first call
 //    before any stream capture.  The address is kept per device and per
 //    context: after a cudaDeviceReset the next call looks it up again.
-//  - every call writes all the scratch it later reads (split points, carries),
+//  - every call writes all the scratch it later reads,
 //    so nothing has to be cleared between calls; but all calls share the one
 //    array: calls that overlap on the GPU (different streams, or a graph
 //    replayed concurrently) race on it and must be serialised by the caller.
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = 16u << 20;
-constexpr int kNoAllocTile = MergeShape<1>::tile;  // 2048 merge items
-// per tile: split point (int2) + carry_row + has_end + carry and head values
-// (kMaxK slots of up to 8 bytes each, the layout csr_merge_kernel uses)
-constexpr size_t kNoAllocTileBytes = sizeof(int2) + 4 + 4 + 2 * kMaxK * 8;
-constexpr int64_t kNoAllocMaxTiles = (int64_t)((kNoAllocScratchBytes - 4 * 256 - sizeof(int2)) / kNoAllocTileBytes);
+constexpr size_t kNoAllocWindowBytes = 4 + 4 + 2 * 8;  // carry_row, has_end, carry and head values
+constexpr int64_t kNoAllocMaxItems = 238594048;
+static_assert((kNoAllocMaxItems / kMergeItems + 1) * kNoAllocWindowBytes + 4 * 256 <= kNoAllocScratchBytes);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -953,43 +953,26 @@ extern "C" sspmv_status sspmv_LeSpMV_csr_noalloc(double alpha, const sspmv_csr *
     SSPMV_TRY(check_spmm_args(&A->f, 1, x, 1, y, 1));
     const int64_t m = A->f.num_rows, nnz = A->f.num_nnzs;
     if (m == 0) return SSPMV_OK;
-    const int64_t tiles = std::max<int64_t>((m + nnz + kNoAllocTile - 1) / kNoAllocTile, 1);
-    if (tiles > kNoAllocMaxTiles)
+    if (m + nnz > kNoAllocMaxItems)
         return fail(SSPMV_INVALID_ARG,
-                    "sspmv_LeSpMV_csr_noalloc: num_rows + num_nnzs = %lld exceeds the fixed scratch limit of %lld "
-                    "(%lld tiles of %d); use sspmv_LeSpMV_csr",
-                    (long long)(m + nnz), (long long)(kNoAllocMaxTiles * kNoAllocTile), (long long)kNoAllocMaxTiles,
-                    kNoAllocTile);
+                    "sspmv_LeSpMV_csr_noalloc: num_rows + num_nnzs = %lld exceeds the fixed scratch limit of %lld; "
+                    "use sspmv_LeSpMV_csr",
+                    (long long)(m + nnz), (long long)kNoAllocMaxItems);
     void *base = nullptr;
     SSPMV_TRY(noalloc_scratch(&base));
+    MergePlan q;
+    q.windows = merge_windows(m, nnz);
     unsigned char *b = (unsigned char *)base;
-    size_t off = 0;
-    int2 *coords = (int2 *)(b + off);
-    off = align256(off + (size_t)(tiles + 1) * sizeof(int2));
-    int32_t *carry_row = (int32_t *)(b + off);
-    off = align256(off + (size_t)tiles * 4);
-    int32_t *has_end = (int32_t *)(b + off);
-    off = align256(off + (size_t)tiles * 4);
-    unsigned char *carry_val = b + off;
-    off = align256(off + (size_t)tiles * kMaxK * 8);
-    unsigned char *head_val = b + off;
-    merge_path_search<<<grid_for(tiles + 1, 256), 256, 0, cu(s)>>>(tiles, kNoAllocTile, (int)m, (int)nnz,
-                                                                    A->row_offset, coords);
-    SSPMV_LAUNCH_CHECK();
+    q.carry_row = (int32_t *)b;
+    b += align256((size_t)q.windows * 4);
+    q.has_end = (int32_t *)b;
+    b += align256((size_t)q.windows * 4);
+    q.carry_val = b;
+    b += align256((size_t)q.windows * 8);
+    q.head_val = b;
     return dispatch_value(A->f.value_type, [&](auto tag) -> sspmv_status {
         using V = decltype(tag);
-        const size_t smem = (size_t)kNoAllocTile * sizeof(V) + ((size_t)kNoAllocTile + 1) * 4;
-        csr_merge_kernel<V, 1><<<(unsigned)tiles, kBlock, smem, cu(s)>>>(
-            (int)m, A->row_offset, A->col_index, (const V *)A->values, (const V *)x, 1, (V)alpha, (V)beta, (V *)y, 1,
-            coords, carry_row, has_end, (V *)carry_val, (V *)head_val);
-        SSPMV_LAUNCH_CHECK();
-        if (tiles > 1) {
-            csr_merge_fixup<V, 1><<<grid_for(tiles, 256), 256, 0, cu(s)>>>(
-                tiles, (int)m, A->row_offset, coords, carry_row, has_end, (const V *)carry_val, (const V *)head_val,
-                (V)alpha, (V)beta, (V *)y, 1);
-            SSPMV_LAUNCH_CHECK();
-        }
-        return SSPMV_OK;
+        return run_merge<V, 1>(A, q, (V)alpha, (const V *)x, 1, (V)beta, (V *)y, 1, s);
     });
 }
 
