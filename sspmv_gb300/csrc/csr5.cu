@@ -400,6 +400,7 @@ __global__ void __launch_bounds__(kC5Block, (c5_min_ctas<V, K, SIG>())) csr5_ker
     const StreamView A, const C5Shape g, const V *__restrict__ x, int64_t ldx, int xvec, V alpha, V beta,
     V *__restrict__ y, int64_t ldy, V *__restrict__ tail_val, V *__restrict__ head_val) {
     const int64_t w = (int64_t)blockIdx.x * (kC5Block / 32) + (threadIdx.x >> 5);
+    let_next_start();
     if (w >= A.windows) return;
     c5_window<V, K, SIG, PLAIN>(A, g, x, ldx, xvec, alpha, beta, y, ldy, w, tail_val, head_val);
 }

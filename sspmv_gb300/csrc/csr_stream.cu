@@ -401,9 +401,18 @@ __device__ __forceinline__ void stream_split_row(bool any, const int4 sp, const 
                                                  const StreamSlots<V> &sl, V alpha, V beta, V *__restrict__ y,
                                                  int64_t ldy) {
     const int lane = threadIdx.x & (kSplitLanes - 1);
-    V tot[K];
+    V tot[K], y_old[K];
 #pragma unroll
-    for (int q = 0; q < K; q++) tot[q] = V(0);
+    for (int q = 0; q < K; q++) tot[q] = y_old[q] = V(0);
+    V *yp = y;
+    if (any && lane == 0) {  // nothing the windows write: loaded while they still run
+        yp += (int64_t)(nzrow ? __ldg(nzrow + sp.z) : sp.z) * ldy;
+        if (beta != V(0)) {
+#pragma unroll
+            for (int q = 0; q < K; q++) y_old[q] = yp[q];
+        }
+    }
+    wait_for_previous();
     if (any) {
         for (int u = sp.x + lane; u <= sp.y; u += kSplitLanes) {
             const V *p = (u == sp.y ? sl.head_val : sl.tail_val) + (u + sl.shift) * kMaxK;
@@ -414,9 +423,8 @@ __device__ __forceinline__ void stream_split_row(bool any, const int4 sp, const 
 #pragma unroll
     for (int q = 0; q < K; q++) tot[q] = warp_sum(tot[q], kSplitLanes);
     if (any && lane == 0) {
-        V *yp = y + (int64_t)(nzrow ? __ldg(nzrow + sp.z) : sp.z) * ldy;
 #pragma unroll
-        for (int q = 0; q < K; q++) yp[q] = scaled(alpha, tot[q], beta, beta == V(0) ? V(0) : yp[q]);
+        for (int q = 0; q < K; q++) yp[q] = scaled(alpha, tot[q], beta, y_old[q]);
     }
 }
 
@@ -437,6 +445,7 @@ __global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K>())) csr_stream_
     const StreamSlots<V> sl, int xvec, int yvec) {
     const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
     __shared__ __align__(16) V s_y[kWarps][PLAIN ? 1 : StreamShape<V, K>::kStage * K];
+    let_next_start();
     if (w >= A.windows) return;
     stream_window<V, K, PLAIN>(A, x, xrow, alpha, beta, y, yrow, w, sl, xvec != 0, yvec != 0,
                                s_y[threadIdx.x >> 5]);
@@ -660,15 +669,15 @@ StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, co
 }
 
 template <typename V, int K>
-sspmv_status launch_stream_view(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta, V *y,
-                                int64_t ldy, sspmv_stream_t s) {
+sspmv_status launch_stream_windows(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta,
+                                   V *y, int64_t ldy, sspmv_stream_t s) {
     const StreamSlots<V> sl{(V *)sp.tail_val, (V *)sp.head_val, 0};
     const uint32_t xrow = (uint32_t)(ldx * (int64_t)sizeof(V)), yrow = (uint32_t)(ldy * (int64_t)sizeof(V));
     const auto kernel = alpha == V(1) && beta == V(0) ? csr_stream_kernel<V, K, true> : csr_stream_kernel<V, K, false>;
     kernel<<<grid_for(v.windows, kWarps), kBlock, 0, cu(s)>>>(v, x, xrow, alpha, beta, y, yrow, sl,
                                                               xrow_vec(x, ldx, sizeof(V), K), yrow_vec(y, ldy, K));
     SSPMV_LAUNCH_CHECK();
-    return launch_split_rows<V, K>(v, sp, alpha, beta, y, ldy, s);
+    return SSPMV_OK;
 }
 
 template <typename V, int K>
@@ -676,16 +685,16 @@ sspmv_status launch_split_rows(const StreamView &v, StreamPlan &sp, V alpha, V b
                                sspmv_stream_t s) {
     if (v.nsplit == 0) return SSPMV_OK;
     const StreamSlots<V> sl{(V *)sp.tail_val, (V *)sp.head_val, 0};
-    csr_split_kernel<V, K><<<grid_for(v.nsplit * kSplitLanes, 256), 256, 0, cu(s)>>>(v.nsplit, v.split, v.nzrow, sl,
-                                                                                      alpha, beta, y, ldy);
+    SSPMV_CUDA_TRY(launch_behind(csr_split_kernel<V, K>, grid_for(v.nsplit * kSplitLanes, 256), 256, cu(s), v.nsplit,
+                                 v.split, v.nzrow, sl, alpha, beta, y, ldy));
     SSPMV_LAUNCH_CHECK();
     return SSPMV_OK;
 }
 
-#define SSPMV_STREAM_INST(V, K)                                                                              \
-    template sspmv_status launch_stream_view<V, K>(const StreamView &, StreamPlan &, V, const V *, int64_t, V, \
-                                                   V *, int64_t, sspmv_stream_t);                            \
-    template sspmv_status launch_split_rows<V, K>(const StreamView &, StreamPlan &, V, V, V *, int64_t,          \
+#define SSPMV_STREAM_INST(V, K)                                                                                \
+    template sspmv_status launch_stream_windows<V, K>(const StreamView &, StreamPlan &, V, const V *, int64_t, \
+                                                      V, V *, int64_t, sspmv_stream_t);                        \
+    template sspmv_status launch_split_rows<V, K>(const StreamView &, StreamPlan &, V, V, V *, int64_t,        \
                                                   sspmv_stream_t);
 SSPMV_STREAM_INST(float, 1)
 SSPMV_STREAM_INST(float, 2)

@@ -70,8 +70,8 @@ constexpr int sliced_min_ctas() {
     return !FLAT ? 8 : S > 10 ? 4 : S > 8 ? 5 : S > 6 ? 6 : 7;
 }
 
-template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false>
-__global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sliced_spmv_kernel(
+template <typename V, int K, int S, bool PLAIN, bool FLAT>
+__device__ __forceinline__ void sliced_row(
     int m, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
     const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
     V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap) {
@@ -125,6 +125,18 @@ __global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sl
     V *yp = y + row * ldy;
 #pragma unroll
     for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, s[q], beta, yp + q);
+}
+
+template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false>
+__global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sliced_spmv_kernel(
+    int m, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
+    const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
+    V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap) {
+    let_next_start();
+    sliced_row<V, K, S, PLAIN, FLAT>(m, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
+    // the long rows' kernel before this one shares nothing with it; one block
+    // outlasts it, so that what follows is behind both
+    if (blockIdx.x == 0) wait_for_previous();
 }
 
 // Plan building: stored length of every stored row (padding is a suffix:
@@ -401,18 +413,24 @@ template <typename V, int K>
 sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, int64_t ldx, V beta, V *y,
                            int64_t ldy, sspmv_stream_t s) {
     const int64_t nov = p && stream_takes_strides(ldx, ldy, sizeof(V)) ? p->extra_i[1] : 0;
-    if (nov > 0)  // the long rows first: the thread pass fills in behind them
-        SSPMV_TRY((launch_stream_view<V, K>(stream_view(p->stream, p->extra_i[4], (const int32_t *)p->extra[1],
-                                                        p->extra[2]),
-                                            p->stream, alpha, x, ldx, beta, y, ldy, s)));
+    StreamView lv;
+    if (nov > 0) {  // the long rows first: the thread pass starts under their last wave
+        lv = stream_view(p->stream, p->extra_i[4], (const int32_t *)p->extra[1], p->extra[2]);
+        SSPMV_TRY((launch_stream_windows<V, K>(lv, p->stream, alpha, x, ldx, beta, y, ldy, s)));
+    }
     // A thread per row and no grid stride: a fixed grid gave the same blocks the
     // long rows at the head of every sigma slice (4M rows FP32, sigma = 4096:
     // 580 us so, 328 with blocks scheduled as they finish).
     const unsigned grid = grid_for(v.m, kBlock);
     const int xvec = xrow_vec(x, ldx, sizeof(V), K);
+    cudaError_t behind = cudaSuccess;
     auto go = [&](auto kernel) {
-        kernel<<<grid, kBlock, 0, cu(s)>>>((int)v.m, v.C, v.chunk_ptr, v.reorder, v.col, (const V *)v.val, x, ldx,
-                                           xvec, alpha, beta, y, ldy, nov > 0 ? p->extra_i[2] : kNoCap);
+        const auto args = [&](auto launch) {
+            launch((int)v.m, v.C, v.chunk_ptr, v.reorder, v.col, (const V *)v.val, x, ldx, xvec, alpha, beta, y, ldy,
+                   nov > 0 ? p->extra_i[2] : kNoCap);
+        };
+        if (nov > 0) args([&](auto... a) { behind = launch_behind(kernel, grid, kBlock, cu(s), a...); });
+        else args([&](auto... a) { kernel<<<grid, kBlock, 0, cu(s)>>>(a...); });
     };
     if constexpr (K == 1) {
         const bool plain = alpha == V(1) && beta == V(0);  // y = sum
@@ -434,8 +452,9 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
     } else {
         go(sliced_spmv_kernel<V, K, 4>);
     }
+    SSPMV_CUDA_TRY(behind);
     SSPMV_LAUNCH_CHECK();
-    return SSPMV_OK;
+    return nov > 0 ? launch_split_rows<V, K>(lv, p->stream, alpha, beta, y, ldy, s) : SSPMV_OK;
 }
 
 sspmv_status spmm_sliced(const sspmv_features *f, const SlicedView &v, double alpha, int32_t k, const void *X,

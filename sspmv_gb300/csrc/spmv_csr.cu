@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(kMergeBlock, (merge_ctas<V, K>())) csr_merge_k
     __shared__ unsigned short s_row[kMergeWarps][kMergeItems];
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t w = (int64_t)blockIdx.x * kMergeWarps + wi;
+    let_next_start();
     if (w >= windows) return;  // warp-uniform
     uint32_t *ends = s_ends[wi];
     unsigned short *rows = s_row[wi];
@@ -257,6 +258,7 @@ __global__ void csr_merge_fixup(int64_t windows, const int32_t *__restrict__ car
                                 const int32_t *__restrict__ has_end, const V *__restrict__ carry_val,
                                 const V *__restrict__ head_val, V alpha, V beta, V *__restrict__ y, int64_t ldy) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    wait_for_previous();
     if (t - (threadIdx.x & 31) >= windows) return;  // whole warp past the end
     const int r = t < windows ? carry_row[t] : -1;
     V tot[K];
@@ -284,8 +286,8 @@ sspmv_status run_merge(const sspmv_csr *A, const MergePlan &q, V alpha, const V 
     else go(csr_merge_kernel<V, K, false>);
     SSPMV_LAUNCH_CHECK();
     if (q.windows > 1) {
-        csr_merge_fixup<V, K><<<grid_for(q.windows, 256), 256, 0, cu(s)>>>(
-            q.windows, q.carry_row, q.has_end, (const V *)q.carry_val, (const V *)q.head_val, alpha, beta, y, ldy);
+        SSPMV_CUDA_TRY(launch_behind(csr_merge_fixup<V, K>, grid_for(q.windows, 256), 256, cu(s), q.windows, q.carry_row,
+                                     q.has_end, (const V *)q.carry_val, (const V *)q.head_val, alpha, beta, y, ldy));
         SSPMV_LAUNCH_CHECK();
     }
     return SSPMV_OK;
