@@ -111,17 +111,19 @@ sspmv_status exclusive_scan(const T *in, T *out, int64_t n, T *h_total, sspmv_st
 
 // ------------------------------------------------------------ radix sort --
 constexpr int kSortBlock = 256;
-constexpr int kSortRounds = 16;
-constexpr int kSortTile = kSortBlock * kSortRounds;  // 4096 keys per CTA
+// Keys per CTA: kSortBlock * rounds, as few rounds (1 to 16) as leave four CTAs a
+// SM: with 16 always, 500k keys were 123 CTAs of 16 serial rounds.  SELL-c-R of
+// 1M rows, FP32, build and product: 1629 -> 1500 us.
+constexpr int kMaxSortRounds = 16;
 constexpr int kSortWarps = kSortBlock / 32;
 
 __global__ void __launch_bounds__(kSortBlock) radix_hist(const uint64_t *__restrict__ keys, int64_t n, int shift,
-                                                       int32_t *__restrict__ hist, int64_t ntiles) {
+                                                       int32_t *__restrict__ hist, int64_t ntiles, int rounds) {
     __shared__ int32_t sh[256];
     sh[threadIdx.x] = 0;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    for (int r = 0; r < kSortRounds; r++) {
+    const int64_t base = (int64_t)blockIdx.x * kSortBlock * rounds;
+    for (int r = 0; r < rounds; r++) {
         int64_t i = base + (int64_t)r * kSortBlock + threadIdx.x;
         if (i < n) atomicAdd(&sh[(keys[i] >> shift) & 0xff], 1);
     }
@@ -133,14 +135,15 @@ __global__ void __launch_bounds__(kSortBlock) radix_hist(const uint64_t *__restr
 __global__ void __launch_bounds__(kSortBlock) radix_scatter(const uint64_t *__restrict__ kin,
                                                           const uint32_t *__restrict__ vin, uint64_t *__restrict__ kout,
                                                           uint32_t *__restrict__ vout, int64_t n, int shift,
-                                                          const int32_t *__restrict__ hist, int64_t ntiles) {
+                                                          const int32_t *__restrict__ hist, int64_t ntiles,
+                                                          int rounds) {
     __shared__ int32_t s_off[256];      // global position of the next key of digit d
     __shared__ int32_t s_cnt[kSortWarps][256];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     s_off[threadIdx.x] = hist[(int64_t)threadIdx.x * ntiles + blockIdx.x];
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
+    const int64_t base = (int64_t)blockIdx.x * kSortBlock * rounds;
     const unsigned lt_mask = (1u << lane) - 1u;
-    for (int r = 0; r < kSortRounds; r++) {
+    for (int r = 0; r < rounds; r++) {
 #pragma unroll
         for (int w = 0; w < kSortWarps; w++) s_cnt[w][threadIdx.x] = 0;
         __syncthreads();
@@ -194,7 +197,8 @@ sspmv_status exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t n, int3
 
 sspmv_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int end_bit, sspmv_stream_t s) {
     if (n <= 1 || end_bit <= 0) return SSPMV_OK;
-    const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
+    const int rounds = (int)std::min<int64_t>(kMaxSortRounds, 1 + n / (kSortBlock * 4 * (int64_t)num_sms()));
+    const int64_t tile = (int64_t)kSortBlock * rounds, ntiles = (n + tile - 1) / tile;
     uint64_t *k2 = nullptr;
     uint32_t *v2 = nullptr;
     int32_t *hist = nullptr;
@@ -204,12 +208,12 @@ sspmv_status radix_sort_pairs(uint64_t *keys, uint32_t *vals, int64_t n, int end
     uint64_t *ka = keys, *kb = k2;
     uint32_t *va = vals, *vb = v2;
     for (int shift = 0; st == SSPMV_OK && shift < end_bit; shift += 8) {
-        radix_hist<<<(unsigned)ntiles, kSortBlock, 0, cu(s)>>>(ka, n, shift, hist, ntiles);
+        radix_hist<<<(unsigned)ntiles, kSortBlock, 0, cu(s)>>>(ka, n, shift, hist, ntiles, rounds);
         note_launch();
         if (cudaGetLastError() != cudaSuccess) { st = fail(SSPMV_CUDA_ERROR, "radix_hist launch failed"); break; }
         st = exclusive_scan_i32(hist, hist, ntiles * 256, nullptr, s);
         if (st != SSPMV_OK) break;
-        radix_scatter<<<(unsigned)ntiles, kSortBlock, 0, cu(s)>>>(ka, va, kb, vb, n, shift, hist, ntiles);
+        radix_scatter<<<(unsigned)ntiles, kSortBlock, 0, cu(s)>>>(ka, va, kb, vb, n, shift, hist, ntiles, rounds);
         note_launch();
         if (cudaGetLastError() != cudaSuccess) { st = fail(SSPMV_CUDA_ERROR, "radix_scatter launch failed"); break; }
         std::swap(ka, kb);

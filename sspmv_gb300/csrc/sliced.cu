@@ -127,16 +127,19 @@ __device__ __forceinline__ void sliced_row(
     for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, s[q], beta, yp + q);
 }
 
-template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false>
+// BEHIND: launched behind the long rows' kernel (launch_behind), with which it
+// shares nothing; one block outlasts that kernel, so that what follows is behind
+// both.  Not for the forms of more slots (narrow ELL), whose loads the compiler
+// no longer keeps in flight with the wait after them (20 -> 28 us).
+template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false, bool BEHIND = false>
 __global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sliced_spmv_kernel(
     int m, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
     const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
     V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap) {
-    let_next_start();
+    if constexpr (BEHIND) let_next_start();
     sliced_row<V, K, S, PLAIN, FLAT>(m, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
-    // the long rows' kernel before this one shares nothing with it; one block
-    // outlasts it, so that what follows is behind both
-    if (blockIdx.x == 0) wait_for_previous();
+    if constexpr (BEHIND)
+        if (blockIdx.x == 0) wait_for_previous();
 }
 
 // Plan building: stored length of every stored row (padding is a suffix:
@@ -216,35 +219,47 @@ __global__ void __launch_bounds__(kBlock) cap_stats(int64_t m, const int32_t *__
     }
 }
 
-// Rows past the cap: a flag each, and their length.
-__global__ void overflow_flags(int64_t m, int64_t cap, const int32_t *__restrict__ len, int32_t *__restrict__ flag,
-                               int32_t *__restrict__ over) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
-        const bool past = (int64_t)len[i] > cap;
-        flag[i] = past;
-        over[i] = past ? len[i] : 0;
-    }
+// Rows past the cap: a one in the upper word and their length in the lower, so
+// that one scan counts both.
+__global__ void overflow_flags(int64_t m, int64_t cap, const int32_t *__restrict__ len, int64_t *__restrict__ flag) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
+        flag[i] = (int64_t)len[i] > cap ? (int64_t(1) << 32) + len[i] : 0;
 }
 
-// pos / off: the scans of flag and over.  Stored position, y row and first
-// compact element of every overflow row (optr[nov] = novf).
-__global__ void overflow_rows(int64_t m, int64_t cap, const int32_t *__restrict__ len, const int32_t *__restrict__ pos,
-                              const int32_t *__restrict__ off, const int32_t *__restrict__ reorder, int64_t nov,
-                              int32_t novf, int32_t *__restrict__ rows, int32_t *__restrict__ yrow,
-                              int32_t *__restrict__ optr) {
+// pos: the scan of the flags.  Stored position, y row and first compact element
+// of every overflow row (optr[nov] = novf).
+__global__ void overflow_rows(int64_t m, int64_t cap, const int32_t *__restrict__ len, const int64_t *__restrict__ pos,
+                              const int32_t *__restrict__ reorder, int64_t nov, int32_t novf,
+                              int32_t *__restrict__ rows, int32_t *__restrict__ yrow, int32_t *__restrict__ optr) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
         if (i == 0) optr[nov] = novf;
         if ((int64_t)len[i] <= cap) continue;
-        const int32_t o = pos[i];
+        const int32_t o = (int32_t)(pos[i] >> 32);
         rows[o] = (int32_t)i;
         yrow[o] = reorder ? reorder[i] : (int32_t)i;
-        optr[o] = off[i];
+        optr[o] = (int32_t)pos[i];
     }
 }
 
-// Copies the overflow rows out of the slab: a block per kCopyTile consecutive
-// elements of the compact arrays (so that a row of 50k elements does not keep
-// one warp), each element's row by binary search among the block's rows.
+// The last of the ascending p[0 .. n) that is <= e, p[0] being: the warp's lanes
+// together, 32 probes a step.
+template <typename T>
+__device__ __forceinline__ int64_t warp_last_le(const T *__restrict__ p, int64_t n, T e, int lane) {
+    int64_t lo = 0, hi = n - 1;
+    while (lo < hi) {  // warp-uniform
+        const int64_t step = (hi - lo + 31) >> 5, at = lo + (lane + 1) * step;
+        const int64_t next = lo + __popc(__ballot_sync(0xffffffffu, at <= hi && __ldg(p + min(at, hi)) <= e)) * step;
+        hi = min(hi, next + step - 1);
+        lo = next;
+    }
+    return lo;
+}
+
+// Copies the overflow rows out of the slab: a warp per 256 consecutive elements
+// of the compact arrays (so that a row of 50k elements does not keep one warp),
+// eight a lane with their loads in flight together; each element's row is the
+// one before's or one soon after.  3.5M elements FP64, C = 4: 43 us (51 with a
+// binary search and one element in flight at a time).
 constexpr int kCopyTile = 2048;
 
 template <typename V>
@@ -254,31 +269,47 @@ __global__ void __launch_bounds__(kBlock) copy_overflow(int64_t nov, int32_t nov
                                                         const int64_t *__restrict__ chunk_ptr,
                                                         const int32_t *__restrict__ col, const V *__restrict__ val,
                                                         int32_t *__restrict__ ocol, V *__restrict__ oval) {
-    __shared__ int s_row[2];
-    const int64_t e0 = (int64_t)blockIdx.x * kCopyTile, e1 = min(e0 + (int64_t)kCopyTile, (int64_t)novf);
-    if (threadIdx.x < 2) {  // rows of the block's first and last element
-        const int64_t e = threadIdx.x ? e1 - 1 : e0;
-        int64_t lo = 0, hi = nov - 1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi + 1) >> 1;
-            if (optr[mid] <= e) lo = mid;
-            else hi = mid - 1;
+    constexpr int U = kCopyTile / kBlock;
+    const int lane = threadIdx.x & 31;
+    const int64_t e0 = (int64_t)blockIdx.x * kCopyTile + (threadIdx.x >> 5) * (32 * U);  // the warp's elements
+    if (e0 >= novf) return;  // warp-uniform
+    const int64_t r1 = warp_last_le(optr, nov, (int32_t)(min(e0 + 32 * U, (int64_t)novf) - 1), lane);
+    int64_t r = warp_last_le(optr, r1 + 1, (int32_t)e0, lane);
+    int64_t i[U], k[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {  // the row of each element: this one's or soon after
+        const int64_t e = min(e0 + u * 32 + lane, (int64_t)novf - 1);
+        if (r < r1 && __ldg(optr + r + 1) <= e) {
+            int64_t hi = r1;
+            r++;
+            while (r < hi) {
+                const int64_t mid = (r + hi + 1) >> 1;
+                if (__ldg(optr + mid) <= e) r = mid;
+                else hi = mid - 1;
+            }
         }
-        s_row[threadIdx.x] = (int)lo;
+        k[u] = e - __ldg(optr + r);
+        i[u] = __ldg(rows + r);
     }
-    __syncthreads();
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += kBlock) {
-        int lo = s_row[0], hi = s_row[1];
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(optr + mid) <= e) lo = mid;
-            else hi = mid - 1;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t c = div_nonneg(i[u], C);
+        k[u] = __ldg(chunk_ptr + c) + k[u] * C + (i[u] - c * C);
+    }
+    int32_t oc[U];
+    V ov[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        oc[u] = col[k[u]];
+        ov[u] = val[k[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t e = e0 + u * 32 + lane;
+        if (e < novf) {
+            ocol[e] = oc[u];
+            oval[e] = ov[u];
         }
-        const int64_t i = __ldg(rows + lo);
-        const int64_t c = div_nonneg(i, C);
-        const int64_t src = __ldg(chunk_ptr + c) + (e - __ldg(optr + lo)) * C + (i - c * C);
-        ocol[e] = col[src];
-        oval[e] = val[src];
     }
 }
 
@@ -348,7 +379,8 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
     const int64_t m = v.m;
     const unsigned grid = grid_for(m, 256, (int64_t)num_sms() * 32);
     const size_t sv = vsize(f->value_type);
-    int32_t *len = nullptr, *pos = nullptr, *off = nullptr, *rows = nullptr, *optr = nullptr;
+    int32_t *len = nullptr, *rows = nullptr, *optr = nullptr;
+    int64_t *pos = nullptr;
     CapStats *dst = nullptr;
     CapList caps = kCaps;
     if (p->param > 0) caps.cap[0] = p->param;
@@ -373,7 +405,6 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
         int32_t *yrow = nullptr, *ocol = nullptr;
         unsigned char *oval = nullptr;
         SSPMV_TRY(dalloc(&pos, (size_t)m, s));
-        SSPMV_TRY(dalloc(&off, (size_t)m, s));
         SSPMV_TRY(dalloc(&rows, (size_t)nov, s));
         SSPMV_TRY(dalloc(&optr, (size_t)nov + 1, s));
         // each kept buffer belongs to the plan as soon as it exists (free_overflow)
@@ -383,11 +414,10 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
         p->extra[1] = ocol;
         SSPMV_TRY(dalloc(&oval, (size_t)novf * sv, s));
         p->extra[2] = oval;
-        overflow_flags<<<grid, 256, 0, cu(s)>>>(m, cap, len, pos, off);
+        overflow_flags<<<grid, 256, 0, cu(s)>>>(m, cap, len, pos);
         SSPMV_LAUNCH_CHECK();
-        SSPMV_TRY(exclusive_scan_i32(pos, pos, m, nullptr, s));
-        SSPMV_TRY(exclusive_scan_i32(off, off, m, nullptr, s));
-        overflow_rows<<<grid, 256, 0, cu(s)>>>(m, cap, len, pos, off, v.reorder, nov, (int32_t)novf, rows, yrow, optr);
+        SSPMV_TRY(exclusive_scan_i64(pos, pos, m, nullptr, s));
+        overflow_rows<<<grid, 256, 0, cu(s)>>>(m, cap, len, pos, v.reorder, nov, (int32_t)novf, rows, yrow, optr);
         SSPMV_LAUNCH_CHECK();
         SSPMV_TRY(dispatch_value(f->value_type, [&](auto tag) -> sspmv_status {
             using V = decltype(tag);
@@ -399,7 +429,7 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
         return ensure_stream_plan(p->stream, nov, novf, optr, yrow, f->value_type, s);
     };
     const sspmv_status st = build();
-    for (void *t : {(void *)len, (void *)pos, (void *)off, (void *)rows, (void *)optr, (void *)dst}) dfree(t, s);
+    for (void *t : {(void *)len, (void *)pos, (void *)rows, (void *)optr, (void *)dst}) dfree(t, s);
     SSPMV_TRY(st);
     p->extra_i[1] = nov;
     p->extra_i[2] = nov > 0 ? cap : kNoCap;
@@ -423,20 +453,28 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
     // 580 us so, 328 with blocks scheduled as they finish).
     const unsigned grid = grid_for(v.m, kBlock);
     const int xvec = xrow_vec(x, ldx, sizeof(V), K);
-    cudaError_t behind = cudaSuccess;
     auto go = [&](auto kernel) {
-        const auto args = [&](auto launch) {
-            launch((int)v.m, v.C, v.chunk_ptr, v.reorder, v.col, (const V *)v.val, x, ldx, xvec, alpha, beta, y, ldy,
-                   nov > 0 ? p->extra_i[2] : kNoCap);
-        };
-        if (nov > 0) args([&](auto... a) { behind = launch_behind(kernel, grid, kBlock, cu(s), a...); });
-        else args([&](auto... a) { kernel<<<grid, kBlock, 0, cu(s)>>>(a...); });
+        kernel<<<grid, kBlock, 0, cu(s)>>>((int)v.m, v.C, v.chunk_ptr, v.reorder, v.col, (const V *)v.val, x, ldx,
+                                           xvec, alpha, beta, y, ldy, nov > 0 ? p->extra_i[2] : kNoCap);
+        return cudaSuccess;
     };
+    auto go_behind = [&](auto kernel) {
+        return launch_behind(kernel, grid, kBlock, cu(s), (int)v.m, v.C, v.chunk_ptr, v.reorder, v.col,
+                             (const V *)v.val, x, ldx, xvec, alpha, beta, y, ldy, p->extra_i[2]);
+    };
+    cudaError_t launched = cudaSuccess;
     if constexpr (K == 1) {
         const bool plain = alpha == V(1) && beta == V(0);  // y = sum
         auto slots = [&](auto tag) {
             constexpr int S = decltype(tag)::value;
             constexpr bool flat = S > 4 && sizeof(V) == 4;  // only ELL takes S > 4
+            if constexpr (S == 4) {
+                if (nov > 0) {
+                    launched = plain ? go_behind(sliced_spmv_kernel<V, K, S, true, false, true>)
+                                     : go_behind(sliced_spmv_kernel<V, K, S, false, false, true>);
+                    return;
+                }
+            }
             if (plain) go(sliced_spmv_kernel<V, K, S, true, flat>);
             else go(sliced_spmv_kernel<V, K, S, false, flat>);
         };
@@ -450,9 +488,9 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
         else if (w <= 10) slots(std::integral_constant<int, 10>());
         else slots(std::integral_constant<int, 12>());
     } else {
-        go(sliced_spmv_kernel<V, K, 4>);
+        launched = nov > 0 ? go_behind(sliced_spmv_kernel<V, K, 4, false, false, true>) : go(sliced_spmv_kernel<V, K, 4>);
     }
-    SSPMV_CUDA_TRY(behind);
+    SSPMV_CUDA_TRY(launched);
     SSPMV_LAUNCH_CHECK();
     return nov > 0 ? launch_split_rows<V, K>(lv, p->stream, alpha, beta, y, ldy, s) : SSPMV_OK;
 }
@@ -491,6 +529,151 @@ __global__ void sell_sort_keys(int64_t m, int64_t sigma, int32_t maxlen, const i
         keys[p] = (uint64_t)(row / sigma) * (uint64_t)(maxlen + 1) + (uint64_t)(maxlen - len);
         vals[p] = (uint32_t)row;
     }
+}
+
+// The same order by a block per whole slices, in shared memory: slices of up to
+// kSortRows rows (shorter ones several to a block).  A stable radix sort of
+// 8-bit digits of (longest - length) over the block's rows in descending order,
+// then of the slice where there are several; a warp ranks 32 IT consecutive
+// rows, 32 at a time.  SELL-c-sigma (16384, 4) of 500k rows: 23.6 us; the
+// same by the radix sort of all rows (three passes of five launches, and the
+// longest row read back for the keys) 137.
+constexpr int kSortThreads = 1024;
+constexpr int kSortRows = 16 * kSortThreads;
+constexpr int kSortSlices = 256;  // slices a block takes at most
+
+template <int IT>
+constexpr size_t sort_smem() {
+    return (size_t)kSortThreads * IT * (sizeof(uint32_t) + sizeof(uint16_t)) + 32 * 256 * sizeof(uint16_t);
+}
+
+template <int IT>
+__global__ void __launch_bounds__(kSortThreads) sell_sort_slices(int64_t m, int64_t sigma, int64_t seg,
+                                                                 const int32_t *__restrict__ rp,
+                                                                 int32_t *__restrict__ reorder) {
+    constexpr unsigned kFull = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char sort_smem_raw[];
+    uint32_t *s_key = reinterpret_cast<uint32_t *>(sort_smem_raw);
+    uint16_t *s_idx = reinterpret_cast<uint16_t *>(s_key + kSortThreads * IT);
+    uint16_t *s_cnt = s_idx + kSortThreads * IT;  // [warp][digit]: the warp's rows, then their first place
+    __shared__ uint32_t s_first[256];             // place of the first row of a digit
+    __shared__ uint32_t s_longest;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t b0 = (int64_t)blockIdx.x * seg;
+    const int n = (int)min(seg, m - b0);
+    uint16_t *cnt = s_cnt + warp * 256;
+    uint32_t key[IT];
+    uint16_t idx[IT];
+    if (threadIdx.x == 0) s_longest = 0;
+    __syncthreads();
+    uint32_t most = 0;
+#pragma unroll
+    for (int u = 0; u < IT; u++) {
+        const int t = (warp * IT + u) * 32 + lane;
+        idx[u] = t < n ? (uint16_t)(n - 1 - t) : 0;
+        key[u] = t < n ? (uint32_t)(rp[b0 + idx[u] + 1] - rp[b0 + idx[u]]) : 0;
+        most = max(most, key[u]);
+    }
+    most = __reduce_max_sync(kFull, most);
+    if (lane == 0) atomicMax(&s_longest, most);
+    __syncthreads();
+    most = s_longest;
+#pragma unroll
+    for (int u = 0; u < IT; u++) key[u] = most - key[u];
+
+    const int digits = (39 - __clz(most | 1)) / 8;  // of the lengths; one pass more for the slices
+    for (int pass = 0; pass < digits + (seg > sigma ? 1 : 0); pass++) {
+        auto digit = [&](int u) {
+            return pass < digits ? (int)(key[u] >> (8 * pass)) & 0xff : (int)((uint32_t)idx[u] / (uint32_t)sigma);
+        };
+        for (int d = lane; d < 128; d += 32) reinterpret_cast<uint32_t *>(cnt)[d] = 0;
+        __syncwarp();
+        uint16_t rank[IT];
+#pragma unroll
+        for (int u = 0; u < IT; u++) {
+            const bool valid = (warp * IT + u) * 32 + lane < n;
+            const int d = valid ? digit(u) : 256;
+            const unsigned peers = __match_any_sync(kFull, d);
+            const int before = valid ? cnt[d] : 0;
+            rank[u] = (uint16_t)(before + __popc(peers & ((1u << lane) - 1u)));
+            __syncwarp();
+            if (valid && lane == __ffs(peers) - 1) cnt[d] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            uint32_t run = 0;
+            for (int w = 0; w < 32; w++) {
+                const uint32_t c = s_cnt[w * 256 + threadIdx.x];
+                s_cnt[w * 256 + threadIdx.x] = (uint16_t)run;
+                run += c;
+            }
+            s_first[threadIdx.x] = run;
+        }
+        __syncthreads();
+        if (warp == 0) {  // exclusive scan of the 256 digits, 8 a lane
+            uint32_t v[8], sum = 0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                v[q] = s_first[lane * 8 + q];
+                sum += v[q];
+            }
+            uint32_t inc = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t up = __shfl_up_sync(kFull, inc, o);
+                if (lane >= o) inc += up;
+            }
+            uint32_t run = inc - sum;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                s_first[lane * 8 + q] = run;
+                run += v[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < IT; u++) {
+            if ((warp * IT + u) * 32 + lane < n) {
+                const int d = digit(u);
+                const int pos = (int)s_first[d] + cnt[d] + rank[u];
+                s_key[pos] = key[u];
+                s_idx[pos] = idx[u];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < IT; u++) {
+            const int t = (warp * IT + u) * 32 + lane;
+            if (t < n) {
+                key[u] = s_key[t];
+                idx[u] = s_idx[t];
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int u = 0; u < IT; u++) {
+        const int t = (warp * IT + u) * 32 + lane;
+        if (t < n) reorder[b0 + t] = (int32_t)(b0 + idx[u]);
+    }
+}
+
+sspmv_status sort_slices(int64_t m, int64_t sigma, const int32_t *rp, int32_t *reorder, sspmv_stream_t s) {
+    const int64_t seg = sigma * std::max<int64_t>(1, std::min<int64_t>(kSortSlices, 2 * kSortThreads / sigma));
+    auto go = [&](auto tag) -> sspmv_status {
+        constexpr int IT = decltype(tag)::value;
+        SSPMV_CUDA_TRY(cudaFuncSetAttribute(sell_sort_slices<IT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)sort_smem<IT>()));
+        sell_sort_slices<IT><<<(unsigned)((m + seg - 1) / seg), kSortThreads, sort_smem<IT>(), cu(s)>>>(m, sigma, seg, rp,
+                                                                                                      reorder);
+        SSPMV_LAUNCH_CHECK();
+        return SSPMV_OK;
+    };
+    if (seg <= 2 * kSortThreads) return go(std::integral_constant<int, 2>());
+    if (seg <= 4 * kSortThreads) return go(std::integral_constant<int, 4>());
+    if (seg <= 8 * kSortThreads) return go(std::integral_constant<int, 8>());
+    return go(std::integral_constant<int, 16>());
 }
 
 __global__ void copy_u32_to_i32(int64_t n, const uint32_t *__restrict__ in, int32_t *__restrict__ out) {
@@ -542,59 +725,79 @@ __global__ void chunk_widths(int64_t nchunks, int32_t C, int32_t align, int32_t 
     }
 }
 
-// Copies the CSR rows into the slab, padding included: a block per kFillTile
-// consecutive slots, each slot's chunk by binary search among the block's
-// chunks (a chunk as wide as a 38k-nonzero row is spread over many blocks).
-// Writes are consecutive; neighbouring slots read C rows at a time, and the
-// block's 2048 / C slots of each row share their cache lines.  For chunks of
-// up to kFillChunk rows: SELL-c-sigma (16384, 4) of 500k power-law rows FP64
-// 704 us with a thread per row (the rows of 256 and more by the block that
-// holds them, all the longest in one block) after two fills, now 94 us.
+// Copies the CSR rows into the slab, padding included: a warp per 256
+// consecutive slots, eight a lane with their loads in flight together; a slot's
+// chunk is the one before's or one soon after (a chunk as wide as a 38k-nonzero
+// row is spread over many blocks).  Writes are consecutive; neighbouring slots
+// read C rows at a time, and the warp's 256 / C slots of each row share their
+// sectors.  For chunks of up to kFillChunk rows: SELL-c-sigma (16384, 4) of 500k
+// power-law rows FP64 704 us with a thread per row (the rows of 256 and more by
+// the block that holds them, all the longest in one block) after two fills, 94
+// with a binary search for each slot, now 71 (242 MB: 36 us).
 constexpr int kFillTile = 2048;
 constexpr int kFillChunk = 256;
 
 template <typename V>
-__global__ void __launch_bounds__(256) sliced_fill_slots(int64_t m, int32_t C, int64_t nchunks, int64_t total,
+__global__ void __launch_bounds__(256, 6) sliced_fill_slots(int64_t m, int32_t C, int64_t nchunks, int64_t total,
                                                          const int64_t *__restrict__ chunk_ptr,
                                                          const int32_t *__restrict__ reorder,
                                                          const int32_t *__restrict__ rp,
                                                          const int32_t *__restrict__ ci, const V *__restrict__ cv,
                                                          int32_t *__restrict__ col, V *__restrict__ val) {
-    __shared__ int64_t s_chunk[2];
-    const int64_t e0 = (int64_t)blockIdx.x * kFillTile, e1 = min(e0 + (int64_t)kFillTile, total);
-    if (threadIdx.x < 2) {  // chunks of the block's first and last slot: the last that start there or before
-        const int64_t e = threadIdx.x ? e1 - 1 : e0;
-        int64_t lo = 0, hi = nchunks - 1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi + 1) >> 1;
-            if (chunk_ptr[mid] <= e) lo = mid;
-            else hi = mid - 1;
-        }
-        s_chunk[threadIdx.x] = lo;
-    }
-    __syncthreads();
-    const int64_t c0 = s_chunk[0], c1 = s_chunk[1];
-#pragma unroll 4
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += 256) {
-        int64_t lo = c0, hi = c1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi + 1) >> 1;
-            if (__ldg(chunk_ptr + mid) <= e) lo = mid;
-            else hi = mid - 1;
-        }
-        const int64_t at = e - __ldg(chunk_ptr + lo), k = div_nonneg(at, C), i = lo * C + (at - k * C);
-        int32_t oc = -1;
-        V ov = V(0);
-        if (i < m) {
-            const int64_t r = reorder ? __ldg(reorder + i) : i;
-            const int64_t s0 = __ldg(rp + r);
-            if (s0 + k < __ldg(rp + r + 1)) {
-                oc = __ldg(ci + s0 + k);
-                ov = __ldg(cv + s0 + k);
+    constexpr int U = kFillTile / 256;
+    const int lane = threadIdx.x & 31;
+    const int64_t e0 = (int64_t)blockIdx.x * kFillTile + (threadIdx.x >> 5) * (32 * U);  // the warp's slots
+    if (e0 >= total) return;  // warp-uniform
+    const int64_t c1 = warp_last_le(chunk_ptr, nchunks, min(e0 + 32 * U, total) - 1, lane);
+    int64_t c = warp_last_le(chunk_ptr, c1 + 1, e0, lane);
+    int64_t row[U];
+    int32_t k[U];  // slot within the row; -1: no such row
+#pragma unroll
+    for (int u = 0; u < U; u++) {  // the chunk of each slot: this one's or soon after
+        const int64_t e = e0 + u * 32 + lane;
+        k[u] = -1;
+        row[u] = 0;
+        if (e < total) {
+            if (c < c1 && __ldg(chunk_ptr + c + 1) <= e) {
+                int64_t hi = c1;
+                c++;
+                while (c < hi) {
+                    const int64_t mid = (c + hi + 1) >> 1;
+                    if (__ldg(chunk_ptr + mid) <= e) c = mid;
+                    else hi = mid - 1;
+                }
+            }
+            const int64_t at = e - __ldg(chunk_ptr + c), kk = div_nonneg(at, C), i = c * C + (at - kk * C);
+            if (i < m) {
+                k[u] = (int32_t)kk;
+                row[u] = i;
             }
         }
-        col[e] = oc;
-        val[e] = ov;
+    }
+    if (reorder) {
+#pragma unroll
+        for (int u = 0; u < U; u++) row[u] = __ldg(reorder + row[u]);
+    }
+    int32_t at[U];  // nonzero of the slot, -1: padding
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int32_t s0 = __ldg(rp + row[u]), s1 = __ldg(rp + row[u] + 1);
+        at[u] = k[u] >= 0 && k[u] < s1 - s0 ? s0 + k[u] : -1;
+    }
+    int32_t oc[U];
+    V ov[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        oc[u] = __ldg(ci + max(at[u], 0));
+        ov[u] = __ldg(cv + max(at[u], 0));
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t e = e0 + u * 32 + lane;
+        if (e < total) {
+            col[e] = at[u] >= 0 ? oc[u] : -1;
+            val[e] = at[u] >= 0 ? ov[u] : V(0);
+        }
     }
 }
 
@@ -672,29 +875,35 @@ sspmv_status build_sliced(const sspmv_csr *A, int32_t C, int32_t align, int64_t 
     const int64_t m = A->f.num_rows;
     const int32_t vt = A->f.value_type;
     b.nchunks = (m + C - 1) / C;
-    int32_t maxlen = 0;
-    SSPMV_TRY(max_row_length(A->row_offset, m, &maxlen, s));
     const unsigned g = grid_for(m, 256, (int64_t)num_sms() * 16);
     sspmv_status st = SSPMV_OK;
     if (sigma > 0) {
-        uint64_t *keys = nullptr;
-        uint32_t *vals = nullptr;
         st = dalloc(&b.reorder, (size_t)m, s);
-        if (st == SSPMV_OK) st = dalloc(&keys, (size_t)m, s);
-        if (st == SSPMV_OK) st = dalloc(&vals, (size_t)m, s);
         if (st == SSPMV_OK && m > 0) {
-            sell_sort_keys<<<g, 256, 0, cu(s)>>>(m, sigma, maxlen, A->row_offset, keys, vals);
-            note_launch();
-            const uint64_t nslices = (uint64_t)((m + sigma - 1) / sigma);
-            const uint64_t maxkey = (nslices - 1) * (uint64_t)(maxlen + 1) + (uint64_t)maxlen;
-            st = radix_sort_pairs(keys, vals, m, bits_for(maxkey), s);
-            if (st == SSPMV_OK) {
-                copy_u32_to_i32<<<g, 256, 0, cu(s)>>>(m, vals, b.reorder);
-                note_launch();
+            if (sigma <= kSortRows) {
+                st = sort_slices(m, sigma, A->row_offset, b.reorder, s);
+            } else {
+                int32_t maxlen = 0;
+                uint64_t *keys = nullptr;
+                uint32_t *vals = nullptr;
+                st = max_row_length(A->row_offset, m, &maxlen, s);
+                if (st == SSPMV_OK) st = dalloc(&keys, (size_t)m, s);
+                if (st == SSPMV_OK) st = dalloc(&vals, (size_t)m, s);
+                if (st == SSPMV_OK) {
+                    sell_sort_keys<<<g, 256, 0, cu(s)>>>(m, sigma, maxlen, A->row_offset, keys, vals);
+                    note_launch();
+                    const uint64_t nslices = (uint64_t)((m + sigma - 1) / sigma);
+                    const uint64_t maxkey = (nslices - 1) * (uint64_t)(maxlen + 1) + (uint64_t)maxlen;
+                    st = radix_sort_pairs(keys, vals, m, bits_for(maxkey), s);
+                }
+                if (st == SSPMV_OK) {
+                    copy_u32_to_i32<<<g, 256, 0, cu(s)>>>(m, vals, b.reorder);
+                    note_launch();
+                }
+                dfree(keys, s);
+                dfree(vals, s);
             }
         }
-        dfree(keys, s);
-        dfree(vals, s);
         if (st != SSPMV_OK) { b.release(s); return st; }
     }
     st = dalloc(&b.width, (size_t)b.nchunks, s);
