@@ -202,6 +202,20 @@ __device__ __forceinline__ T warp_sum(T v, unsigned width = 32) {
     return v;
 }
 
+// The last of the ascending p[0 .. n) that is <= e, p[0] being: the warp's lanes
+// together, 32 probes a step.
+template <typename T>
+__device__ __forceinline__ int64_t warp_last_le(const T *__restrict__ p, int64_t n, T e, int lane) {
+    int64_t lo = 0, hi = n - 1;
+    while (lo < hi) {  // warp-uniform
+        const int64_t step = (hi - lo + 31) >> 5, at = lo + (lane + 1) * step;
+        const int64_t next = lo + __popc(__ballot_sync(0xffffffffu, at <= hi && __ldg(p + min(at, hi)) <= e)) * step;
+        hi = min(hi, next + step - 1);
+        lo = next;
+    }
+    return lo;
+}
+
 // A kernel that follows another in one call and needs its results only late, or
 // not at all: launched by launch_behind it may start once every block of the
 // kernel before it has started (that kernel calls let_next_start); what it needs

@@ -501,26 +501,22 @@ __global__ void stream_end_bits(int64_t m, const int32_t *__restrict__ rp, uint3
         }
 }
 
-// First row r with rp[r] >= e (m if none).
-__device__ __forceinline__ int first_row_from(const int32_t *__restrict__ rp, int m, int64_t e) {
-    int lo = 0, hi = m;
-    while (lo < hi) {
-        const int mid = lo + ((hi - lo) >> 1);
-        if (rp[mid] < e) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
+// First row r with rp[r] >= e (m if none): the warp's lanes together.
+__device__ __forceinline__ int first_row_from(const int32_t *__restrict__ rp, int m, int64_t e, int lane) {
+    return e > 0 ? (int)warp_last_le(rp, m, (int32_t)(e - 1), lane) + 1 : 0;
 }
 
 // Window records, and the list of split rows (in any order: each is summed
-// on its own); nsplit starts at zero.
+// on its own); nsplit starts at zero.  A warp per window, for the searches.
 __global__ void stream_windows(int64_t nw, int T, int over, int m, int64_t nnz, const int32_t *__restrict__ rp,
                                const int32_t *__restrict__ pos, int4 *__restrict__ rec, int4 *__restrict__ split,
                                unsigned long long *__restrict__ nsplit) {
-    const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= nw) return;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (w >= nw) return;  // warp-uniform
     const int64_t a = w * T, b = min(a + T, nnz);
-    const int r = first_row_from(rp, m, a), r2 = first_row_from(rp, m, b);
+    const int r = first_row_from(rp, m, a, lane), r2 = first_row_from(rp, m, b, lane);
+    if (lane != 0) return;
     auto ordinal = [&](int row) { return pos && row < m ? pos[row] : row; };
     int64_t eA = rp[r], eB;
     int first = ordinal(r), flags = 0;
@@ -627,7 +623,7 @@ sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const in
         SSPMV_TRY(dalloc(&q.rec, (size_t)nw, s));
         q.nsplit = (int64_t)h[1];
         SSPMV_TRY(dalloc(&q.split, (size_t)q.nsplit, s));
-        stream_windows<<<grid_for(nw, 128), 128, 0, cu(s)>>>(nw, T, over, (int)m, nnz, row_offset, pos, q.rec, q.split,
+        stream_windows<<<grid_for(nw, 8), 256, 0, cu(s)>>>(nw, T, over, (int)m, nnz, row_offset, pos, q.rec, q.split,
                                                              count + 2);
         SSPMV_LAUNCH_CHECK();
         if (q.nsplit > 0) {

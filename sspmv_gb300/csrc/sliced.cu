@@ -241,20 +241,6 @@ __global__ void overflow_rows(int64_t m, int64_t cap, const int32_t *__restrict_
     }
 }
 
-// The last of the ascending p[0 .. n) that is <= e, p[0] being: the warp's lanes
-// together, 32 probes a step.
-template <typename T>
-__device__ __forceinline__ int64_t warp_last_le(const T *__restrict__ p, int64_t n, T e, int lane) {
-    int64_t lo = 0, hi = n - 1;
-    while (lo < hi) {  // warp-uniform
-        const int64_t step = (hi - lo + 31) >> 5, at = lo + (lane + 1) * step;
-        const int64_t next = lo + __popc(__ballot_sync(0xffffffffu, at <= hi && __ldg(p + min(at, hi)) <= e)) * step;
-        hi = min(hi, next + step - 1);
-        lo = next;
-    }
-    return lo;
-}
-
 // Copies the overflow rows out of the slab: a warp per 256 consecutive elements
 // of the compact arrays (so that a row of 50k elements does not keep one warp),
 // eight a lane with their loads in flight together; each element's row is the
