@@ -407,7 +407,7 @@ sspmv_status coo_pass(const sspmv_coo *A, Plan *p, V alpha, const V *x, int64_t 
     if (A->f.kernel_flag != 1 && nnz > 0 && stream_takes_strides(ldx, ldy, sizeof(V))) {
         SSPMV_TRY(ensure_coo_stream_plan(A, p, s));
         return launch_stream_view<V, K>(stream_view(p->stream, nnz, A->col_index, A->values), p->stream, alpha, x, ldx,
-                                        beta, y, ldy, s);
+                                        beta, y, ldy, A->f.num_cols, s);
     }
     const int tile = CooShape<K>::tile;
     const int which = K <= 4 ? 0 : 1;

@@ -68,10 +68,10 @@ constexpr unsigned kFull = 0xffffffffu;
 // Resident CTAs per SM the register budget is set for: the best of 16 to 24
 // (FP32) and 12 to 18 (FP64) for K = 1; spills and fewer warps cost about the
 // same beyond.
-template <typename V, int K>
+template <typename V, int K, bool BIG = false>
 constexpr int stream_min_ctas() {
     if (K == 1) return sizeof(V) == 8 ? 15 : 20;
-    return sizeof(V) == 8 ? 12 : 14;
+    return BIG ? 10 : sizeof(V) == 8 ? 12 : 14;
 }
 
 // Elements per window: whole steps of 256 less what the last row may run past
@@ -82,7 +82,8 @@ int window_size(int64_t nnz, int32_t value_type) {
     return 256 * window_steps(nnz, 256, 256 - kOver, ctas * kWarps) - kOver;
 }
 
-template <typename V, int K>
+// BIG: X does not fit in L2, a gather is a random HBM access.
+template <typename V, int K, bool BIG = false>
 struct StreamShape {
     static constexpr int G = K * (int)sizeof(V) > 16 ? K * (int)sizeof(V) / 16 : 1;  // lanes per row of X
     static constexpr int KL = K / G;                                                 // columns per lane
@@ -96,7 +97,7 @@ struct StreamShape {
     // and each 8 elements are summed on their own first: long chains of adds to
     // a large sum would lose more bits than the rows' sums lose in chunks.
     static constexpr bool kSeed = sizeof(V) == 8;
-    static constexpr int kHot = KL * sizeof(V) == 16 ? 4 : 8;  // gathers of a lane in flight together
+    static constexpr int kHot = KL * sizeof(V) == 16 && !BIG ? 4 : 8;  // gathers of a lane in flight together
 };
 
 // End bits of the 8 G elements at e0 (a multiple of 8 G; the mask is padded
@@ -143,12 +144,19 @@ __device__ __forceinline__ V scaled(V alpha, V sum, V beta, V y) {
     return beta == V(0) ? alpha * sum : fma(alpha, sum, beta * y);
 }
 
-template <typename V, int KL>
+template <typename V, int KL, bool BIG = false>
 __device__ __forceinline__ void st_cols(V *__restrict__ p, bool vec, const V (&o)[KL]) {
     if constexpr (KL * sizeof(V) == 16) {
         if (vec) {
-            if constexpr (sizeof(V) == 8) *reinterpret_cast<double2 *>(p) = make_double2(o[0], o[1]);
-            else *reinterpret_cast<float4 *>(p) = make_float4(o[0], o[1], o[2], o[3]);
+            if constexpr (sizeof(V) == 8) {
+                const double2 v = make_double2(o[0], o[1]);
+                if constexpr (BIG) __stcs(reinterpret_cast<double2 *>(p), v);  // leaves L2 to X
+                else *reinterpret_cast<double2 *>(p) = v;
+            } else {
+                const float4 v = make_float4(o[0], o[1], o[2], o[3]);
+                if constexpr (BIG) __stcs(reinterpret_cast<float4 *>(p), v);
+                else *reinterpret_cast<float4 *>(p) = v;
+            }
             return;
         }
     }
@@ -166,12 +174,12 @@ struct StreamSlots {
 
 // Window w of a matrix, run by one warp.  s_y: the warp's kStage * K values of
 // shared memory (not PLAIN).
-template <typename V, int K, bool PLAIN>
+template <typename V, int K, bool PLAIN, bool BIG = false>
 __device__ __forceinline__ void stream_window(const StreamView &A, const V *__restrict__ x, uint32_t xrow, V alpha,
                                               V beta, V *__restrict__ y, uint32_t yrow, const int64_t w,
                                               const StreamSlots<V> &sl, bool xvec, bool yvec,
                                               V *__restrict__ s_y) {
-    using S = StreamShape<V, K>;
+    using S = StreamShape<V, K, BIG>;
     constexpr int G = S::G, KL = S::KL, NG = S::NG, kStep = S::kStep, kStage = S::kStage, kHot = S::kHot;
     constexpr bool kSeed = S::kSeed;
     const int lane = threadIdx.x & 31, gi = lane / G, q0 = (lane % G) * KL;
@@ -218,7 +226,7 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
         // row `idx` of the step is complete
         auto finished = [&](int idx, const V(&sum)[KL]) {
             if constexpr (PLAIN) {
-                st_cols<V, KL>(y_of(row + idx), yvec, sum);
+                st_cols<V, KL, BIG>(y_of(row + idx), yvec, sum);
             } else if (K == 1 || idx < kStage) {
                 st_cols<V, KL>(s_y + idx * K + q0, true, sum);
             } else {
@@ -226,7 +234,7 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
                 V o[KL];
 #pragma unroll
                 for (int q = 0; q < KL; q++) o[q] = scaled(alpha, sum[q], beta, beta == V(0) ? V(0) : yp[q]);
-                st_cols<V, KL>(yp, yvec, o);
+                st_cols<V, KL, BIG>(yp, yvec, o);
             }
         };
         V y_old[PLAIN ? 1 : KL];  // y of the step's first finished rows, loaded under the gathers
@@ -353,7 +361,7 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
                 for (int q = 0; q < KL; q++)
                     o[q] = scaled(alpha, s_y[i * K + q0 + q], beta,
                                   i < NG ? y_old[q] : beta == V(0) ? V(0) : yp[q]);
-                st_cols<V, KL>(yp, yvec, o);
+                st_cols<V, KL, BIG>(yp, yvec, o);
             }
             __syncwarp();
         }
@@ -439,15 +447,15 @@ __global__ void __launch_bounds__(256) csr_split_kernel(int64_t n, const int4 *_
 
 // PLAIN: alpha == 1 and beta == 0 (y = sum): row writes carry no FP64
 // multiply.
-template <typename V, int K, bool PLAIN>
-__global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K>())) csr_stream_kernel(
+template <typename V, int K, bool PLAIN, bool BIG = false>
+__global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K, BIG>())) csr_stream_kernel(
     const StreamView A, const V *__restrict__ x, uint32_t xrow, V alpha, V beta, V *__restrict__ y, uint32_t yrow,
     const StreamSlots<V> sl, int xvec, int yvec) {
     const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
     __shared__ __align__(16) V s_y[kWarps][PLAIN ? 1 : StreamShape<V, K>::kStage * K];
     let_next_start();
     if (w >= A.windows) return;
-    stream_window<V, K, PLAIN>(A, x, xrow, alpha, beta, y, yrow, w, sl, xvec != 0, yvec != 0,
+    stream_window<V, K, PLAIN, BIG>(A, x, xrow, alpha, beta, y, yrow, w, sl, xvec != 0, yvec != 0,
                                s_y[threadIdx.x >> 5]);
 }
 
@@ -664,14 +672,32 @@ StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, co
     return v;
 }
 
+// An X of more bytes than this does not stay in L2 (129 MB, less what the matrix
+// and Y take): its gathers wait for HBM, and the form with twice the gathers in
+// flight, fewer warps and Y written past L2 is the faster one (FP32, k = 8: 4.2M
+// rows 755 us, 715 so; FP64, k = 4, 4M rows: 814, 800), where with X in L2 it is
+// the slower one (2M rows FP32 231 us, 251 so).  For rows of X of 32 bytes: with
+// 64 the registers do not hold it (FP64, k = 8, 2M rows: 650, 655 so).
+constexpr int64_t kBigX = int64_t(100) << 20;
+
 template <typename V, int K>
 sspmv_status launch_stream_windows(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta,
-                                   V *y, int64_t ldy, sspmv_stream_t s) {
+                                   V *y, int64_t ldy, int64_t cols, sspmv_stream_t s) {
     const StreamSlots<V> sl{(V *)sp.tail_val, (V *)sp.head_val, 0};
     const uint32_t xrow = (uint32_t)(ldx * (int64_t)sizeof(V)), yrow = (uint32_t)(ldy * (int64_t)sizeof(V));
-    const auto kernel = alpha == V(1) && beta == V(0) ? csr_stream_kernel<V, K, true> : csr_stream_kernel<V, K, false>;
-    kernel<<<grid_for(v.windows, kWarps), kBlock, 0, cu(s)>>>(v, x, xrow, alpha, beta, y, yrow, sl,
-                                                              xrow_vec(x, ldx, sizeof(V), K), yrow_vec(y, ldy, K));
+    auto go = [&](auto kernel) {
+        kernel<<<grid_for(v.windows, kWarps), kBlock, 0, cu(s)>>>(v, x, xrow, alpha, beta, y, yrow, sl,
+                                                                  xrow_vec(x, ldx, sizeof(V), K), yrow_vec(y, ldy, K));
+    };
+    const bool plain = alpha == V(1) && beta == V(0);
+    bool big = false;
+    if constexpr (K * sizeof(V) == 32) {
+        big = cols * ldx * (int64_t)sizeof(V) > kBigX;
+        if (big && plain) go(csr_stream_kernel<V, K, true, true>);
+        else if (big) go(csr_stream_kernel<V, K, false, true>);
+    }
+    if (!big && plain) go(csr_stream_kernel<V, K, true>);
+    else if (!big) go(csr_stream_kernel<V, K, false>);
     SSPMV_LAUNCH_CHECK();
     return SSPMV_OK;
 }
@@ -689,7 +715,7 @@ sspmv_status launch_split_rows(const StreamView &v, StreamPlan &sp, V alpha, V b
 
 #define SSPMV_STREAM_INST(V, K)                                                                                \
     template sspmv_status launch_stream_windows<V, K>(const StreamView &, StreamPlan &, V, const V *, int64_t, \
-                                                      V, V *, int64_t, sspmv_stream_t);                        \
+                                                      V, V *, int64_t, int64_t, sspmv_stream_t);               \
     template sspmv_status launch_split_rows<V, K>(const StreamView &, StreamPlan &, V, V, V *, int64_t,        \
                                                   sspmv_stream_t);
 SSPMV_STREAM_INST(float, 1)

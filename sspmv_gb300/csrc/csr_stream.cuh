@@ -52,9 +52,10 @@ inline bool stream_takes_strides(int64_t ldx, int64_t ldy, size_t value_bytes) {
 
 // Y = alpha * A * X + beta * Y on the rows of the plan, K right-hand sides
 // (1, 2, 4 or 8), but for the split rows, whose pieces it leaves: one launch.
+// cols: rows of X.
 template <typename V, int K>
 sspmv_status launch_stream_windows(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta,
-                                   V *y, int64_t ldy, sspmv_stream_t s);
+                                   V *y, int64_t ldy, int64_t cols, sspmv_stream_t s);
 
 // Finishes the rows whose pieces a kernel over the plan's windows has left in
 // tail_val and head_val: one launch, none without such rows.  It follows that
@@ -65,8 +66,8 @@ sspmv_status launch_split_rows(const StreamView &v, StreamPlan &sp, V alpha, V b
 
 template <typename V, int K>
 inline sspmv_status launch_stream_view(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta,
-                                       V *y, int64_t ldy, sspmv_stream_t s) {
-    SSPMV_TRY((launch_stream_windows<V, K>(v, sp, alpha, x, ldx, beta, y, ldy, s)));
+                                       V *y, int64_t ldy, int64_t cols, sspmv_stream_t s) {
+    SSPMV_TRY((launch_stream_windows<V, K>(v, sp, alpha, x, ldx, beta, y, ldy, cols, s)));
     return launch_split_rows<V, K>(v, sp, alpha, beta, y, ldy, s);
 }
 

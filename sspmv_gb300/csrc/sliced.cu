@@ -308,6 +308,7 @@ struct SlicedView {
     const void *val;
     int64_t nchunks;  // 0: ELL
     int32_t width;    // ELL
+    int64_t cols;     // rows of X
 };
 
 // Cost model of the cap, in picoseconds of GB300 time (fitted to measured
@@ -432,7 +433,7 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
     StreamView lv;
     if (nov > 0) {  // the long rows first: the thread pass starts under their last wave
         lv = stream_view(p->stream, p->extra_i[4], (const int32_t *)p->extra[1], p->extra[2]);
-        SSPMV_TRY((launch_stream_windows<V, K>(lv, p->stream, alpha, x, ldx, beta, y, ldy, s)));
+        SSPMV_TRY((launch_stream_windows<V, K>(lv, p->stream, alpha, x, ldx, beta, y, ldy, v.cols, s)));
     }
     // A thread per row and no grid stride: a fixed grid gave the same blocks the
     // long rows at the head of every sigma slice (4M rows FP32, sigma = 4096:
@@ -1034,7 +1035,7 @@ extern "C" sspmv_status sspmv_spmm_ell(double alpha, const sspmv_ell *A, int32_t
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     Plan *p = get_plan(&A->f);
     SlicedView v{A->f.num_rows, (int32_t)std::max<int64_t>(A->f.num_rows, 1), (const int64_t *)p->extra[0], nullptr,
-                 A->col_index, A->values, 0, A->max_row_width};
+                 A->col_index, A->values, 0, A->max_row_width, A->f.num_cols};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1109,7 +1110,7 @@ extern "C" sspmv_status sspmv_spmm_sell(double alpha, const sspmv_s_ell *A, int3
                                         double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->sliceWidth,   A->chunk_ptr,   nullptr,
-                 A->col_index,  A->values,     A->chunk_num, 0};
+                 A->col_index,  A->values,     A->chunk_num, 0, A->f.num_cols};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1183,7 +1184,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_sigma(double alpha, const sspmv_sell_c
                                                 int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, 0};
+                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1252,7 +1253,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_R(double alpha, const sspmv_sell_c_R *
                                             int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, 0};
+                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 

@@ -770,7 +770,7 @@ sspmv_status launch_stream(const sspmv_csr *A, Plan *p, V alpha, const V *x, int
         return launch_merge<V, K>(A, p, alpha, x, ldx, beta, y, ldy, s);
     StreamView v;
     SSPMV_TRY(csr_stream_view(A, &v, s));
-    return launch_stream_view<V, K>(v, p->stream, alpha, x, ldx, beta, y, ldy, s);
+    return launch_stream_view<V, K>(v, p->stream, alpha, x, ldx, beta, y, ldy, A->f.num_cols, s);
 }
 
 // kernel_flag 0 (default): stream kernel (merge-path for a matrix without
