@@ -272,10 +272,11 @@ sspmv_status sspmv_spmm_csr(double alpha, const sspmv_csr *A, int32_t k, const v
  * device memory at SpMV time: a solver or serving loop whose device heap is
  * owned by its own pool allocator, a latency-bound loop that cannot take
  * cudaMalloc's implicit device synchronisation, a component held to a device
- * memory budget enforced elsewhere.  Its scratch (the pieces of rows
- * that cross windows) lives in one fixed 16 MiB device array that every GPU loading this
- * library keeps until exit; no per-matrix plan is built and nothing is
- * allocated.  Limit: num_rows + num_nnzs <= 238,594,048; larger matrices return SSPMV_INVALID_ARG.  The first call
+ * memory budget enforced elsewhere.  Its scratch (the pieces of rows that
+ * cross windows) lives in one fixed 16 MiB device array that every GPU loading
+ * this library keeps until exit; no per-matrix plan is built and nothing is
+ * allocated.  Limit: num_rows + num_nnzs <= 238,594,048; larger matrices
+ * return SSPMV_INVALID_ARG.  The first call
  * on a device (and the first after a cudaDeviceReset of it) looks up the
  * array's address with that device current: make it before any stream
  * capture.  All calls share the array: calls that overlap on
