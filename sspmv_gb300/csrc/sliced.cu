@@ -64,19 +64,20 @@ constexpr int kBlock = 256;
 // and orders a load after another's use; in FP64, whose pipe is the bound,
 // that form at full occupancy is the faster one (banded 2M 56 us against 63
 // FLAT).
+// Four slots in FP64 with registers for 6 CTAs: S-ELL, 2.9M banded rows, 103 us
+// at 8, 93 so; in FP32 75 and 73, but 4x4 block rows 44.1 and 45.5.
 template <typename V, int K, int S, bool FLAT>
 constexpr int sliced_min_ctas() {
     if (K > 1) return K * sizeof(V) <= 16 ? 6 : 4;
-    return !FLAT ? 8 : S > 10 ? 4 : S > 8 ? 5 : S > 6 ? 6 : 7;
+    if (!FLAT) return sizeof(V) == 8 && S == 4 ? 6 : 8;
+    return S > 10 ? 4 : S > 8 ? 5 : S > 6 ? 6 : 7;
 }
 
 template <typename V, int K, int S, bool PLAIN, bool FLAT>
 __device__ __forceinline__ void sliced_row(
-    int m, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
+    int64_t i, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
     const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
     V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
     const int64_t c = div_nonneg(i, C);
     const int r = (int)(i - c * C);
     const int64_t base = ld_stream(chunk_ptr + c);
@@ -131,13 +132,19 @@ __device__ __forceinline__ void sliced_row(
 // shares nothing; one block outlasts that kernel, so that what follows is behind
 // both.  Not for the forms of more slots (narrow ELL), whose loads the compiler
 // no longer keeps in flight with the wait after them (20 -> 28 us).
-template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false, bool BEHIND = false>
+template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false, bool BEHIND = false, bool STRIDE = false>
 __global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sliced_spmv_kernel(
     int m, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
     const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
     V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap) {
     if constexpr (BEHIND) let_next_start();
-    sliced_row<V, K, S, PLAIN, FLAT>(m, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if constexpr (STRIDE) {
+        for (; i < m; i += (int64_t)gridDim.x * blockDim.x)
+            sliced_row<V, K, S, PLAIN, FLAT>(i, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
+    } else if (i < m) {
+        sliced_row<V, K, S, PLAIN, FLAT>(i, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
+    }
     if constexpr (BEHIND)
         if (blockIdx.x == 0) wait_for_previous();
 }
@@ -309,6 +316,7 @@ struct SlicedView {
     int64_t nchunks;  // 0: ELL
     int32_t width;    // ELL
     int64_t cols;     // rows of X
+    int64_t nnz;
 };
 
 // Cost model of the cap, in picoseconds of GB300 time (fitted to measured
@@ -426,6 +434,12 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
     return SSPMV_OK;
 }
 
+// FP32, short rows of about one length (no row past the cap, at most this many
+// nonzeros on average): 16 blocks a SM striding over the rows are faster than a
+// block per 256 (S-ELL, 2.9M banded rows of 9: 69 us against 75), with longer
+// rows slower (1M uniform rows of 20: 113 against 107).
+constexpr int64_t kStrideRow = 12;
+
 template <typename V, int K>
 sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, int64_t ldx, V beta, V *y,
                            int64_t ldy, sspmv_stream_t s) {
@@ -438,7 +452,7 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
     // A thread per row and no grid stride: a fixed grid gave the same blocks the
     // long rows at the head of every sigma slice (4M rows FP32, sigma = 4096:
     // 580 us so, 328 with blocks scheduled as they finish).
-    const unsigned grid = grid_for(v.m, kBlock);
+    unsigned grid = grid_for(v.m, kBlock);
     const int xvec = xrow_vec(x, ldx, sizeof(V), K);
     auto go = [&](auto kernel) {
         kernel<<<grid, kBlock, 0, cu(s)>>>((int)v.m, v.C, v.chunk_ptr, v.reorder, v.col, (const V *)v.val, x, ldx,
@@ -459,6 +473,14 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
                 if (nov > 0) {
                     launched = plain ? go_behind(sliced_spmv_kernel<V, K, S, true, false, true>)
                                      : go_behind(sliced_spmv_kernel<V, K, S, false, false, true>);
+                    return;
+                }
+            }
+            if constexpr (S == 4 && sizeof(V) == 4) {
+                if (v.nchunks > 0 && nov == 0 && v.nnz <= kStrideRow * v.m) {
+                    grid = grid_for(v.m, kBlock, (int64_t)num_sms() * 16);
+                    if (plain) go(sliced_spmv_kernel<V, K, S, true, false, false, true>);
+                    else go(sliced_spmv_kernel<V, K, S, false, false, false, true>);
                     return;
                 }
             }
@@ -1035,7 +1057,7 @@ extern "C" sspmv_status sspmv_spmm_ell(double alpha, const sspmv_ell *A, int32_t
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     Plan *p = get_plan(&A->f);
     SlicedView v{A->f.num_rows, (int32_t)std::max<int64_t>(A->f.num_rows, 1), (const int64_t *)p->extra[0], nullptr,
-                 A->col_index, A->values, 0, A->max_row_width, A->f.num_cols};
+                 A->col_index, A->values, 0, A->max_row_width, A->f.num_cols, A->f.num_nnzs};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1110,7 +1132,7 @@ extern "C" sspmv_status sspmv_spmm_sell(double alpha, const sspmv_s_ell *A, int3
                                         double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->sliceWidth,   A->chunk_ptr,   nullptr,
-                 A->col_index,  A->values,     A->chunk_num, 0, A->f.num_cols};
+                 A->col_index,  A->values,     A->chunk_num, 0, A->f.num_cols, A->f.num_nnzs};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1184,7 +1206,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_sigma(double alpha, const sspmv_sell_c
                                                 int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols};
+                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols, A->f.num_nnzs};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1253,7 +1275,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_R(double alpha, const sspmv_sell_c_R *
                                             int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols};
+                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols, A->f.num_nnzs};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
