@@ -154,8 +154,9 @@ __global__ void __launch_bounds__(kMergeBlock, (merge_ctas<V, K>())) csr_merge_k
 #pragma unroll
         for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, sum[q], beta, yp + q);
     };
-    for (int e = j0 < j1 ? b : j1; e < j1; e += 256) {  // warp-uniform
-        const uint32_t e0 = (uint32_t)e + 8u * lane;
+    // unsigned: the last step's e + 256 may pass INT_MAX (nnz up to 2^31 - 1)
+    for (uint32_t e = j0 < j1 ? b : j1; e < (uint32_t)j1; e += 256) {  // warp-uniform
+        const uint32_t e0 = e + 8u * lane;
         const unsigned in = in_window<8>(e0, j0, j1);
         int c[8];
         V a[8];
