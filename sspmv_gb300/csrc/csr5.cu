@@ -209,7 +209,7 @@ __global__ void c5_transpose(int64_t nnz, int32_t p, int32_t sigma, int32_t omeg
 
 // ------------------------------------------------------------------ SpMV --
 struct C5Shape {
-    int32_t sigma, omega, tiles;  // the last tile is stored in CSR order
+    int32_t sigma, omega, tiles;  // tile tiles - 1 (and what follows) is stored in CSR order
 };
 
 // One window (rows that cross its ends are split), one warp.  A tile inside
@@ -251,10 +251,10 @@ __device__ __forceinline__ void c5_window(const StreamView &A, const C5Shape g, 
     for (int q = 0; q < K; q++) carry[q] = V(0);
     bool later = false;
     const int64_t wend = min((w + 1) * (int64_t)A.window, (int64_t)A.nnz);
-    for (int64_t b = w * (int64_t)A.window; b < wend; b += 32 * sigma) {  // warp-uniform
+    for (int64_t b = w * (int64_t)A.window; b < wend; b += 32 * (int64_t)sigma) {  // warp-uniform
         const int64_t e0 = b + (int64_t)lane * sigma;  // this lane's nonzeros e0 .. e0 + sigma - 1
         const int64_t t = e0 / tile;
-        const bool csr_order = t == (int64_t)g.tiles - 1;
+        const bool csr_order = t >= (int64_t)g.tiles - 1;
         const int64_t p0 = csr_order ? e0 : t * tile + xl;
         const int64_t step = csr_order ? 1 : g.omega;
         const int nv = (int)max((int64_t)0, min((int64_t)sigma, (int64_t)A.nnz - e0));
@@ -405,6 +405,14 @@ __global__ void __launch_bounds__(kC5Block, (c5_min_ctas<V, K, SIG>())) csr5_ker
     c5_window<V, K, SIG, PLAIN>(A, g, x, ldx, xvec, alpha, beta, y, ldy, w, tail_val, head_val);
 }
 
+// Nonzeros per window: whole steps of 32 sigma.  Where these pass the 32-bit
+// range one window covers the matrix, whose nonzeros are fewer.
+int c5_window_size(int64_t nnz, int sigma, int warps_per_sm) {
+    const int64_t step = 32 * (int64_t)sigma;
+    if (step > INT32_MAX / 5) return (int)std::min<int64_t>(step, INT32_MAX);
+    return (int)step * window_steps(nnz, (int)step, (int)step, warps_per_sm);
+}
+
 template <typename V, int K>
 __global__ void csr5_no_nonzeros(int64_t m, V beta, V *__restrict__ y, int64_t ldy) {
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m; r += (int64_t)gridDim.x * blockDim.x)
@@ -423,23 +431,24 @@ sspmv_status csr5_pass(const sspmv_csr5 *A, Plan *pl, V alpha, const V *x, int64
     }
     if (A->_p > 1 && A->omega != 4 && A->omega != 8 && A->omega != 16 && A->omega != 32)
         return fail(SSPMV_NOT_SUPPORTED, "CSR5 SpMV supports omega in {4, 8, 16, 32}");
+    // A single tile is in CSR order whatever its shape: steps of 16 a lane
+    // (with the format's sigma one of more nonzeros than the matrix would leave
+    // them all to one lane).
+    const C5Shape g = A->_p > 1 ? C5Shape{A->sigma, A->omega, A->_p} : C5Shape{16, 32, 1};
     const int ctas = A->f.value_type == SSPMV_F64 ? c5_min_ctas<double, 1, 16>() : c5_min_ctas<float, 1, 16>();
-    const int steps = window_steps(nnz, 32 * A->sigma, 32 * A->sigma, ctas * (kC5Block / 32));
     SSPMV_TRY(ensure_stream_plan(pl->stream, m, nnz, A->row_offset, nullptr, A->f.value_type, s,
-                                 32 * A->sigma * steps, 0));
+                                 c5_window_size(nnz, g.sigma, ctas * (kC5Block / 32)), 0));
     const StreamView v = stream_view(pl->stream, nnz, A->col_index, A->values);
-    // a single tile is in CSR order whatever omega is
-    const C5Shape g{A->sigma, A->_p > 1 ? A->omega : 32, A->_p};
     const unsigned grid = grid_for(v.windows, kC5Block / 32);
     V *tv = (V *)pl->stream.tail_val, *hv = (V *)pl->stream.head_val;
     auto go = [&](auto kernel) {
         kernel<<<grid, kC5Block, 0, cu(s)>>>(v, g, x, ldx, xrow_vec(x, ldx, sizeof(V), K), alpha, beta, y, ldy, tv, hv);
     };
     const bool plain = alpha == V(1) && beta == V(0);  // y = sum
-    if (A->sigma == 16) {
+    if (g.sigma == 16) {
         if (plain) go(csr5_kernel<V, K, 16, true>);
         else go(csr5_kernel<V, K, 16, false>);
-    } else if (A->sigma == 32) {
+    } else if (g.sigma == 32) {
         if (plain) go(csr5_kernel<V, K, 32, true>);
         else go(csr5_kernel<V, K, 32, false>);
     } else {
