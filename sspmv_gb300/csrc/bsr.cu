@@ -214,9 +214,24 @@ __global__ void __launch_bounds__(kStreamBlock, (bsr_ctas<V, C>())) bsr_stream_k
     constexpr int B = BsrShape<V, C>::B;
     constexpr bool kSeed = sizeof(V) == 8;
     const int64_t w = (int64_t)blockIdx.x * (kStreamBlock / 32) + (threadIdx.x >> 5);
-    if (w >= A.windows) return;  // warp-uniform
     const int r = 1 << lr, NG = 32 >> lr;
     const int lane = threadIdx.x & 31, g = lane >> lr, q = lane & (r - 1);
+    if (w >= A.windows) {  // warp-uniform: block rows without blocks, y = beta * y, 256 rows a warp
+        const int64_t t0 = (w - A.windows) * kEmptyUnit + lane;
+        int64_t i[8];
+        V old[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int64_t t = t0 + 32 * u;
+            i[u] = (t >> lr) < A.nempty ? ((int64_t)__ldg(A.empty + (t >> lr)) << lr) + (t & (r - 1)) : m;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) old[u] = !PLAIN && beta != V(0) && i[u] < m ? y[i[u]] : V(0);
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (i[u] < m) y[i[u]] = PLAIN || beta == V(0) ? V(0) : beta * old[u];
+        return;
+    }
     const int64_t rc = (int64_t)r * C;
     const int4 rec = __ldg(A.rec + w);
     const uint32_t eA = (uint32_t)rec.x, eB = (uint32_t)rec.y;
@@ -331,13 +346,6 @@ __global__ void __launch_bounds__(kStreamBlock, (bsr_ctas<V, C>())) bsr_stream_k
         carry = kSeed || nend > 0 ? open : carry + open;
         row += nend;
     }
-    if (A.nempty > 0) {  // block rows without blocks: y = beta * y, this window's share of the list
-        const int64_t i0 = A.nempty * w / A.windows, i1 = A.nempty * (w + 1) / A.windows;
-        for (int64_t t = lane; t < (i1 - i0) << lr; t += 32) {
-            const int64_t i = ((int64_t)__ldg(A.empty + i0 + (t >> lr)) << lr) + (t & (r - 1));
-            if (i < m) y[i] = beta == V(0) ? V(0) : beta * y[i];
-        }
-    }
 }
 
 // out[0]: lane slots the thread-per-row kernel spends (every warp of 32 rows,
@@ -421,7 +429,7 @@ sspmv_status launch_bsr_stream(const sspmv_bsr *A, Plan *p, V alpha, const V *x,
     const int xvec = reinterpret_cast<uintptr_t>(x) % run == 0 ? 1 : 0;
     const int dvec = reinterpret_cast<uintptr_t>(A->block_data) % run == 0 ? 1 : 0;
     auto go = [&](auto kernel) {
-        kernel<<<grid_for(v.windows, kStreamBlock / 32), kStreamBlock, 0, cu(s)>>>(
+        kernel<<<grid_for(v.windows + empty_units((int64_t)v.nempty << lr), kStreamBlock / 32), kStreamBlock, 0, cu(s)>>>(
             v, (int)A->f.num_rows, (int)A->f.num_cols, lr, (const V *)A->block_data, dvec, x, xvec, alpha, beta, y);
     };
     if (alpha == V(1) && beta == V(0)) go(bsr_stream_kernel<V, C, true>);  // y = sum

@@ -374,14 +374,6 @@ __device__ __forceinline__ void c5_window(const StreamView &A, const C5Shape g, 
         row += nend;
         later = true;
     }
-    if (A.nempty > 0) {  // rows without nonzeros: this window's share of the list
-        const int64_t i0 = A.nempty * w / A.windows, i1 = A.nempty * (w + 1) / A.windows;
-        for (int64_t i = i0 + lane; i < i1; i += 32) {
-            V *ye = y + (int64_t)__ldg(A.empty + i) * ldy;
-#pragma unroll
-            for (int q = 0; q < K; q++) ye[q] = beta == V(0) ? V(0) : beta * ye[q];
-        }
-    }
     if ((rec.w & 2) && lane == 0) {
         V *cp = tail_val + w * kMaxK;
 #pragma unroll
@@ -401,7 +393,10 @@ __global__ void __launch_bounds__(kC5Block, (c5_min_ctas<V, K, SIG>())) csr5_ker
     V *__restrict__ y, int64_t ldy, V *__restrict__ tail_val, V *__restrict__ head_val) {
     const int64_t w = (int64_t)blockIdx.x * (kC5Block / 32) + (threadIdx.x >> 5);
     let_next_start();
-    if (w >= A.windows) return;
+    if (w >= A.windows) {  // rows without nonzeros
+        scale_empty_rows<V, K>(A, w - A.windows, PLAIN ? V(0) : beta, y, (uint64_t)ldy * sizeof(V), false);
+        return;
+    }
     c5_window<V, K, SIG, PLAIN>(A, g, x, ldx, xvec, alpha, beta, y, ldy, w, tail_val, head_val);
 }
 
@@ -439,7 +434,7 @@ sspmv_status csr5_pass(const sspmv_csr5 *A, Plan *pl, V alpha, const V *x, int64
     SSPMV_TRY(ensure_stream_plan(pl->stream, m, nnz, A->row_offset, nullptr, A->f.value_type, s,
                                  c5_window_size(nnz, g.sigma, ctas * (kC5Block / 32)), 0));
     const StreamView v = stream_view(pl->stream, nnz, A->col_index, A->values);
-    const unsigned grid = grid_for(v.windows, kC5Block / 32);
+    const unsigned grid = grid_for(v.windows + empty_units(v.nempty), kC5Block / 32);
     V *tv = (V *)pl->stream.tail_val, *hv = (V *)pl->stream.head_val;
     auto go = [&](auto kernel) {
         kernel<<<grid, kC5Block, 0, cu(s)>>>(v, g, x, ldx, xrow_vec(x, ldx, sizeof(V), K), alpha, beta, y, ldy, tv, hv);

@@ -43,9 +43,9 @@
 // one's pieces in window order, a warp per row.  (The last warp to finish,
 // found by a counter per row, adding the pieces instead cost a memory fence per
 // window: power-law 4M FP32 365 us against 303.)  Rows without nonzeros are a
-// list, shared evenly by the windows.  No atomics on y: sums depend on the
-// matrix alone, and a request's batch runs the same windows with the same
-// code, so its result does not depend on the batch.
+// list, which warps behind the windows' write (scale_empty_rows).  No atomics
+// on y: sums depend on the matrix alone, and a request's batch runs the same
+// windows with the same code, so its result does not depend on the batch.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -142,26 +142,6 @@ __device__ __forceinline__ void ld_cols(const V *__restrict__ p, bool vec, V (&o
 template <typename V>
 __device__ __forceinline__ V scaled(V alpha, V sum, V beta, V y) {
     return beta == V(0) ? alpha * sum : fma(alpha, sum, beta * y);
-}
-
-template <typename V, int KL, bool BIG = false>
-__device__ __forceinline__ void st_cols(V *__restrict__ p, bool vec, const V (&o)[KL]) {
-    if constexpr (KL * sizeof(V) == 16) {
-        if (vec) {
-            if constexpr (sizeof(V) == 8) {
-                const double2 v = make_double2(o[0], o[1]);
-                if constexpr (BIG) __stcs(reinterpret_cast<double2 *>(p), v);  // leaves L2 to X
-                else *reinterpret_cast<double2 *>(p) = v;
-            } else {
-                const float4 v = make_float4(o[0], o[1], o[2], o[3]);
-                if constexpr (BIG) __stcs(reinterpret_cast<float4 *>(p), v);
-                else *reinterpret_cast<float4 *>(p) = v;
-            }
-            return;
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < KL; q++) p[q] = o[q];
 }
 
 // Where the pieces of split rows are left (slot = window plus the matrix's
@@ -382,9 +362,8 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
         ebits = load_ends<G>(A.ends, e0, A.nnz);
     }
 
-    // rows without nonzeros: this window's share of the list
-    if (A.nempty > 0) {
-        const int64_t i0 = A.nempty * w / A.windows, i1 = A.nempty * (w + 1) / A.windows;
+    if (A.nshared > 0) {  // the rows without nonzeros: this window's share
+        const int64_t i0 = A.nshared * w / A.windows, i1 = A.nshared * (w + 1) / A.windows;
         for (int64_t i = i0 + lane; i < i1; i += 32) {
             V *ye = reinterpret_cast<V *>(reinterpret_cast<char *>(y) + (uint64_t)(uint32_t)__ldg(A.empty + i) * yrow);
 #pragma unroll
@@ -454,7 +433,10 @@ __global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K, BIG>())) csr_st
     const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
     __shared__ __align__(16) V s_y[kWarps][PLAIN ? 1 : StreamShape<V, K>::kStage * K];
     let_next_start();
-    if (w >= A.windows) return;
+    if (w >= A.windows) {
+        if (A.nshared == 0) scale_empty_rows<V, K>(A, w - A.windows, PLAIN ? V(0) : beta, y, yrow, yvec != 0);
+        return;
+    }
     stream_window<V, K, PLAIN, BIG>(A, x, xrow, alpha, beta, y, yrow, w, sl, xvec != 0, yvec != 0,
                                s_y[threadIdx.x >> 5]);
 }
@@ -667,6 +649,7 @@ StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, co
     v.nnz = (uint32_t)nnz;
     v.window = sp.window;
     v.nempty = (int32_t)sp.nempty;
+    v.nshared = sp.nempty <= sp.windows / 8 ? (int32_t)sp.nempty : 0;
     v.nsplit = (int32_t)sp.nsplit;
     v.vec = ((reinterpret_cast<uintptr_t>(col) | reinterpret_cast<uintptr_t>(val)) & 15) == 0;
     return v;
@@ -686,8 +669,8 @@ sspmv_status launch_stream_windows(const StreamView &v, StreamPlan &sp, V alpha,
     const StreamSlots<V> sl{(V *)sp.tail_val, (V *)sp.head_val, 0};
     const uint32_t xrow = (uint32_t)(ldx * (int64_t)sizeof(V)), yrow = (uint32_t)(ldy * (int64_t)sizeof(V));
     auto go = [&](auto kernel) {
-        kernel<<<grid_for(v.windows, kWarps), kBlock, 0, cu(s)>>>(v, x, xrow, alpha, beta, y, yrow, sl,
-                                                                  xrow_vec(x, ldx, sizeof(V), K), yrow_vec(y, ldy, K));
+        kernel<<<grid_for(v.windows + (v.nshared > 0 ? 0 : empty_units(v.nempty)), kWarps), kBlock, 0, cu(s)>>>(
+            v, x, xrow, alpha, beta, y, yrow, sl, xrow_vec(x, ldx, sizeof(V), K), yrow_vec(y, ldy, K));
     };
     const bool plain = alpha == V(1) && beta == V(0);
     bool big = false;
@@ -744,7 +727,8 @@ __device__ __forceinline__ int batch_item_of(const BatchItem *__restrict__ items
     return lo;
 }
 
-// Persistent stream kernel over the windows of every request of group g:
+// Persistent stream kernel over the windows of every request of group g and
+// then the units of their lists of rows without nonzeros:
 // warp i of the grid takes global windows i, i + warps, ...  A request is cut
 // into the windows a lone sspmv_spmm_csr call uses (the matrix's own plan),
 // and the pieces of its split rows go to per-batch slots, so its result does
@@ -765,6 +749,12 @@ __global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K>() * 3 / 4)) csr
         stream_window<V, K, false>(q->view, (const V *)q->x, (uint32_t)(q->ldx * (int64_t)sizeof(V)), (V)q->alpha,
                                    (V)q->beta, (V *)q->y, (uint32_t)(q->ldy * (int64_t)sizeof(V)),
                                    gw - q->window_begin, sl, q->xvec != 0, q->yvec != 0, s_y[threadIdx.x >> 5]);
+    }
+    const int64_t units = hdr->total_empties[g];
+    for (int64_t gu = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5); gu < units; gu += warps) {
+        const BatchItem *q = items + batch_item_of(items, n, gu, &BatchItem::empty_begin);
+        scale_empty_rows<V, K>(q->view, gu - q->empty_begin, (V)q->beta, (V *)q->y,
+                               (uint64_t)q->ldy * sizeof(V), q->yvec != 0);
     }
 }
 

@@ -32,6 +32,7 @@ struct BatchItem {
     double alpha, beta;
     int64_t window_begin;  // first global window of this item in its group
     int64_t split_begin;   // first global split row likewise
+    int64_t empty_begin;   // first global unit of rows without nonzeros likewise
     int32_t xvec;          // X rows aligned for vector loads (xrow_vec)
     int32_t yvec;          // Y rows likewise
 };
@@ -41,6 +42,7 @@ struct BatchHeader {
     int32_t n_items[kBatchGroups];
     int64_t total_windows[kBatchGroups];
     int64_t total_splits[kBatchGroups];
+    int64_t total_empties[kBatchGroups];
     int64_t slot_base[kBatchGroups];     // first split-row slot of each group
 };
 

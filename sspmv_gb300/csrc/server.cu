@@ -601,7 +601,7 @@ void Server::issue(Batch &b) {
     }
     BatchItem *items = reinterpret_cast<BatchItem *>(w.h_in + sizeof(BatchHeader));
     int fill[kBatchGroups] = {0};
-    int64_t group_tiles[kBatchGroups] = {0}, group_splits[kBatchGroups] = {0};
+    int64_t group_tiles[kBatchGroups] = {0}, group_splits[kBatchGroups] = {0}, group_empties[kBatchGroups] = {0};
     uint32_t mask = 0;
     for (Request *r : b.reqs) {
         if (r->group < 0) continue;
@@ -617,10 +617,12 @@ void Server::issue(Batch &b) {
         it.beta = r->r.beta;
         it.window_begin = group_tiles[g];
         it.split_begin = group_splits[g];
+        it.empty_begin = group_empties[g];
         it.xvec = xrow_vec(r->d_x, r->r.ldx, g >= 4 ? 8 : 4, r->r.k);
         it.yvec = xrow_vec(r->d_y, r->r.ldy, g >= 4 ? 8 : 4, r->r.k);
         group_tiles[g] += M.view.windows;
         group_splits[g] += M.view.nsplit;
+        group_empties[g] += M.view.nshared > 0 ? 0 : empty_units(M.view.nempty);
         mask |= 1u << g;
     }
     int64_t carry = 0;
@@ -628,6 +630,7 @@ void Server::issue(Batch &b) {
         hdr.n_items[g] = counts[g];
         hdr.total_windows[g] = group_tiles[g];
         hdr.total_splits[g] = group_splits[g];
+        hdr.total_empties[g] = group_empties[g];
         hdr.slot_base[g] = carry;
         carry += group_tiles[g];
     }
