@@ -51,29 +51,37 @@ constexpr int kBlock = 256;
 // puts them in the same sectors).  Moving only the part of a row past the cap
 // (the thread's partial sum, a CSR pass over short tails, a warp per 2048
 // elements of long ones and a pass that adds the three) took five launches one
-// after another: SELL-c-sigma (4096, 32) on power-law 1M FP64 146 us, two
-// launches now 102.
+// after another: SELL-c-sigma (4096, 32) on power-law 1M FP64 136 us of GPU time,
+// now 84 in three launches that overlap.
 
 // S: slots of a row whose loads are in flight together (column and value
 // loads of S slots, then their x gathers, then the FMAs in slot order).
-// FLAT (ELL of up to 12 slots in FP32): a row's slots loaded unconditionally
+// FLAT (ELL of up to 12 slots in FP32, but 7 and 8): a row's slots loaded unconditionally
 // (a slot past the width reads the last one again, padding gathers x[0]) with
 // registers for all of them: two memory latencies per row instead of two per
-// four slots -- banded 1M FP32 27 -> 21 us, 5-point Laplacian 1M 18.4 -> 15 us.
+// four slots -- banded 1M FP32 24.9 -> 17.9 us, 5-point Laplacian 1M 15.6 -> 11.9.
 // With a test around each load the compiler holds a thread to 32 registers
 // and orders a load after another's use; in FP64, whose pipe is the bound,
 // that form at full occupancy is the faster one (banded 2M 56 us against 63
 // FLAT).
-// Four slots in FP64 with registers for 6 CTAs: S-ELL, 2.9M banded rows, 103 us
-// at 8, 93 so; in FP32 75 and 73, but 4x4 block rows 44.1 and 45.5.
-template <typename V, int K, int S, bool FLAT>
+// Four slots in FP64 with registers for 6 CTAs (S-ELL, 2.9M banded rows, 115 us
+// at 8, 94 so), except (WAVE) for a grid that 8 take in one wave and 6 do not
+// (254,620 banded rows, 14.3 us at 6, 10.9 so), for one wave of long rows (200k
+// rows of 64, 58 and 48) and for chunks of one or two slots (1M rows of 2, 12.4
+// and 11.0).
+template <typename V, int K, int S, bool FLAT, bool WAVE>
 constexpr int sliced_min_ctas() {
     if (K > 1) return K * sizeof(V) <= 16 ? 6 : 4;
-    if (!FLAT) return sizeof(V) == 8 && S == 4 ? 6 : 8;
+    if (!FLAT) return sizeof(V) == 8 && S == 4 && !WAVE ? 6 : 8;
     return S > 10 ? 4 : S > 8 ? 5 : S > 6 ? 6 : 7;
 }
 
-template <typename V, int K, int S, bool PLAIN, bool FLAT>
+// TWO: S slots at a time while there are S, without a test around each load,
+// then one by one: S-ELL in FP32, 5-point Laplacian 4M 79 us with tested loads,
+// 66 so, and 61 without a grid that strides over the rows; FP64, 1M rows of 30,
+// 147 and 114.  Otherwise the loads of a step are tested and those past the width
+// left out: for the widths that would be read mostly one by one.
+template <typename V, int K, int S, bool PLAIN, bool FLAT, bool TWO>
 __device__ __forceinline__ void sliced_row(
     int64_t i, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
     const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
@@ -88,29 +96,17 @@ __device__ __forceinline__ void sliced_row(
     V s[K];
 #pragma unroll
     for (int q = 0; q < K; q++) s[q] = V(0);
-    for (int64_t k = 0; k < w; k += S) {
-        int cc[S];
-        V aa[S];
+    if constexpr (TWO) {
+        int64_t k = 0;
+        bool open = true;
+        for (; k + S <= w; k += S) {
+            int cc[S];
+            V aa[S];
 #pragma unroll
-        for (int u = 0; u < S; u++) {
-            cc[u] = -1;
-            aa[u] = V(0);
-            if (FLAT || k + u < w) {
-                const int64_t at = (FLAT ? min(k + u, w - 1) : k + u) * C;
-                cc[u] = ld_stream(cp + at);
-                aa[u] = ld_stream(vp + at);
+            for (int u = 0; u < S; u++) {
+                cc[u] = ld_stream(cp + (k + u) * C);
+                aa[u] = ld_stream(vp + (k + u) * C);
             }
-            if (FLAT && k + u >= w) cc[u] = -1;
-        }
-        if constexpr (K == 1) {
-            V xv[S];
-#pragma unroll
-            for (int u = 0; u < S; u++)
-                xv[u] = FLAT ? ld_x(x + (int64_t)max(cc[u], 0) * ldx) : cc[u] >= 0 ? ld_x(x + (int64_t)cc[u] * ldx) : V(0);
-#pragma unroll
-            for (int u = 0; u < S; u++)
-                if (cc[u] >= 0) s[0] += aa[u] * xv[u];  // never 0 * x[0]: x may hold Inf or NaN
-        } else {
 #pragma unroll
             for (int u = 0; u < S; u++)
                 if (cc[u] >= 0) {
@@ -119,8 +115,55 @@ __device__ __forceinline__ void sliced_row(
 #pragma unroll
                     for (int q = 0; q < K; q++) s[q] += aa[u] * xr[q];
                 }
+            if (cc[S - 1] < 0) {  // padding is a suffix of the row
+                open = false;
+                break;
+            }
         }
-        if (cc[S - 1] < 0) break;  // padding is a suffix of the row
+        for (; open && k < w; k++) {
+            const int cc = ld_stream(cp + k * C);
+            if (cc < 0) break;
+            const V aa = ld_stream(vp + k * C);
+            V xr[K];
+            ld_xrow<V, K>(x, cc, ldx, xvec, xr);
+#pragma unroll
+            for (int q = 0; q < K; q++) s[q] += aa * xr[q];
+        }
+    } else {
+        for (int64_t k = 0; k < w; k += S) {
+            int cc[S];
+            V aa[S];
+#pragma unroll
+            for (int u = 0; u < S; u++) {
+                cc[u] = -1;
+                aa[u] = V(0);
+                if (FLAT || k + u < w) {
+                    const int64_t at = (FLAT ? min(k + u, w - 1) : k + u) * C;
+                    cc[u] = ld_stream(cp + at);
+                    aa[u] = ld_stream(vp + at);
+                }
+                if (FLAT && k + u >= w) cc[u] = -1;
+            }
+            if constexpr (K == 1) {
+                V xv[S];
+#pragma unroll
+                for (int u = 0; u < S; u++)
+                    xv[u] = FLAT ? ld_x(x + (int64_t)max(cc[u], 0) * ldx) : cc[u] >= 0 ? ld_x(x + (int64_t)cc[u] * ldx) : V(0);
+#pragma unroll
+                for (int u = 0; u < S; u++)
+                    if (cc[u] >= 0) s[0] += aa[u] * xv[u];  // never 0 * x[0]: x may hold Inf or NaN
+            } else {
+#pragma unroll
+                for (int u = 0; u < S; u++)
+                    if (cc[u] >= 0) {
+                        V xr[K];
+                        ld_xrow<V, K>(x, cc[u], ldx, xvec, xr);
+#pragma unroll
+                        for (int q = 0; q < K; q++) s[q] += aa[u] * xr[q];
+                    }
+            }
+            if (cc[S - 1] < 0) break;  // padding is a suffix of the row
+        }
     }
     const int64_t row = reorder ? (int64_t)ld_stream(reorder + i) : i;
     V *yp = y + row * ldy;
@@ -132,8 +175,9 @@ __device__ __forceinline__ void sliced_row(
 // shares nothing; one block outlasts that kernel, so that what follows is behind
 // both.  Not for the forms of more slots (narrow ELL), whose loads the compiler
 // no longer keeps in flight with the wait after them (20 -> 28 us).
-template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false, bool BEHIND = false, bool STRIDE = false>
-__global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sliced_spmv_kernel(
+template <typename V, int K, int S, bool PLAIN = false, bool FLAT = false, bool BEHIND = false, bool STRIDE = false,
+          bool WAVE = false, bool TWO = STRIDE>
+__global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT, WAVE>())) sliced_spmv_kernel(
     int m, int C, const int64_t *__restrict__ chunk_ptr, const int32_t *__restrict__ reorder,
     const int32_t *__restrict__ col, const V *__restrict__ val, const V *__restrict__ x, int64_t ldx, int xvec,
     V alpha, V beta, V *__restrict__ y, int64_t ldy, int64_t cap) {
@@ -141,9 +185,10 @@ __global__ void __launch_bounds__(kBlock, (sliced_min_ctas<V, K, S, FLAT>())) sl
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (STRIDE) {
         for (; i < m; i += (int64_t)gridDim.x * blockDim.x)
-            sliced_row<V, K, S, PLAIN, FLAT>(i, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
+            sliced_row<V, K, S, PLAIN, FLAT, TWO>(i, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
     } else if (i < m) {
-        sliced_row<V, K, S, PLAIN, FLAT>(i, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy, cap);
+        sliced_row<V, K, S, PLAIN, FLAT, TWO>(i, C, chunk_ptr, reorder, col, val, x, ldx, xvec, alpha, beta, y, ldy,
+                                               cap);
     }
     if constexpr (BEHIND)
         if (blockIdx.x == 0) wait_for_previous();
@@ -316,31 +361,43 @@ struct SlicedView {
     int64_t nchunks;  // 0: ELL
     int32_t width;    // ELL
     int64_t cols;     // rows of X
-    int64_t nnz;
+    int32_t align;    // of the chunks' widths
+    bool sorted;      // by length over the whole matrix (SELL-c-R)
 };
 
 // Cost model of the cap, in picoseconds of GB300 time (fitted to measured
 // times of power-law matrices of 0.1-4M rows at caps of 1 to 512).  A nonzero
 // costs kNnzPs in either kernel, its x gather; the thread pass no less than
 // kWarpSlotPs per warp and slot it runs (a warp runs as many slots as its
-// longest row within the cap), plus its longest thread's chain, kSlotChainPs
-// per slot (1M rows FP64, sigma = 4096: caps of 32, 128, 512 take 115, 171, 396
-// us); the overflow kOvfRowPs per row and kOvfLaunchPs for its launches.
+// longest row within the cap), nor than a warp of average length's chain,
+// kSlotChainPs per slot, plus what its longest thread's chain goes on beyond
+// that (1M rows FP64, sigma = 4096: caps of 32, 128, 512 take 115, 171, 396 us;
+// 1M even rows of 50 have no such rest: 185 us in the thread pass, 212 through the
+// stream kernel); the overflow kOvfRowPs per row and kOvfLaunchPs for its
+// launches.
 constexpr double kWarpSlotPs = 73.0;
 constexpr double kSlotChainPs = 0.5e6;
 constexpr double kNnzPs = 3.9;
 constexpr double kOvfRowPs = 20.0;
 constexpr double kOvfLaunchPs = 4.0e6;
+// Rows sorted by length over the whole matrix leave no lane of a warp idle, and the
+// longest ones start first: without very long ones they stay in the thread pass
+// (SELL-c-R, 1.5M 4x4 block rows of up to 28: FP32 27.3 us with a cap of 8, 19.5
+// without; k = 2 28.3 and 20.9; FP64 32.0 and 26.9).
+constexpr int64_t kShortRow = 64;
+constexpr int64_t kWholeRows = 500000;
 constexpr CapList kCaps = {{8, 12, 16, 24, 32, 48, 64, 96, 128, 256, 512, kNoCap}};
 
 // The candidate of least modelled time (ties: no cap, then the largest).
-int choose_cap(const CapStats (&st)[kNumCaps], int64_t total_nnz) {
+int choose_cap(const CapStats (&st)[kNumCaps], int64_t m, int64_t total_nnz) {
+    const double warps = (double)((m + 31) / 32);
     int best = kNumCaps - 1;
     double best_cost = 0;
     for (int t = kNumCaps - 1; t >= 0; t--) {
-        const double thread = std::max(kWarpSlotPs * (double)st[t].slots,
-                                       kNnzPs * (double)(total_nnz - (int64_t)st[t].nnz)) +
-                              kSlotChainPs * (double)st[t].longest;
+        const double average = (double)st[t].slots / warps;
+        const double thread = std::max({kWarpSlotPs * (double)st[t].slots,
+                                        kNnzPs * (double)(total_nnz - (int64_t)st[t].nnz), kSlotChainPs * average}) +
+                              kSlotChainPs * ((double)st[t].longest - average);
         const double cost = thread + kNnzPs * (double)st[t].nnz + kOvfRowPs * (double)st[t].rows +
                             (st[t].rows > 0 ? kOvfLaunchPs : 0.0);
         if (t == kNumCaps - 1 || cost < best_cost) {
@@ -364,7 +421,8 @@ void free_overflow(Plan *p, sspmv_stream_t s) {
 // sspmv_set_kernel changes the cap).  extra[0] y row of every overflow row
 // (the stream plan's row list), extra[1] / extra[2] their columns / values;
 // p->stream the stream plan; extra_i[1] overflow rows, [2] the cap, [3] the
-// kernel parameter the plan was built for, [4] overflow nonzeros, [7] built.
+// kernel parameter the plan was built for, [4] overflow nonzeros, [5] the
+// longest row, [7] built.
 sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, Plan *p, sspmv_stream_t s) {
     if (p->extra_i[7] && p->extra_i[3] == p->param) return SSPMV_OK;
     std::lock_guard<PlanMutex> g(plan_mutex());
@@ -379,7 +437,7 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
     CapStats *dst = nullptr;
     CapList caps = kCaps;
     if (p->param > 0) caps.cap[0] = p->param;
-    int64_t nov = 0, novf = 0, cap = kNoCap;
+    int64_t nov = 0, novf = 0, cap = kNoCap, longest = 0;
     auto build = [&]() -> sspmv_status {
         SSPMV_TRY(dalloc(&len, (size_t)m, s));
         SSPMV_TRY(dalloc(&dst, kNumCaps, s));
@@ -391,8 +449,10 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
         CapStats st[kNumCaps];
         SSPMV_CUDA_TRY(cudaMemcpyAsync(st, dst, sizeof(st), cudaMemcpyDeviceToHost, cu(s)));
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
-        const int pick = p->param > 0 ? 0 : choose_cap(st, f->num_nnzs);
+        const bool whole = v.sorted && m > kWholeRows && st[kNumCaps - 1].longest <= (unsigned long long)kShortRow;
+        const int pick = p->param > 0 ? 0 : whole ? kNumCaps - 1 : choose_cap(st, m, f->num_nnzs);
         cap = caps.cap[pick];
+        longest = (int64_t)st[kNumCaps - 1].longest;
         nov = (int64_t)st[pick].rows;
         novf = (int64_t)st[pick].nnz;
         if (novf > 0x7fffffff) return fail(SSPMV_NOT_SUPPORTED, "overflow of the long rows exceeds the int32 range");
@@ -430,20 +490,19 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
     p->extra_i[2] = nov > 0 ? cap : kNoCap;
     p->extra_i[3] = p->param;
     p->extra_i[4] = novf;
+    p->extra_i[5] = longest;
     p->extra_i[7] = 1;
     return SSPMV_OK;
 }
 
-// FP32, short rows of about one length (no row past the cap, at most this many
-// nonzeros on average): 16 blocks a SM striding over the rows are faster than a
-// block per 256 (S-ELL, 2.9M banded rows of 9: 69 us against 75), with longer
-// rows slower (1M uniform rows of 20: 113 against 107).
-constexpr int64_t kStrideRow = 12;
-
 template <typename V, int K>
 sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, int64_t ldx, V beta, V *y,
                            int64_t ldy, sspmv_stream_t s) {
-    const int64_t nov = p && stream_takes_strides(ldx, ldy, sizeof(V)) ? p->extra_i[1] : 0;
+    // Two or four FP32 right-hand sides on many rows, none very long: the thread
+    // pass alone, whatever the cap (S-ELL, block rows, k = 2: 3M rows 84.5 us with
+    // it, 70 so, 1M 30.4 and 27.6, but 100k 5.9 and 8.4).
+    const bool whole = p && sizeof(V) == 4 && (K == 2 || K == 4) && v.m > kWholeRows && p->extra_i[5] <= kShortRow;
+    const int64_t nov = p && !whole && stream_takes_strides(ldx, ldy, sizeof(V)) ? p->extra_i[1] : 0;
     StreamView lv;
     if (nov > 0) {  // the long rows first: the thread pass starts under their last wave
         lv = stream_view(p->stream, p->extra_i[4], (const int32_t *)p->extra[1], p->extra[2]);
@@ -468,36 +527,63 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
         const bool plain = alpha == V(1) && beta == V(0);  // y = sum
         auto slots = [&](auto tag) {
             constexpr int S = decltype(tag)::value;
-            constexpr bool flat = S > 4 && sizeof(V) == 4;  // only ELL takes S > 4
-            if constexpr (S == 4) {
-                if (nov > 0) {
-                    launched = plain ? go_behind(sliced_spmv_kernel<V, K, S, true, false, true>)
-                                     : go_behind(sliced_spmv_kernel<V, K, S, false, false, true>);
-                    return;
-                }
-            }
-            if constexpr (S == 4 && sizeof(V) == 4) {
-                if (v.nchunks > 0 && nov == 0 && v.nnz <= kStrideRow * v.m) {
-                    grid = grid_for(v.m, kBlock, (int64_t)num_sms() * 16);
-                    if (plain) go(sliced_spmv_kernel<V, K, S, true, false, false, true>);
-                    else go(sliced_spmv_kernel<V, K, S, false, false, false, true>);
-                    return;
-                }
-            }
+            constexpr bool flat = S > 4 && sizeof(V) == 4;
             if (plain) go(sliced_spmv_kernel<V, K, S, true, flat>);
             else go(sliced_spmv_kernel<V, K, S, false, flat>);
         };
-        // ELL: all slots of a narrow row at once; wider rows and the chunked
-        // formats, whose rows differ in length, four at a time (six and eight
-        // were slower on power-law and uniform rows).
-        const int w = v.nchunks > 0 || v.width > 12 ? 4 : v.width;
-        if (w <= 4) slots(std::integral_constant<int, 4>());
-        else if (w <= 6) slots(std::integral_constant<int, 6>());
-        else if (w <= 8) slots(std::integral_constant<int, 8>());
-        else if (w <= 10) slots(std::integral_constant<int, 10>());
-        else slots(std::integral_constant<int, 12>());
+        // the widest chunk
+        const int64_t w = v.nchunks > 0 ? (p->extra_i[5] + v.align - 1) / v.align * v.align : v.width;
+        const bool ell = v.nchunks == 0;
+        if (nov > 0) {
+            launched = plain ? go_behind(sliced_spmv_kernel<V, K, 4, true, false, true, false, false, true>)
+                             : go_behind(sliced_spmv_kernel<V, K, 4, false, false, true, false, false, true>);
+        } else if (w <= 3 || (sizeof(V) == 8 && !ell && (w == 6 || w == 7)) || (ell && w == 4)) {
+            // tested loads, where the slots left over would be read one by one
+            // (S-ELL without padding, 1M rows of 3, FP64: 22.1 us so, 17.9 tested;
+            // of 7 36.6 and 32.7; FP32, of 3, 17.6 and 15.5)
+            bool wave = false;
+            if constexpr (sizeof(V) == 8) {
+                wave = w <= 2;
+                if (wave && plain) go(sliced_spmv_kernel<V, K, 4, true, false, false, false, true>);
+                else if (wave) go(sliced_spmv_kernel<V, K, 4, false, false, false, false, true>);
+            }
+            if (!wave) slots(std::integral_constant<int, 4>());
+        } else if (!ell || w > 12 || (sizeof(V) == 4 && (w == 7 || w == 8))) {
+            // rows of many lengths, or of more slots than registers hold at once
+            // (ELL of 8 random columns, 1M rows, FP32: 35.3 us with all of them
+            // in flight, 31.7 so)
+            bool wave = false;
+            if constexpr (sizeof(V) == 8) {
+                wave = (int64_t)grid <= 8 * num_sms() && ((int64_t)grid > 6 * num_sms() || w > 32);
+                if (wave && plain) go(sliced_spmv_kernel<V, K, 4, true, false, false, false, true, true>);
+                else if (wave) go(sliced_spmv_kernel<V, K, 4, false, false, false, false, true, true>);
+            }
+            if (!wave && plain) go(sliced_spmv_kernel<V, K, 4, true, false, false, false, false, true>);
+            else if (!wave) go(sliced_spmv_kernel<V, K, 4, false, false, false, false, false, true>);
+        } else if (w <= 6 || (sizeof(V) == 4 && w > 10)) {  // 12 at once: 53.3 us, 6 and 6: 45.0
+            slots(std::integral_constant<int, 6>());
+        } else if (w <= 8) {
+            if constexpr (sizeof(V) == 8) slots(std::integral_constant<int, 8>());
+        } else if (w <= 10) {
+            slots(std::integral_constant<int, 10>());
+        } else {
+            if constexpr (sizeof(V) == 8) slots(std::integral_constant<int, 12>());
+        }
     } else {
-        launched = nov > 0 ? go_behind(sliced_spmv_kernel<V, K, 4, false, false, true>) : go(sliced_spmv_kernel<V, K, 4>);
+        // Two FP32 right-hand sides, and any number on rows sorted by length:
+        // a fixed grid striding over the rows (5-point Laplacian 1M, FP32, k = 2,
+        // 18.1 us in blocks of 256 rows, 16.2 so; SELL-c-R of block rows k = 8
+        // 42.2 and 36.7), otherwise blocks (banded FP32 k = 4 28.0 and 29.2,
+        // FP64 k = 2 42 and 50).
+        const bool stride = (K == 2 && sizeof(V) == 4) || (K > 2 && v.sorted) || (whole && !v.reorder && p->extra_i[1] > 0);
+        if (nov > 0) {
+            launched = go_behind(sliced_spmv_kernel<V, K, 4, false, false, true>);
+        } else if (stride) {
+            grid = grid_for(v.m, kBlock, (int64_t)num_sms() * 16);
+            go(sliced_spmv_kernel<V, K, 4, false, false, false, true>);
+        } else {
+            go(sliced_spmv_kernel<V, K, 4>);
+        }
     }
     SSPMV_CUDA_TRY(launched);
     SSPMV_LAUNCH_CHECK();
@@ -1057,7 +1143,7 @@ extern "C" sspmv_status sspmv_spmm_ell(double alpha, const sspmv_ell *A, int32_t
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     Plan *p = get_plan(&A->f);
     SlicedView v{A->f.num_rows, (int32_t)std::max<int64_t>(A->f.num_rows, 1), (const int64_t *)p->extra[0], nullptr,
-                 A->col_index, A->values, 0, A->max_row_width, A->f.num_cols, A->f.num_nnzs};
+                 A->col_index, A->values, 0, A->max_row_width, A->f.num_cols, 1, false};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1132,7 +1218,7 @@ extern "C" sspmv_status sspmv_spmm_sell(double alpha, const sspmv_s_ell *A, int3
                                         double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->sliceWidth,   A->chunk_ptr,   nullptr,
-                 A->col_index,  A->values,     A->chunk_num, 0, A->f.num_cols, A->f.num_nnzs};
+                 A->col_index,  A->values,     A->chunk_num, 0, A->f.num_cols, A->alignment, false};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1206,7 +1292,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_sigma(double alpha, const sspmv_sell_c
                                                 int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols, A->f.num_nnzs};
+                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols, A->alignment, A->sliceWidth_Sigma >= A->f.num_rows};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
@@ -1275,7 +1361,7 @@ extern "C" sspmv_status sspmv_spmm_sell_c_R(double alpha, const sspmv_sell_c_R *
                                             int64_t ldx, double beta, void *Y, int64_t ldy, sspmv_stream_t s) {
     if (!A) return fail(SSPMV_INVALID_ARG, "null matrix");
     SlicedView v{A->f.num_rows, A->chunkWidth_C,   A->chunk_ptr,   A->reorder,
-                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols, A->f.num_nnzs};
+                 A->col_index,  A->values,         A->validchunkNum, 0, A->f.num_cols, A->alignment, true};
     return spmm_sliced(&A->f, v, alpha, k, X, ldx, beta, Y, ldy, s);
 }
 
