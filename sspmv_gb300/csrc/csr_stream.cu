@@ -68,10 +68,10 @@ constexpr unsigned kFull = 0xffffffffu;
 // Resident CTAs per SM the register budget is set for: the best of 16 to 24
 // (FP32) and 12 to 18 (FP64) for K = 1; spills and fewer warps cost about the
 // same beyond.
-template <typename V, int K, bool BIG = false>
+template <typename V, int K, bool BIG = false, bool PLAIN = true>
 constexpr int stream_min_ctas() {
     if (K == 1) return sizeof(V) == 8 ? 15 : 20;
-    return BIG ? 10 : sizeof(V) == 8 ? 12 : 14;
+    return BIG ? (PLAIN ? 10 : 8) : sizeof(V) == 8 ? 12 : 14;
 }
 
 // Elements per window: whole steps of 256 less what the last row may run past
@@ -82,7 +82,8 @@ int window_size(int64_t nnz, int32_t value_type) {
     return 256 * window_steps(nnz, 256, 256 - kOver, ctas * kWarps) - kOver;
 }
 
-// BIG: X does not fit in L2, a gather is a random HBM access.
+// BIG: X does not fit in L2, a gather is a random HBM access: a step's columns
+// and values are all loaded before its gathers.
 template <typename V, int K, bool BIG = false>
 struct StreamShape {
     static constexpr int G = K * (int)sizeof(V) > 16 ? K * (int)sizeof(V) / 16 : 1;  // lanes per row of X
@@ -168,9 +169,11 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
     // the first step's loads wait for nothing but the window's index; a
     // group's elements are 8 G consecutive ones, taken 8 at a time
     uint32_t e0 = (uint32_t)w * (uint32_t)A.window + 8u * G * gi;
-    int c[8];
-    V a[8];
-    load_cols8(A.col, e0, A.nnz, vec, c);
+    constexpr int NB = BIG ? G : 1;  // blocks of 8 elements loaded together
+    int cb[NB][8];
+    V ab[NB][8];
+#pragma unroll
+    for (int j = 0; j < NB; j++) load_cols8(A.col, e0 + 8 * j, A.nnz, vec, cb[j]);
     unsigned ebits = load_ends<G>(A.ends, e0, A.nnz);
     const int4 rec = __ldg(A.rec + w);
     const uint32_t eA = (uint32_t)rec.x, eB = (uint32_t)rec.y;
@@ -186,7 +189,8 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
     bool later = false;
 
     for (;;) {
-        load_vals8<V>(val, e0, A.nnz, vec, a);
+#pragma unroll
+        for (int j = 0; j < NB; j++) load_vals8<V>(val, e0 + 8 * j, A.nnz, vec, ab[j]);
         // from the end bits, under the loads: rows ended before this group
         // (pos) and in the whole step (nend), and the groups back to the one
         // whose last end opened this group's running sum (dist)
@@ -249,7 +253,9 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
                     sum[q] = V(0);
                 }
             }
-            if (j > 0) {
+            int(&c)[8] = cb[NB > 1 ? j : 0];
+            V(&a)[8] = ab[NB > 1 ? j : 0];
+            if (NB == 1 && j > 0) {
                 load_cols8(A.col, e0 + 8 * j, A.nnz, vec, c);
                 load_vals8<V>(val, e0 + 8 * j, A.nnz, vec, a);
             }
@@ -358,7 +364,8 @@ __device__ __forceinline__ void stream_window(const StreamView &A, const V *__re
         row += nend;
         if (!more) break;
         later = true;
-        load_cols8(A.col, e0, A.nnz, vec, c);
+#pragma unroll
+        for (int j = 0; j < NB; j++) load_cols8(A.col, e0 + 8 * j, A.nnz, vec, cb[j]);
         ebits = load_ends<G>(A.ends, e0, A.nnz);
     }
 
@@ -427,7 +434,7 @@ __global__ void __launch_bounds__(256) csr_split_kernel(int64_t n, const int4 *_
 // PLAIN: alpha == 1 and beta == 0 (y = sum): row writes carry no FP64
 // multiply.
 template <typename V, int K, bool PLAIN, bool BIG = false>
-__global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K, BIG>())) csr_stream_kernel(
+__global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K, BIG, PLAIN>())) csr_stream_kernel(
     const StreamView A, const V *__restrict__ x, uint32_t xrow, V alpha, V beta, V *__restrict__ y, uint32_t yrow,
     const StreamSlots<V> sl, int xvec, int yvec) {
     const int64_t w = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
@@ -656,12 +663,15 @@ StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, co
 }
 
 // An X of more bytes than this does not stay in L2 (129 MB, less what the matrix
-// and Y take): its gathers wait for HBM, and the form with twice the gathers in
-// flight, fewer warps and Y written past L2 is the faster one (FP32, k = 8: 4.2M
-// rows 755 us, 715 so; FP64, k = 4, 4M rows: 814, 800), where with X in L2 it is
-// the slower one (2M rows FP32 231 us, 251 so).  For rows of X of 32 bytes: with
-// 64 the registers do not hold it (FP64, k = 8, 2M rows: 650, 655 so).
-constexpr int64_t kBigX = int64_t(100) << 20;
+// and Y take): its gathers wait for HBM, and the form that loads all of a step's
+// columns and values before its first gathers, with twice the gathers in flight,
+// fewer warps and Y written past L2 is the faster one.  For rows of X of 32 bytes
+// (of 64 the registers do not hold it).  FP32, k = 8: 83 MB power-law 314 us, 297
+// so, uniform 278 and 241, banded 144 and 152; 64 MB power-law 214 and 222; 512 MB
+// 5.02 ms and 4.72.  With alpha and beta 83 MB 396 and 415, 96 MB 488 and 490,
+// 134 MB 804 and 783.  FP64, k = 4: 96 MB 541 and 531, 64 MB 337 and 351.
+constexpr int64_t kBigX = int64_t(80) << 20;
+constexpr int64_t kBigXScaled = int64_t(100) << 20;
 
 template <typename V, int K>
 sspmv_status launch_stream_windows(const StreamView &v, StreamPlan &sp, V alpha, const V *x, int64_t ldx, V beta,
@@ -675,7 +685,7 @@ sspmv_status launch_stream_windows(const StreamView &v, StreamPlan &sp, V alpha,
     const bool plain = alpha == V(1) && beta == V(0);
     bool big = false;
     if constexpr (K * sizeof(V) == 32) {
-        big = cols * ldx * (int64_t)sizeof(V) > kBigX;
+        big = cols * ldx * (int64_t)sizeof(V) > (plain ? kBigX : kBigXScaled);
         if (big && plain) go(csr_stream_kernel<V, K, true, true>);
         else if (big) go(csr_stream_kernel<V, K, false, true>);
     }
