@@ -350,13 +350,18 @@ __global__ void __launch_bounds__(kStreamBlock, (bsr_ctas<V, C>())) bsr_stream_k
 
 // out[0]: lane slots the thread-per-row kernel spends (every warp of 32 rows,
 // 32 / r block rows, runs as many block iterations as its longest block row);
-// out[1]: block rows without blocks, for the stream plan.
-__global__ void bsr_row_kernel_slots(int64_t mb, int lr, const int32_t *__restrict__ row_ptr,
-                                     unsigned long long *__restrict__ out) {
+// out[1]: block rows without blocks, and tiles[b].x the block's with, for the
+// stream plan.
+__global__ void __launch_bounds__(kBlock) bsr_row_kernel_slots(int64_t mb, int64_t rows, int lr,
+                                                               const int32_t *__restrict__ row_ptr,
+                                                               unsigned long long *__restrict__ out,
+                                                               int2 *__restrict__ tiles) {
+    __shared__ int s_empty[kBlock / 32];
     const int64_t per = 32 >> lr;
-    const int64_t groups = (mb + per - 1) / per;
-    unsigned long long acc = 0, empty = 0;
-    for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < groups; w += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t w0 = (int64_t)blockIdx.x * rows / per, w1 = min(w0 + rows / per, (mb + per - 1) / per);
+    unsigned long long acc = 0;
+    int empty = 0;
+    for (int64_t w = w0 + threadIdx.x; w < w1; w += kBlock) {
         int32_t mx = 0;
         const int64_t b1 = min(mb, (w + 1) * per);
         for (int64_t b = w * per; b < b1; b++) {
@@ -370,8 +375,13 @@ __global__ void bsr_row_kernel_slots(int64_t mb, int lr, const int32_t *__restri
     empty = warp_sum(empty);
     if ((threadIdx.x & 31) == 0) {
         if (acc) atomicAdd(out, acc);
-        if (empty) atomicAdd(out + 1, empty);
+        s_empty[threadIdx.x >> 5] = empty;
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < kBlock / 32; w++) empty += s_empty[w];
+    if (empty) atomicAdd(out + 1, (unsigned long long)empty);
+    tiles[blockIdx.x] = make_int2((int)(min(rows, mb - blockIdx.x * rows) - empty), 0);
 }
 
 int log2_exact(int64_t v) {
@@ -390,27 +400,30 @@ constexpr double kStreamWaste = 2.0;
 
 // extra_i[2], decided once and published in one word: bits 0-1, 1 = block-stream
 // kernel, 2 = thread-per-row kernel; above them the block rows without blocks.
+// extra[3]: for the block-stream kernel, the tiles' counts until its plan is built.
 sspmv_status choose_bsr_kernel(const sspmv_bsr *A, Plan *p, sspmv_stream_t s) {
     if (p->extra_i[2]) return SSPMV_OK;
     std::lock_guard<PlanMutex> guard(plan_mutex());
     if (p->extra_i[2]) return SSPMV_OK;
     const int lr = log2_exact(A->blockDim_r);
+    const int64_t rows = stream_tile_rows(A->mb), tiles = (A->mb + rows - 1) / rows;
     unsigned long long *d = nullptr, h[2] = {0, 0};
-    SSPMV_TRY(dalloc(&d, 2, s));
+    SSPMV_TRY(dalloc(&d, 2 + (size_t)tiles, s));  // the sums, then the tiles
+    int2 *tile = (int2 *)(d + 2);
     auto body = [&]() -> sspmv_status {
         SSPMV_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(h), cu(s)));
-        const int64_t groups = (A->mb + (32 >> lr) - 1) / (32 >> lr);
-        bsr_row_kernel_slots<<<grid_for(groups, 256, (int64_t)num_sms() * 16), 256, 0, cu(s)>>>(A->mb, lr, A->row_ptr,
-                                                                                              d);
+        bsr_row_kernel_slots<<<(unsigned)tiles, kBlock, 0, cu(s)>>>(A->mb, rows, lr, A->row_ptr, d, tile);
         SSPMV_LAUNCH_CHECK();
         SSPMV_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, cu(s)));
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
         return SSPMV_OK;
     };
     const sspmv_status st = body();
-    dfree(d, s);
+    const bool stream = st == SSPMV_OK && (double)h[0] > kStreamWaste * (double)A->nnzb;
+    if (stream) p->extra[3] = d;
+    else dfree(d, s);
     if (st != SSPMV_OK) return st;
-    p->extra_i[2] = ((int64_t)h[1] << 2) | ((double)h[0] > kStreamWaste * (double)A->nnzb ? 1 : 2);
+    p->extra_i[2] = ((int64_t)h[1] << 2) | (stream ? 1 : 2);
     return SSPMV_OK;
 }
 
@@ -421,9 +434,15 @@ sspmv_status launch_bsr_stream(const sspmv_bsr *A, Plan *p, V alpha, const V *x,
     const int64_t mean = A->mb > 0 ? (A->nnzb + A->mb - 1) / A->mb : 1;
     const int slack = (int)std::min<int64_t>(step / 4, mean + 1);
     const int n = window_steps(A->nnzb, step, step - slack, bsr_ctas<V, C>() * (kStreamBlock / 32));
-    const int64_t chosen = p->extra_i[2];
-    SSPMV_TRY(ensure_stream_plan(p->stream, A->mb, A->nnzb, A->row_ptr, nullptr, A->f.value_type, s,
-                                 step * n - slack, 0x7fffffff, chosen ? chosen >> 2 : -1));
+    if (!p->stream.window) {
+        std::lock_guard<PlanMutex> guard(plan_mutex());
+        const unsigned long long *d = (const unsigned long long *)p->extra[3];
+        SSPMV_TRY(ensure_stream_plan(p->stream, A->mb, A->nnzb, A->row_ptr, nullptr, A->f.value_type, s,
+                                     step * n - slack, 0x7fffffff, d ? p->extra_i[2] >> 2 : -1,
+                                     d ? (const int2 *)(d + 2) : nullptr));
+        dfree(p->extra[3], s);
+        p->extra[3] = nullptr;
+    }
     const StreamView v = stream_view(p->stream, A->nnzb, A->block_colindex, A->block_data);
     const size_t run = std::min<size_t>(16, C * sizeof(V));
     const int xvec = reinterpret_cast<uintptr_t>(x) % run == 0 ? 1 : 0;

@@ -37,12 +37,14 @@ int window_steps(int64_t nnz, int step, int first, int warps_per_sm);
 // row_map: y row of each row (rows then all nonempty; null: the row itself),
 // owned by the caller and kept as long as the plan.
 // window, over: elements per window and past it that its warp may read to
-// finish a row (0, -1: the stream kernel's own).  nempty: the rows without
-// elements where the caller has counted them and `over` leaves no row to split
-// (-1: counted here, which waits for the device).
+// finish a row (0, -1: the stream kernel's own).  nempty, counted: the rows
+// without elements and, per tile of stream_tile_rows(m) rows, .x of those with,
+// where the caller has counted them and `over` leaves no row to split (null:
+// counted here, which waits for the device).
+int64_t stream_tile_rows(int64_t m);  // a multiple of 1024
 sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
                                 const int32_t *row_map, int32_t value_type, sspmv_stream_t s, int window = 0,
-                                int over = -1, int64_t nempty = -1);
+                                int over = -1, int64_t nempty = -1, const int2 *counted = nullptr);
 void free_stream_plan(StreamPlan &sp, sspmv_stream_t s);
 StreamView stream_view(const StreamPlan &sp, int64_t nnz, const int32_t *col, const void *val);
 

@@ -36,9 +36,10 @@ struct StreamPlan {
     void *tail_val = nullptr;  // [windows * kMaxK] piece of the split row that goes on past the window
     void *head_val = nullptr;  // [windows * kMaxK] last piece of the split row that ends in the window
     int32_t *nzrow = nullptr;  // y row of the i-th nonempty row (null: i itself)
-    bool owns_nzrow = false;
     int32_t *empty = nullptr;  // rows without nonzeros
     int64_t nempty = 0;
+    unsigned char *slab = nullptr;  // the allocation that holds all of these (but a caller's nzrow)
+    int64_t bytes = 0;              // of it
 };
 
 struct Plan {
