@@ -37,10 +37,10 @@ int window_steps(int64_t nnz, int step, int first, int warps_per_sm);
 // row_map: y row of each row (rows then all nonempty; null: the row itself),
 // owned by the caller and kept as long as the plan.
 // window, over: elements per window and past it that its warp may read to
-// finish a row (0, -1: the stream kernel's own).  nempty, counted: the rows
-// without elements and, per tile of stream_tile_rows(m) rows, .x of those with,
-// where the caller has counted them and `over` leaves no row to split (null:
-// counted here, which waits for the device).
+// finish a row (0, -1: the stream kernel's own).  nempty: the rows without
+// elements where the caller has counted them and no row is split (-1: counted
+// here, which waits for the device); counted: if there are any, per tile of
+// stream_tile_rows(m) rows, .x of those with elements.
 int64_t stream_tile_rows(int64_t m);  // a multiple of 1024
 sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const int32_t *row_offset,
                                 const int32_t *row_map, int32_t value_type, sspmv_stream_t s, int window = 0,
@@ -110,6 +110,9 @@ __device__ __forceinline__ void scale_empty_rows(const StreamView &A, int64_t un
         }
     }
 }
+
+// Rows of at most this many elements are never split (0, -1 for window, over).
+constexpr int kStreamWholeRow = 33;
 
 // The kernel steps through X and Y in 32-bit byte strides.
 inline bool stream_takes_strides(int64_t ldx, int64_t ldy, size_t value_bytes) {

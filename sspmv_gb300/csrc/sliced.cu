@@ -379,7 +379,7 @@ constexpr double kWarpSlotPs = 73.0;
 constexpr double kSlotChainPs = 0.5e6;
 constexpr double kNnzPs = 3.9;
 constexpr double kOvfRowPs = 20.0;
-constexpr double kOvfLaunchPs = 4.0e6;
+constexpr double kOvfLaunchPs = 5.0e6;
 // Rows sorted by length over the whole matrix leave no lane of a warp idle, and the
 // longest ones start first: without very long ones they stay in the thread pass
 // (SELL-c-R, 1.5M 4x4 block rows of up to 28: FP32 27.3 us with a cap of 8, 19.5
@@ -410,17 +410,15 @@ int choose_cap(const CapStats (&st)[kNumCaps], int64_t m, int64_t total_nnz) {
 
 void free_overflow(Plan *p, sspmv_stream_t s) {
     free_stream_plan(p->stream, s);
-    for (int e : {0, 1, 2}) {
-        dfree(p->extra[e], s);
-        p->extra[e] = nullptr;
-    }
+    dfree(p->extra[0], s);
+    p->extra[0] = nullptr;
     p->extra_i[1] = p->extra_i[4] = 0;
 }
 
 // Overflow plan of a sliced matrix, built on its first SpMV (and again after
-// sspmv_set_kernel changes the cap).  extra[0] y row of every overflow row
-// (the stream plan's row list), extra[1] / extra[2] their columns / values;
-// p->stream the stream plan; extra_i[1] overflow rows, [2] the cap, [3] the
+// sspmv_set_kernel changes the cap).  extra[0] y row of every overflow row (the
+// stream plan's row list), then, extra_i[8] and [9] bytes on, their columns and
+// values; p->stream the stream plan; extra_i[1] overflow rows, [2] the cap, [3] the
 // kernel parameter the plan was built for, [4] overflow nonzeros, [5] the
 // longest row, [7] built.
 sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, Plan *p, sspmv_stream_t s) {
@@ -432,43 +430,42 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
     const int64_t m = v.m;
     const unsigned grid = grid_for(m, 256, (int64_t)num_sms() * 32);
     const size_t sv = vsize(f->value_type);
-    int32_t *len = nullptr, *rows = nullptr, *optr = nullptr;
-    int64_t *pos = nullptr;
-    CapStats *dst = nullptr;
+    unsigned char *stats = nullptr, *temp = nullptr;  // lengths and the caps' statistics; positions and row lists
     CapList caps = kCaps;
     if (p->param > 0) caps.cap[0] = p->param;
     int64_t nov = 0, novf = 0, cap = kNoCap, longest = 0;
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     auto build = [&]() -> sspmv_status {
-        SSPMV_TRY(dalloc(&len, (size_t)m, s));
-        SSPMV_TRY(dalloc(&dst, kNumCaps, s));
-        SSPMV_CUDA_TRY(cudaMemsetAsync(dst, 0, kNumCaps * sizeof(CapStats), cu(s)));
+        CapStats st[kNumCaps];
+        SSPMV_TRY(dalloc(&stats, up(sizeof(st)) + (size_t)m * 4, s));
+        CapStats *dst = (CapStats *)stats;
+        int32_t *len = (int32_t *)(stats + up(sizeof(st)));
+        SSPMV_CUDA_TRY(cudaMemsetAsync(dst, 0, sizeof(st), cu(s)));
         stored_row_lengths<<<grid, 256, 0, cu(s)>>>(m, v.C, v.chunk_ptr, v.col, len);
         SSPMV_LAUNCH_CHECK();
         cap_stats<<<grid_for(m, kBlock, (int64_t)num_sms() * 4), kBlock, 0, cu(s)>>>(m, len, caps, dst);
         SSPMV_LAUNCH_CHECK();
-        CapStats st[kNumCaps];
         SSPMV_CUDA_TRY(cudaMemcpyAsync(st, dst, sizeof(st), cudaMemcpyDeviceToHost, cu(s)));
         SSPMV_CUDA_TRY(cudaStreamSynchronize(cu(s)));
-        const bool whole = v.sorted && m > kWholeRows && st[kNumCaps - 1].longest <= (unsigned long long)kShortRow;
+        longest = (int64_t)st[kNumCaps - 1].longest;
+        const bool whole = v.sorted && m > kWholeRows && longest <= kShortRow;
         const int pick = p->param > 0 ? 0 : whole ? kNumCaps - 1 : choose_cap(st, m, f->num_nnzs);
         cap = caps.cap[pick];
-        longest = (int64_t)st[kNumCaps - 1].longest;
         nov = (int64_t)st[pick].rows;
         novf = (int64_t)st[pick].nnz;
         if (novf > 0x7fffffff) return fail(SSPMV_NOT_SUPPORTED, "overflow of the long rows exceeds the int32 range");
         if (nov == 0) return SSPMV_OK;
-        int32_t *yrow = nullptr, *ocol = nullptr;
-        unsigned char *oval = nullptr;
-        SSPMV_TRY(dalloc(&pos, (size_t)m, s));
-        SSPMV_TRY(dalloc(&rows, (size_t)nov, s));
-        SSPMV_TRY(dalloc(&optr, (size_t)nov + 1, s));
-        // each kept buffer belongs to the plan as soon as it exists (free_overflow)
-        SSPMV_TRY(dalloc(&yrow, (size_t)nov, s));
-        p->extra[0] = yrow;
-        SSPMV_TRY(dalloc(&ocol, (size_t)novf, s));
-        p->extra[1] = ocol;
-        SSPMV_TRY(dalloc(&oval, (size_t)novf * sv, s));
-        p->extra[2] = oval;
+        const size_t rows_at = up((size_t)m * 8), optr_at = rows_at + up((size_t)nov * 4);
+        SSPMV_TRY(dalloc(&temp, optr_at + ((size_t)nov + 1) * 4, s));
+        int64_t *pos = (int64_t *)temp;
+        int32_t *rows = (int32_t *)(temp + rows_at), *optr = (int32_t *)(temp + optr_at);
+        const size_t col_at = up((size_t)nov * 4), val_at = col_at + up((size_t)novf * 4);
+        unsigned char *kept = nullptr;  // the plan's as soon as it exists (free_overflow)
+        SSPMV_TRY(dalloc(&kept, val_at + (size_t)novf * sv, s));
+        p->extra[0] = kept;
+        p->extra_i[8] = (int64_t)col_at;
+        p->extra_i[9] = (int64_t)val_at;
+        int32_t *yrow = (int32_t *)kept, *ocol = (int32_t *)(kept + col_at);
         overflow_flags<<<grid, 256, 0, cu(s)>>>(m, cap, len, pos);
         SSPMV_LAUNCH_CHECK();
         SSPMV_TRY(exclusive_scan_i64(pos, pos, m, nullptr, s));
@@ -477,14 +474,17 @@ sspmv_status ensure_overflow_plan(const sspmv_features *f, const SlicedView &v, 
         SSPMV_TRY(dispatch_value(f->value_type, [&](auto tag) -> sspmv_status {
             using V = decltype(tag);
             copy_overflow<V><<<grid_for(novf, kCopyTile), kBlock, 0, cu(s)>>>(
-                nov, (int32_t)novf, v.C, rows, optr, v.chunk_ptr, v.col, (const V *)v.val, ocol, (V *)oval);
+                nov, (int32_t)novf, v.C, rows, optr, v.chunk_ptr, v.col, (const V *)v.val, ocol, (V *)(kept + val_at));
             SSPMV_LAUNCH_CHECK();
             return SSPMV_OK;
         }));
-        return ensure_stream_plan(p->stream, nov, novf, optr, yrow, f->value_type, s);
+        // no empty rows, and no split ones to wait for if all are short
+        return ensure_stream_plan(p->stream, nov, novf, optr, yrow, f->value_type, s, 0, -1,
+                                  longest <= kStreamWholeRow ? 0 : -1);
     };
     const sspmv_status st = build();
-    for (void *t : {(void *)len, (void *)pos, (void *)rows, (void *)optr, (void *)dst}) dfree(t, s);
+    dfree(stats, s);
+    dfree(temp, s);
     SSPMV_TRY(st);
     p->extra_i[1] = nov;
     p->extra_i[2] = nov > 0 ? cap : kNoCap;
@@ -505,7 +505,8 @@ sspmv_status launch_sliced(const SlicedView &v, Plan *p, V alpha, const V *x, in
     const int64_t nov = p && !whole && stream_takes_strides(ldx, ldy, sizeof(V)) ? p->extra_i[1] : 0;
     StreamView lv;
     if (nov > 0) {  // the long rows first: the thread pass starts under their last wave
-        lv = stream_view(p->stream, p->extra_i[4], (const int32_t *)p->extra[1], p->extra[2]);
+        const unsigned char *kept = (const unsigned char *)p->extra[0];
+        lv = stream_view(p->stream, p->extra_i[4], (const int32_t *)(kept + p->extra_i[8]), kept + p->extra_i[9]);
         SSPMV_TRY((launch_stream_windows<V, K>(lv, p->stream, alpha, x, ldx, beta, y, ldy, v.cols, s)));
     }
     // A thread per row and no grid stride: a fixed grid gave the same blocks the
