@@ -5,6 +5,7 @@
 #include <cstring>
 #include <cuda.h>
 #include <mutex>
+#include <unordered_map>
 
 #include "common.cuh"
 #include "csr_stream.cuh"
@@ -69,39 +70,57 @@ constexpr int kMaxDevices = 64;
 struct DevicePool {
     cudaMemPool_t pool = nullptr;
     unsigned long long ctx = 0;
+    int64_t live_bytes = 0, live_blocks = 0;
+    uint64_t threshold = 0;  // release threshold set
+    bool used = false;       // since it was last emptied
+};
+struct Block {
+    size_t bytes;
+    int dev;
 };
 std::mutex g_pool_mutex;
 DevicePool g_pools[kMaxDevices];
-std::atomic<long long> g_live_blocks{0};
+std::unordered_map<void *, Block> g_blocks;  // live ones
+
+// The release threshold bounds all that the pool holds, live blocks included: it
+// follows them, in steps (a call each), so that kPoolKeepBytes more are kept.
+// g_pool_mutex held.
+cudaError_t follow_live(DevicePool &d) {
+    const uint64_t want = (uint64_t)d.live_bytes / kPoolStepBytes * kPoolStepBytes + kPoolKeepBytes;
+    if (want == d.threshold) return cudaSuccess;
+    uint64_t v = want;
+    const cudaError_t e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &v);
+    if (e == cudaSuccess) d.threshold = want;
+    return e;
+}
 
 // The current device's pool, made on first use (and again after a
 // cudaDeviceReset ended the context it belonged to).
-cudaError_t current_pool(cudaMemPool_t *out) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+cudaError_t current_pool(int *dev, cudaMemPool_t *out) {
+    cudaError_t e = cudaGetDevice(dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    if (*dev < 0 || *dev >= kMaxDevices) return cudaErrorInvalidDevice;
     unsigned long long ctx = current_context_id();
-    if (ctx == 0 && (e = cudaSetDevice(dev)) == cudaSuccess) ctx = current_context_id();  // no context yet: made here
+    if (ctx == 0 && (e = cudaSetDevice(*dev)) == cudaSuccess) ctx = current_context_id();  // no context yet: made here
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> g(g_pool_mutex);
-    DevicePool &d = g_pools[dev];
+    DevicePool &d = g_pools[*dev];
     if (!d.pool || d.ctx != ctx) {
         cudaMemPoolProps props;
         std::memset(&props, 0, sizeof(props));
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
-        uint64_t keep = kPoolKeepBytes;
-        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e != cudaSuccess) {
-            cudaMemPoolDestroy(pool);
+        props.location.id = *dev;
+        DevicePool fresh;
+        fresh.ctx = ctx;
+        if ((e = cudaMemPoolCreate(&fresh.pool, &props)) != cudaSuccess) return e;
+        if ((e = follow_live(fresh)) != cudaSuccess) {
+            cudaMemPoolDestroy(fresh.pool);
             return e;
         }
-        d.pool = pool;
-        d.ctx = ctx;
+        for (auto it = g_blocks.begin(); it != g_blocks.end();)  // went with the old context
+            it = it->second.dev == *dev ? g_blocks.erase(it) : std::next(it);
+        d = fresh;
     }
     *out = d.pool;
     return cudaSuccess;
@@ -109,8 +128,9 @@ cudaError_t current_pool(cudaMemPool_t *out) {
 }  // namespace
 
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
+    int dev = 0;
     cudaMemPool_t pool = nullptr;
-    cudaError_t e = current_pool(&pool);
+    cudaError_t e = current_pool(&dev, &pool);
     if (e != cudaSuccess) return e;
     e = cudaMallocFromPoolAsync(p, bytes, pool, s);
     if (e == cudaErrorMemoryAllocation) {  // once more with nothing kept back
@@ -118,24 +138,53 @@ cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(p, bytes, pool, s);
     }
-    if (e == cudaSuccess) g_live_blocks.fetch_add(1, std::memory_order_relaxed);
-    return e;
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> g(g_pool_mutex);
+    DevicePool &d = g_pools[dev];
+    g_blocks[*p] = Block{bytes, dev};
+    d.live_bytes += (int64_t)bytes;
+    d.live_blocks++;
+    d.used = true;
+    follow_live(d);
+    return cudaSuccess;
 }
 
 void pool_free(void *p, cudaStream_t s) {
+    {
+        std::lock_guard<std::mutex> g(g_pool_mutex);
+        const auto it = g_blocks.find(p);
+        if (it != g_blocks.end()) {
+            DevicePool &d = g_pools[it->second.dev];
+            d.live_bytes -= (int64_t)it->second.bytes;
+            d.live_blocks--;
+            g_blocks.erase(it);
+            follow_live(d);
+        }
+    }
     cudaFreeAsync(p, s);
-    g_live_blocks.fetch_sub(1, std::memory_order_relaxed);
+}
+
+void give_back_idle_pools() {
+    cudaMemPool_t idle[kMaxDevices];
+    int n = 0;
+    {
+        std::lock_guard<std::mutex> g(g_pool_mutex);
+        for (DevicePool &d : g_pools)
+            if (d.pool && d.used && d.live_blocks == 0) {
+                d.used = false;
+                idle[n++] = d.pool;
+            }
+    }
+    if (n == 0) return;
+    cudaStreamSynchronize(nullptr);  // the frees just queued
+    for (int i = 0; i < n; i++) cudaMemPoolTrimTo(idle[i], 0);
 }
 
 DeleteScope::DeleteScope() {
     if (g_delete_nosync == 0) cudaDeviceSynchronize();
 }
 DeleteScope::~DeleteScope() {
-    if (g_delete_nosync != 0 || g_live_blocks.load(std::memory_order_relaxed) != 0) return;
-    cudaMemPool_t pool = nullptr;
-    if (current_pool(&pool) != cudaSuccess) return;
-    cudaStreamSynchronize(nullptr);  // the frees just queued
-    cudaMemPoolTrimTo(pool, 0);
+    if (g_delete_nosync == 0) give_back_idle_pools();
 }
 
 PlanMutex &plan_mutex() {

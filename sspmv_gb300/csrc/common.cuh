@@ -46,15 +46,21 @@ inline cudaStream_t cu(sspmv_stream_t s) { return reinterpret_cast<cudaStream_t>
 // ---------------------------------------------------------------- memory --
 // Library-owned device allocations are stream ordered, from a memory pool of
 // the library's own (one per device and context) that keeps up to
-// kPoolKeepBytes of freed memory for the next allocation.  The device's default
-// pool keeps none: it unmaps freed memory at the next synchronisation and maps
-// it again, 0.4 of the 1.1 ms a 500k-row matrix took to convert and multiply
-// for the first time (1121 -> 713 us).  What is kept goes back to the
-// device when the last matrix is deleted, and when an allocation fails.
+// kPoolKeepBytes of freed memory, beside the live blocks, for the next
+// allocation.  The device's default pool keeps none: it unmaps freed memory at
+// the next synchronisation and maps it again, 0.4 of the 1.1 ms a 500k-row
+// matrix took to convert and multiply for the first time (1121 -> 713 us).  All
+// that is kept goes back to the device when a matrix or a request server is
+// deleted and no live block is left on it, and when an allocation fails; a
+// program that only releases plans (sspmv_release_plan) keeps its up to 1 GiB.
+// Settings of the device's default pool do not reach this one.
 // Safe from any thread and stream: the pool orders reuse by stream.
 constexpr uint64_t kPoolKeepBytes = 1ull << 30;
+constexpr uint64_t kPoolStepBytes = 64ull << 20;
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
 void pool_free(void *p, cudaStream_t s);
+// Empties the pools without live blocks.
+void give_back_idle_pools();
 
 template <typename T>
 sspmv_status dalloc(T **p, size_t count, sspmv_stream_t s) {
@@ -79,8 +85,8 @@ struct DeleteWithoutDeviceSync {
     DeleteWithoutDeviceSync();
     ~DeleteWithoutDeviceSync();
 };
-// The body of an sspmv_delete_<fmt>: waits on entry; when the last live block
-// of the library went with the matrix, the pool's kept memory is given back.
+// The body of an sspmv_delete_<fmt>: waits on entry; when a device's last live
+// block went with the matrix, what its pool kept is given back.
 struct DeleteScope {
     DeleteScope();
     ~DeleteScope();

@@ -313,6 +313,7 @@ void Server::shutdown() {
         cudaStreamDestroy(load_stream);
     }
     if (capture_stream) cudaStreamDestroy(capture_stream);
+    give_back_idle_pools();
 }
 
 // -------------------------------------------------------------- residency --
