@@ -128,6 +128,11 @@ cudaError_t current_pool(int *dev, cudaMemPool_t *out) {
 }  // namespace
 
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
+    // Under capture the block belongs to the graph, whatever pool is named, and a
+    // pool cannot be made (it ends the capture).
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
+    if (capture == cudaStreamCaptureStatusActive) return cudaMallocAsync(p, bytes, s);
     int dev = 0;
     cudaMemPool_t pool = nullptr;
     cudaError_t e = current_pool(&dev, &pool);
@@ -153,7 +158,7 @@ void pool_free(void *p, cudaStream_t s) {
     {
         std::lock_guard<std::mutex> g(g_pool_mutex);
         const auto it = g_blocks.find(p);
-        if (it != g_blocks.end()) {
+        if (it != g_blocks.end()) {  // not a graph's
             DevicePool &d = g_pools[it->second.dev];
             d.live_bytes -= (int64_t)it->second.bytes;
             d.live_blocks--;
