@@ -169,6 +169,12 @@ void pool_free(void *p, cudaStream_t s) {
     cudaFreeAsync(p, s);
 }
 
+int64_t block_bytes(const void *p) {
+    std::lock_guard<std::mutex> g(g_pool_mutex);
+    const auto it = g_blocks.find(const_cast<void *>(p));
+    return it == g_blocks.end() ? 0 : (int64_t)it->second.bytes;
+}
+
 void give_back_idle_pools() {
     cudaMemPool_t idle[kMaxDevices];
     int n = 0;
@@ -202,6 +208,16 @@ Plan *get_plan(const sspmv_features *f) {
     std::lock_guard<PlanMutex> g(plan_mutex());
     if (!f->priv) const_cast<sspmv_features *>(f)->priv = new (std::nothrow) Plan();
     return reinterpret_cast<Plan *>(f->priv);
+}
+
+int64_t plan_bytes(const sspmv_features *f) {
+    const Plan *p = reinterpret_cast<const Plan *>(f->priv);
+    if (!p) return 0;
+    std::lock_guard<PlanMutex> g(plan_mutex());
+    int64_t n = block_bytes(p->stream.slab) + block_bytes(p->merge.carry_row) + block_bytes(p->merge.has_end) +
+                block_bytes(p->merge.carry_val) + block_bytes(p->merge.head_val);
+    for (const void *e : p->extra) n += block_bytes(e);
+    return n;
 }
 
 void free_plan(sspmv_features *f, sspmv_stream_t s) {

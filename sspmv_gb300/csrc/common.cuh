@@ -59,6 +59,8 @@ constexpr uint64_t kPoolKeepBytes = 1ull << 30;
 constexpr uint64_t kPoolStepBytes = 64ull << 20;
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
 void pool_free(void *p, cudaStream_t s);
+// Bytes asked for in a live block (0 for anything else).
+int64_t block_bytes(const void *p);
 // Empties the pools without live blocks.
 void give_back_idle_pools();
 

@@ -671,7 +671,6 @@ sspmv_status ensure_stream_plan(StreamPlan &sp, int64_t m, int64_t nnz, const in
         q.head_val = q.slab + head;
         q.nzrow = lists ? (int32_t *)(q.slab + nz) : const_cast<int32_t *>(row_map);
         q.empty = (int32_t *)(q.slab + em);
-        q.bytes = (int64_t)bytes;
         if (lists) SSPMV_TRY(dalloc(&pos, (size_t)m, s));
         SSPMV_CUDA_TRY(cudaMemsetAsync(q.ends, 0, words * 4, cu(s)));
         auto fill = [&](auto kernel) {

@@ -39,7 +39,6 @@ struct StreamPlan {
     int32_t *empty = nullptr;  // rows without nonzeros
     int64_t nempty = 0;
     unsigned char *slab = nullptr;  // the allocation that holds all of these (but a caller's nzrow)
-    int64_t bytes = 0;              // of it
 };
 
 struct Plan {
@@ -58,6 +57,7 @@ using PlanMutex = std::recursive_mutex;
 PlanMutex &plan_mutex();
 Plan *get_plan(const sspmv_features *f);  // creates an empty plan if needed
 void free_plan(sspmv_features *f, sspmv_stream_t s);
+int64_t plan_bytes(const sspmv_features *f);  // device memory of the plan as it is
 
 // Allocates (once) the merge-path scratch of a matrix.
 sspmv_status ensure_merge_plan(MergePlan &mp, int64_t m, int64_t nnz, int32_t value_type, sspmv_stream_t s);

@@ -70,7 +70,8 @@ struct Matrix {
     const void *h_val = nullptr;
     bool resident = false;
     DeviceMatrix dev;
-    int64_t bytes = 0;
+    int64_t bytes = 0;       // counted against the budget
+    bool counted = false;    // with the plan that the first product builds
     int64_t refs = 0;        // requests in batches not yet completed (or being formed)
     uint64_t last_use = 0;   // LRU clock
     StreamView view;                     // CSR: what the batched stream kernel reads
@@ -123,22 +124,44 @@ struct Batch {
     sspmv_status st = SSPMV_OK;
 };
 
-// Device bytes a resident matrix holds (arrays; plans counted at a bound of
-// their window records and split-row slots).
+// The features of a resident matrix, whose plan hangs off them.
+const sspmv_features &features_of(const Matrix &M) {
+    const DeviceMatrix &d = M.dev;
+    switch (M.fmt) {
+    case SSPMV_FMT_COO: return d.coo.f;
+    case SSPMV_FMT_ELL: return d.ell.f;
+    case SSPMV_FMT_SELL: return d.sell.f;
+    case SSPMV_FMT_SELL_C_SIGMA: return d.scs.f;
+    case SSPMV_FMT_SELL_C_R: return d.scr.f;
+    case SSPMV_FMT_DIA: return d.dia.f;
+    case SSPMV_FMT_BSR: return d.bsr.f;
+    case SSPMV_FMT_CSR5: return d.csr5.f;
+    default: return d.csr.f;
+    }
+}
+
+// Most that the plan of a CSR matrix takes while it is built: end bits, records
+// and pieces of windows of 224 nonzeros, row lists and their positions.
+int64_t stream_plan_bound(int64_t m, int64_t nnz, int64_t V) {
+    return nnz / 8 + (nnz / 224 + 1) * (2 * (int64_t)sizeof(int4) + 2 * kMaxK * V) + 8 * m + (1 << 16);
+}
+
+// Device bytes a resident matrix holds: its arrays, and its plan as it is (CSR's
+// is built with the matrix, the other formats' by the first product).
 int64_t device_bytes(const Matrix &M) {
     const int64_t V = (int64_t)vsize(M.vt), m = M.m, nnz = M.nnz;
-    const int64_t plan = 2 * ((m + nnz) / 1024 + 2) * 152;
+    const int64_t plan = plan_bytes(&features_of(M));
     const DeviceMatrix &d = M.dev;
     switch (M.fmt) {
     case SSPMV_FMT_CSR: return (m + 1) * 4 + nnz * (4 + V) + plan;
     case SSPMV_FMT_COO: return nnz * (8 + V) + plan;
-    case SSPMV_FMT_ELL: return m * (int64_t)d.ell.max_row_width * (4 + V);
+    case SSPMV_FMT_ELL: return m * (int64_t)d.ell.max_row_width * (4 + V) + plan;
     case SSPMV_FMT_SELL: return d.sell.total_slots * (4 + V) + (int64_t)d.sell.chunk_num * 12 + 8 + plan;
     case SSPMV_FMT_SELL_C_SIGMA:
         return d.scs.total_slots * (4 + V) + (int64_t)d.scs.validchunkNum * 12 + 8 + m * 4 + plan;
     case SSPMV_FMT_SELL_C_R: return d.scr.total_slots * (4 + V) + (int64_t)d.scr.validchunkNum * 12 + 8 + m * 4 + plan;
-    case SSPMV_FMT_DIA: return (int64_t)d.dia.stride * d.dia.complete_ndiags * V + (int64_t)d.dia.complete_ndiags * 8;
-    case SSPMV_FMT_BSR: return d.bsr.nnzb * (d.bsr.blockNNZ * V + 4) + (d.bsr.mb + 1) * 4;
+    case SSPMV_FMT_DIA: return (int64_t)d.dia.stride * d.dia.complete_ndiags * V + (int64_t)d.dia.complete_ndiags * 8 + plan;
+    case SSPMV_FMT_BSR: return d.bsr.nnzb * (d.bsr.blockNNZ * V + 4) + (d.bsr.mb + 1) * 4 + plan;
     case SSPMV_FMT_CSR5:
         return (m + 1) * 4 + nnz * (4 + V) + ((int64_t)d.csr5._p + 1) * 8 +
                (int64_t)d.csr5._p * d.csr5.omega * d.csr5.num_packets * 4 + (int64_t)d.csr5.num_offsets * 4 + plan;
@@ -365,6 +388,7 @@ sspmv_status Server::load(Matrix &M) {
     M.ev_stream = nullptr;
     M.resident = true;
     M.bytes = device_bytes(M);
+    M.counted = false;
     return SSPMV_OK;
 }
 
@@ -378,9 +402,10 @@ sspmv_status Server::ensure_resident(Matrix &M, bool *wait) {
     // transient peak of a load: the CSR plus a converted copy (padding allowed for)
     const int64_t need = M.fmt == SSPMV_FMT_CSR ? csr_bytes + 2 * ((M.m + M.nnz) / 1024 + 2) * 152 : 3 * csr_bytes;
     if (need > cfg.hbm_budget_bytes) return fail(SSPMV_BUDGET_EXCEEDED, "matrix %d alone exceeds the HBM budget", M.id);
+    const int64_t with_plan = M.fmt == SSPMV_FMT_CSR ? csr_bytes + stream_plan_bound(M.m, M.nnz, V) : need;
     {
         std::lock_guard<std::mutex> g(mu);
-        if (make_room(need) != SSPMV_OK) {
+        if (make_room(std::min(std::max(need, with_plan), cfg.hbm_budget_bytes)) != SSPMV_OK) {
             *wait = true;
             return SSPMV_BUDGET_EXCEEDED;
         }
@@ -684,6 +709,14 @@ void Server::issue(Batch &b) {
                   reinterpret_cast<sspmv_stream_t>(cs));
         cudaEventRecord(M.ev, cs);
         M.ev_stream = cs;
+        if (!M.counted) {  // its plan is built now
+            const int64_t bytes = device_bytes(M);
+            std::lock_guard<std::mutex> g(mu);
+            resident_bytes += bytes - M.bytes;
+            M.bytes = bytes;
+            M.counted = true;
+            make_room(0);
+        }
     }
     for (int a = 0; a < kAuxStreams; a++)
         if (used[a]) {
