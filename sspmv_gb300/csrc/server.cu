@@ -124,6 +124,17 @@ struct Batch {
     sspmv_status st = SSPMV_OK;
 };
 
+constexpr int64_t kServedAloneRun = 256;
+
+int64_t longest_empty_run(const int32_t *rp, int64_t m) {
+    int64_t longest = 0, run = 0;
+    for (int64_t i = 0; i < m; i++) {
+        run = rp[i + 1] == rp[i] ? run + 1 : 0;
+        longest = std::max(longest, run);
+    }
+    return longest;
+}
+
 // The features of a resident matrix, whose plan hangs off them.
 const sspmv_features &features_of(const Matrix &M) {
     const DeviceMatrix &d = M.dev;
@@ -367,7 +378,10 @@ sspmv_status Server::load(Matrix &M) {
         M.dev.csr = csr;
         if (M.nnz > 0) st = csr_stream_view(&M.dev.csr, &M.view, s);
         M.chunks = (M.nnz + 255) / 256;
-        M.batchable = st == SSPMV_OK && M.nnz > 0;
+        // A matrix that no batch holds is served on its own if it has a long run of
+        // empty rows, and refused if it has none.
+        M.batchable = st == SSPMV_OK && M.nnz > 0 &&
+                      (M.chunks <= cfg.max_batch_tiles || longest_empty_run(M.h_rp, M.m) <= kServedAloneRun);
     } else {
         st = convert(&csr, M, s);
         cudaStreamSynchronize(load_stream);
@@ -744,7 +758,8 @@ void Server::issue(Batch &b) {
     if (mask) {
         stats.batched_requests += begin;
         stats.graph_launches += cfg.use_graphs ? 1 : 0;
-        for (int q = 0; q < kBatchGroups; q++) stats.batched_tiles += group_tiles[q];
+        for (const Request *r : b.reqs)
+            if (r->group >= 0) stats.batched_tiles += r->mat->chunks;
     }
 }
 
