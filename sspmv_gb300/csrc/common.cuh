@@ -232,7 +232,7 @@ __device__ __forceinline__ int64_t warp_last_le(const T *__restrict__ p, int64_t
 // block that calls it, so the grid after it is ordered behind both.  Only inside
 // a call, behind a kernel of the library: the call's first kernel is launched as
 // any other.  SELL-C-sigma of 1M power-law rows, FP64 (long rows' kernel, thread
-// pass, split rows): 102 us one after the other, 89 so.
+// pass, split rows): 102 us one after the other, 85 so.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

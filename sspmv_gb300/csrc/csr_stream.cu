@@ -21,8 +21,8 @@
 // lane that ends it.  An earlier form that marked row starts in shared memory
 // (row_offset read per chunk, a five-step prefix scan, a second launch for rows
 // crossing 256-element chunks) took, per SpMV: 1024^2 Laplacian FP64 33.4 us
-// (now 21.2), uniform 2M x 32 FP64 315 us (271), banded 2M FP64 85 us (60),
-// power-law 4M FP32 with alpha and beta 339 us (272).  Columns
+// (now 20.7), uniform 2M x 32 FP64 315 us (271), banded 2M FP64 85 us (60),
+// power-law 4M FP32 with alpha and beta 339 us (268).  Columns
 // loaded a step ahead, a cp.async.bulk L2 prefetch of later windows and all
 // finished rows through shared memory were slower, too (fewer warps, or more
 // queued accesses).
@@ -34,13 +34,13 @@
 // collected in shared memory, up to kStage per step, and scaled (y read) 32 /
 // G rows at a time: scattered multiplies would cost a full warp instruction of
 // the FP64 pipe each.  SpMM on power-law rows, before and now: 1M FP64 k = 4
-// 297 -> 192 us, k = 8 448 -> 331 us, 2M FP32 k = 8 318 -> 232 us; with alpha
+// 297 -> 192 us, k = 8 448 -> 331 us, 2M FP32 k = 8 318 -> 229 us; with alpha
 // and beta FP64 k = 8 banded 372 -> 245 us.
 //
 // A warp reads up to kOver elements past its window to finish its last row.
 // A row that goes on further is split: every window it meets leaves its piece
 // and a second kernel (launched only when the matrix has split rows) adds each
-// one's pieces in window order, a warp per row.  (The last warp to finish,
+// one's pieces in a fixed order, eight lanes a row.  (The last warp to finish,
 // found by a counter per row, adding the pieces instead cost a memory fence per
 // window: power-law 4M FP32 365 us against 303.)  Rows without nonzeros are a
 // list, which warps behind the windows' write (scale_empty_rows).  No atomics
@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(kBlock, (stream_min_ctas<V, K>() * 3 / 4)) csr
     }
 }
 
-// The split rows of every request of group g, a warp each.
+// The split rows of every request of group g, kSplitLanes lanes each.
 template <typename V, int K>
 __global__ void __launch_bounds__(256) csr_batch_split_kernel(int g, const BatchHeader *__restrict__ hdr,
                                                               const BatchItem *__restrict__ all_items,

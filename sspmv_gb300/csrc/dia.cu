@@ -118,7 +118,7 @@ __global__ void dia_fill(int64_t m, int64_t stride, const int32_t *__restrict__ 
 
 // One thread per row, a block per 256 rows, four diagonals' values in flight.
 // FP64 is bound by the FP64 pipe (2M rows of 9 diagonals: 35.6 us of FMAs at its
-// rate; 39.6 us, 41.7 with a fixed grid striding over the rows), FP32 by the
+// rate; 38.9 us, 41.0 with a fixed grid striding over the rows), FP32 by the
 // latency of the x loads (1M rows of 9: 14.4 us).  Eight diagonals in flight
 // (fewer warps) measured 70 us, two or four rows a thread 43.4 and 41.9.
 template <typename V, int K, bool PLAIN = false>

@@ -347,8 +347,9 @@ __global__ void __launch_bounds__(kBlock, (VS == 1 && K == 1) ? (sizeof(V) == 4 
                     for (int r = 0; r < K; r++) s[r] += a[q] * xr[q][r];
                 }
         } else if (row < m) {
-            int j = rs + sub;
-            for (; j + 3 * VS < re; j += 4 * VS) {  // four independent gathers in flight
+            uint32_t j = rs + sub;  // unsigned: j + 4 * VS may pass INT_MAX at the last nonzeros
+            const uint32_t je = re;
+            for (; j + 3 * VS < je; j += 4 * VS) {  // four independent gathers in flight
                 int c[4];
                 V a[4];
 #pragma unroll
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kBlock, (VS == 1 && K == 1) ? (sizeof(V) == 4 
                     for (int r = 0; r < K; r++) s[r] += a[u] * xr[r];
                 }
             }
-            for (; j < re; j += VS) {
+            for (; j < je; j += VS) {
                 const int c = ld_stream(col_index + j);
                 const V a = ld_stream(values + j);
                 V xr[K];
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(kBlock) csr_rowblock_kernel(int64_t nb, int m,
                         rs = r < pend ? ps[r - ap] : ld_stream(rp + r);
                         re = r + 1 < pend ? ps[r + 1 - ap] : ld_stream(rp + r + 1);
                     }
-                    for (int e = rs + sub; e < re; e += L) sum += vs[e - av];
+                    for (uint32_t e = rs + sub; e < (uint32_t)re; e += L) sum += vs[e - av];
                 }
                 if constexpr (L > 1) sum = warp_sum(sum, L);
                 if (i < nr && sub == 0) {

@@ -15,7 +15,9 @@ keeps no state between calls:
   2-D x: the library's SpMM (sspmv_spmm_csr, one pass for up to 8 columns,
          the same merge-path kernel) on a matrix wrapped for this call; its
          plan is built in stream order and released in stream order after the
-         call (sspmv_release_plan), nothing waits for the device.
+         call (sspmv_release_plan), nothing waits for the device.  That memory
+         goes back to the library's pool, which keeps up to 1 GiB of it for
+         the next call; under a stream capture it belongs to the graph.
 
 A fake implementation gives shapes to tracing.
 """

@@ -19,7 +19,7 @@ def arrays():
 
 
 @pytest.mark.parametrize("k", [1, 8])
-@pytest.mark.parametrize("flag", [0, 2], ids=["stream", "merge"])
+@pytest.mark.parametrize("flag", [0, 1, 2], ids=["stream", "vector", "merge"])
 def test_csr_of_int_max_nonzeros(arrays, flag, k):
     import torch
     from sspmv_gb300 import _lib
