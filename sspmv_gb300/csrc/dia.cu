@@ -121,14 +121,15 @@ __global__ void dia_fill(int64_t m, int64_t stride, const int32_t *__restrict__ 
 // rate; 38.9 us, 41.0 with a fixed grid striding over the rows), FP32 by the
 // latency of the x loads (1M rows of 9: 14.4 us).  Eight diagonals in flight
 // (fewer warps) measured 70 us, two or four rows a thread 43.4 and 41.9.
-template <typename V, int K, bool PLAIN = false>
+// STRIDE: the fixed grid, for one FP32 right-hand side with alpha and beta (3M rows
+// 34.0 us in blocks of 256 rows, 32.4 so).
+template <typename V, int K, bool PLAIN = false, bool STRIDE = false>
 __global__ void __launch_bounds__(kBlock) dia_spmv_kernel(int m, int n, int nd, int64_t stride,
                                                         const int64_t *__restrict__ offsets,
                                                         const V *__restrict__ data, const V *__restrict__ x,
                                                         int64_t ldx, int xvec, V alpha, V beta, V *__restrict__ y,
                                                         int64_t ldy) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < m) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x) {
         V s[K];
 #pragma unroll
         for (int q = 0; q < K; q++) s[q] = V(0);
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(kBlock) dia_spmv_kernel(int m, int n, int nd, 
         V *yp = y + i * ldy;
 #pragma unroll
         for (int q = 0; q < K; q++) yp[q] = row_out(PLAIN, alpha, s[q], beta, yp + q);
+        if constexpr (!STRIDE) break;
     }
 }
 
@@ -352,13 +354,16 @@ sspmv_status launch_dia(const sspmv_dia *A, V alpha, const V *x, int64_t ldx, V 
         sspmv_status st = SSPMV_OK;
         if (try_dia_staged<V>(A, alpha, x, ldx, beta, y, ldy, s, &st)) return st;
     }
-    const unsigned grid = grid_for(A->f.num_rows, kBlock);
+    const bool plain = K == 1 && alpha == V(1) && beta == V(0);  // y = sum
+    const bool stride = K == 1 && sizeof(V) == 4 && !plain;
+    const unsigned grid = grid_for(A->f.num_rows, kBlock, stride ? (int64_t)num_sms() * 16 : 0);
     auto go = [&](auto kernel) {
         kernel<<<grid, kBlock, 0, cu(s)>>>((int)A->f.num_rows, (int)A->f.num_cols, A->complete_ndiags, A->stride,
                                            A->diag_offsets, (const V *)A->diag_data, x, ldx,
                                            xrow_vec(x, ldx, sizeof(V), K), alpha, beta, y, ldy);
     };
-    if (K == 1 && alpha == V(1) && beta == V(0)) go(dia_spmv_kernel<V, K, K == 1>);  // y = sum
+    if (plain) go(dia_spmv_kernel<V, K, K == 1>);
+    else if (stride) go(dia_spmv_kernel<V, K, false, K == 1 && sizeof(V) == 4>);
     else go(dia_spmv_kernel<V, K>);
     SSPMV_LAUNCH_CHECK();
     return SSPMV_OK;
