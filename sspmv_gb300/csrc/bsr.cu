@@ -160,10 +160,13 @@ __global__ void __launch_bounds__(kBlock) bsr_spmv_kernel(int m, int n, int r, i
 // TB/s there: a chain of two dependent loads (the block's column, then x) at 32
 // warps a SM.  The next step's columns and blocks loaded before this step's
 // sums measured 19.6 us (more registers, fewer warps).
-template <typename V, int C>
+// SMALL: a matrix that leaves most warps idle takes one block a group, half a step
+// of them a window: more warps and the shortest chain, which is its time (4,000
+// rows, 2x2 FP64, 5.6 us with four blocks a group, 2.7 so).
+template <typename V, int C, bool SMALL = false>
 struct BsrShape {
     static constexpr int kWords = (int)(C * sizeof(V) / 4);             // 4-byte words of a block's row
-    static constexpr int B = kWords >= 16 ? 1 : kWords <= 4 ? 4 : 16 / kWords;  // up to 16 words a lane in flight
+    static constexpr int B = SMALL || kWords >= 16 ? 1 : kWords <= 4 ? 4 : 16 / kWords;  // up to 16 words a lane in flight
 };
 
 // Resident CTAs per SM the register budget is set for: 2M rows of 4x4 blocks,
@@ -206,12 +209,12 @@ __device__ __forceinline__ void ld_run(const V *__restrict__ p, bool vec, V (&ou
     for (int e = 0; e < C; e++) out[e] = STREAM ? ld_stream(p + e) : ld_x(p + e);
 }
 
-template <typename V, int C, bool PLAIN>
+template <typename V, int C, bool PLAIN, bool SMALL>
 __global__ void __launch_bounds__(kStreamBlock, (bsr_ctas<V, C>())) bsr_stream_kernel(
     const StreamView A, int m, int n, int lr, const V *__restrict__ data, int dvec, const V *__restrict__ x, int xvec, V alpha,
     V beta, V *__restrict__ y) {
     constexpr unsigned kFull = 0xffffffffu;
-    constexpr int B = BsrShape<V, C>::B;
+    constexpr int B = BsrShape<V, C, SMALL>::B;
     constexpr bool kSeed = sizeof(V) == 8;
     const int64_t w = (int64_t)blockIdx.x * (kStreamBlock / 32) + (threadIdx.x >> 5);
     const int r = 1 << lr, NG = 32 >> lr;
@@ -430,15 +433,24 @@ sspmv_status choose_bsr_kernel(const sspmv_bsr *A, Plan *p, sspmv_stream_t s) {
 template <typename V, int C>
 sspmv_status launch_bsr_stream(const sspmv_bsr *A, Plan *p, V alpha, const V *x, V beta, V *y, sspmv_stream_t s) {
     // windows of whole steps less a block row's overhang; never split
-    const int lr = log2_exact(A->blockDim_r), step = BsrShape<V, C>::B * (32 >> lr);
+    const int lr = log2_exact(A->blockDim_r), groups = 32 >> lr, step = BsrShape<V, C>::B * groups;
     const int64_t mean = A->mb > 0 ? (A->nnzb + A->mb - 1) / A->mb : 1;
     const int slack = (int)std::min<int64_t>(step / 4, mean + 1);
-    const int n = window_steps(A->nnzb, step, step - slack, bsr_ctas<V, C>() * (kStreamBlock / 32));
+    const int warps = bsr_ctas<V, C>() * (kStreamBlock / 32);
+    const int64_t slots = (int64_t)num_sms() * warps;
+    // one wave of half steps, of one block a group or of B: a window and what its
+    // last block row goes on past it in one step (100k rows, 4x4 FP32, 4.4 us in
+    // windows of whole steps, 3.7 so)
+    const bool small = A->nnzb <= slots * std::max(1, groups / 2) && step > groups;
+    const bool half = !small && A->nnzb <= slots * std::max(1, step / 2);
+    const int window = small   ? std::max(1, groups / 2)
+                       : half  ? std::max(1, step / 2)
+                               : step * window_steps(A->nnzb, step, step - slack, warps) - slack;
     if (!p->stream.window) {
         std::lock_guard<PlanMutex> guard(plan_mutex());
         const unsigned long long *d = (const unsigned long long *)p->extra[3];
         SSPMV_TRY(ensure_stream_plan(p->stream, A->mb, A->nnzb, A->row_ptr, nullptr, A->f.value_type, s,
-                                     step * n - slack, 0x7fffffff, d ? p->extra_i[2] >> 2 : -1,
+                                     window, 0x7fffffff, d ? p->extra_i[2] >> 2 : -1,
                                      d ? (const int2 *)(d + 2) : nullptr));
         dfree(p->extra[3], s);
         p->extra[3] = nullptr;
@@ -451,8 +463,11 @@ sspmv_status launch_bsr_stream(const sspmv_bsr *A, Plan *p, V alpha, const V *x,
         kernel<<<grid_for(v.windows + empty_units((int64_t)v.nempty << lr), kStreamBlock / 32), kStreamBlock, 0, cu(s)>>>(
             v, (int)A->f.num_rows, (int)A->f.num_cols, lr, (const V *)A->block_data, dvec, x, xvec, alpha, beta, y);
     };
-    if (alpha == V(1) && beta == V(0)) go(bsr_stream_kernel<V, C, true>);  // y = sum
-    else go(bsr_stream_kernel<V, C, false>);
+    const bool plain = alpha == V(1) && beta == V(0);  // y = sum
+    if (small && plain) go(bsr_stream_kernel<V, C, true, true>);
+    else if (small) go(bsr_stream_kernel<V, C, false, true>);
+    else if (plain) go(bsr_stream_kernel<V, C, true, false>);
+    else go(bsr_stream_kernel<V, C, false, false>);
     SSPMV_LAUNCH_CHECK();
     return SSPMV_OK;
 }
