@@ -252,7 +252,8 @@ sspmv_status sspmv_delete_csr(sspmv_csr *A);
 /* ---------------- SpMV / SpMM ---------------- */
 /* LeSpMV_csr (src/spmv_csr.cpp:165-185).  kernel_flag 0 (default):
  * nonzero-split stream kernel; 2: nnz-balanced merge-path
- * kernel; 1: vector-per-row kernel (param: lanes per row, 1..32); 3: row-block
+ * kernel; 1: vector-per-row kernel (param: lanes per row, 1..32; a matrix
+ * within 128 nonzeros of 2^31 runs the default kernel); 3: row-block
  * kernel for matrices whose rows all have at most 64 nonzeros (one CTA per
  * block of whole rows, param: nonzeros per block window, 512..4096; one
  * right-hand side; other matrices and k > 1 run the default kernel); 4:

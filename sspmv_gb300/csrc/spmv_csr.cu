@@ -296,6 +296,11 @@ sspmv_status run_merge(const sspmv_csr *A, const MergePlan &q, V alpha, const V 
 
 constexpr int kVecHoist = 6;
 
+// The vector kernel's element index runs up to 127 past a row's last element in an
+// int: matrices with more nonzeros run the default kernel.  (An unsigned or 64-bit
+// index costs 10 to 25% with two or more lanes per row.)
+constexpr int64_t kVecMaxNnz = INT32_MAX - 128;
+
 template <typename V, int K, int VS, bool PLAIN = false>
 __global__ void __launch_bounds__(kBlock, (VS == 1 && K == 1) ? (sizeof(V) == 4 ? 6 : 5) : 1) csr_vector_kernel(
     int m, const int32_t *__restrict__ row_offset, const int32_t *__restrict__ col_index,
@@ -347,9 +352,8 @@ __global__ void __launch_bounds__(kBlock, (VS == 1 && K == 1) ? (sizeof(V) == 4 
                     for (int r = 0; r < K; r++) s[r] += a[q] * xr[q][r];
                 }
         } else if (row < m) {
-            uint32_t j = rs + sub;  // unsigned: j + 4 * VS may pass INT_MAX at the last nonzeros
-            const uint32_t je = re;
-            for (; j + 3 * VS < je; j += 4 * VS) {  // four independent gathers in flight
+            int j = rs + sub;
+            for (; j + 3 * VS < re; j += 4 * VS) {  // four independent gathers in flight
                 int c[4];
                 V a[4];
 #pragma unroll
@@ -365,7 +369,7 @@ __global__ void __launch_bounds__(kBlock, (VS == 1 && K == 1) ? (sizeof(V) == 4 
                     for (int r = 0; r < K; r++) s[r] += a[u] * xr[r];
                 }
             }
-            for (; j < je; j += VS) {
+            for (; j < re; j += VS) {
                 const int c = ld_stream(col_index + j);
                 const V a = ld_stream(values + j);
                 V xr[K];
@@ -783,7 +787,8 @@ sspmv_status launch_stream(const sspmv_csr *A, Plan *p, V alpha, const V *x, int
 template <typename V, int K>
 sspmv_status csr_pass(const sspmv_csr *A, Plan *p, V alpha, const V *x, int64_t ldx, V beta, V *y,
                       int64_t ldy, sspmv_stream_t s) {
-    if (A->f.kernel_flag == 1) return launch_vector<V, K>(A, p, alpha, x, ldx, beta, y, ldy, s);
+    if (A->f.kernel_flag == 1 && A->f.num_nnzs <= kVecMaxNnz)
+        return launch_vector<V, K>(A, p, alpha, x, ldx, beta, y, ldy, s);
     if (A->f.kernel_flag == 2) return launch_merge<V, K>(A, p, alpha, x, ldx, beta, y, ldy, s);
     if constexpr (K == 1) {
         if (A->f.kernel_flag == 3) {
