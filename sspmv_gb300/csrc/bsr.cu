@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kBlock) bsr_spmv_kernel(int m, int n, int r, i
 // finishes the block rows that start in its window, so one launch and no
 // pieces; r must be a power of two <= 32.  With one block per group and step,
 // a scan for each, block_row read per block and values one at a time: 2M rows
-// of 4x4 blocks FP32 23.2 us, now 19.2 (FP64 54.0, now 40.0).  It moves 2.5
+// of 4x4 blocks FP32 22.5 us, now 17.1 (FP64 50.8, now 34.7).  It moves 3.2
 // TB/s there: a chain of two dependent loads (the block's column, then x) at 32
 // warps a SM.  The next step's columns and blocks loaded before this step's
 // sums measured 19.6 us (more registers, fewer warps).
